@@ -161,6 +161,349 @@ attn_generic_kernel(const T *__restrict__ q, T *__restrict__ out, const T *__res
   }
 }
 
+// ---------------------------------------------------------------------------------------------------
+// The same attention in float for pages of 64 keys, head sizes up to 256 that are multiples of 4, and no pooled blocks:
+// a page's keys (a segment) are brought to shared memory once and serve many rows.  A score is the sum of four partial
+// dot products (d mod 4, each in increasing d); a segment's scores have one maximum; its probabilities are added pairwise
+// by a warp (keys i and i + 32 first); its weighted values are added in the order of the keys; segments are merged one after
+// the other from the lowest.  Both kernels keep that order, so a row's result depends neither on the kernel nor on the batch.
+//
+//   tile    a block per (64 rows of one prompt, query head) that walks the segments: prompts
+//   split   a block per (token, kv head, segment), for all query heads of the kv head, and a merge: single tokens, whose
+//           few rows leave the GPU to the segments
+//
+// 16 heads of 128 on 8 kv heads: two tokens behind 200 and 500 keys 7.4 + 4.2 us in a decode step (850 us with a warp a token
+// and head, whose lanes read rows of 512 bytes each for themselves); prompts of 201 and 500 tokens 181 us.
+#define SEG 64
+#define F32_MAX_HD 256
+#define F32_MAX_GROUP 32
+#define F32_PART_EXTRA 2                                            // maximum and sum in front of a part's values
+
+struct F32Attn {
+  const float *q, *cache, *sink, *gate;
+  float *out, *parts;
+  const int *tok_pos, *tok_seq, *page_table, *tiles;
+  int P, nh, nkv, hd, window, planes, q_stride, gate_stride, chunk, keep_first, v_heads, segments;
+  float scale, softcap;
+};
+
+__device__ __forceinline__ int lowest_key(const F32Attn &p, int pos) {
+  return p.chunk > 0 ? (pos / p.chunk) * p.chunk : (p.window > 0 ? max(0, pos - p.window + 1) : 0);
+}
+// may a token whose window starts at `lo` see `key` (at most the token's own position)?
+__device__ __forceinline__ bool sees(const F32Attn &p, int lo, int key) { return key >= lo || key < p.keep_first; }
+__device__ __forceinline__ bool sees_segment(const F32Attn &p, int lo, int pos, int seg) {
+  return seg * SEG <= pos && (seg * SEG + SEG > lo || seg * SEG < p.keep_first);
+}
+
+__device__ __forceinline__ void bring_panel(float *to, const float *from, int hd, int tid, int threads) {
+  for (int i = tid; i < SEG * (hd / 4); i += threads) {
+    const int r = i / (hd / 4), c = i % (hd / 4) * 4;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(to + r * (hd + 4) + c)),
+                 "l"(from + (size_t)r * hd + c));
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+}
+__device__ __forceinline__ const float *panel_of(const F32Attn &p, int seq, int seg, int kvh, bool values) {
+  const size_t page = (size_t)p.page_table[(size_t)seq * p.P + seg];
+  const int plane = values ? p.planes - 1 : 0, head = values && p.planes == 2 ? kvh % p.v_heads : kvh;
+  return p.cache + ((page * p.planes + plane) * p.nkv + head) * ((size_t)SEG * p.hd);
+}
+__device__ __forceinline__ float scored(const F32Attn &p, float4 d) {
+  const float s = ((d.x + d.y) + (d.z + d.w)) * p.scale;
+  return p.softcap > 0.f ? p.softcap * tanhf(s / p.softcap) : s;
+}
+__device__ __forceinline__ void dot4(float4 &d, const float4 a, const float4 b) {
+  d.x = fmaf(a.x, b.x, d.x);
+  d.y = fmaf(a.y, b.y, d.y);
+  d.z = fmaf(a.z, b.z, d.z);
+  d.w = fmaf(a.w, b.w, d.w);
+}
+// One warp: a row's 64 scores in shared memory (-inf: not seen) become probabilities against their maximum.
+__device__ __forceinline__ void soften(float *row, int lane, float &m, float &l) {
+  const float a = row[lane], b = row[lane + 32];
+  m = warp_max(fmaxf(a, b));
+  const float pa = a == -INFINITY ? 0.f : expf(a - m), pb = b == -INFINITY ? 0.f : expf(b - m);
+  row[lane] = pa;
+  row[lane + 32] = pb;
+  l = warp_sum(pa + pb);
+}
+// Adds a part (maximum m, times e) to a running one: the factors for what is there and for what comes.
+__device__ __forceinline__ void merge_factors(float &m, float m_part, float &old_factor, float &new_factor) {
+  const float m_new = fmaxf(m, m_part);
+  old_factor = expf(m - m_new);                                     // 0 in front of the first part
+  new_factor = expf(m_part - m_new);
+  m = m_new;
+}
+__device__ __forceinline__ float merged(float there, float old_factor, float part, float new_factor) {
+  return fmaf(part, new_factor, __fmul_rn(there, old_factor));
+}
+__device__ __forceinline__ float last_factor(const F32Attn &p, int t, int h, float m, float l) {
+  if (p.sink) l += expf(p.sink[h] - m);
+  float f = 1.f / l;
+  if (p.gate) f *= 1.f / (1.f + expf(-p.gate[(size_t)t * p.gate_stride + h]));
+  return f;
+}
+
+#define F32_TILE_ROWS 64
+template <int HD4>                                                  // float4 columns of a row per thread: ceil(hd / 64)
+__global__ void __launch_bounds__(256)
+attn_f32_tile_kernel(F32Attn p) {
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];
+  const int hd = p.hd, pitch = hd + 4;
+  float *Qs = sm, *Ks = Qs + F32_TILE_ROWS * pitch, *Vs = Ks + SEG * pitch, *Ps = Vs + SEG * pitch;
+  float *row_m = Ps + F32_TILE_ROWS * (SEG + 4), *row_l = row_m + F32_TILE_ROWS, *old_f = row_l + F32_TILE_ROWS,
+        *new_f = old_f + F32_TILE_ROWS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
+  const int *tile = p.tiles + 4 * blockIdx.x;
+  const int seq = tile[0], t0 = tile[1], rows = tile[2], pos0 = tile[3], h = blockIdx.y, kvh = h / (p.nh / p.nkv);
+  for (int i = tid; i < F32_TILE_ROWS * (hd / 4); i += 256) {
+    const int r = i / (hd / 4), c = i % (hd / 4) * 4;
+    *(float4 *)(Qs + r * pitch + c) =
+        r < rows ? *(const float4 *)(p.q + (size_t)(t0 + r) * p.q_stride + (size_t)h * hd + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (tid < F32_TILE_ROWS) {
+    row_m[tid] = -INFINITY;
+    row_l[tid] = 0.f;
+  }
+  float4 O[4][HD4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < HD4; ++j) O[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int last_pos = pos0 + rows - 1, lo0 = lowest_key(p, pos0);
+  for (int seg = 0; seg * SEG <= last_pos; ++seg) {
+    if (!sees_segment(p, lo0, last_pos, seg)) continue;             // the first row's window starts lowest
+    __syncthreads();                                                // the last segment's panels and probabilities are read
+    bring_panel(Ks, panel_of(p, seq, seg, kvh, false), hd, tid, 256);
+    bring_panel(Vs, panel_of(p, seq, seg, kvh, true), hd, tid, 256);
+    asm volatile("cp.async.wait_group 1;\n" ::);
+    __syncthreads();
+    float4 S[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) S[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int d = 0; d < hd; d += 4) {
+      float4 k[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = *(const float4 *)(Ks + (tx + 16 * j) * pitch + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 q = *(const float4 *)(Qs + (ty + 16 * i) * pitch + d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dot4(S[i][j], q, k[j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = ty + 16 * i, pos = pos0 + r, lo = lowest_key(p, pos);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = seg * SEG + tx + 16 * j;
+        Ps[r * (SEG + 4) + tx + 16 * j] = r < rows && key <= pos && sees(p, lo, key) ? scored(p, S[i][j]) : -INFINITY;
+      }
+    }
+    __syncthreads();
+    for (int r = warp; r < F32_TILE_ROWS; r += 8) {
+      float m, l;
+      soften(Ps + r * (SEG + 4), lane, m, l);
+      if (lane == 0) {
+        float of = 1.f, nf = 0.f;                                   // nothing of the segment is seen: all stays
+        if (m != -INFINITY) {
+          float there = row_m[r];
+          merge_factors(there, m, of, nf);
+          row_m[r] = there;
+          row_l[r] = merged(row_l[r], of, l, nf);
+        }
+        old_f[r] = of;
+        new_f[r] = nf;
+      }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    float4 acc[4][HD4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < HD4; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int n_keys = min(SEG, last_pos - seg * SEG + 1);
+    for (int key = 0; key < n_keys; ++key) {
+      float4 v[HD4];
+#pragma unroll
+      for (int j = 0; j < HD4; ++j)
+        if (64 * j + 4 * tx < hd) v[j] = *(const float4 *)(Vs + key * pitch + 64 * j + 4 * tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float pr = Ps[(ty + 16 * i) * (SEG + 4) + key];
+        if (pr != 0.f)                                              // a value that is not seen is not touched, whatever it holds
+#pragma unroll
+          for (int j = 0; j < HD4; ++j)
+            if (64 * j + 4 * tx < hd) {
+              acc[i][j].x = fmaf(pr, v[j].x, acc[i][j].x);
+              acc[i][j].y = fmaf(pr, v[j].y, acc[i][j].y);
+              acc[i][j].z = fmaf(pr, v[j].z, acc[i][j].z);
+              acc[i][j].w = fmaf(pr, v[j].w, acc[i][j].w);
+            }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float of = old_f[ty + 16 * i], nf = new_f[ty + 16 * i];
+      if (nf != 0.f || of != 1.f)
+#pragma unroll
+        for (int j = 0; j < HD4; ++j) {
+          O[i][j].x = merged(O[i][j].x, of, acc[i][j].x, nf);
+          O[i][j].y = merged(O[i][j].y, of, acc[i][j].y, nf);
+          O[i][j].z = merged(O[i][j].z, of, acc[i][j].z, nf);
+          O[i][j].w = merged(O[i][j].w, of, acc[i][j].w, nf);
+        }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = ty + 16 * i;
+    if (r >= rows) continue;
+    const float f = last_factor(p, t0 + r, h, row_m[r], row_l[r]);
+    float *op = p.out + (size_t)(t0 + r) * p.nh * hd + (size_t)h * hd;
+#pragma unroll
+    for (int j = 0; j < HD4; ++j)
+      if (64 * j + 4 * tx < hd)
+        *(float4 *)(op + 64 * j + 4 * tx) = make_float4(O[i][j].x * f, O[i][j].y * f, O[i][j].z * f, O[i][j].w * f);
+  }
+}
+
+__global__ void __launch_bounds__(128)
+attn_f32_split_kernel(F32Attn p) {
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];
+  const int hd = p.hd, pitch = hd + 4, group = p.nh / p.nkv, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int seg = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
+  const int pos = p.tok_pos[t], seq = p.tok_seq[t], lo = lowest_key(p, pos);
+  if (!sees_segment(p, lo, pos, seg)) return;
+  float *Ks = sm, *Vs = Ks + SEG * pitch, *Qs = Vs + SEG * pitch, *Ps = Qs + group * pitch;
+  bring_panel(Ks, panel_of(p, seq, seg, kvh, false), hd, tid, 128);
+  bring_panel(Vs, panel_of(p, seq, seg, kvh, true), hd, tid, 128);
+  for (int i = tid; i < group * (hd / 4); i += 128) {
+    const int r = i / (hd / 4), c = i % (hd / 4) * 4;
+    *(float4 *)(Qs + r * pitch + c) = *(const float4 *)(p.q + (size_t)t * p.q_stride + (size_t)(kvh * group + r) * hd + c);
+  }
+  asm volatile("cp.async.wait_group 1;\n" ::);
+  __syncthreads();
+  const int j = tid & (SEG - 1), key = seg * SEG + j;
+  for (int r = tid / SEG; r < group; r += 128 / SEG) {
+    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int c = 0; c < hd; c += 4) dot4(d, *(const float4 *)(Qs + r * pitch + c), *(const float4 *)(Ks + j * pitch + c));
+    Ps[r * (SEG + 4) + j] = key <= pos && sees(p, lo, key) ? scored(p, d) : -INFINITY;
+  }
+  __syncthreads();
+  const size_t part_size = hd + F32_PART_EXTRA;
+  float *part = p.parts + (((size_t)t * p.nh + kvh * group) * p.segments + seg) * part_size;
+  for (int r = warp; r < group; r += 4) {
+    float m, l;
+    soften(Ps + r * (SEG + 4), lane, m, l);
+    if (lane == 0) {
+      part[r * p.segments * part_size] = m;
+      part[r * p.segments * part_size + 1] = l;
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __syncthreads();
+  const int n_keys = min(SEG, pos - seg * SEG + 1);
+  for (int i = tid; i < group * hd; i += 128) {
+    const int r = i / hd, d = i % hd;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < n_keys; ++k) {
+      const float pr = Ps[r * (SEG + 4) + k];
+      if (pr != 0.f) acc = fmaf(pr, Vs[k * pitch + d], acc);
+    }
+    part[r * p.segments * part_size + F32_PART_EXTRA + d] = acc;
+  }
+}
+
+// a block per (token, head); a thread per value
+__global__ void __launch_bounds__(F32_MAX_HD)
+attn_f32_merge_kernel(F32Attn p) {
+  pdl_launch();
+  pdl_wait();
+  const int t = blockIdx.x / p.nh, h = blockIdx.x % p.nh, d = threadIdx.x;
+  const int pos = p.tok_pos[t], lo = lowest_key(p, pos);
+  const size_t part_size = p.hd + F32_PART_EXTRA;
+  const float *part = p.parts + (size_t)blockIdx.x * p.segments * part_size;
+  float m = -INFINITY, l = 0.f, o = 0.f;
+#pragma unroll 4
+  for (int seg = 0; seg * SEG <= pos; ++seg) {
+    if (!sees_segment(p, lo, pos, seg)) continue;
+    const float *s = part + seg * part_size;
+    const float part_m = s[0], part_l = s[1], v = d < p.hd ? s[F32_PART_EXTRA + d] : 0.f;
+    float of, nf;
+    merge_factors(m, part_m, of, nf);
+    l = merged(l, of, part_l, nf);
+    o = merged(o, of, v, nf);
+  }
+  if (d < p.hd) p.out[(size_t)t * p.nh * p.hd + (size_t)h * p.hd + d] = o * last_factor(p, t, h, m, l);
+}
+
+template <int HD4>
+static int launch_f32_tiles(const F32Attn &p, int n_tiles, cudaStream_t stream) {
+  static G2bPerDevice done;
+  auto bytes = [](int hd) { return sizeof(float) * ((size_t)(F32_TILE_ROWS + 2 * SEG) * (hd + 4) + F32_TILE_ROWS * (SEG + 4) + 4 * F32_TILE_ROWS); };
+  const int dev = g2b_current_device();
+  if (dev < 0 || !done.value[dev]) {
+    if (cudaFuncSetAttribute(attn_f32_tile_kernel<HD4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(64 * HD4)) != cudaSuccess)
+      G2B_REFUSE("attn_f32: %zu bytes of shared memory are not available", bytes(64 * HD4));
+    if (dev >= 0) done.value[dev] = 1;
+  }
+  g2b_launch(attn_f32_tile_kernel<HD4>, dim3(n_tiles, p.nh), dim3(256), bytes(p.hd), stream, p);
+  return g2b_check_launch("attn_f32");
+}
+
+// Float attention over pages of 64 keys (see above).  `tiles` [n_tiles, 4] (sequence, first token, rows up to 64, position of
+// the first row): the step's rows in tiles; null: a token by itself, with `parts` of n_tokens * nh * segments * (hd + 2)
+// floats for the segments, of which there are as many as the longest sequence has pages.
+extern "C" int g2b_attn_f32(const float *q, float *out, const float *cache, const int *tok_pos, const int *tok_seq,
+                            const int *page_table, int P, int n_tokens, int nh, int nkv, int hd, int window, float scale,
+                            const float *sink, int planes, int q_stride, const float *gate, int gate_stride, int chunk, float softcap,
+                            int keep_first, int v_heads, const int *tiles, int n_tiles, float *parts, int segments,
+                            cudaStream_t stream) {
+  if (n_tokens <= 0) return 0;
+  if (v_heads <= 0) v_heads = nkv;
+  if (hd <= 0 || hd > F32_MAX_HD || hd % 4 || q_stride % 4 || (uintptr_t)q % 16 || (uintptr_t)out % 16 || (uintptr_t)cache % 16)
+    G2B_REFUSE("attn_f32: head size %d (a multiple of 4 up to %d) with rows on 16 bytes", hd, F32_MAX_HD);
+  if (nkv <= 0 || nh % nkv || nh / nkv > F32_MAX_GROUP) G2B_REFUSE("attn_f32: %d heads on %d kv heads", nh, nkv);
+  if (v_heads > nkv || nkv % v_heads) G2B_REFUSE("attn_f32: %d key heads on %d value heads", nkv, v_heads);
+  if (chunk < 0 || (chunk > 0 && window > 0)) G2B_REFUSE("attn_f32: a chunk of %d keys with a window of %d", chunk, window);
+  if (keep_first < 0 || (keep_first > 0 && window <= 0)) G2B_REFUSE("attn_f32: %d first tokens kept need a window", keep_first);
+  if (planes != 1 && planes != 2) G2B_REFUSE("attn_f32: %d panels per page and kv head (1 or 2)", planes);
+  const F32Attn p{q, cache, sink, gate, out, parts, tok_pos, tok_seq, page_table, tiles, P, nh, nkv, hd, window, planes, q_stride, gate_stride,
+                  chunk, keep_first, v_heads, segments, scale, softcap};
+  if (tiles) {
+    if (hd <= 64) return launch_f32_tiles<1>(p, n_tiles, stream);
+    if (hd <= 128) return launch_f32_tiles<2>(p, n_tiles, stream);
+    return launch_f32_tiles<4>(p, n_tiles, stream);
+  }
+  if (!parts || segments <= 0 || segments > P) G2B_REFUSE("attn_f32: %d segments of a table of %d pages need their parts", segments, P);
+  if (n_tokens > 65535 || nkv > 65535) G2B_REFUSE("attn_f32: %d tokens of %d kv heads are too many for one launch", n_tokens, nkv);
+  static G2bPerDevice done;
+  auto bytes = [](int d, int group) { return sizeof(float) * ((size_t)(2 * SEG + group) * (d + 4) + group * (SEG + 4)); };
+  const int dev = g2b_current_device();
+  if (dev < 0 || !done.value[dev]) {
+    const size_t most = bytes(F32_MAX_HD, F32_MAX_GROUP);
+    if (cudaFuncSetAttribute(attn_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess)
+      G2B_REFUSE("attn_f32: %zu bytes of shared memory are not available", most);
+    if (dev >= 0) done.value[dev] = 1;
+  }
+  g2b_launch(attn_f32_split_kernel, dim3(segments, nkv, n_tokens), dim3(128), bytes(hd, nh / nkv), stream, p);
+  if (int rc = g2b_check_launch("attn_f32")) return rc;
+  g2b_launch(attn_f32_merge_kernel, dim3(n_tokens * nh), dim3((hd + 31) / 32 * 32), 0, stream, p);
+  return g2b_check_launch("attn_f32");
+}
+
 extern "C" int g2b_attn_generic(const void *q, void *out, int dtype, const void *cache,
                                 const int *tok_pos, const int *tok_seq, const int *page_table,
                                 int P, int n_tokens, int nh, int nkv, int hd, int page_size,

@@ -719,6 +719,42 @@ def attn_generic(q, out, cache_pages, tok_pos, tok_seq, page_table, n_heads, n_k
           pooled.shape[3] if pool else 0, float(softcap), int(keep_first), int(v_heads), _stream())
 
 
+F32_PARTS_MOST = 512 << 20        # bytes of scratch that the segments of single tokens may take
+
+
+def attn_f32(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window, scale, sink=None, planes: int = 2,
+             gate=None, chunk: int = 0, softcap: float = 0.0, keep_first: int = 0, v_heads: int = 0) -> bool:
+    """``attn_generic`` in float over pages of 64 keys, for a whole step: prompts in the step's tiles, single tokens a
+    segment of keys at a time.  False when the sizes or the alignment are not the kernels'."""
+    if q.dtype != torch.float32 or cache_pages.dtype != torch.float32 or out.dtype != torch.float32 or page_size != 64 or \
+            head_dim % 4 or head_dim > 256 or n_heads // n_kv_heads > 32 or q.stride(0) % 4 or q.stride(1) != 1 or \
+            not out.is_contiguous() or any(t.data_ptr() % 16 for t in (q, out, cache_pages)) or \
+            (gate is not None and (gate.stride(1) != 1 or gate.dtype != torch.float32)):
+        return False
+    if sink is not None:
+        _need(sink, torch.float32, "sink")
+    tiles, parts, segments = (None, None, 0)
+    if ctx.attn_tiles is None or ctx.all_single:
+        segments = -(-ctx.max_kv_len // page_size)
+        shape = (q.shape[0], n_heads, segments, head_dim + 2)
+        if segments < 1 or segments > ctx.page_table.shape[1] or q.shape[0] > 65535 or \
+                4 * shape[0] * shape[1] * shape[2] * shape[3] > F32_PARTS_MOST:
+            return False
+        parts = ctx.workspace.buffer("attn.f32.parts", shape, torch.float32)
+    else:
+        tiles = ctx.attn_tiles
+    f = _fn("attn_generic.cu", "g2b_attn_f32",
+            [c_void_p] * 6 + [c_int] * 6 + [c_float, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_float, c_int, c_int,
+                                            c_void_p, c_int, c_void_p, c_int, c_void_p])
+    _call(f, _ptr(q), _ptr(out), _ptr(cache_pages), _ptr(ctx.tok_pos), _ptr(ctx.tok_seq), _ptr(ctx.page_table),
+          ctx.page_table.shape[1], q.shape[0], n_heads, n_kv_heads, head_dim, window, scale, _ptr(sink), planes, q.stride(0),
+          _ptr(gate), gate.stride(0) if gate is not None else 0, int(chunk), float(softcap), int(keep_first), int(v_heads),
+          _ptr(tiles), ctx.n_attn_tiles if tiles is not None else 0, _ptr(parts), segments, _stream())
+    if tiles is None:
+        count_launches(1)                          # the segments, then their merge
+    return True
+
+
 def attention(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window,
               scale, sink=None, planes: int = 2, gate=None, chunk: int = 0, pooled=None, pool: int = 0,
               softcap: float = 0.0, keep_first: int = 0, v_heads: int = 0) -> None:
@@ -738,6 +774,9 @@ def attention(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size
                                        page_size, window, scale, sink, planes, gate, chunk,
                                        softcap=softcap, keep_first=keep_first, v_heads=v_heads):
             return
+    elif attn_f32(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window, scale, sink, planes, gate, chunk,
+                  softcap, keep_first, v_heads):
+        return
     attn_generic(q, out, cache_pages, ctx.tok_pos, ctx.tok_seq, ctx.page_table, n_heads,
                  n_kv_heads, head_dim, page_size, window, scale, sink, planes, gate, chunk,
                  softcap=softcap, keep_first=keep_first, v_heads=v_heads)

@@ -1,11 +1,11 @@
-"""The float32 path's product at the edges of their tiles, against 64-bit arithmetic, and the rule that a row's bits do
+"""The float32 path's kernels at the edges of their tiles, against 64-bit arithmetic, and the rule that a row's bits do
 not depend on the rows beside it."""
 import math
 
 import pytest
 import torch
 
-from test_gpu_kernels import DEV, rnd
+from test_gpu_kernels import DEV, make_paged, rnd
 
 pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -24
@@ -46,3 +46,73 @@ def test_product_keeps_infinities_and_nan_in_their_rows():
         kernels.gemm_simt(a[:M], w, out)
         bad = (~torch.isfinite(out)).any(1).nonzero().flatten().tolist()
         assert bad == [r for r in (3, 40) if r < M]
+
+
+def ctx_of(lens, q_lens, table, tiles):
+    from gguf2bin_b200.engine.workspace import Workspace
+    from gguf2bin_b200.parts.base import StepContext
+    pos, seq, rows, t0 = [], [], [], 0
+    for b, (l, n) in enumerate(zip(lens, q_lens)):
+        rows += [(b, t0 + r, min(64, n - r), l - n + r) for r in range(0, n, 64)]
+        pos += range(l - n, l)
+        seq += [b] * n
+        t0 += n
+    as_int = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    return StepContext(n_tokens=t0, n_seqs=len(lens), tok_ids=None, tok_pos=as_int(pos), tok_seq=as_int(seq), page_table=table,
+                       page_size=64, workspace=Workspace(DEV), dtype=torch.float32, max_kv_len=max(lens),
+                       attn_tiles=as_int(rows) if tiles else None, n_attn_tiles=len(rows))
+
+
+OPTIONS = [dict(), dict(window=37), dict(window=70, keep_first=5), dict(window=64, keep_first=130), dict(chunk=50),
+           dict(softcap=3.0, sink=True, gate=True), dict(v_heads=1), dict(planes=1)]
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 128), (6, 2, 20), (5, 1, 64), (2, 2, 256), (3, 1, 132)])
+@pytest.mark.parametrize("options", OPTIONS, ids=lambda o: "-".join(o) or "plain")
+def test_attention_tiles_and_segments(nh, nkv, hd, options):
+    """A whole prompt, a prompt behind a past, a few tokens and one: every row from the tile kernel and from the kernel of
+    segments alike, bit for bit, and within the 32-bit bound of the kernel that walks keys one by one."""
+    from gguf2bin_b200 import kernels
+    if options.get("v_heads", nkv) > nkv or nkv % options.get("v_heads", nkv):
+        pytest.skip("fewer key heads than value heads")
+    lens, q_lens = [130, 321, 64, 200], [130, 65, 3, 1]
+    cache, table, _, Vs = make_paged(4, lens, nkv, hd, 64, torch.float32, seed=7)
+    T = sum(q_lens)
+    planes = options.get("planes", 2)
+    if planes == 1:
+        cache = cache[:, :1].contiguous()
+    wide = rnd(T, nh * hd + 4, seed=8)
+    q = wide[:, :nh * hd]
+    sink = rnd(nh, seed=9) if options.get("sink") else None
+    gate = rnd(T, nh, seed=10) if options.get("gate") else None
+    scale = 1 / math.sqrt(hd)
+    more = {k: v for k, v in options.items() if k in ("softcap", "keep_first", "v_heads", "chunk")}
+    window = options.get("window", 0)
+    outs = []
+    for tiles in (True, False):
+        out = torch.full((T, nh * hd), math.nan, device=DEV)
+        assert kernels.attn_f32(q, out, cache, ctx_of(lens, q_lens, table, tiles), nh, nkv, hd, 64, window, scale, sink, planes, gate, **more)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    ctx = ctx_of(lens, q_lens, table, False)
+    ref = torch.empty(T, nh * hd, device=DEV)
+    kernels.attn_generic(q, ref, cache, ctx.tok_pos, ctx.tok_seq, table, nh, nkv, hd, 64, window, scale, sink, planes, gate, **more)
+    # a score of standard normal vectors is off by at most (hd + 2) eps |q||k| scale <~ hd eps 4 sqrt(hd), in either kernel;
+    # a probability by twice that and a few eps for the exponential and the sum of up to 321 keys
+    score = (hd + 2) * EPS * 4 * math.sqrt(hd)
+    bound = 2 * (2 * score + 400 * EPS) * cache.abs().max().item()
+    assert (outs[0] - ref).abs().max().item() <= bound
+
+
+@pytest.mark.parametrize("tiles", [True, False])
+def test_attention_reads_no_value_that_is_not_seen(tiles):
+    """NaN in the rows of a page behind a sequence's end, and in another token's future, reaches no result."""
+    from gguf2bin_b200 import kernels
+    lens, q_lens = [100], [100]
+    cache, table, Ks, Vs = make_paged(1, lens, 1, 64, 64, torch.float32, seed=3)
+    last = int(table[0, 1])
+    cache[last, :, :, 36:] = math.nan
+    cache[last, :, :, 35] = math.nan                    # the last token's own key and value
+    q, out = rnd(100, 64, seed=4), torch.empty(100, 64, device=DEV)
+    assert kernels.attn_f32(q, out, cache, ctx_of(lens, q_lens, table, tiles), 1, 1, 64, 64, 0, 0.125)
+    assert torch.isfinite(out[:99]).all() and torch.isnan(out[99]).all()
