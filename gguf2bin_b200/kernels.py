@@ -725,7 +725,8 @@ F32_PARTS_MOST = 512 << 20        # bytes of scratch that the segments of single
 def attn_f32(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window, scale, sink=None, planes: int = 2,
              gate=None, chunk: int = 0, softcap: float = 0.0, keep_first: int = 0, v_heads: int = 0) -> bool:
     """``attn_generic`` in float over pages of 64 keys, for a whole step: prompts in the step's tiles, single tokens a
-    segment of keys at a time.  False when the sizes or the alignment are not the kernels'."""
+    segment of keys at a time.  False when the sizes or the alignment are not the kernels', or when the step says neither
+    its tiles nor its longest sequence and where to put the segments' parts."""
     if q.dtype != torch.float32 or cache_pages.dtype != torch.float32 or out.dtype != torch.float32 or page_size != 64 or \
             head_dim % 4 or head_dim > 256 or n_heads // n_kv_heads > 32 or q.stride(0) % 4 or q.stride(1) != 1 or \
             not out.is_contiguous() or any(t.data_ptr() % 16 for t in (q, out, cache_pages)) or \
@@ -733,16 +734,15 @@ def attn_f32(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size,
         return False
     if sink is not None:
         _need(sink, torch.float32, "sink")
-    tiles, parts, segments = (None, None, 0)
-    if ctx.attn_tiles is None or ctx.all_single:
-        segments = -(-ctx.max_kv_len // page_size)
+    tiles, parts, segments = getattr(ctx, "attn_tiles", None), None, 0
+    if tiles is None or ctx.all_single:
+        tiles, workspace = None, getattr(ctx, "workspace", None)
+        segments = -(-getattr(ctx, "max_kv_len", 0) // page_size)
         shape = (q.shape[0], n_heads, segments, head_dim + 2)
-        if segments < 1 or segments > ctx.page_table.shape[1] or q.shape[0] > 65535 or \
+        if workspace is None or segments < 1 or segments > ctx.page_table.shape[1] or q.shape[0] > 65535 or \
                 4 * shape[0] * shape[1] * shape[2] * shape[3] > F32_PARTS_MOST:
             return False
-        parts = ctx.workspace.buffer("attn.f32.parts", shape, torch.float32)
-    else:
-        tiles = ctx.attn_tiles
+        parts = workspace.buffer("attn.f32.parts", shape, torch.float32)
     f = _fn("attn_generic.cu", "g2b_attn_f32",
             [c_void_p] * 6 + [c_int] * 6 + [c_float, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_float, c_int, c_int,
                                             c_void_p, c_int, c_void_p, c_int, c_void_p])
