@@ -1225,8 +1225,8 @@ def moe_gemm(a, row_pair, pairs_per_token: int, w, n_out: int, plan, n_real: int
 
 def moe_gemv(a, row_pair, pairs_per_token: int, gather: bool, idx, w, n_out: int, plan, n_real: int, n_rows: int,
              swiglu: bool, out, blocked: bool = False, form: GluForm = SILU) -> bool:
-    """``moe_gemm`` for a step of few rows: a warp per four output columns of one row, the weight rows
-    streamed with 16-byte loads.  ``gather``: row r reads a[pair / pairs_per_token], else a[r].  False
+    """``moe_gemm`` for a step of few rows, the weight rows streamed with 16-byte loads: in bfloat16 once for all rows of
+    an expert (``swiglu`` in the blocked layout), else by a warp per four output columns of one row.  ``gather``: row r reads a[pair / pairs_per_token], else a[r].  False
     when the sizes do not allow 16-byte loads (the caller then takes ``moe_gemm``)."""
     if w.dtype != a.dtype:
         raise KernelError("moe_gemv: activations and expert matrices must have one dtype")

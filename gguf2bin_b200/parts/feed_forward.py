@@ -212,7 +212,7 @@ class RoutedExperts:
     grouped product for gate and up with the activation in its epilogue and one for down; nothing
     comes back to the host, so the step may be replayed from a CUDA graph."""
     graph_safe = True
-    FEW_ROWS = 128            # (token, choice) pairs up to which every row streams its expert's matrices by itself
+    FEW_ROWS = 128            # (token, choice) pairs up to which the experts' matrices are streamed past their rows
     MANY_ROWS = 48            # rows an expert on average from which its product runs on the tcgen05 kernel
 
     def __init__(self, spec: PartSpec, hidden_size: int, dtype: torch.dtype, device):
@@ -361,7 +361,7 @@ class RoutedExperts:
             wt = self.w_gate_up.dtype                     # matrices stored in 32-bit keep their products there
             mid = ws.buffer("moe.mid", (n_pairs, self.inter), wt)
             a = h if h.dtype == wt else h.to(wt)
-            # few rows (decoding): every row streams its expert's matrices.  Many rows an expert (a prompt
+            # few rows (decoding): the experts' matrices are streamed past their rows.  Many rows an expert (a prompt
             # step in bfloat16): the rows gathered side by side, then the tcgen05 kernel over each expert's
             # range.  Else tiles of rows per expert on mma.sync or the CUDA cores.
             few = n_pairs <= self.FEW_ROWS

@@ -1,0 +1,57 @@
+"""Few rows through routed experts' matrices in bfloat16: every row of every expert, whatever the plan, against 64-bit products."""
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, rnd
+
+pytestmark = pytest.mark.gpu
+
+
+def plan_of(idx, E):
+    from gguf2bin_b200 import kernels
+    n = idx.numel()
+    max_tiles = -(-n // kernels.moe_tile_rows()) + E
+    plan = torch.zeros(E + 2 + 3 * max_tiles, dtype=torch.int32, device=DEV)
+    row_pair, pair_row = (torch.full((n,), -1, dtype=torch.int32, device=DEV) for _ in range(2))
+    kernels.moe_plan(idx, E, max_tiles, plan, row_pair, pair_row)
+    return plan, row_pair, pair_row
+
+
+@pytest.mark.parametrize("T,top,E,spread", [(1, 1, 1, 1), (1, 4, 16, 18), (8, 3, 16, 16), (9, 2, 3, 3), (16, 8, 16, 16), (33, 3, 5, 2), (128, 1, 4, 1)])
+@pytest.mark.parametrize("N,K", [(8, 8), (24, 264), (40, 248), (1000, 512), (768, 1032), (48, 6000)])
+def test_rows_of_experts(T, top, E, spread, N, K):
+    """``spread``: experts that are chosen at all; from E on an expert has no matrices and its pairs no rows."""
+    from gguf2bin_b200 import kernels
+    g = torch.Generator().manual_seed(T + N)
+    idx = torch.randint(spread, (T, top), generator=g).to(torch.int32).to(DEV)
+    a, w = rnd(T, K, dtype=torch.bfloat16, seed=1), rnd(E, N, K, dtype=torch.bfloat16, seed=2)
+    plan, row_pair, pair_row = plan_of(idx, E)
+    used = int(plan[1 + E])
+    own = rnd(T * top, K, dtype=torch.bfloat16, seed=3)
+    pairs = torch.arange(T * top, device=DEV)
+    chosen = idx.flatten().long()
+    real = chosen < E
+    rows = pair_row[pairs[real]].long()
+    assert (pair_row[pairs[~real]] == -1).all() and used == int(real.sum())
+    for gather in (True, False):
+        src = a[pairs[real] // top] if gather else own[rows]
+        out = torch.full((T * top, N), float("nan"), device=DEV)
+        assert kernels.moe_gemv(a if gather else own, row_pair, top, gather, idx, w, N, plan, E, T * top, False, out)
+        ref = torch.einsum("rk,rnk->rn", src.double(), w[chosen[real]].double())
+        size = torch.einsum("rk,rnk->rn", src.double().abs(), w[chosen[real]].double().abs())
+        # products of bfloat16 are exact in 32 bits: only the sum of K rounds, at most K eps of the magnitudes
+        assert ((out[rows].double() - ref).abs() <= K * 2.0 ** -23 * size).all()
+        assert torch.isnan(out[used:]).all()
+        if N % 16:
+            continue
+        half = N // 2                                             # gates and ups, eight of each in turn
+        mid = torch.full((T * top, half), float("nan"), dtype=torch.bfloat16, device=DEV)
+        if half % 8:
+            continue
+        assert kernels.moe_gemv(a if gather else own, row_pair, top, gather, idx, w, half, plan, E, T * top, True, mid, True)
+        both = ref.view(-1, half // 8, 2, 8)
+        gate, up = both[:, :, 0].flatten(1), both[:, :, 1].flatten(1)
+        want = gate * torch.sigmoid(gate) * up
+        err = K * 2.0 ** -23 * size.view(-1, half // 8, 2, 8)
+        slack = 1.2 * err[:, :, 0].flatten(1) * up.abs() + (gate.abs() + 1) * err[:, :, 1].flatten(1)      # |silu'| < 1.1
+        assert ((mid[rows].double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-6).all()
