@@ -885,69 +885,65 @@ moe_combine_kernel(const float *__restrict__ rows, const int *__restrict__ pair_
   }
 }
 
-// The combination, then the sum's RMS norm (times a weight) added to the stream, and the new stream
-// once more in the compute type: what a layer whose sublayer outputs are normed does behind its routed
-// feed-forward, in one pass.  A thread keeps its share of the row (rows of up to 4,096 entries).
-#define MCN_PER 16
-template <typename T>
-__global__ void __launch_bounds__(256)
-moe_combine_norm_add_kernel(const float *__restrict__ rows, const int *__restrict__ pair_row,
-                            const float *__restrict__ weight, float *__restrict__ x, const float *__restrict__ norm_w,
-                            float eps, int top, int Hw, T *__restrict__ cast_out) {
+// The same four neighbours a thread, the choices' rows fetched four at a time (a token of a decode step is a few threads, whose
+// time is the chain from the pairs to their rows).
+__global__ void __launch_bounds__(128)
+moe_combine4_kernel(const float *__restrict__ rows, const int *__restrict__ pair_row, const float *__restrict__ weight,
+                    const float *__restrict__ x_self, int top, int Hw, float *__restrict__ out, int accumulate) {
   pdl_launch();
   pdl_wait();
-  __shared__ float scratch[32];
-  const int t = blockIdx.x;
-  float *xr = x + (size_t)t * Hw;
-  float keep[MCN_PER], own[MCN_PER];
-  float ss = 0.f;
+  const int t = blockIdx.x, j = (blockIdx.y * 128 + threadIdx.x) * 4;
+  if (j >= Hw) return;
+  float4 *to = reinterpret_cast<float4 *>(out + (size_t)t * Hw + j);
+  const float4 there = accumulate ? *to : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int r0 = 0; r0 < top; r0 += 4) {
+    const float *src[4];
+    float wt[4];
+    float4 v[4];
 #pragma unroll
-  for (int i = 0; i < MCN_PER; ++i) {
-    const int j = threadIdx.x + 256 * i;
-    float acc = 0.f;
-    own[i] = 0.f;
-    if (j < Hw) {
-      own[i] = xr[j];
-      for (int r = 0; r < top; ++r) {
-        const int row = pair_row[(size_t)t * top + r];
-        acc = fmaf(weight[(size_t)t * top + r], row >= 0 ? rows[(size_t)row * Hw + j] : own[i], acc);
-      }
+    for (int i = 0; i < 4; ++i) {
+      const size_t at = (size_t)t * top + min(r0 + i, top - 1);
+      const int row = pair_row[at];
+      wt[i] = weight[at];
+      src[i] = (row >= 0 ? rows + (size_t)row * Hw : x_self + (size_t)t * Hw) + j;
     }
-    keep[i] = acc;
-    ss = fmaf(acc, acc, ss);
-  }
-  ss = block_sum(ss, scratch);
-  const float inv = 1.f / sqrtf(ss / (float)Hw + eps);
 #pragma unroll
-  for (int i = 0; i < MCN_PER; ++i) {
-    const int j = threadIdx.x + 256 * i;
-    if (j < Hw) {
-      const float v = own[i] + (keep[i] * inv) * (norm_w ? norm_w[j] : 1.f);
-      xr[j] = v;
-      if (cast_out) cast_out[(size_t)t * Hw + j] = from_f32<T>(v);
-    }
+    for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4 *>(src[i]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (r0 + i < top)
+        a.x = fmaf(wt[i], v[i].x, a.x), a.y = fmaf(wt[i], v[i].y, a.y), a.z = fmaf(wt[i], v[i].z, a.z), a.w = fmaf(wt[i], v[i].w, a.w);
   }
+  *to = accumulate ? make_float4(there.x + a.x, there.y + a.y, there.z + a.z, there.w + a.w) : a;
 }
 
+// The combination, then the sum's RMS norm (times a weight) added to the stream, and the new stream
+// once more in the compute type (join.cuh): what a layer whose sublayer outputs are normed does behind its routed
+// feed-forward, in one pass.
+#define MCN_MOST 4096
 extern "C" int g2b_moe_combine_norm_add(const float *rows, const int *pair_row, const float *weight, float *x,
                                         const float *norm_w, float eps, int T_tokens, int top, int Hw, void *cast_out,
                                         int dtype, cudaStream_t stream) {
-  if (T_tokens <= 0) return 0;
-  if (Hw > 256 * MCN_PER) G2B_REFUSE("moe_combine_norm_add: rows of %d entries (at most %d)", Hw, 256 * MCN_PER);
-  if (dtype == G2B_F32)
-    g2b_launch(moe_combine_norm_add_kernel<float>, dim3(T_tokens), dim3(256), 0, stream, rows, pair_row, weight, x, norm_w,
-               eps, top, Hw, (float *)cast_out);
-  else if (dtype == G2B_BF16)
-    g2b_launch(moe_combine_norm_add_kernel<bf16>, dim3(T_tokens), dim3(256), 0, stream, rows, pair_row, weight, x, norm_w,
-               eps, top, Hw, (bf16 *)cast_out);
-  else
-    G2B_REFUSE("moe_combine_norm_add: unknown dtype %d", dtype);
+  if (T_tokens <= 0 || Hw <= 0) return 0;
+  if (Hw > MCN_MOST) G2B_REFUSE("moe_combine_norm_add: rows of %d entries (at most %d)", Hw, MCN_MOST);
+  const JoinTail a = {norm_w, eps, nullptr, nullptr, 0.f, cast_out, 1};
+  const JoinExperts from = {rows, pair_row, weight, nullptr, top};
+  const bool aligned = !(((uintptr_t)x | (uintptr_t)rows | (uintptr_t)norm_w | (uintptr_t)cast_out) & 15);
+  if (dtype == G2B_F32) launch_join<float>(x, from, a, T_tokens, Hw, aligned, stream);
+  else if (dtype == G2B_BF16) launch_join<bf16>(x, from, a, T_tokens, Hw, aligned, stream);
+  else G2B_REFUSE("moe_combine_norm_add: unknown dtype %d", dtype);
   return g2b_check_launch("moe_combine_norm_add");
 }
 
 extern "C" int g2b_moe_combine(const float *rows, const int *pair_row, const float *weight, const float *x_self, int T,
                                int top, int Hw, float *out, int accumulate, cudaStream_t stream) {
   if (T <= 0) return 0;
+  if (Hw % 4 == 0 && top > 0 && !(((uintptr_t)rows | (uintptr_t)x_self | (uintptr_t)out) & 15) && (Hw + 511) / 512 <= 65535) {
+    g2b_launch(moe_combine4_kernel, dim3(T, (Hw + 511) / 512), dim3(128), 0, stream, rows, pair_row, weight, x_self, top, Hw, out,
+               accumulate);
+    return g2b_check_launch("moe_combine");
+  }
   g2b_launch(moe_combine_kernel, dim3(T), dim3(256), 0, stream, rows, pair_row, weight, x_self, T, top, Hw, out, accumulate);
   return g2b_check_launch("moe_combine");
 }
@@ -958,7 +954,7 @@ extern "C" int g2b_moe_combine_join(const float *rows, const int *pair_row, cons
                                     float *x, const float *w, float eps, const float *add, int n_rows, int H,
                                     const float *next_w, float next_eps, void *next, int dtype, cudaStream_t stream) {
   if (n_rows <= 0 || H <= 0) return 0;
-  const JoinTail a = {w, eps, add, next_w, next_eps, next};
+  const JoinTail a = {w, eps, add, next_w, next_eps, next, 0};
   const JoinExperts from = {rows, pair_row, weight, base, top};
   const bool aligned = !(((uintptr_t)x | (uintptr_t)rows | (uintptr_t)base | (uintptr_t)w | (uintptr_t)add | (uintptr_t)next_w |
                           (uintptr_t)next) & 15);

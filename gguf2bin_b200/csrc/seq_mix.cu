@@ -1257,69 +1257,33 @@ extern "C" int g2b_gate_mul(const void *o, int hd, const void *gate, int gate_st
 // ---------------------------------------------------------------------------
 // x += norm(y) * w; the new x once more in the compute type
 // ---------------------------------------------------------------------------
-#define NORM_ADD_PER 16       // elements a thread keeps of a row of up to 4,096
+// The rounding alone (no result to add): the stream in the compute type.
 template <typename T>
 __global__ void __launch_bounds__(256)
-norm_add_kernel(float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ w, float eps, int Hw,
-                T *__restrict__ cast_out) {
+cast_rows_kernel(const float *__restrict__ x, long long n, T *__restrict__ out) {
   pdl_launch();
   pdl_wait();
-  __shared__ float scratch[32];
-  const int t = blockIdx.x;
-  float *xr = x + (size_t)t * Hw;
-  const bool held = Hw <= 256 * NORM_ADD_PER;          // the row of y stays in registers: one pass over it
-  float keep[NORM_ADD_PER];
-  float inv = 0.f;
-  if (y) {
-    const float *yr = y + (size_t)t * Hw;
-    float ss = 0.f;
-    if (held) {
-#pragma unroll
-      for (int i = 0; i < NORM_ADD_PER; ++i) {
-        const int j = threadIdx.x + 256 * i;
-        keep[i] = j < Hw ? yr[j] : 0.f;
-        ss = fmaf(keep[i], keep[i], ss);
-      }
-    } else {
-      for (int j = threadIdx.x; j < Hw; j += blockDim.x) ss = fmaf(yr[j], yr[j], ss);
-    }
-    ss = block_sum(ss, scratch);
-    inv = 1.f / sqrtf(ss / (float)Hw + eps);
-  }
-  if (held) {
-#pragma unroll
-    for (int i = 0; i < NORM_ADD_PER; ++i) {
-      const int j = threadIdx.x + 256 * i;
-      if (j < Hw) {
-        float v = xr[j];
-        if (y) {
-          v += (keep[i] * inv) * (w ? w[j] : 1.f);
-          xr[j] = v;
-        }
-        if (cast_out) cast_out[(size_t)t * Hw + j] = from_f32<T>(v);
-      }
-    }
-    return;
-  }
-  for (int j = threadIdx.x; j < Hw; j += blockDim.x) {
-    float v = xr[j];
-    if (y) {
-      v += (y[(size_t)t * Hw + j] * inv) * (w ? w[j] : 1.f);
-      xr[j] = v;
-    }
-    if (cast_out) cast_out[(size_t)t * Hw + j] = from_f32<T>(v);
-  }
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) out[i] = from_f32<T>(x[i]);
 }
 
+// x += norm(y) * w, and the new x rounded (join.cuh)
 extern "C" int g2b_norm_add(float *x, const float *y, const float *w, float eps, int T_tokens, int Hw, void *cast_out,
                             int dtype, cudaStream_t stream) {
-  if (T_tokens <= 0) return 0;
-  if (dtype == G2B_F32)
-    g2b_launch(norm_add_kernel<float>, dim3(T_tokens), dim3(256), 0, stream, x, y, w, eps, Hw, (float *)cast_out);
-  else if (dtype == G2B_BF16)
-    g2b_launch(norm_add_kernel<bf16>, dim3(T_tokens), dim3(256), 0, stream, x, y, w, eps, Hw, (bf16 *)cast_out);
-  else
-    G2B_REFUSE("norm_add: unknown dtype %d", dtype);
+  if (T_tokens <= 0 || Hw <= 0) return 0;
+  if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("norm_add: unknown dtype %d", dtype);
+  if (!y) {
+    if (!cast_out) return 0;
+    const long long n = (long long)T_tokens * Hw, blocks = (n + 255) / 256;
+    const dim3 grid((unsigned)(blocks < 4096 ? blocks : 4096));
+    if (dtype == G2B_F32) g2b_launch(cast_rows_kernel<float>, grid, dim3(256), 0, stream, x, n, (float *)cast_out);
+    else g2b_launch(cast_rows_kernel<bf16>, grid, dim3(256), 0, stream, x, n, (bf16 *)cast_out);
+    return g2b_check_launch("norm_add");
+  }
+  const JoinTail a = {w, eps, nullptr, nullptr, 0.f, cast_out, 1};
+  const JoinRow from = {y};
+  const bool aligned = !(((uintptr_t)x | (uintptr_t)y | (uintptr_t)w | (uintptr_t)cast_out) & 15);
+  if (dtype == G2B_F32) launch_join<float>(x, from, a, T_tokens, Hw, aligned, stream);
+  else launch_join<bf16>(x, from, a, T_tokens, Hw, aligned, stream);
   return g2b_check_launch("norm_add");
 }
 
@@ -1329,7 +1293,7 @@ extern "C" int g2b_norm_add(float *x, const float *y, const float *w, float eps,
 extern "C" int g2b_norm_join(float *x, const float *y, const float *w, float eps, const float *add, int n_rows, int H,
                              const float *next_w, float next_eps, void *next, int dtype, cudaStream_t stream) {
   if (n_rows <= 0 || H <= 0) return 0;
-  const JoinTail a = {w, eps, add, next_w, next_eps, next};
+  const JoinTail a = {w, eps, add, next_w, next_eps, next, 0};
   const JoinRow from = {y};
   const bool aligned = !(((uintptr_t)x | (uintptr_t)y | (uintptr_t)w | (uintptr_t)add | (uintptr_t)next_w | (uintptr_t)next) & 15);
   if (dtype == G2B_F32) launch_join<float>(x, from, a, n_rows, H, aligned, stream);
