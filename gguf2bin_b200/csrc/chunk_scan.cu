@@ -1,0 +1,654 @@
+// The state scan of a prompt in chunks: per head a state S [V columns of D], a token at a time
+//   S <- g_t S + s_t v_t k_t^T   (column c: S_c <- g_t S_c + s_t v_t[c] k_t),   o_t[c] = S_c . q_t
+// with g, s numbers per token and head (or one g per head and s = 1).  seq_mix.cu has the recurrence as it stands; a prompt
+// of thousands of tokens is a chain of dependent steps there, whatever the GPU could do beside it.
+//
+// Here a sequence is cut into segments, a segment into chunks of 64 tokens, and inside a chunk the recurrence is products:
+//   with D_ij = g_(j+1) ... g_i, c_i = g_0 ... g_i (from the chunk's start) and the state S at the chunk's start
+//   o_i = c_i (S q_i) + sum_(j<=i) (q_i . k_j) D_ij s_j v_j,      S' = c_last S + sum_j D_(last,j) s_j v_j k_j^T.
+// The decays are products of the g's themselves, in the order of the tokens (no logarithms, no quotients), so a g of zero is
+// exact, and everything is 32-bit multiply-adds as before.
+//   1. chunk_segment<false>: every segment by itself from a zero state: its own contribution, and the product of its g's
+//   2. chunk_carry: along a sequence, S at every segment's start from the contributions; the sequence's state in the end
+//   3. chunk_segment<true>: every segment from its start state: the outputs
+// A block of 256 threads takes a segment of one head and 64 columns; the state's share (64 x D) stays in registers (32 a
+// thread), q, k and v of the next chunk are on their way while one is computed.  Shared-memory reads bound it: 8 loads of 16
+// bytes feed 64 multiply-adds.  2,048 tokens, 8 heads of 128 x 256: 58 + 23 + 86 us (551 us as a chain); 1,501 tokens at
+// most in four sequences, 64 heads of 128 x 64 and 8 of 128 x 257, on average: 146 + 21 + 334 us (697 us).
+#include "common.cuh"
+
+G2B_DEFINE_LAST_ERROR
+
+#define CHUNK 64
+#define COLS 64
+#define THREADS 256
+#define MAX_D 128
+#define P_PITCH (CHUNK + 4)
+
+struct ChunkArgs {
+  const float *qf, *kf;       // [T, G, D] prepared
+  const void *v;              // compute type, rows of a wider buffer
+  int v_stride, H, G, D, V, Vin;        // V: columns of a head's state; Vin: value size in `v` (columns beyond: 1)
+  const float *decay;         // [H], or null:
+  const float *gates;         // [T, 2H]: g, then s
+  float *state;               // [slots, H, V, D]
+  const int *seq_meta;
+  int n_seqs, seg;            // tokens of a segment, a multiple of CHUNK
+  float *parts;               // [segments, H, V, D]: contributions, then start states
+  float *part_decay;          // [segments, H]
+  float *out;                 // [T, H*V]
+};
+
+// The sequence and the place in it of segment `idx` of the step (sequences one after another); false behind the last one.
+__device__ __forceinline__ bool find_segment(const int *meta, int n_seqs, int seg, int idx, int &b, int &place) {
+  const int lane = threadIdx.x & 31;
+  int before = 0;
+  for (int b0 = 0; b0 < n_seqs; b0 += 32) {
+    const int mine = b0 + lane < n_seqs ? (meta[4 * (b0 + lane) + 1] + seg - 1) / seg : 0;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned behind = __ballot_sync(0xffffffffu, before + upto > idx);
+    if (behind) {
+      const int at = __ffs(behind) - 1;
+      b = b0 + at;
+      place = idx - before - __shfl_sync(0xffffffffu, upto - mine, at);
+      return true;
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return false;
+}
+
+__device__ __forceinline__ void copy16(float *dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ float dot4(const float4 &a, const float4 &b, float acc) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
+}
+__device__ __forceinline__ float4 scale4(const float4 &a, float f) { return make_float4(a.x * f, a.y * f, a.z * f, a.w * f); }
+__device__ __forceinline__ void add4(float4 &a, float f, const float4 &b) {
+  a.x = fmaf(f, b.x, a.x), a.y = fmaf(f, b.y, a.y), a.z = fmaf(f, b.z, a.z), a.w = fmaf(f, b.w, a.w);
+}
+
+template <typename T, bool OUT>
+__global__ void __launch_bounds__(THREADS, OUT ? 1 : 2)
+chunk_segment_kernel(const ChunkArgs a) {
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];
+  const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, col0 = blockIdx.x * COLS;
+  int b, place;
+  if (!find_segment(a.seq_meta, a.n_seqs, a.seg, blockIdx.z, b, place)) return;
+  const int first = a.seq_meta[4 * b] + place * a.seg, n = min(a.seg, a.seq_meta[4 * b + 1] - place * a.seg);
+  const int qk_head = h / (H / a.G), tid = threadIdx.x;
+  float *K = sm, *Vs = K + 2 * CHUNK * pitch;            // two buffers of K and of V
+  // decays and strengths of the chunk's tokens; from the token on: to the end of its sixteen, of the chunk times its strength;
+  // up to the token: from its sixteen's start; the sixteens' products; in_block[B][i][j] = D_ij inside sixteen B
+  float *g = Vs + 2 * CHUNK * COLS, *s = g + CHUNK, *tail16 = s + CHUNK, *tail = tail16 + CHUNK, *head = tail + CHUNK, *block = head + CHUNK,
+        *in_block = block + 4;
+  float *Q = in_block + CHUNK * 17, *S = Q + 2 * CHUNK * pitch, *P = S + COLS * pitch;            // OUT only
+  // this thread's share of the state: columns 4 vy .. + 3, entries 4 dx .. + 3 and 64 further
+  const int dx = tid & 15, vy = tid >> 4;
+  const size_t head_state = (size_t)V * D;
+  float *part = a.parts + ((size_t)blockIdx.z * H + h) * head_state;
+  float4 st[4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int c = col0 + 4 * vy + i, d = 4 * dx + 64 * m;
+      st[i][m] = OUT && c < V && d < D ? *reinterpret_cast<const float4 *>(part + (size_t)c * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  float whole = 1.f;                                     // the product of the segment's g's
+  const T *vg = (const T *)a.v;
+  T rv[16];                                              // the next chunk's values, decay and strength, on their way
+  float rg = 1.f, rs = 0.f;
+  auto fetch = [&](int t0, int buf) {
+    const int nt = min(CHUNK, n - t0);
+    for (int i = tid; i < CHUNK * (D / 4); i += THREADS) {
+      const int r = i / (D / 4), c = i % (D / 4) * 4;
+      float *kd = K + (buf * CHUNK + r) * pitch + c, *qd = Q + (buf * CHUNK + r) * pitch + c;
+      const size_t at = ((size_t)(first + t0 + r) * a.G + qk_head) * D + c;
+      if (r < nt) {
+        copy16(kd, a.kf + at);
+        if (OUT) copy16(qd, a.qf + at);
+      } else {
+        *reinterpret_cast<float4 *>(kd) = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (OUT) *reinterpret_cast<float4 *>(qd) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    const int c = col0 + (tid & 63);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {                       // nothing here waits for a load
+      const int r = (tid >> 6) + 4 * i;
+      rv[i] = from_f32<T>(c < V && c >= a.Vin ? 1.f : 0.f);
+      if (r < nt && c < a.Vin) rv[i] = vg[(size_t)(first + t0 + r) * a.v_stride + (size_t)h * a.Vin + c];
+    }
+    if (tid < CHUNK) {
+      rg = 1.f;
+      rs = tid < nt ? 1.f : 0.f;
+      if (tid < nt) {
+        const size_t at = (size_t)(first + t0 + tid) * 2 * H + h;
+        if (a.decay) rg = a.decay[h];
+        else rg = a.gates[at], rs = a.gates[at + H];
+      }
+    }
+  };
+  fetch(0, 0);
+  int buf = 0;
+  for (int t0 = 0; t0 < n; t0 += CHUNK, buf ^= 1) {
+    const int nt = min(CHUNK, n - t0);
+    const bool more = t0 + CHUNK < n;
+    float *Vc = Vs + buf * CHUNK * COLS;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) Vc[((tid >> 6) + 4 * i) * COLS + (tid & 63)] = to_f32(rv[i]);
+    if (tid < CHUNK) {
+      g[tid] = rg;
+      s[tid] = rs;
+    }
+    if (OUT)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+          if (4 * dx + 64 * m < D) *reinterpret_cast<float4 *>(S + (4 * vy + i) * pitch + 4 * dx + 64 * m) = st[i][m];
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    if (more) fetch(t0 + CHUNK, buf ^ 1);
+    if (tid < CHUNK) {                                   // the decays from token `tid` on, to the end of its sixteen
+      const int b16 = tid & ~15, j = tid & 15;
+      float d = 1.f;
+      in_block[tid * 17 + j] = 1.f;                      // row i of its sixteen: in_block[(b16 + i) * 17 + j]
+      if (j == 0) head[tid] = g[tid];
+      for (int i = j + 1; i < 16; ++i) {
+        d *= g[b16 + i];
+        in_block[(b16 + i) * 17 + j] = d;
+        if (j == 0) head[b16 + i] = g[b16] * d;
+      }
+      tail16[tid] = d;
+      if (j == 0) block[tid >> 4] = g[b16] * d;
+    }
+    const float *Kc = K + buf * CHUNK * pitch;
+    if (OUT) {
+      const int tx = tid & 15, ty = tid >> 4;            // tokens ty + 16 i, columns (or keys) tx + 16 j
+      const float *Qc = Q + buf * CHUNK * pitch;
+      float p[4][4], o[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[i][j] = o[i][j] = 0.f;
+#pragma unroll 2
+      for (int d = 0; d < D; d += 4) {
+        float4 q[4], k[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4 *>(Qc + (ty + 16 * i) * pitch + d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(Kc + (tx + 16 * j) * pitch + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j <= i) p[i][j] = dot4(q[i], k[j], p[i][j]);       // later keys are not seen
+#pragma unroll
+        for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(S + (tx + 16 * j) * pitch + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[i][j] = dot4(q[i], k[j], o[i][j]);
+      }
+      __syncthreads();                                   // all decays stand
+      if (tid < CHUNK) {
+        float f = s[tid] * tail16[tid];
+        for (int B = (tid >> 4) + 1; B < 4; ++B) f *= block[B];
+        tail[tid] = f;
+      }
+      float before = 1.f;                                // the sixteens in front
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = ty + 16 * i;
+        const float up = head[r];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[i][j] *= before * up;
+        before *= block[i];
+        float between = up;                              // the sixteens between the key's and the row's, and the row's up to it
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+          if (j > i) continue;
+          const int t = tx + 16 * j;
+          if (j == i) {
+            p[i][j] = tx <= ty ? p[i][j] * (in_block[r * 17 + tx] * s[t]) : 0.f;
+          } else {
+            p[i][j] *= tail16[t] * between * s[t];
+            between *= block[j];
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) P[(ty + 16 * i) * P_PITCH + tx + 16 * j] = p[i][j];
+      __syncwarp();                                      // a row's 16 threads are one half of a warp
+      // sixteen tokens at a time, for the rows that see them; later values are not touched, whatever they hold
+#pragma unroll
+      for (int tb = 0; tb < 4; ++tb)
+#pragma unroll 1
+        for (int t = 16 * tb; t < 16 * tb + 16; t += 4) {
+          float x[4][4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[e][j] = Vc[(t + e) * COLS + tx + 16 * j];
+#pragma unroll
+          for (int i = tb; i < 4; ++i) {
+            const int r = ty + 16 * i;
+            const float4 w = *reinterpret_cast<const float4 *>(P + r * P_PITCH + t);
+            const bool all = i > tb;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (all || t <= r) o[i][j] = fmaf(w.x, x[0][j], o[i][j]);
+              if (all || t + 1 <= r) o[i][j] = fmaf(w.y, x[1][j], o[i][j]);
+              if (all || t + 2 <= r) o[i][j] = fmaf(w.z, x[2][j], o[i][j]);
+              if (all || t + 3 <= r) o[i][j] = fmaf(w.w, x[3][j], o[i][j]);
+            }
+          }
+        }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int r = ty + 16 * i, c = col0 + tx + 16 * j;
+          if (r < nt && c < V) a.out[(size_t)(first + t0 + r) * H * V + (size_t)h * V + c] = o[i][j];
+        }
+    } else {
+      __syncthreads();
+      if (tid < CHUNK) {
+        float f = s[tid] * tail16[tid];
+        for (int B = (tid >> 4) + 1; B < 4; ++B) f *= block[B];
+        tail[tid] = f;
+      }
+    }
+    __syncthreads();                                     // `tail` stands
+    if (!OUT || more) {
+      const float all = (block[0] * block[1]) * (block[2] * block[3]);
+      whole *= all;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) st[i][m] = scale4(st[i][m], all);
+#pragma unroll 4
+      for (int t = 0; t < nt; ++t) {
+        const float f = tail[t];
+        const float4 x = *reinterpret_cast<const float4 *>(Vc + t * COLS + 4 * vy);
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+          if (4 * dx + 64 * m < D) {
+            const float4 k = *reinterpret_cast<const float4 *>(Kc + t * pitch + 4 * dx + 64 * m);
+            add4(st[0][m], f * x.x, k);
+            add4(st[1][m], f * x.y, k);
+            add4(st[2][m], f * x.z, k);
+            add4(st[3][m], f * x.w, k);
+          }
+      }
+    }
+    __syncthreads();                                     // g, tail, S and P are written again
+  }
+  if (!OUT) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int c = col0 + 4 * vy + i, d = 4 * dx + 64 * m;
+        if (c < V && d < D) *reinterpret_cast<float4 *>(part + (size_t)c * D + d) = st[i][m];
+      }
+    if (tid == 0 && blockIdx.x == 0) a.part_decay[(size_t)blockIdx.z * H + h] = whole;
+  }
+}
+
+// Four neighbours of a sequence's state a thread, along the sequence's segments.
+__global__ void __launch_bounds__(THREADS)
+chunk_carry_kernel(const ChunkArgs a) {
+  pdl_launch();
+  pdl_wait();
+  const int b = blockIdx.y, lane = threadIdx.x & 31;
+  int before = 0;                                        // segments of the sequences in front
+  for (int b0 = 0; b0 < b; b0 += 32) {
+    int c = b0 + lane < b ? (a.seq_meta[4 * (b0 + lane) + 1] + a.seg - 1) / a.seg : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    before += c;
+  }
+  const size_t size = (size_t)a.H * a.V * a.D, e = ((size_t)blockIdx.x * THREADS + threadIdx.x) * 4;
+  if (e >= size) return;
+  const int h = (int)(e / ((size_t)a.V * a.D)), segments = (a.seq_meta[4 * b + 1] + a.seg - 1) / a.seg;
+  float4 *kept = reinterpret_cast<float4 *>(a.state + (size_t)a.seq_meta[4 * b + 3] * size + e);
+  float4 s = *kept;
+  for (int i0 = 0; i0 < segments; i0 += 4) {
+    float4 x[4];
+    float g[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const size_t at = (size_t)before + min(i0 + i, segments - 1);
+      x[i] = *reinterpret_cast<const float4 *>(a.parts + at * size + e);
+      g[i] = a.part_decay[at * a.H + h];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i0 + i < segments) {
+        *reinterpret_cast<float4 *>(a.parts + ((size_t)before + i0 + i) * size + e) = s;
+        s = make_float4(fmaf(g[i], s.x, x[i].x), fmaf(g[i], s.y, x[i].y), fmaf(g[i], s.z, x[i].z), fmaf(g[i], s.w, x[i].w));
+      }
+  }
+  *kept = s;
+}
+
+template <typename T, bool OUT>
+static int launch_segments(const ChunkArgs &a, dim3 grid, cudaStream_t stream) {
+  static G2bPerDevice done;
+  auto bytes = [](int D) {
+    return sizeof(float) * ((size_t)2 * CHUNK * (D + 4) * (OUT ? 2 : 1) + 2 * CHUNK * COLS + 5 * CHUNK + 4 + CHUNK * 17 +
+                            (OUT ? (size_t)COLS * (D + 4) + CHUNK * P_PITCH : 0));
+  };
+  const int dev = g2b_current_device();
+  if (dev < 0 || !done.value[dev]) {
+    if (cudaFuncSetAttribute(chunk_segment_kernel<T, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(MAX_D)) != cudaSuccess)
+      G2B_REFUSE("chunk_scan: %zu bytes of shared memory are not available", bytes(MAX_D));
+    if (dev >= 0) done.value[dev] = 1;
+  }
+  g2b_launch(chunk_segment_kernel<T, OUT>, grid, dim3(THREADS), bytes(a.D), stream, a);
+  return g2b_check_launch("chunk_scan");
+}
+
+// `segments`: how many there can be (n_tokens / seg + n_seqs); parts [segments, H, V, D], part_decay [segments, H].
+extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D, int Vin,
+                              int extra_one, const float *decay, const float *gates, float *state, const int *seq_meta, int n_seqs,
+                              int seg, int segments, float *parts, float *part_decay, float *out, cudaStream_t stream) {
+  const int V = Vin + (extra_one ? 1 : 0);
+  if (n_seqs <= 0 || segments <= 0) return 0;
+  if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("chunk_scan: unknown dtype %d", dtype);
+  if (D <= 0 || D > MAX_D || D % 4) G2B_REFUSE("chunk_scan: key size %d (a multiple of 4 up to %d)", D, MAX_D);
+  if (G <= 0 || H % G) G2B_REFUSE("chunk_scan: %d heads are not a multiple of %d query/key heads", H, G);
+  if (!decay == !gates) G2B_REFUSE("chunk_scan: a decay per head or gates, not both");
+  if (seg <= 0 || seg % CHUNK) G2B_REFUSE("chunk_scan: segments of %d tokens (a multiple of %d)", seg, CHUNK);
+  if (H > 65535 || segments > 65535 || n_seqs > 65535) G2B_REFUSE("chunk_scan: %d heads, %d segments are too many", H, segments);
+  if (((uintptr_t)qf | (uintptr_t)kf | (uintptr_t)state | (uintptr_t)parts) & 15) G2B_REFUSE("chunk_scan: a buffer is off 16 bytes");
+  const ChunkArgs a = {qf, kf, v, v_stride, H, G, D, V, Vin, decay, gates, state, seq_meta, n_seqs, seg, parts, part_decay, out};
+  const dim3 grid((V + COLS - 1) / COLS, H, segments);
+  if (int rc = dtype == G2B_F32 ? launch_segments<float, false>(a, grid, stream) : launch_segments<bf16, false>(a, grid, stream)) return rc;
+  const size_t quads = (size_t)H * V * D / 4;
+  g2b_launch(chunk_carry_kernel, dim3((unsigned)((quads + THREADS - 1) / THREADS), n_seqs), dim3(THREADS), 0, stream, a);
+  if (int rc = g2b_check_launch("chunk_scan")) return rc;
+  return dtype == G2B_F32 ? launch_segments<float, true>(a, grid, stream) : launch_segments<bf16, true>(a, grid, stream);
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// the gated delta rule in chunks
+// ---------------------------------------------------------------------------------------------------------
+//   S <- g_t S;  u_t = b_t (v_t - S k_t);  S <- S + u_t k_t^T;  o_t = S q_t
+// Inside a chunk of 32 tokens, with D_ij and c_i as above and the state S at the chunk's start, the u solve a triangular system
+//   u_i + sum_(j<i) A_ij u_j = b_i v_i - b_i c_i S k_i,   A_ij = b_i D_ij (k_i . k_j),
+// whose right side is linear in S: U = U0 - W S^T with (I + A) U0 = (b_i v_i) and (I + A) W = (b_i c_i k_i).
+//   1. delta_chunk: every chunk by itself (none needs the state): U0, W by substitution, a column a thread, and the
+//      products P_ij = D_ij (q_i . k_j) of the outputs
+//   2. delta_walk: along the sequence, a chunk a step: U = U0 - W S^T, o_i = c_i S q_i + sum_(j<=i) P_ij u_j,
+//      S' = c_last S + sum_j D_(last,j) u_j k_j^T.  A block has 8 columns of a head; the next chunk's operands are on their way.
+// The substitution takes the tokens in their order, as the recurrence does; all is 32-bit.  The walk's chain of products, read
+// from shared memory, bounds it.  2,048 tokens, 8 heads of 128 x 128: 60 + 219 us (714 us a token after a token).
+#define DELTA_CHUNK 32
+#define DELTA_COLS 8
+#define DELTA_WALK 128
+
+struct DeltaArgs {
+  const float *qf, *kf;       // [T, G, D] prepared
+  const void *v;              // compute type, rows of a wider buffer
+  int v_stride, H, G, D, V;
+  const float *ab;            // [T, 2H]: decay input, then write-strength input
+  const float *A_log, *dt_bias;
+  float *state;               // [slots, H, V, D]
+  const int *seq_meta;
+  int n_seqs;
+  float *U0, *W, *P, *decays; // [chunks, H, 32, V], [.., 32, D], [.., 32, 32], [.., 64]: c, then the decays to the chunk's end
+  float *out;                 // [T, H*V]
+};
+
+template <typename T>
+__global__ void __launch_bounds__(THREADS)
+delta_chunk_kernel(const DeltaArgs a) {
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];
+  __shared__ __align__(16) float M[DELTA_CHUNK][DELTA_CHUNK + 4];         // D_ij, then A_ij
+  __shared__ float g[DELTA_CHUNK], beta[DELTA_CHUNK], c[DELTA_CHUNK];
+  const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, tid = threadIdx.x, qk_head = h / (H / a.G);
+  int b, place;
+  if (!find_segment(a.seq_meta, a.n_seqs, DELTA_CHUNK, blockIdx.x, b, place)) return;
+  const int first = a.seq_meta[4 * b] + place * DELTA_CHUNK, nt = min(DELTA_CHUNK, a.seq_meta[4 * b + 1] - place * DELTA_CHUNK);
+  float *K = sm, *Q = K + DELTA_CHUNK * pitch;
+  for (int i = tid; i < DELTA_CHUNK * (D / 4); i += THREADS) {
+    const int r = i / (D / 4), d = i % (D / 4) * 4;
+    const size_t at = ((size_t)(first + r) * a.G + qk_head) * D + d;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4 *>(K + r * pitch + d) = r < nt ? *reinterpret_cast<const float4 *>(a.kf + at) : zero;
+    *reinterpret_cast<float4 *>(Q + r * pitch + d) = r < nt ? *reinterpret_cast<const float4 *>(a.qf + at) : zero;
+  }
+  if (tid < DELTA_CHUNK) {
+    float x = 1.f, y = 0.f;
+    if (tid < nt) {
+      const float *ab = a.ab + (size_t)(first + tid) * 2 * H;
+      const float z = ab[h] + a.dt_bias[h];
+      x = expf(-expf(a.A_log[h]) * (fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)))));
+      y = 1.f / (1.f + expf(-ab[H + h]));
+    }
+    g[tid] = x;
+    beta[tid] = y;
+  }
+  __syncthreads();
+  const size_t item = (size_t)blockIdx.x * H + h;
+  if (tid < DELTA_CHUNK) {
+    float d = 1.f;
+    M[tid][tid] = 1.f;
+    for (int i = tid + 1; i < DELTA_CHUNK; ++i) {
+      d *= g[i];
+      M[i][tid] = d;
+    }
+    a.decays[item * 64 + DELTA_CHUNK + tid] = d;
+  }
+  const int i = tid >> 3, j0 = tid & 7;
+  float kk[4] = {0.f, 0.f, 0.f, 0.f}, qk[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int d = 0; d < D; d += 4) {
+    const float4 ki = *reinterpret_cast<const float4 *>(K + i * pitch + d), qi = *reinterpret_cast<const float4 *>(Q + i * pitch + d);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const float4 kj = *reinterpret_cast<const float4 *>(K + (j0 + 8 * m) * pitch + d);
+      kk[m] = dot4(ki, kj, kk[m]);
+      qk[m] = dot4(qi, kj, qk[m]);
+    }
+  }
+  __syncthreads();                                       // the decays stand
+  if (tid < DELTA_CHUNK) {
+    c[tid] = g[0] * M[tid][0];
+    a.decays[item * 64 + tid] = c[tid];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int j = j0 + 8 * m;
+    const float d = j <= i ? M[i][j] : 0.f;
+    a.P[(item * DELTA_CHUNK + i) * DELTA_CHUNK + j] = j <= i ? d * qk[m] : 0.f;
+    M[i][j] = j < i ? beta[i] * d * kk[m] : 0.f;
+  }
+  __syncthreads();
+  const T *vg = (const T *)a.v;
+  for (int col = tid; col < V + D; col += THREADS) {
+    float x[DELTA_CHUNK];
+#pragma unroll
+    for (int r = 0; r < DELTA_CHUNK; ++r) {
+      float y;
+      if (col < V) y = r < nt ? beta[r] * to_f32(vg[(size_t)(first + r) * a.v_stride + (size_t)h * V + col]) : 0.f;
+      else y = beta[r] * c[r] * K[r * pitch + col - V];
+      x[r] = y;
+    }
+#pragma unroll
+    for (int r = 1; r < DELTA_CHUNK; ++r) {
+      float y = x[r];
+#pragma unroll
+      for (int j = 0; j < r; j += 4) {
+        const float4 m = *reinterpret_cast<const float4 *>(&M[r][j]);
+        y = fmaf(-m.x, x[j], y);
+        if (j + 1 < r) y = fmaf(-m.y, x[j + 1], y);
+        if (j + 2 < r) y = fmaf(-m.z, x[j + 2], y);
+        if (j + 3 < r) y = fmaf(-m.w, x[j + 3], y);
+      }
+      x[r] = y;
+    }
+    float *to = col < V ? a.U0 + item * DELTA_CHUNK * V + col : a.W + item * DELTA_CHUNK * D + col - V;
+    const int step = col < V ? V : D;
+#pragma unroll
+    for (int r = 0; r < DELTA_CHUNK; ++r) to[(size_t)r * step] = x[r];
+  }
+}
+
+__global__ void __launch_bounds__(DELTA_WALK)
+delta_walk_kernel(const DeltaArgs a) {
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];
+  const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31;
+  const int qk_head = h / (H / a.G), col0 = blockIdx.x * DELTA_COLS;
+  int before = 0;                                        // chunks of the sequences in front
+  for (int b0 = 0; b0 < b; b0 += 32) {
+    int n = b0 + lane < b ? (a.seq_meta[4 * (b0 + lane) + 1] + DELTA_CHUNK - 1) / DELTA_CHUNK : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    before += n;
+  }
+  const int first = a.seq_meta[4 * b], n = a.seq_meta[4 * b + 1], slot = a.seq_meta[4 * b + 3];
+  // two buffers, each: W, Q, K [32, pitch], P [32, 36], U0 [32, 8], decays [64]
+  const int rows = DELTA_CHUNK * pitch, P_AT = 3 * rows, U_AT = P_AT + DELTA_CHUNK * 36, G_AT = U_AT + DELTA_CHUNK * DELTA_COLS,
+            SIZE = G_AT + 64;
+  float *S = sm + 2 * SIZE, *U = S + DELTA_COLS * pitch;                 // S [8, pitch], U [32, 8]
+  auto fetch = [&](int t0, int buf) {
+    float *to = sm + buf * SIZE;
+    const size_t item = (size_t)(before + t0 / DELTA_CHUNK) * H + h;
+    const int nt = min(DELTA_CHUNK, n - t0);
+    for (int i = tid; i < DELTA_CHUNK * (D / 4); i += DELTA_WALK) {
+      const int r = i / (D / 4), d = i % (D / 4) * 4;
+      const size_t at = ((size_t)(first + t0 + min(r, nt - 1)) * a.G + qk_head) * D + d;      // rows behind the last are not used
+      copy16(to + r * pitch + d, a.W + (item * DELTA_CHUNK + r) * D + d);
+      copy16(to + rows + r * pitch + d, a.qf + at);
+      copy16(to + 2 * rows + r * pitch + d, a.kf + at);
+    }
+    for (int i = tid; i < DELTA_CHUNK * (DELTA_CHUNK / 4); i += DELTA_WALK)
+      copy16(to + P_AT + (i / 8) * 36 + (i % 8) * 4, a.P + item * DELTA_CHUNK * DELTA_CHUNK + i * 4);
+    if (tid < DELTA_CHUNK * 2) {
+      const int r = tid >> 1, q = (tid & 1) * 4;
+      if (col0 + q < V) copy16(to + U_AT + r * DELTA_COLS + q, a.U0 + (item * DELTA_CHUNK + r) * V + col0 + q);
+    }
+    if (tid >= 64 && tid < 80) copy16(to + G_AT + (tid - 64) * 4, a.decays + item * 64 + (tid - 64) * 4);
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  // this thread's share of the state: column cs, entries 4 dx .. + 3 and 64 further
+  const int cs = tid >> 4, dx = tid & 15;
+  float *kept = a.state + (((size_t)slot * H + h) * V + col0 + cs) * D;
+  float4 st[2];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    const int d = 4 * dx + 64 * m;
+    st[m] = col0 + cs < V && d < D ? *reinterpret_cast<const float4 *>(kept + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (d < D) *reinterpret_cast<float4 *>(S + cs * pitch + d) = st[m];
+  }
+  for (int i = tid; i < 2 * DELTA_CHUNK * DELTA_COLS; i += DELTA_WALK)   // columns behind the last hold zeros
+    sm[(i / (DELTA_CHUNK * DELTA_COLS)) * SIZE + U_AT + i % (DELTA_CHUNK * DELTA_COLS)] = 0.f;
+  __syncthreads();
+  fetch(0, 0);
+  const int r0 = tid >> 3, cc = tid & 7;                 // tokens r0 and r0 + 16, column cc
+  int buf = 0;
+  for (int t0 = 0; t0 < n; t0 += DELTA_CHUNK, buf ^= 1) {
+    const int nt = min(DELTA_CHUNK, n - t0);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();                                     // the chunk's operands and S are in place
+    if (t0 + DELTA_CHUNK < n) fetch(t0 + DELTA_CHUNK, buf ^ 1);
+    const float *W = sm + buf * SIZE, *Q = W + rows, *K = Q + rows, *P = W + P_AT, *U0 = W + U_AT, *G = W + G_AT;
+    float ws[2] = {0.f, 0.f}, qs[2] = {0.f, 0.f};
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+      const float4 s = *reinterpret_cast<const float4 *>(S + cc * pitch + d);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        ws[m] = dot4(*reinterpret_cast<const float4 *>(W + (r0 + 16 * m) * pitch + d), s, ws[m]);
+        qs[m] = dot4(*reinterpret_cast<const float4 *>(Q + (r0 + 16 * m) * pitch + d), s, qs[m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) U[(r0 + 16 * m) * DELTA_COLS + cc] = U0[(r0 + 16 * m) * DELTA_COLS + cc] - ws[m];
+    __syncthreads();                                     // U stands, and S is read
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int r = r0 + 16 * m;
+      float o = G[r] * qs[m];
+#pragma unroll
+      for (int j = 0; j < 16 + 16 * m; j += 4) {
+        const float4 p = *reinterpret_cast<const float4 *>(P + r * 36 + j);
+        if (j <= r) o = fmaf(p.x, U[j * DELTA_COLS + cc], o);            // later tokens are not touched, whatever they hold
+        if (j + 1 <= r) o = fmaf(p.y, U[(j + 1) * DELTA_COLS + cc], o);
+        if (j + 2 <= r) o = fmaf(p.z, U[(j + 2) * DELTA_COLS + cc], o);
+        if (j + 3 <= r) o = fmaf(p.w, U[(j + 3) * DELTA_COLS + cc], o);
+      }
+      if (r < nt && col0 + cc < V) a.out[(size_t)(first + t0 + r) * H * V + (size_t)h * V + col0 + cc] = o;
+    }
+    const float all = G[DELTA_CHUNK - 1];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) st[m] = scale4(st[m], all);
+#pragma unroll 4
+    for (int j = 0; j < nt; ++j) {
+      const float f = G[DELTA_CHUNK + j] * U[j * DELTA_COLS + cs];
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+        if (4 * dx + 64 * m < D) add4(st[m], f, *reinterpret_cast<const float4 *>(K + j * pitch + 4 * dx + 64 * m));
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+      if (4 * dx + 64 * m < D) *reinterpret_cast<float4 *>(S + cs * pitch + 4 * dx + 64 * m) = st[m];
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    const int d = 4 * dx + 64 * m;
+    if (col0 + cs < V && d < D) *reinterpret_cast<float4 *>(kept + d) = st[m];
+  }
+}
+
+// `chunks`: how many there can be (n_tokens / 32 + n_seqs).
+extern "C" int g2b_delta_scan(int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D, int V,
+                              const float *ab, const float *A_log, const float *dt_bias, float *state, const int *seq_meta, int n_seqs,
+                              int chunks, float *U0, float *W, float *P, float *decays, float *out, cudaStream_t stream) {
+  if (n_seqs <= 0 || chunks <= 0) return 0;
+  if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("delta_scan: unknown dtype %d", dtype);
+  if (D <= 0 || D > MAX_D || D % 4 || V <= 0 || V % 4) G2B_REFUSE("delta_scan: key size %d (a multiple of 4 up to %d), value size %d (of 4)", D, MAX_D, V);
+  if (G <= 0 || H % G) G2B_REFUSE("delta_scan: %d heads are not a multiple of %d query/key heads", H, G);
+  if (H > 65535 || n_seqs > 65535) G2B_REFUSE("delta_scan: %d heads, %d sequences are too many", H, n_seqs);
+  if (((uintptr_t)qf | (uintptr_t)kf | (uintptr_t)state | (uintptr_t)U0 | (uintptr_t)W | (uintptr_t)P | (uintptr_t)decays) & 15)
+    G2B_REFUSE("delta_scan: a buffer is off 16 bytes");
+  const DeltaArgs a = {qf, kf, v, v_stride, H, G, D, V, ab, A_log, dt_bias, state, seq_meta, n_seqs, U0, W, P, decays, out};
+  auto prep_bytes = [](int d) { return sizeof(float) * (size_t)2 * DELTA_CHUNK * (d + 4); };
+  auto walk_bytes = [](int d) {
+    return sizeof(float) * ((size_t)2 * (3 * DELTA_CHUNK * (d + 4) + DELTA_CHUNK * 36 + DELTA_CHUNK * DELTA_COLS + 64) + DELTA_COLS * (d + 4) +
+                            DELTA_CHUNK * DELTA_COLS);
+  };
+  static G2bPerDevice done;
+  const int dev = g2b_current_device();
+  if (dev < 0 || !done.value[dev]) {
+    if (cudaFuncSetAttribute(delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_bytes(MAX_D)) != cudaSuccess)
+      G2B_REFUSE("delta_scan: %zu bytes of shared memory are not available", walk_bytes(MAX_D));
+    if (dev >= 0) done.value[dev] = 1;
+  }
+  if (dtype == G2B_F32) g2b_launch(delta_chunk_kernel<float>, dim3(chunks, H), dim3(THREADS), prep_bytes(D), stream, a);
+  else g2b_launch(delta_chunk_kernel<bf16>, dim3(chunks, H), dim3(THREADS), prep_bytes(D), stream, a);
+  if (int rc = g2b_check_launch("delta_scan")) return rc;
+  g2b_launch(delta_walk_kernel, dim3((V + DELTA_COLS - 1) / DELTA_COLS, H, n_seqs), dim3(DELTA_WALK), walk_bytes(D), stream, a);
+  return g2b_check_launch("delta_scan");
+}

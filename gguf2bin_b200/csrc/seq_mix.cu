@@ -1016,6 +1016,25 @@ static void launch_scan_prompt(const PScanArgs &a, dim3 grid, size_t smem, cudaS
   else g2b_launch(state_scan_prompt_kernel<T, MODE, 32>, grid, dim3(PSCAN_THREADS), smem, stream, a);
 }
 
+// The preparation alone: q and k of the step turned or divided by their norms, scaled, in float [T, G, D].
+extern "C" int g2b_scan_prep(int dtype, const void *q, int q_stride, const void *k, int k_stride, int n_tokens, int G, int D,
+                             const float *rope, int rot, int interleaved, float q_scale, float k_scale, int unit_norm, float unit_eps,
+                             float *qf, float *kf, cudaStream_t stream) {
+  if (n_tokens <= 0) return 0;
+  if (D <= 0 || D > SCAN_MAX_D) G2B_REFUSE("state_scan: key size %d outside 1..%d", D, SCAN_MAX_D);
+  if (rope && (rot <= 0 || rot > D || (rot & 1))) G2B_REFUSE("state_scan: %d rotated entries of a head of %d", rot, D);
+  const dim3 grid((unsigned)(((long long)n_tokens * G + 3) / 4));
+  if (dtype == G2B_F32)
+    g2b_launch(scan_prep_kernel<float>, grid, dim3(128), 0, stream, (const float *)q, q_stride, (const float *)k, k_stride, n_tokens, G, D,
+               (const float2 *)rope, rot, interleaved, q_scale, k_scale, unit_norm, unit_eps, qf, kf);
+  else if (dtype == G2B_BF16)
+    g2b_launch(scan_prep_kernel<bf16>, grid, dim3(128), 0, stream, (const bf16 *)q, q_stride, (const bf16 *)k, k_stride, n_tokens, G, D,
+               (const float2 *)rope, rot, interleaved, q_scale, k_scale, unit_norm, unit_eps, qf, kf);
+  else
+    G2B_REFUSE("state_scan: unknown dtype %d", dtype);
+  return g2b_check_launch("state_scan_prep");
+}
+
 extern "C" int g2b_state_scan_prompt(int mode, int dtype, const void *q, int q_stride, const void *k, int k_stride,
                                      const void *v, int v_stride, int H, int G, int D, int V, const float *rope, int rot,
                                      int interleaved, float q_scale, float k_scale, int unit_norm, float unit_eps,

@@ -946,6 +946,34 @@ def short_conv(x, w32, ring, ctx, out, act: bool = True, bias=None) -> None:
         count_launches(1)
 
 
+DELTA_CHUNK = 32                  # tokens of a chunk of the gated delta rule (csrc/chunk_scan.cu)
+CHUNK_PARTS_MOST = 1 << 30        # bytes of scratch that the segments' states, or the delta rule's chunks, may take
+
+
+def _chunk_segment(n_tokens: int, n_seqs: int, heads: int, cols: int, dim: int) -> int:
+    """Tokens of a segment of the scan in chunks (csrc/chunk_scan.cu), 0 where the scan of a token after a token is taken: key
+    sizes that the kernel has not, prompts of less than 96 tokens on average, whose chain is no longer than the
+    chunked scan's launches, and states that do not fit the scratch.  The longest of 256, 128 and 64 tokens that
+    leaves four blocks for every SM, longer where the scratch asks for it."""
+    if dim % 4 or dim > 128 or n_tokens < 96 * n_seqs or heads > 65535:
+        return 0
+    blocks = heads * -(-cols // 64)
+    seg = next((s for s in (256, 128) if n_tokens // s * blocks >= 4 * 148), 64)
+    while 4 * (n_tokens // seg + n_seqs) * heads * cols * dim > CHUNK_PARTS_MOST:
+        if seg > n_tokens:
+            return 0
+        seg *= 2
+    return seg if n_tokens // seg + n_seqs <= 65535 else 0
+
+
+def _delta_chunks(n_tokens: int, n_seqs: int, heads: int, dim: int, v_dim: int) -> int:
+    """Chunks of the gated delta rule over a prompt, 0 where it goes a token after a token: _chunk_segment's rule on sizes
+    and lengths, with the scratch of the chunks' own products."""
+    chunks = n_tokens // DELTA_CHUNK + n_seqs
+    fits = 4 * chunks * heads * (DELTA_CHUNK * (v_dim + dim + DELTA_CHUNK) + 64) <= CHUNK_PARTS_MOST and chunks <= 65535
+    return chunks if fits and v_dim % 4 == 0 and _chunk_segment(n_tokens, 1, heads, 1, dim) and n_tokens >= 96 * n_seqs else 0
+
+
 def state_scan(q, k, v, state, ctx, out32, heads, qk_heads, qk_dim, v_dim, *, decay=None, ab=None, a_log=None,
                dt_bias=None, rope=None, rotary_dim: int = 0, interleaved: bool = False, q_scale: float = 1.0,
                k_scale: float = 1.0, unit_eps: Optional[float] = None, gates=None, ones_column: bool = False) -> None:
@@ -985,6 +1013,39 @@ def state_scan(q, k, v, state, ctx, out32, heads, qk_heads, qk_dim, v_dim, *, de
         # that fetches the next tokens while it works on the ones it has
         qf = ctx.workspace.buffer("scan.q", (T, qk_heads * qk_dim), torch.float32)
         kf = ctx.workspace.buffer("scan.k", (T, qk_heads * qk_dim), torch.float32)
+        chunks = seg = 0
+        if not state.data_ptr() & 15:
+            if mode == 1:
+                chunks = _delta_chunks(T, ctx.n_seqs, heads, qk_dim, v_dim)
+            else:
+                seg = _chunk_segment(T, ctx.n_seqs, heads, cols, qk_dim)
+        if seg or chunks:
+            f = _fn("seq_mix.cu", "g2b_scan_prep",
+                    [c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_float, c_float, c_int,
+                     c_float, c_void_p, c_void_p, c_void_p])
+            _call(f, _code(q.dtype), _ptr(q), _dense_rows(q, "q"), _ptr(k), _dense_rows(k, "k"), T, qk_heads, qk_dim, _ptr(rope),
+                  rotary_dim, 1 if interleaved else 0, q_scale, k_scale, 0 if unit_eps is None else 1, unit_eps or 0.0, _ptr(qf),
+                  _ptr(kf), _stream())
+            if chunks:
+                u0, w_, p_, dec = (ctx.workspace.buffer("delta." + n, (chunks, heads, *shape), torch.float32) for n, shape in (
+                    ("u0", (DELTA_CHUNK, v_dim)), ("w", (DELTA_CHUNK, qk_dim)), ("p", (DELTA_CHUNK, DELTA_CHUNK)), ("decays", (64,))))
+                f = _fn("chunk_scan.cu", "g2b_delta_scan",
+                        [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p] * 5 + [c_int] * 2 + [c_void_p] * 6)
+                _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim, _ptr(ab),
+                      _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, chunks, _ptr(u0), _ptr(w_), _ptr(p_),
+                      _ptr(dec), _ptr(out32), _stream())
+                count_launches(1)
+                return
+            segments = T // seg + ctx.n_seqs
+            parts = ctx.workspace.buffer("scan.parts", (segments, heads, cols, qk_dim), torch.float32)
+            decays = ctx.workspace.buffer("scan.part_decay", (segments, heads), torch.float32)
+            f = _fn("chunk_scan.cu", "g2b_chunk_scan",
+                    [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p] * 4 + [c_int] * 3 + [c_void_p] * 4)
+            _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim,
+                  1 if ones_column else 0, _ptr(decay), _ptr(gates), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, seg, segments,
+                  _ptr(parts), _ptr(decays), _ptr(out32), _stream())
+            count_launches(2)
+            return
         f = _fn("seq_mix.cu", "g2b_state_scan_prompt",
                 types + [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p])
         _call(f, *common, _ptr(ctx.seq_meta), T, ctx.n_seqs, _ptr(qf), _ptr(kf), _ptr(out32),
