@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -24
 
 
-@pytest.mark.parametrize("N,K", [(1, 4), (4, 64), (17, 60), (64, 68), (65, 132), (130, 516), (1024, 3072), (4800, 1028), (9000, 96)])
+@pytest.mark.parametrize("N,K", [(1, 4), (4, 64), (17, 60), (300, 800), (64, 68), (65, 132), (130, 516), (1024, 3072), (4800, 1028), (9000, 96)])
 def test_product_of_few_and_many_rows(N, K):
     """M on either side of every switch of kernel.  A sum of chunks of 64 in 32-bit is off by at most about
     (64 + K / 64) eps times the sum of the magnitudes."""
