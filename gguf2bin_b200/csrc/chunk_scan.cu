@@ -7,14 +7,17 @@
 //   with D_ij = g_(j+1) ... g_i, c_i = g_0 ... g_i (from the chunk's start) and the state S at the chunk's start
 //   o_i = c_i (S q_i) + sum_(j<=i) (q_i . k_j) D_ij s_j v_j,      S' = c_last S + sum_j D_(last,j) s_j v_j k_j^T.
 // The decays are products of the g's themselves, in the order of the tokens (no logarithms, no quotients), so a g of zero is
-// exact, and everything is 32-bit multiply-adds as before.
+// exact.  They are taken in 64 bits and rounded once, and what carries a state over a chunk or a segment is a pair of floats: the
+// rounding of one factor would fall on a whole state, again with every chunk.  All else is 32-bit multiply-adds, in sums of 16
+// that are added up, which rounds less than the chain of single tokens does (decay per head, 2,048 tokens, against 64 bits:
+// outputs 1.5e-7, states 1.2e-7, token by token 4.9e-7 and 5.7e-7; gates 0.9e-7 and 0.8e-7, 1.3e-7 and 0.9e-7).
 //   1. chunk_segment<false>: every segment by itself from a zero state: its own contribution, and the product of its g's
 //   2. chunk_carry: along a sequence, S at every segment's start from the contributions; the sequence's state in the end
 //   3. chunk_segment<true>: every segment from its start state: the outputs
 // A block of 256 threads takes a segment of one head and 64 columns; the state's share (64 x D) stays in registers (32 a
 // thread), q, k and v of the next chunk are on their way while one is computed.  Shared-memory reads bound it: 8 loads of 16
-// bytes feed 64 multiply-adds.  2,048 tokens, 8 heads of 128 x 256: 58 + 23 + 86 us (551 us as a chain); 1,501 tokens at
-// most in four sequences, 64 heads of 128 x 64 and 8 of 128 x 257, on average: 146 + 21 + 334 us (697 us).
+// bytes feed 64 multiply-adds.  2,048 tokens, 8 heads of 128 x 256: 64 + 26 + 95 us (551 us as a chain); 1,501 tokens at
+// most in four sequences, 64 heads of 128 x 64 and 8 of 128 x 257, on average: 164 + 23 + 372 us (697 us).
 #include "common.cuh"
 
 G2B_DEFINE_LAST_ERROR
@@ -35,7 +38,7 @@ struct ChunkArgs {
   const int *seq_meta;
   int n_seqs, seg;            // tokens of a segment, a multiple of CHUNK
   float *parts;               // [segments, H, V, D]: contributions, then start states
-  float *part_decay;          // [segments, H]
+  float2 *part_decay;         // [segments, H]: the product of the g's, and what its rounding left
   float *out;                 // [T, H*V]
 };
 
@@ -69,9 +72,17 @@ __device__ __forceinline__ void copy16(float *dst, const float *src) {
 __device__ __forceinline__ float dot4(const float4 &a, const float4 &b, float acc) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
-__device__ __forceinline__ float4 scale4(const float4 &a, float f) { return make_float4(a.x * f, a.y * f, a.z * f, a.w * f); }
 __device__ __forceinline__ void add4(float4 &a, float f, const float4 &b) {
   a.x = fmaf(f, b.x, a.x), a.y = fmaf(f, b.y, a.y), a.z = fmaf(f, b.z, a.z), a.w = fmaf(f, b.w, a.w);
+}
+
+__device__ __forceinline__ float2 two_floats(double x) {
+  const float hi = (float)x;
+  return make_float2(hi, (float)(x - (double)hi));
+}
+__device__ __forceinline__ float4 carry4(const float4 &a, float2 f, const float4 &b) {       // f a + b
+  return make_float4(fmaf(f.x, a.x, fmaf(f.y, a.x, b.x)), fmaf(f.x, a.y, fmaf(f.y, a.y, b.y)), fmaf(f.x, a.z, fmaf(f.y, a.z, b.z)),
+                     fmaf(f.x, a.w, fmaf(f.y, a.w, b.w)));
 }
 
 template <typename T, bool OUT>
@@ -88,8 +99,8 @@ chunk_segment_kernel(const ChunkArgs a) {
   float *K = sm, *Vs = K + 2 * CHUNK * pitch;            // two buffers of K and of V
   // decays and strengths of the chunk's tokens; from the token on: to the end of its sixteen, of the chunk times its strength;
   // up to the token: from its sixteen's start; the sixteens' products; in_block[B][i][j] = D_ij inside sixteen B
-  float *g = Vs + 2 * CHUNK * COLS, *s = g + CHUNK, *tail16 = s + CHUNK, *tail = tail16 + CHUNK, *head = tail + CHUNK, *block = head + CHUNK,
-        *in_block = block + 4;
+  double *tail16 = reinterpret_cast<double *>(Vs + 2 * CHUNK * COLS), *head = tail16 + CHUNK, *block = head + CHUNK;
+  float *g = reinterpret_cast<float *>(block + 4), *s = g + CHUNK, *tail = s + CHUNK, *in_block = tail + CHUNK;
   float *Q = in_block + CHUNK * 17, *S = Q + 2 * CHUNK * pitch, *P = S + COLS * pitch;            // OUT only
   // this thread's share of the state: columns 4 vy .. + 3, entries 4 dx .. + 3 and 64 further
   const int dx = tid & 15, vy = tid >> 4;
@@ -103,7 +114,7 @@ chunk_segment_kernel(const ChunkArgs a) {
       const int c = col0 + 4 * vy + i, d = 4 * dx + 64 * m;
       st[i][m] = OUT && c < V && d < D ? *reinterpret_cast<const float4 *>(part + (size_t)c * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-  float whole = 1.f;                                     // the product of the segment's g's
+  double whole = 1.0;                                    // the product of the segment's g's
   const T *vg = (const T *)a.v;
   T rv[16];                                              // the next chunk's values, decay and strength, on their way
   float rg = 1.f, rs = 0.f;
@@ -162,12 +173,12 @@ chunk_segment_kernel(const ChunkArgs a) {
     if (more) fetch(t0 + CHUNK, buf ^ 1);
     if (tid < CHUNK) {                                   // the decays from token `tid` on, to the end of its sixteen
       const int b16 = tid & ~15, j = tid & 15;
-      float d = 1.f;
+      double d = 1.0;
       in_block[tid * 17 + j] = 1.f;                      // row i of its sixteen: in_block[(b16 + i) * 17 + j]
       if (j == 0) head[tid] = g[tid];
       for (int i = j + 1; i < 16; ++i) {
         d *= g[b16 + i];
-        in_block[(b16 + i) * 17 + j] = d;
+        in_block[(b16 + i) * 17 + j] = (float)d;
         if (j == 0) head[b16 + i] = g[b16] * d;
       }
       tail16[tid] = d;
@@ -182,40 +193,54 @@ chunk_segment_kernel(const ChunkArgs a) {
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) p[i][j] = o[i][j] = 0.f;
+#pragma unroll 1
+      for (int d0 = 0; d0 < D; d0 += 16) {
+        float p16[4][4], o16[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) p16[i][j] = o16[i][j] = 0.f;
+        const int d1 = min(d0 + 16, D);
 #pragma unroll 2
-      for (int d = 0; d < D; d += 4) {
-        float4 q[4], k[4];
+        for (int d = d0; d < d1; d += 4) {
+          float4 q[4], k[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4 *>(Qc + (ty + 16 * i) * pitch + d);
+          for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4 *>(Qc + (ty + 16 * i) * pitch + d);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(Kc + (tx + 16 * j) * pitch + d);
+          for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(Kc + (tx + 16 * j) * pitch + d);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (j <= i) p16[i][j] = dot4(q[i], k[j], p16[i][j]); // later keys are not seen
+#pragma unroll
+          for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(S + (tx + 16 * j) * pitch + d);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o16[i][j] = dot4(q[i], k[j], o16[i][j]);
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (j <= i) p[i][j] = dot4(q[i], k[j], p[i][j]);       // later keys are not seen
-#pragma unroll
-        for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(S + (tx + 16 * j) * pitch + d);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) o[i][j] = dot4(q[i], k[j], o[i][j]);
+          for (int j = 0; j < 4; ++j) p[i][j] += p16[i][j], o[i][j] += o16[i][j];
       }
       __syncthreads();                                   // all decays stand
       if (tid < CHUNK) {
-        float f = s[tid] * tail16[tid];
+        double f = (double)s[tid] * tail16[tid];
         for (int B = (tid >> 4) + 1; B < 4; ++B) f *= block[B];
-        tail[tid] = f;
+        tail[tid] = (float)f;
       }
-      float before = 1.f;                                // the sixteens in front
+      double before = 1.0;                               // the sixteens in front
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = ty + 16 * i;
-        const float up = head[r];
+        const double up = head[r];
+        const float from_start = (float)(before * up);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[i][j] *= before * up;
+        for (int j = 0; j < 4; ++j) o[i][j] *= from_start;
         before *= block[i];
-        float between = up;                              // the sixteens between the key's and the row's, and the row's up to it
+        double between = up;                             // the sixteens between the key's and the row's, and the row's up to it
 #pragma unroll
         for (int j = 3; j >= 0; --j) {
           if (j > i) continue;
@@ -223,7 +248,7 @@ chunk_segment_kernel(const ChunkArgs a) {
           if (j == i) {
             p[i][j] = tx <= ty ? p[i][j] * (in_block[r * 17 + tx] * s[t]) : 0.f;
           } else {
-            p[i][j] *= tail16[t] * between * s[t];
+            p[i][j] *= (float)(tail16[t] * between * (double)s[t]);
             between *= block[j];
           }
         }
@@ -235,7 +260,12 @@ chunk_segment_kernel(const ChunkArgs a) {
       __syncwarp();                                      // a row's 16 threads are one half of a warp
       // sixteen tokens at a time, for the rows that see them; later values are not touched, whatever they hold
 #pragma unroll
-      for (int tb = 0; tb < 4; ++tb)
+      for (int tb = 0; tb < 4; ++tb) {
+        float o16[4][4];
+#pragma unroll
+        for (int i = tb; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o16[i][j] = 0.f;
 #pragma unroll 1
         for (int t = 16 * tb; t < 16 * tb + 16; t += 4) {
           float x[4][4];
@@ -250,13 +280,18 @@ chunk_segment_kernel(const ChunkArgs a) {
             const bool all = i > tb;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              if (all || t <= r) o[i][j] = fmaf(w.x, x[0][j], o[i][j]);
-              if (all || t + 1 <= r) o[i][j] = fmaf(w.y, x[1][j], o[i][j]);
-              if (all || t + 2 <= r) o[i][j] = fmaf(w.z, x[2][j], o[i][j]);
-              if (all || t + 3 <= r) o[i][j] = fmaf(w.w, x[3][j], o[i][j]);
+              if (all || t <= r) o16[i][j] = fmaf(w.x, x[0][j], o16[i][j]);
+              if (all || t + 1 <= r) o16[i][j] = fmaf(w.y, x[1][j], o16[i][j]);
+              if (all || t + 2 <= r) o16[i][j] = fmaf(w.z, x[2][j], o16[i][j]);
+              if (all || t + 3 <= r) o16[i][j] = fmaf(w.w, x[3][j], o16[i][j]);
             }
           }
         }
+#pragma unroll
+        for (int i = tb; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[i][j] += o16[i][j];
+      }
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -267,32 +302,42 @@ chunk_segment_kernel(const ChunkArgs a) {
     } else {
       __syncthreads();
       if (tid < CHUNK) {
-        float f = s[tid] * tail16[tid];
+        double f = (double)s[tid] * tail16[tid];
         for (int B = (tid >> 4) + 1; B < 4; ++B) f *= block[B];
-        tail[tid] = f;
+        tail[tid] = (float)f;
       }
     }
     __syncthreads();                                     // `tail` stands
     if (!OUT || more) {
-      const float all = (block[0] * block[1]) * (block[2] * block[3]);
+      const double all = (block[0] * block[1]) * (block[2] * block[3]);
+      const float2 f2 = two_floats(all);
       whole *= all;
+#pragma unroll 1
+      for (int tb = 0; tb < nt; tb += 16) {
+        float4 sum[4][2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int m = 0; m < 2; ++m) st[i][m] = scale4(st[i][m], all);
+          for (int m = 0; m < 2; ++m) sum[i][m] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int t1 = min(tb + 16, nt);
 #pragma unroll 4
-      for (int t = 0; t < nt; ++t) {
-        const float f = tail[t];
-        const float4 x = *reinterpret_cast<const float4 *>(Vc + t * COLS + 4 * vy);
+        for (int t = tb; t < t1; ++t) {
+          const float f = tail[t];
+          const float4 x = *reinterpret_cast<const float4 *>(Vc + t * COLS + 4 * vy);
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
-          if (4 * dx + 64 * m < D) {
-            const float4 k = *reinterpret_cast<const float4 *>(Kc + t * pitch + 4 * dx + 64 * m);
-            add4(st[0][m], f * x.x, k);
-            add4(st[1][m], f * x.y, k);
-            add4(st[2][m], f * x.z, k);
-            add4(st[3][m], f * x.w, k);
-          }
+          for (int m = 0; m < 2; ++m)
+            if (4 * dx + 64 * m < D) {
+              const float4 k = *reinterpret_cast<const float4 *>(Kc + t * pitch + 4 * dx + 64 * m);
+              add4(sum[0][m], f * x.x, k);
+              add4(sum[1][m], f * x.y, k);
+              add4(sum[2][m], f * x.z, k);
+              add4(sum[3][m], f * x.w, k);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int m = 0; m < 2; ++m) st[i][m] = carry4(st[i][m], tb ? make_float2(1.f, 0.f) : f2, sum[i][m]);
       }
     }
     __syncthreads();                                     // g, tail, S and P are written again
@@ -305,7 +350,7 @@ chunk_segment_kernel(const ChunkArgs a) {
         const int c = col0 + 4 * vy + i, d = 4 * dx + 64 * m;
         if (c < V && d < D) *reinterpret_cast<float4 *>(part + (size_t)c * D + d) = st[i][m];
       }
-    if (tid == 0 && blockIdx.x == 0) a.part_decay[(size_t)blockIdx.z * H + h] = whole;
+    if (tid == 0 && blockIdx.x == 0) a.part_decay[(size_t)blockIdx.z * H + h] = two_floats(whole);
   }
 }
 
@@ -329,7 +374,7 @@ chunk_carry_kernel(const ChunkArgs a) {
   float4 s = *kept;
   for (int i0 = 0; i0 < segments; i0 += 4) {
     float4 x[4];
-    float g[4];
+    float2 g[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const size_t at = (size_t)before + min(i0 + i, segments - 1);
@@ -340,7 +385,7 @@ chunk_carry_kernel(const ChunkArgs a) {
     for (int i = 0; i < 4; ++i)
       if (i0 + i < segments) {
         *reinterpret_cast<float4 *>(a.parts + ((size_t)before + i0 + i) * size + e) = s;
-        s = make_float4(fmaf(g[i], s.x, x[i].x), fmaf(g[i], s.y, x[i].y), fmaf(g[i], s.z, x[i].z), fmaf(g[i], s.w, x[i].w));
+        s = carry4(s, g[i], x[i]);
       }
   }
   *kept = s;
@@ -350,7 +395,7 @@ template <typename T, bool OUT>
 static int launch_segments(const ChunkArgs &a, dim3 grid, cudaStream_t stream) {
   static G2bPerDevice done;
   auto bytes = [](int D) {
-    return sizeof(float) * ((size_t)2 * CHUNK * (D + 4) * (OUT ? 2 : 1) + 2 * CHUNK * COLS + 5 * CHUNK + 4 + CHUNK * 17 +
+    return sizeof(float) * ((size_t)2 * CHUNK * (D + 4) * (OUT ? 2 : 1) + 2 * CHUNK * COLS + 7 * CHUNK + 8 + CHUNK * 17 +
                             (OUT ? (size_t)COLS * (D + 4) + CHUNK * P_PITCH : 0));
   };
   const int dev = g2b_current_device();
@@ -363,10 +408,10 @@ static int launch_segments(const ChunkArgs &a, dim3 grid, cudaStream_t stream) {
   return g2b_check_launch("chunk_scan");
 }
 
-// `segments`: how many there can be (n_tokens / seg + n_seqs); parts [segments, H, V, D], part_decay [segments, H].
+// `segments`: how many there can be (n_tokens / seg + n_seqs); parts [segments, H, V, D], part_decay [segments, H, 2].
 extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D, int Vin,
                               int extra_one, const float *decay, const float *gates, float *state, const int *seq_meta, int n_seqs,
-                              int seg, int segments, float *parts, float *part_decay, float *out, cudaStream_t stream) {
+                              int seg, int segments, float *parts, float2 *part_decay, float *out, cudaStream_t stream) {
   const int V = Vin + (extra_one ? 1 : 0);
   if (n_seqs <= 0 || segments <= 0) return 0;
   if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("chunk_scan: unknown dtype %d", dtype);
@@ -396,11 +441,13 @@ extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const
 //      products P_ij = D_ij (q_i . k_j) of the outputs
 //   2. delta_walk: along the sequence, a chunk a step: U = U0 - W S^T, o_i = c_i S q_i + sum_(j<=i) P_ij u_j,
 //      S' = c_last S + sum_j D_(last,j) u_j k_j^T.  A block has 8 columns of a head; the next chunk's operands are on their way.
-// The substitution takes the tokens in their order, as the recurrence does; all is 32-bit.  The walk's chain of products, read
-// from shared memory, bounds it.  2,048 tokens, 8 heads of 128 x 128: 60 + 219 us (714 us a token after a token).
+// The substitution takes the tokens in their order, as the recurrence does; decays and sums as above (errors against 64 bits as
+// token by token: outputs 1.5e-7, states 1.1e-7).  The walk's chain of products, read
+// from shared memory, bounds it.  2,048 tokens, 8 heads of 128 x 128: 40 + 250 us (714 us a token after a token).
 #define DELTA_CHUNK 32
 #define DELTA_COLS 8
 #define DELTA_WALK 128
+#define DELTA_DECAYS (2 * DELTA_CHUNK + 4)
 
 struct DeltaArgs {
   const float *qf, *kf;       // [T, G, D] prepared
@@ -411,7 +458,7 @@ struct DeltaArgs {
   float *state;               // [slots, H, V, D]
   const int *seq_meta;
   int n_seqs;
-  float *U0, *W, *P, *decays; // [chunks, H, 32, V], [.., 32, D], [.., 32, 32], [.., 64]: c, then the decays to the chunk's end
+  float *U0, *W, *P, *decays; // [chunks, H, 32, V], [.., 32, D], [.., 32, 32], [.., 68]: c, the decays to the chunk's end, what c_last's rounding left
   float *out;                 // [T, H*V]
 };
 
@@ -422,7 +469,7 @@ delta_chunk_kernel(const DeltaArgs a) {
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
   __shared__ __align__(16) float M[DELTA_CHUNK][DELTA_CHUNK + 4];         // D_ij, then A_ij
-  __shared__ float g[DELTA_CHUNK], beta[DELTA_CHUNK], c[DELTA_CHUNK];
+  __shared__ float g[DELTA_CHUNK], beta[DELTA_CHUNK], beta_c[DELTA_CHUNK];
   const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, tid = threadIdx.x, qk_head = h / (H / a.G);
   int b, place;
   if (!find_segment(a.seq_meta, a.n_seqs, DELTA_CHUNK, blockIdx.x, b, place)) return;
@@ -449,32 +496,39 @@ delta_chunk_kernel(const DeltaArgs a) {
   __syncthreads();
   const size_t item = (size_t)blockIdx.x * H + h;
   if (tid < DELTA_CHUNK) {
-    float d = 1.f;
+    float *decays = a.decays + item * DELTA_DECAYS;
+    double d = 1.0;
     M[tid][tid] = 1.f;
     for (int i = tid + 1; i < DELTA_CHUNK; ++i) {
       d *= g[i];
-      M[i][tid] = d;
+      M[i][tid] = (float)d;
     }
-    a.decays[item * 64 + DELTA_CHUNK + tid] = d;
+    decays[DELTA_CHUNK + tid] = (float)d;
+    d = g[0];
+    for (int i = 1; i <= tid; ++i) d *= g[i];
+    decays[tid] = (float)d;
+    beta_c[tid] = (float)(d * beta[tid]);
+    if (tid == DELTA_CHUNK - 1) decays[2 * DELTA_CHUNK] = two_floats(d).y;
   }
   const int i = tid >> 3, j0 = tid & 7;
   float kk[4] = {0.f, 0.f, 0.f, 0.f}, qk[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int d0 = 0; d0 < D; d0 += 16) {
+    float kk16[4] = {0.f, 0.f, 0.f, 0.f}, qk16[4] = {0.f, 0.f, 0.f, 0.f};
+    const int d1 = min(d0 + 16, D);
 #pragma unroll 4
-  for (int d = 0; d < D; d += 4) {
-    const float4 ki = *reinterpret_cast<const float4 *>(K + i * pitch + d), qi = *reinterpret_cast<const float4 *>(Q + i * pitch + d);
+    for (int d = d0; d < d1; d += 4) {
+      const float4 ki = *reinterpret_cast<const float4 *>(K + i * pitch + d), qi = *reinterpret_cast<const float4 *>(Q + i * pitch + d);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const float4 kj = *reinterpret_cast<const float4 *>(K + (j0 + 8 * m) * pitch + d);
-      kk[m] = dot4(ki, kj, kk[m]);
-      qk[m] = dot4(qi, kj, qk[m]);
+      for (int m = 0; m < 4; ++m) {
+        const float4 kj = *reinterpret_cast<const float4 *>(K + (j0 + 8 * m) * pitch + d);
+        kk16[m] = dot4(ki, kj, kk16[m]);
+        qk16[m] = dot4(qi, kj, qk16[m]);
+      }
     }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) kk[m] += kk16[m], qk[m] += qk16[m];
   }
   __syncthreads();                                       // the decays stand
-  if (tid < DELTA_CHUNK) {
-    c[tid] = g[0] * M[tid][0];
-    a.decays[item * 64 + tid] = c[tid];
-  }
-  __syncthreads();
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     const int j = j0 + 8 * m;
@@ -490,21 +544,22 @@ delta_chunk_kernel(const DeltaArgs a) {
     for (int r = 0; r < DELTA_CHUNK; ++r) {
       float y;
       if (col < V) y = r < nt ? beta[r] * to_f32(vg[(size_t)(first + r) * a.v_stride + (size_t)h * V + col]) : 0.f;
-      else y = beta[r] * c[r] * K[r * pitch + col - V];
+      else y = beta_c[r] * K[r * pitch + col - V];
       x[r] = y;
     }
 #pragma unroll
     for (int r = 1; r < DELTA_CHUNK; ++r) {
-      float y = x[r];
+      float y[2] = {0.f, 0.f};                           // of the first sixteen tokens, of the others
 #pragma unroll
       for (int j = 0; j < r; j += 4) {
         const float4 m = *reinterpret_cast<const float4 *>(&M[r][j]);
-        y = fmaf(-m.x, x[j], y);
-        if (j + 1 < r) y = fmaf(-m.y, x[j + 1], y);
-        if (j + 2 < r) y = fmaf(-m.z, x[j + 2], y);
-        if (j + 3 < r) y = fmaf(-m.w, x[j + 3], y);
+        float &to = y[j >> 4];
+        to = fmaf(m.x, x[j], to);
+        if (j + 1 < r) to = fmaf(m.y, x[j + 1], to);
+        if (j + 2 < r) to = fmaf(m.z, x[j + 2], to);
+        if (j + 3 < r) to = fmaf(m.w, x[j + 3], to);
       }
-      x[r] = y;
+      x[r] -= y[0] + y[1];
     }
     float *to = col < V ? a.U0 + item * DELTA_CHUNK * V + col : a.W + item * DELTA_CHUNK * D + col - V;
     const int step = col < V ? V : D;
@@ -528,9 +583,9 @@ delta_walk_kernel(const DeltaArgs a) {
     before += n;
   }
   const int first = a.seq_meta[4 * b], n = a.seq_meta[4 * b + 1], slot = a.seq_meta[4 * b + 3];
-  // two buffers, each: W, Q, K [32, pitch], P [32, 36], U0 [32, 8], decays [64]
+  // two buffers, each: W, Q, K [32, pitch], P [32, 36], U0 [32, 8], decays [68]
   const int rows = DELTA_CHUNK * pitch, P_AT = 3 * rows, U_AT = P_AT + DELTA_CHUNK * 36, G_AT = U_AT + DELTA_CHUNK * DELTA_COLS,
-            SIZE = G_AT + 64;
+            SIZE = G_AT + DELTA_DECAYS;
   float *S = sm + 2 * SIZE, *U = S + DELTA_COLS * pitch;                 // S [8, pitch], U [32, 8]
   auto fetch = [&](int t0, int buf) {
     float *to = sm + buf * SIZE;
@@ -549,7 +604,7 @@ delta_walk_kernel(const DeltaArgs a) {
       const int r = tid >> 1, q = (tid & 1) * 4;
       if (col0 + q < V) copy16(to + U_AT + r * DELTA_COLS + q, a.U0 + (item * DELTA_CHUNK + r) * V + col0 + q);
     }
-    if (tid >= 64 && tid < 80) copy16(to + G_AT + (tid - 64) * 4, a.decays + item * 64 + (tid - 64) * 4);
+    if (tid >= 64 && tid < 64 + DELTA_DECAYS / 4) copy16(to + G_AT + (tid - 64) * 4, a.decays + item * DELTA_DECAYS + (tid - 64) * 4);
     asm volatile("cp.async.commit_group;\n" ::);
   };
   // this thread's share of the state: column cs, entries 4 dx .. + 3 and 64 further
@@ -575,14 +630,20 @@ delta_walk_kernel(const DeltaArgs a) {
     if (t0 + DELTA_CHUNK < n) fetch(t0 + DELTA_CHUNK, buf ^ 1);
     const float *W = sm + buf * SIZE, *Q = W + rows, *K = Q + rows, *P = W + P_AT, *U0 = W + U_AT, *G = W + G_AT;
     float ws[2] = {0.f, 0.f}, qs[2] = {0.f, 0.f};
+    for (int d0 = 0; d0 < D; d0 += 16) {
+      float ws16[2] = {0.f, 0.f}, qs16[2] = {0.f, 0.f};
+      const int d1 = min(d0 + 16, D);
 #pragma unroll 4
-    for (int d = 0; d < D; d += 4) {
-      const float4 s = *reinterpret_cast<const float4 *>(S + cc * pitch + d);
+      for (int d = d0; d < d1; d += 4) {
+        const float4 s = *reinterpret_cast<const float4 *>(S + cc * pitch + d);
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        ws[m] = dot4(*reinterpret_cast<const float4 *>(W + (r0 + 16 * m) * pitch + d), s, ws[m]);
-        qs[m] = dot4(*reinterpret_cast<const float4 *>(Q + (r0 + 16 * m) * pitch + d), s, qs[m]);
+        for (int m = 0; m < 2; ++m) {
+          ws16[m] = dot4(*reinterpret_cast<const float4 *>(W + (r0 + 16 * m) * pitch + d), s, ws16[m]);
+          qs16[m] = dot4(*reinterpret_cast<const float4 *>(Q + (r0 + 16 * m) * pitch + d), s, qs16[m]);
+        }
       }
+#pragma unroll
+      for (int m = 0; m < 2; ++m) ws[m] += ws16[m], qs[m] += qs16[m];
     }
 #pragma unroll
     for (int m = 0; m < 2; ++m) U[(r0 + 16 * m) * DELTA_COLS + cc] = U0[(r0 + 16 * m) * DELTA_COLS + cc] - ws[m];
@@ -590,26 +651,33 @@ delta_walk_kernel(const DeltaArgs a) {
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
       const int r = r0 + 16 * m;
-      float o = G[r] * qs[m];
+      float o[2] = {0.f, 0.f};                           // of the first sixteen tokens, of the others
 #pragma unroll
       for (int j = 0; j < 16 + 16 * m; j += 4) {
         const float4 p = *reinterpret_cast<const float4 *>(P + r * 36 + j);
-        if (j <= r) o = fmaf(p.x, U[j * DELTA_COLS + cc], o);            // later tokens are not touched, whatever they hold
-        if (j + 1 <= r) o = fmaf(p.y, U[(j + 1) * DELTA_COLS + cc], o);
-        if (j + 2 <= r) o = fmaf(p.z, U[(j + 2) * DELTA_COLS + cc], o);
-        if (j + 3 <= r) o = fmaf(p.w, U[(j + 3) * DELTA_COLS + cc], o);
+        float &to = o[j >> 4];
+        if (j <= r) to = fmaf(p.x, U[j * DELTA_COLS + cc], to);          // later tokens are not touched, whatever they hold
+        if (j + 1 <= r) to = fmaf(p.y, U[(j + 1) * DELTA_COLS + cc], to);
+        if (j + 2 <= r) to = fmaf(p.z, U[(j + 2) * DELTA_COLS + cc], to);
+        if (j + 3 <= r) to = fmaf(p.w, U[(j + 3) * DELTA_COLS + cc], to);
       }
-      if (r < nt && col0 + cc < V) a.out[(size_t)(first + t0 + r) * H * V + (size_t)h * V + col0 + cc] = o;
+      if (r < nt && col0 + cc < V) a.out[(size_t)(first + t0 + r) * H * V + (size_t)h * V + col0 + cc] = fmaf(G[r], qs[m], o[0] + o[1]);
     }
-    const float all = G[DELTA_CHUNK - 1];
+    const float2 all = make_float2(G[DELTA_CHUNK - 1], G[2 * DELTA_CHUNK]);
 #pragma unroll
-    for (int m = 0; m < 2; ++m) st[m] = scale4(st[m], all);
+    for (int jb = 0; jb < DELTA_CHUNK; jb += 16) {
+      float4 sum[2];
+      sum[0] = sum[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const int j1 = min(jb + 16, nt);
 #pragma unroll 4
-    for (int j = 0; j < nt; ++j) {
-      const float f = G[DELTA_CHUNK + j] * U[j * DELTA_COLS + cs];
+      for (int j = jb; j < j1; ++j) {
+        const float f = G[DELTA_CHUNK + j] * U[j * DELTA_COLS + cs];
 #pragma unroll
-      for (int m = 0; m < 2; ++m)
-        if (4 * dx + 64 * m < D) add4(st[m], f, *reinterpret_cast<const float4 *>(K + j * pitch + 4 * dx + 64 * m));
+        for (int m = 0; m < 2; ++m)
+          if (4 * dx + 64 * m < D) add4(sum[m], f, *reinterpret_cast<const float4 *>(K + j * pitch + 4 * dx + 64 * m));
+      }
+#pragma unroll
+      for (int m = 0; m < 2; ++m) st[m] = carry4(st[m], jb ? make_float2(1.f, 0.f) : all, sum[m]);
     }
 #pragma unroll
     for (int m = 0; m < 2; ++m)
@@ -636,7 +704,7 @@ extern "C" int g2b_delta_scan(int dtype, const float *qf, const float *kf, const
   const DeltaArgs a = {qf, kf, v, v_stride, H, G, D, V, ab, A_log, dt_bias, state, seq_meta, n_seqs, U0, W, P, decays, out};
   auto prep_bytes = [](int d) { return sizeof(float) * (size_t)2 * DELTA_CHUNK * (d + 4); };
   auto walk_bytes = [](int d) {
-    return sizeof(float) * ((size_t)2 * (3 * DELTA_CHUNK * (d + 4) + DELTA_CHUNK * 36 + DELTA_CHUNK * DELTA_COLS + 64) + DELTA_COLS * (d + 4) +
+    return sizeof(float) * ((size_t)2 * (3 * DELTA_CHUNK * (d + 4) + DELTA_CHUNK * 36 + DELTA_CHUNK * DELTA_COLS + DELTA_DECAYS) + DELTA_COLS * (d + 4) +
                             DELTA_CHUNK * DELTA_COLS);
   };
   static G2bPerDevice done;

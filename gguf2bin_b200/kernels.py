@@ -970,7 +970,7 @@ def _delta_chunks(n_tokens: int, n_seqs: int, heads: int, dim: int, v_dim: int) 
     """Chunks of the gated delta rule over a prompt, 0 where it goes a token after a token: _chunk_segment's rule on sizes
     and lengths, with the scratch of the chunks' own products."""
     chunks = n_tokens // DELTA_CHUNK + n_seqs
-    fits = 4 * chunks * heads * (DELTA_CHUNK * (v_dim + dim + DELTA_CHUNK) + 64) <= CHUNK_PARTS_MOST and chunks <= 65535
+    fits = 4 * chunks * heads * (DELTA_CHUNK * (v_dim + dim + DELTA_CHUNK + 2) + 4) <= CHUNK_PARTS_MOST and chunks <= 65535
     return chunks if fits and v_dim % 4 == 0 and _chunk_segment(n_tokens, 1, heads, 1, dim) and n_tokens >= 96 * n_seqs else 0
 
 
@@ -1028,7 +1028,7 @@ def state_scan(q, k, v, state, ctx, out32, heads, qk_heads, qk_dim, v_dim, *, de
                   _ptr(kf), _stream())
             if chunks:
                 u0, w_, p_, dec = (ctx.workspace.buffer("delta." + n, (chunks, heads, *shape), torch.float32) for n, shape in (
-                    ("u0", (DELTA_CHUNK, v_dim)), ("w", (DELTA_CHUNK, qk_dim)), ("p", (DELTA_CHUNK, DELTA_CHUNK)), ("decays", (64,))))
+                    ("u0", (DELTA_CHUNK, v_dim)), ("w", (DELTA_CHUNK, qk_dim)), ("p", (DELTA_CHUNK, DELTA_CHUNK)), ("decays", (2 * DELTA_CHUNK + 4,))))
                 f = _fn("chunk_scan.cu", "g2b_delta_scan",
                         [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p] * 5 + [c_int] * 2 + [c_void_p] * 6)
                 _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim, _ptr(ab),
@@ -1038,7 +1038,7 @@ def state_scan(q, k, v, state, ctx, out32, heads, qk_heads, qk_dim, v_dim, *, de
                 return
             segments = T // seg + ctx.n_seqs
             parts = ctx.workspace.buffer("scan.parts", (segments, heads, cols, qk_dim), torch.float32)
-            decays = ctx.workspace.buffer("scan.part_decay", (segments, heads), torch.float32)
+            decays = ctx.workspace.buffer("scan.part_decay", (segments, heads, 2), torch.float32)
             f = _fn("chunk_scan.cu", "g2b_chunk_scan",
                     [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p] * 4 + [c_int] * 3 + [c_void_p] * 4)
             _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim,
