@@ -74,17 +74,21 @@ extern "C" int g2b_moe_gather(const void *A, int dtype, int a_stride, const int 
 // `sigmoid`: the scores are sigmoids of the logits, each by itself, instead of a softmax over all.
 // `groups` > 1: the experts form that many equal groups of neighbours; a group's score is the sum of its
 // two largest scores (of score + correction); only experts of the `keep` best groups can be chosen.
-__global__ void __launch_bounds__(ROUTE_WARPS * 32)
-moe_route_kernel(const float *__restrict__ z, const float *__restrict__ correction, int T, int N, int top,
-                 int renormalise, int *__restrict__ idx, float *__restrict__ weight, float scale, int sigmoid,
-                 int groups, int keep, const float *__restrict__ bias) {
-  pdl_launch();
-  pdl_wait();
-  extern __shared__ float sm[];                 // per warp: s [N], pick [N], group scores [groups]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * ROUTE_WARPS + warp;
-  if (t >= T) return;
-  float *s = sm + (size_t)warp * (2 * N + groups), *pick = s + N, *gs = pick + N;
+struct Route {
+  const float *z, *correction, *bias;
+  int T, N, top, renormalise, sigmoid, groups, keep;
+  int *idx;
+  float *weight, scale;
+};
+// One warp chooses token t's experts; `s`: 2 N + groups floats of shared memory (scores, what is picked from, group scores).
+__device__ __forceinline__ void route_token(const Route &a, int t, float *s) {
+  const float *z = a.z, *correction = a.correction, *bias = a.bias;
+  const int N = a.N, top = a.top, renormalise = a.renormalise, sigmoid = a.sigmoid, groups = a.groups, keep = a.keep;
+  int *idx = a.idx;
+  float *weight = a.weight;
+  const float scale = a.scale;
+  const int lane = threadIdx.x & 31;
+  float *pick = s + N, *gs = pick + N;
   const float *zr = z + (size_t)t * N;
   if (sigmoid) {
     for (int j = lane; j < N; j += 32) {
@@ -166,6 +170,15 @@ moe_route_kernel(const float *__restrict__ z, const float *__restrict__ correcti
       weight[(size_t)t * top + r] = weight[(size_t)t * top + r] / (chosen_sum + 1e-20f) * scale;
 }
 
+__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+moe_route_kernel(const Route a) {
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ float sm[];
+  const int warp = threadIdx.x >> 5, t = blockIdx.x * ROUTE_WARPS + warp;
+  if (t < a.T) route_token(a, t, sm + (size_t)warp * (2 * a.N + a.groups));
+}
+
 extern "C" int g2b_moe_route(const float *z, const float *correction, int T, int N, int top, int renormalise,
                              int *idx, float *weight, float scale, int sigmoid, int groups, int keep,
                              const float *bias, cudaStream_t stream) {
@@ -176,8 +189,8 @@ extern "C" int g2b_moe_route(const float *z, const float *correction, int T, int
     G2B_REFUSE("moe_route: %d experts in %d groups of which %d are kept, for %d choices", N, groups, keep, top);
   const size_t smem = (size_t)ROUTE_WARPS * (2 * N + groups) * sizeof(float);
   if (smem > 48 * 1024) G2B_REFUSE("moe_route: %d experts are more than a block's shared memory holds", N);
-  g2b_launch(moe_route_kernel, dim3((T + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), smem, stream, z,
-             correction, T, N, top, renormalise, idx, weight, scale, sigmoid, groups, keep, bias);
+  const Route a = {z, correction, bias, T, N, top, renormalise, sigmoid, groups, keep, idx, weight, scale};
+  g2b_launch(moe_route_kernel, dim3((T + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), smem, stream, a);
   return g2b_check_launch("moe_route");
 }
 
@@ -189,11 +202,8 @@ extern "C" int g2b_moe_route(const float *z, const float *correction, int T, int
 // then the tiles as (expert, first row, rows) triples from word PLAN_TILES_AT(E) on
 #define PLAN_TILES_AT(E) ((E) + 2)
 
-__global__ void __launch_bounds__(1024)
-moe_plan_kernel(const int *__restrict__ idx, int n_pairs, int n_real, int tile_rows, int max_tiles,
-                int *__restrict__ plan, int *__restrict__ row_pair, int *__restrict__ pair_row) {
-  pdl_launch();
-  pdl_wait();
+__device__ __forceinline__ void make_plan(const int *idx, int n_pairs, int n_real, int tile_rows, int max_tiles, int *plan, int *row_pair,
+                                          int *pair_row) {
   __shared__ int count[PLAN_MAX_EXPERTS], start[PLAN_MAX_EXPERTS + 1], cursor[PLAN_MAX_EXPERTS];
   for (int e = threadIdx.x; e < n_real; e += blockDim.x) count[e] = 0;
   __syncthreads();
@@ -232,6 +242,30 @@ moe_plan_kernel(const int *__restrict__ idx, int n_pairs, int n_real, int tile_r
   }
 }
 
+__global__ void __launch_bounds__(1024)
+moe_plan_kernel(const int *__restrict__ idx, int n_pairs, int n_real, int tile_rows, int max_tiles,
+                int *__restrict__ plan, int *__restrict__ row_pair, int *__restrict__ pair_row) {
+  pdl_launch();
+  pdl_wait();
+  make_plan(idx, n_pairs, n_real, tile_rows, max_tiles, plan, row_pair, pair_row);
+}
+
+// The few tokens of a decode step: the choice and the plan in one block, a warp a token (one launch instead of two: 5.2 us for
+// one token and 18 experts, 4.0 + 2.8 apart; 5.7 for eight and 16, 4.0 + 3.2).
+__global__ void __launch_bounds__(1024)
+moe_route_plan_kernel(const Route a, int n_real, int tile_rows, int max_tiles, int *plan, int *row_pair, int *pair_row) {
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ float sm[];
+  const int warp = threadIdx.x >> 5;
+  for (int t = warp; t < a.T; t += blockDim.x >> 5) {
+    route_token(a, t, sm + (size_t)warp * (2 * a.N + a.groups));
+    __syncwarp();                               // the next token's scores go where this one's were
+  }
+  __syncthreads();                              // the choices, written to global memory, are seen by the whole block
+  make_plan(a.idx, a.T * a.top, n_real, tile_rows, max_tiles, plan, row_pair, pair_row);
+}
+
 extern "C" int g2b_moe_plan(const int *idx, int n_pairs, int n_real, int tile_rows, int max_tiles, int *plan,
                             int *row_pair, int *pair_row, cudaStream_t stream) {
   if (n_pairs <= 0) return 0;
@@ -239,6 +273,24 @@ extern "C" int g2b_moe_plan(const int *idx, int n_pairs, int n_real, int tile_ro
   g2b_launch(moe_plan_kernel, dim3(1), dim3(1024), 0, stream, idx, n_pairs, n_real, tile_rows, max_tiles, plan, row_pair,
              pair_row);
   return g2b_check_launch("moe_plan");
+}
+
+// Both for a step of few tokens whose scores fit one block.
+extern "C" int g2b_moe_route_plan(const float *z, const float *correction, int T, int N, int top, int renormalise, int *idx,
+                                  float *weight, float scale, int sigmoid, int groups, int keep, const float *bias, int n_real,
+                                  int tile_rows, int max_tiles, int *plan, int *row_pair, int *pair_row, cudaStream_t stream) {
+  if (T <= 0) return 0;
+  if (top < 1 || top > N) G2B_REFUSE("moe_route: %d choices among %d experts", top, N);
+  if (groups < 1) groups = 1;
+  if (groups > 1 && (N % groups || keep < 1 || keep > groups || top > keep * (N / groups)))
+    G2B_REFUSE("moe_route: %d experts in %d groups of which %d are kept, for %d choices", N, groups, keep, top);
+  if (n_real < 0 || n_real > PLAN_MAX_EXPERTS) G2B_REFUSE("moe_plan: %d experts outside 0..%d", n_real, PLAN_MAX_EXPERTS);
+  const int warps = T < 8 ? 8 : T < 32 ? T : 32;
+  const size_t smem = (size_t)warps * (2 * N + groups) * sizeof(float);
+  if (smem > 32 * 1024) G2B_REFUSE("moe_route_plan: %d tokens of %d experts are not one block's", T, N);
+  const Route a = {z, correction, bias, T, N, top, renormalise, sigmoid, groups, keep, idx, weight, scale};
+  g2b_launch(moe_route_plan_kernel, dim3(1), dim3(warps * 32), smem, stream, a, n_real, tile_rows, max_tiles, plan, row_pair, pair_row);
+  return g2b_check_launch("moe_route_plan");
 }
 
 // ---------------------------------------------------------------------------

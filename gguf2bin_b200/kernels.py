@@ -1269,6 +1269,27 @@ def moe_plan(idx, n_real: int, max_tiles: int, plan, row_pair, pair_row) -> None
           _stream())
 
 
+def moe_route_plan(z32, correction, top: int, renormalise: bool, idx, weight, scale: float, score: str, groups: int, keep: int, bias,
+                   n_real: int, max_tiles: int, plan, row_pair, pair_row) -> None:
+    """``moe_route`` and ``moe_plan`` of a step of few tokens in one launch, where its one block holds them; else both."""
+    if score not in ("softmax", "sigmoid"):
+        raise KernelError(f"moe_route: scores are 'softmax' or 'sigmoid', not {score!r}")
+    _need(z32, torch.float32, "router logits")
+    _need(idx, torch.int32, "idx")
+    _need(weight, torch.float32, "weight")
+    f = _fn("moe.cu", "g2b_moe_route_plan",
+            [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_int, c_int, c_int, c_void_p, c_int, c_int,
+             c_int, c_void_p, c_void_p, c_void_p, c_void_p])
+    tokens, n = z32.shape
+    if 4 * min(max(tokens, 8), 32) * (2 * n + max(groups, 1)) <= 32 * 1024:
+        _call(f, _ptr(z32), _ptr(correction), tokens, n, top, 1 if renormalise else 0, _ptr(idx), _ptr(weight), float(scale),
+              1 if score == "sigmoid" else 0, int(groups), int(keep), _ptr(bias), n_real, moe_tile_rows(), max_tiles, _ptr(plan),
+              _ptr(row_pair), _ptr(pair_row), _stream())
+        return
+    moe_route(z32, correction, top, renormalise, idx, weight, scale, score, groups, keep, bias)
+    moe_plan(idx, n_real, max_tiles, plan, row_pair, pair_row)
+
+
 def moe_gemm(a, row_pair, pairs_per_token: int, w, n_out: int, plan, n_real: int, max_tiles: int, swiglu: bool,
              out, blocked: bool = False, form: GluForm = SILU) -> None:
     """Per expert e over its rows: out[row] = a[source of row] . w[e]^T; ``w`` [E, n_out (x2 with

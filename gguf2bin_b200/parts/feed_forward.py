@@ -347,15 +347,19 @@ class RoutedExperts:
         kernels.linear(h, self.w_router, z)
         idx = ws.buffer("moe.idx", (T, top), torch.int32)
         weight = ws.buffer("moe.weight", (T, top), torch.float32)
-        kernels.moe_route(z, self.correction, top, self.renormalise, idx, weight, self.scale, self.score, self.groups,
-                          self.groups_kept, self.router_bias)
         n_pairs = T * top
         tile = kernels.moe_tile_rows()
         max_tiles = -(-n_pairs // tile) + E               # every expert's last tile may be part full
         plan = ws.buffer("moe.plan", (E + 2 + 3 * max_tiles,), torch.int32)
         row_pair = ws.buffer("moe.row_pair", (n_pairs,), torch.int32)
         pair_row = ws.buffer("moe.pair_row", (n_pairs,), torch.int32)
-        kernels.moe_plan(idx, E, max_tiles, plan, row_pair, pair_row)
+        if n_pairs <= self.FEW_ROWS:
+            kernels.moe_route_plan(z, self.correction, top, self.renormalise, idx, weight, self.scale, self.score, self.groups,
+                                   self.groups_kept, self.router_bias, E, max_tiles, plan, row_pair, pair_row)
+        else:
+            kernels.moe_route(z, self.correction, top, self.renormalise, idx, weight, self.scale, self.score, self.groups,
+                              self.groups_kept, self.router_bias)
+            kernels.moe_plan(idx, E, max_tiles, plan, row_pair, pair_row)
         rows32 = ws.buffer("moe.rows", (n_pairs, self.hidden), torch.float32)
         if E:
             wt = self.w_gate_up.dtype                     # matrices stored in 32-bit keep their products there
