@@ -261,110 +261,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
-// ---------------------------------------------------------------------------
-// One product per group of rows (a routed feed-forward's experts): rows first .. end of A (and of C)
-// belong to group e and are multiplied by rows e Nw .. (e + 1) Nw of W.  Where the groups lie is a
-// plan in device memory, made by an earlier kernel of the step:
-//   plan[0]            tiles in use;   plan[1 + e] first row of group e;   plan[1 + n_groups] all rows
-//   plan[n_groups + 2 + 3 t ..]  tile t: (group, first row, rows), tiles of `plan rows` rows each
-// The grid has a CTA per plan tile and column tile; a CTA whose plan tile is not the first of a
-// 128-row tile of its group returns at once, the others compute 128 rows from theirs on (rows
-// beyond the group's end are loaded, they are the next group's or zeros, and never stored).
-// ---------------------------------------------------------------------------
-template <int BN, int STAGES, int EPI>
-__global__ void __launch_bounds__(THREADS)
-gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                       void *__restrict__ Cv, const int *__restrict__ plan, int n_groups, int Nw, int K, int ldc,
-                       int *__restrict__ status, ProductTail glu) {
-  pdl_launch();
-  pdl_wait();                  // the plan is an earlier kernel's output
-  const int tile = blockIdx.y;
-  if (tile >= plan[0]) return;
-  const int *tl = plan + n_groups + 2 + 3 * tile;
-  const int e = tl[0], m0 = tl[1];
-  const int first = plan[1 + e], end = plan[2 + e];
-  if ((m0 - first) % BM) return;
-  const int m_end = min(m0 + BM, end);
-  const int n0 = blockIdx.x * BN, w0 = e * Nw + n0;
-
-  extern __shared__ unsigned char smem_raw[];
-  using S = Smem<BN, STAGES>;
-  unsigned char *smem = reinterpret_cast<unsigned char *>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + S::BARRIER_OFFSET);
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 1);
-  const uint32_t full0 = smem_addr(bars), empty0 = smem_addr(bars + STAGES);
-  const uint32_t acc_bar = smem_addr(bars + 2 * STAGES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nkb = (K + BK - 1) / BK;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 1);
-    }
-    mbar_init(acc_bar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  if (warp == 5) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
-                     smem_addr(tmem_slot)), "r"((uint32_t)BN));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-
-  if (warp == 4) {
-    if (lane == 0 && PRODUCER_RUNS) {
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % STAGES;
-        if (kb >= STAGES && !mbar_wait(empty0 + 8 * s, ((kb / STAGES) - 1) & 1)) {
-          atomicExch(status, ST_PRODUCER_TIMEOUT);
-          break;
-        }
-        const uint32_t a_dst = smem_addr(smem + s * S::STAGE_BYTES);
-        mbar_expect_tx(full0 + 8 * s, S::STAGE_BYTES);
-        tma_load_2d(a_dst, &map_a, kb * BK, m0, full0 + 8 * s);
-        tma_load_2d(a_dst + S::A_BYTES, &map_w, kb * BK, w0, full0 + 8 * s);
-      }
-    }
-  } else if (warp == 5) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_n(BN);
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % STAGES;
-        if (!mbar_wait(full0 + 8 * s, (kb / STAGES) & 1)) {
-          atomicExch(status, ST_MMA_TIMEOUT);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const uint32_t a_addr = smem_addr(smem + s * S::STAGE_BYTES);
-        const uint64_t adesc = desc_k_major(a_addr), bdesc = desc_k_major(a_addr + S::A_BYTES);
-#pragma unroll
-        for (int k = 0; k < BK / 16; ++k)
-          umma_bf16(tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
-        umma_commit(empty0 + 8 * s);
-      }
-      umma_commit(acc_bar);
-    }
-  } else {
-    if (!mbar_wait(acc_bar, 0)) {
-      if (lane == 0) atomicExch(status, ST_EPILOGUE_TIMEOUT);
-    } else {
-      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      epilogue_tile<BN, EPI>(tmem, reinterpret_cast<float *>(smem) + warp * (32 * 33), Cv, m0, n0, m_end, Nw, ldc, warp, lane, glu);
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  if (warp == 5) {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)BN));
-  }
-}
-
 // Epilogue of one 128 x BN tile through shared memory and tile stores.  Warp w owns rows
 // 32w .. 32w+31; a thread owns one row.  Per box of 128 bytes per row (64 bfloat16 or 32 float
 // outputs) the thread writes its row into a 32 x 128-byte staging buffer of its warp in the
@@ -809,6 +705,173 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   // the copies that read this CTA's ring and the arrivals on its barrier are over when every
   // rank has its parts: nobody leaves before
   if (k_parts > 1) cluster_sync_all();
+}
+
+// ---- groups of rows -------------------------------------------------------------------------
+// One product per group of rows (a routed feed-forward's experts): rows first .. end of A (and of C)
+// belong to group e and are multiplied by rows e Nw .. (e + 1) Nw of W.  Where the groups lie is a
+// plan in device memory, made by an earlier kernel of the step:
+//   plan[1 + e] first row of group e;   plan[1 + n_groups] all rows
+// The persistent kernel's roles over the tiles of all groups, which every CTA counts from the plan: of a group, all its row
+// tiles for one column tile after another, so that the CTAs that run together share a group's rows and a few panels of its
+// matrix in the L2.  A tile's last rows may be the next group's (or zeros): they are loaded and multiplied, never stored, which
+// is why the epilogue stores rows itself instead of whole boxes.  15,360 rows in 16 groups, width 4096: gate and up of 3072
+// 556 us, 1,390 TFLOP/s, down 350 us, 1,105 (a CTA a 128 x 128 tile, without a second accumulator: 973 us, 794 TFLOP/s, and 642 us, 602).
+#define GROUPS_MOST 1024
+template <int BN, int STAGES> struct SmemG {
+  static constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = A_BYTES + BN * BK * 2;
+  static constexpr int SCRATCH_OFFSET = STAGES * STAGE_BYTES;                 // 32 x 33 floats a warp of the epilogue
+  static constexpr int BARRIER_OFFSET = SCRATCH_OFFSET + 4 * 32 * 33 * 4;
+  static constexpr int TOTAL = BARRIER_OFFSET + 8 * (2 * STAGES + 4) + 16 + 1024;
+};
+
+template <int BN, int STAGES, int EPI>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, void *Cv, const int *plan,
+                       int n_groups, int Nw, int K, int ldc, int *status, ProductTail glu) {
+  pdl_launch();
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ int starts[GROUPS_MOST + 1];            // row tiles of the groups in front
+  using S = SmemG<BN, STAGES>;
+  unsigned char *smem = reinterpret_cast<unsigned char *>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + S::BARRIER_OFFSET);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
+  const uint32_t full0 = smem_addr(bars), empty0 = smem_addr(bars + STAGES);
+  const uint32_t acc_full0 = smem_addr(bars + 2 * STAGES), acc_empty0 = smem_addr(bars + 2 * STAGES + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nkb = (K + BK - 1) / BK, tiles_n = (Nw + BN - 1) / BN;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(acc_full0 + 8 * b, 1);
+      mbar_init(acc_empty0 + 8 * b, 4);              // one arrival per epilogue warp
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 5) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                     smem_addr(tmem_slot)), "r"((uint32_t)(2 * BN)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+  }
+  pdl_wait();                  // the plan is an earlier kernel's output
+  if (warp == 0) {
+    int before = 0;
+    for (int e0 = 0; e0 < n_groups; e0 += 32) {
+      const int e = e0 + lane, mine = e < n_groups ? (plan[2 + e] - plan[1 + e] + BM - 1) / BM : 0;
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      if (e < n_groups) starts[e] = before + upto - mine;
+      before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (lane == 0) starts[n_groups] = before;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const int n_tiles = starts[n_groups] * tiles_n;
+  // tile t: its group, its first row and the end of its rows, its first column in the group
+  auto tile_at = [&](int t, int &e, int &m0, int &m_end, int &n0) {
+    int lo = 0, hi = n_groups;                       // the last group with no more than t tiles in front that has any
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (starts[mid] * tiles_n <= t) lo = mid;
+      else hi = mid;
+    }
+    e = lo;
+    const int rows = starts[e + 1] - starts[e], within = t - starts[e] * tiles_n, tn = within / rows;
+    const int end = plan[2 + e];
+    m0 = plan[1 + e] + (within - tn * rows) * BM;
+    m_end = min(m0 + BM, end);
+    n0 = tn * BN;
+  };
+
+  if (warp == 4) {
+    if (lane == 0 && PRODUCER_RUNS) {
+      uint32_t g = 0;                                // k-blocks loaded so far, over all tiles
+      bool ok = true;
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+        int e, m0, m_end, n0;
+        tile_at(t, e, m0, m_end, n0);
+        for (int kb = 0; kb < nkb; ++kb, ++g) {
+          const uint32_t s = g % STAGES;
+          if (g >= STAGES && !mbar_wait(empty0 + 8 * s, ((g / STAGES) - 1) & 1)) {
+            atomicExch(status, ST_PRODUCER_TIMEOUT);
+            ok = false;
+            break;
+          }
+          const uint32_t a_dst = smem_addr(smem + s * S::STAGE_BYTES);
+          mbar_expect_tx(full0 + 8 * s, S::STAGE_BYTES);
+          tma_load_2d(a_dst, &map_a, kb * BK, m0, full0 + 8 * s);
+          tma_load_2d(a_dst + S::A_BYTES, &map_w, kb * BK, e * Nw + n0, full0 + 8 * s);
+        }
+      }
+    }
+  } else if (warp == 5) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = idesc_n(BN);
+      uint32_t g = 0, j = 0;                         // k-blocks and tiles so far
+      bool ok = true;
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++j) {
+        const uint32_t buf = j & 1;
+        // the epilogue must have drained this accumulator (it was used by tile j - 2)
+        if (j >= 2 && !mbar_wait(acc_empty0 + 8 * buf, ((j >> 1) - 1) & 1)) {
+          atomicExch(status, ST_MMA_TIMEOUT);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        for (int kb = 0; kb < nkb; ++kb, ++g) {
+          const uint32_t s = g % STAGES;
+          if (!mbar_wait(full0 + 8 * s, (g / STAGES) & 1)) {
+            atomicExch(status, ST_MMA_TIMEOUT);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          const uint32_t a_addr = smem_addr(smem + s * S::STAGE_BYTES);
+          const uint64_t adesc = desc_k_major(a_addr), bdesc = desc_k_major(a_addr + S::A_BYTES);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_bf16(tmem + buf * BN, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_commit(empty0 + 8 * s);
+        }
+        if (ok) umma_commit(acc_full0 + 8 * buf);    // this tile's MMAs have completed
+      }
+    }
+  } else {
+    uint32_t j = 0;
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++j) {
+      const uint32_t buf = j & 1;
+      if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1)) {
+        if (lane == 0) atomicExch(status, ST_EPILOGUE_TIMEOUT);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      int e, m0, m_end, n0;
+      tile_at(t, e, m0, m_end, n0);
+      epilogue_tile<BN, EPI>(tmem + buf * BN, reinterpret_cast<float *>(smem + S::SCRATCH_OFFSET) + warp * (32 * 33), Cv, m0, n0, m_end, Nw,
+                             ldc, warp, lane, glu);
+      // every load of this warp from the accumulator has completed (each is waited for)
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty0 + 8 * buf);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 5) {
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)(2 * BN)));
+  }
 }
 
 // ---- pairs of CTAs -------------------------------------------------------------------------
@@ -1605,10 +1668,10 @@ extern "C" int g2b_gemm_tc(const void *A, const void *W, void *C, int M, int N, 
 }
 
 template <int BN, int STAGES, int EPI>
-static int launch_grouped(const CUtensorMap &ma, const CUtensorMap &mw, void *C, const int *plan, int n_groups, int Nw,
-                          int K, int ldc, int max_tiles, int *status, ProductTail glu, cudaStream_t stream) {
+static int launch_grouped(const CUtensorMap &ma, const CUtensorMap &mw, void *C, int rows, const int *plan, int n_groups, int Nw, int K,
+                          int ldc, int *status, ProductTail glu, cudaStream_t stream) {
   static G2bPerDevice configured;
-  const int smem = Smem<BN, STAGES>::TOTAL;
+  const int smem = SmemG<BN, STAGES>::TOTAL;
   const int cfg_dev = g2b_current_device();
   if (cfg_dev < 0 || !configured.value[cfg_dev]) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_grouped_kernel<BN, STAGES, EPI>,
@@ -1616,9 +1679,9 @@ static int launch_grouped(const CUtensorMap &ma, const CUtensorMap &mw, void *C,
     if (e != cudaSuccess) G2B_REFUSE("gemm_tc: shared memory of %d bytes refused: %s", smem, cudaGetErrorString(e));
     if (cfg_dev >= 0) configured.value[cfg_dev] = 1;
   }
-  dim3 grid((Nw + BN - 1) / BN, max_tiles);
-  g2b_launch(gemm_tc_grouped_kernel<BN, STAGES, EPI>, grid, dim3(THREADS), smem, stream, ma, mw, C, plan, n_groups, Nw, K,
-             ldc, status, glu);
+  const long long most = ((long long)rows / BM + n_groups) * ((Nw + BN - 1) / BN);
+  g2b_launch(gemm_tc_grouped_kernel<BN, STAGES, EPI>, dim3((unsigned)(most < sm_count() ? most : sm_count())), dim3(THREADS), smem, stream,
+             ma, mw, C, plan, n_groups, Nw, K, ldc, status, glu);
   return g2b_check_launch("gemm_tc (grouped)");
 }
 
@@ -1637,18 +1700,24 @@ extern "C" int g2b_gemm_tc_grouped(const void *A, const void *W, void *C, int ro
   if (max_tiles > 65535) G2B_REFUSE("gemm_tc: %d row tiles are too many for one launch", max_tiles);
   if (!status || !plan) G2B_REFUSE("gemm_tc: no status word or no plan");
   if ((long long)n_groups * Nw > 0x7fffffffLL) G2B_REFUSE("gemm_tc: %d groups of %d rows of W", n_groups, Nw);
+  if (n_groups > GROUPS_MOST) G2B_REFUSE("gemm_tc: %d groups (at most %d)", n_groups, GROUPS_MOST);
+  // wide tiles where two rounds of them fill the GPU (a group's last row tile is half full on average)
+  const long long row_tiles = rows / BM + n_groups / 2;
+  const bool wide = Nw >= 256 && row_tiles * ((Nw + 255) / 256) >= 2 * sm_count();
   CUtensorMap ma, mw;
   int rc = make_map(&ma, A, rows, K, lda, BM);
   if (rc) return rc;
-  rc = make_map(&mw, W, n_groups * Nw, K, K, 128);
+  rc = make_map(&mw, W, n_groups * Nw, K, K, wide ? 256 : 128);
   if (rc) return rc;
 #ifndef G2B_ACT
   if (epi == EPI_SWIGLU_BF16)
-    return launch_grouped<128, 6, EPI_SWIGLU_BF16>(ma, mw, C, plan, n_groups, Nw, K, ldc, max_tiles, status, glu, stream);
+    return wide ? launch_grouped<256, 4, EPI_SWIGLU_BF16>(ma, mw, C, rows, plan, n_groups, Nw, K, ldc, status, glu, stream)
+                : launch_grouped<128, 6, EPI_SWIGLU_BF16>(ma, mw, C, rows, plan, n_groups, Nw, K, ldc, status, glu, stream);
 #endif
 #if !defined(G2B_GLU) && !defined(G2B_ACT)
   if (epi == EPI_STORE_F32)
-    return launch_grouped<128, 6, EPI_STORE_F32>(ma, mw, C, plan, n_groups, Nw, K, ldc, max_tiles, status, glu, stream);
+    return wide ? launch_grouped<256, 4, EPI_STORE_F32>(ma, mw, C, rows, plan, n_groups, Nw, K, ldc, status, glu, stream)
+                : launch_grouped<128, 6, EPI_STORE_F32>(ma, mw, C, rows, plan, n_groups, Nw, K, ldc, status, glu, stream);
 #endif
   G2B_REFUSE("gemm_tc: the grouped kernel stores float or gated bfloat16, not epilogue %d", epi);
 }
