@@ -72,6 +72,14 @@ struct JoinExperts {          // y = base + sum_r weight_r * (row of the pair, o
   }
 };
 
+// Four neighbours of either type as floats, and back.
+__device__ __forceinline__ float4 load4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ float4 load4(const bf16 *p) {
+  const uint2 raw = *reinterpret_cast<const uint2 *>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
 __device__ __forceinline__ void join_store4(float *p, const float4 &v) { *reinterpret_cast<float4 *>(p) = v; }
 __device__ __forceinline__ void join_store4(bf16 *p, const float4 &v) {
   uint2 raw;

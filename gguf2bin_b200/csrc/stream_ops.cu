@@ -22,6 +22,7 @@
 // Rings are indexed by position, never by step: a decode step that is taken back and run again
 // at the same position reads what the step before it read.
 #include "common.cuh"
+#include "join.cuh"
 #include "mma.cuh"
 
 G2B_DEFINE_LAST_ERROR
@@ -407,6 +408,69 @@ latent_pair_kernel(const TA *__restrict__ d, int rank, int width, const float *_
   for (int j = lane; j < fill; j += 32) dst[j] = from_f32<TA>(j < n ? (to_f32(src[j]) * inv) * w[j] : 0.f);
 }
 
+// The same for rows in vectors, up to 128 PER entries: a lane keeps PER groups of four neighbours in registers between the sum and
+// the store, every load is on its way before the first is used, and the weights are asked for before the wait for the kernel
+// in front.  Ranks of 128 and 2,048, decode steps and a prompt on average: 6.9 us (21.5 us an entry a lane).
+template <typename TA, int PER>
+__global__ void __launch_bounds__(LPAIR_WARPS * 32)
+latent_pair4_kernel(const TA *d, int rank, int width, const float *__restrict__ d_w, TA *pages, const int *page_table, int P, int page_size,
+                    const int *tok_pos, const int *tok_seq, const TA *e, int e_rank, const float *__restrict__ e_w, TA *e_out, int stride,
+                    float eps, int n_tokens, int parts) {
+  pdl_launch();
+  const int lane = threadIdx.x & 31;
+  const long long item = (long long)blockIdx.x * LPAIR_WARPS + (threadIdx.x >> 5);
+  if (item >= (long long)n_tokens * parts) return;
+  const int t = (int)(item / parts);
+  const bool keys = d && item % parts == 0;
+  const int n = keys ? rank : e_rank;
+  const float *w = keys ? d_w : e_w;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 x[PER], g[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int j = 4 * lane + 128 * i;
+    g[i] = j < n ? *reinterpret_cast<const float4 *>(w + j) : zero;
+  }
+  pdl_wait();
+  const TA *src = (keys ? d : e) + (size_t)t * stride;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int j = 4 * lane + 128 * i;
+    x[i] = j < n ? load4(src + j) : zero;
+  }
+  TA *dst = e_out + (size_t)t * e_rank;
+  if (keys) {
+    const int pos = tok_pos[t];
+    const int page = page_table[(size_t)tok_seq[t] * P + pos / page_size];
+    dst = pages + ((size_t)page * page_size + pos % page_size) * width;
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) ss = fmaf(x[i].x, x[i].x, fmaf(x[i].y, x[i].y, fmaf(x[i].z, x[i].z, fmaf(x[i].w, x[i].w, ss))));
+  const float inv = 1.f / sqrtf(warp_sum(ss) / (float)n + eps);
+  const int fill = keys ? width : n;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int j = 4 * lane + 128 * i;
+    if (j < fill) join_store4(dst + j, make_float4(x[i].x * inv * g[i].x, x[i].y * inv * g[i].y, x[i].z * inv * g[i].z, x[i].w * inv * g[i].w));
+  }
+}
+
+template <typename TA>
+static void launch_latent_pair(const void *d, int rank, int width, const float *d_w, void *pages, const int *page_table, int P, int page_size,
+                               const int *tok_pos, const int *tok_seq, const void *e, int e_rank, const float *e_w, void *e_out, int stride,
+                               float eps, int n_tokens, int parts, cudaStream_t stream) {
+  const unsigned blocks = (unsigned)(((long long)n_tokens * parts + LPAIR_WARPS - 1) / LPAIR_WARPS);
+  const int most = max(d ? width : 0, e ? e_rank : 0);
+  const bool whole = (!d || (rank % 4 == 0 && width % 4 == 0)) && (!e || e_rank % 4 == 0) && stride % 4 == 0 && most <= 2048 &&
+                     !(((uintptr_t)d | (uintptr_t)e | (uintptr_t)pages | (uintptr_t)e_out) & (4 * sizeof(TA) - 1)) &&
+                     !(((uintptr_t)d_w | (uintptr_t)e_w) & 15);
+  auto kernel = !whole ? latent_pair_kernel<TA> : most <= 512 ? latent_pair4_kernel<TA, 4> : most <= 1024 ? latent_pair4_kernel<TA, 8>
+                                                                                           : latent_pair4_kernel<TA, 16>;
+  g2b_launch(kernel, dim3(blocks), dim3(LPAIR_WARPS * 32), 0, stream, (const TA *)d, rank, width, d_w, (TA *)pages, page_table, P, page_size,
+             tok_pos, tok_seq, (const TA *)e, e_rank, e_w, (TA *)e_out, stride, eps, n_tokens, parts);
+}
+
 extern "C" int g2b_latent_pair(const void *d, int rank, int width, const float *d_w, void *pages, const int *page_table,
                                int P, int page_size, const int *tok_pos, const int *tok_seq, const void *e, int e_rank,
                                const float *e_w, void *e_out, int stride, float eps, int n_tokens, int dtype,
@@ -415,15 +479,12 @@ extern "C" int g2b_latent_pair(const void *d, int rank, int width, const float *
   if (n_tokens <= 0 || !parts) return 0;
   if (d && (rank <= 0 || width < rank || page_size <= 0)) G2B_REFUSE("latent_pair: rank %d in rows of %d", rank, width);
   if (e && e_rank <= 0) G2B_REFUSE("latent_pair: query rank %d", e_rank);
-  const unsigned blocks = (unsigned)(((long long)n_tokens * parts + LPAIR_WARPS - 1) / LPAIR_WARPS);
   if (dtype == G2B_F32)
-    g2b_launch(latent_pair_kernel<float>, dim3(blocks), dim3(LPAIR_WARPS * 32), 0, stream, (const float *)d, rank, width, d_w,
-               (float *)pages, page_table, P, page_size, tok_pos, tok_seq, (const float *)e, e_rank, e_w, (float *)e_out,
-               stride, eps, n_tokens, parts);
+    launch_latent_pair<float>(d, rank, width, d_w, pages, page_table, P, page_size, tok_pos, tok_seq, e, e_rank, e_w, e_out, stride, eps, n_tokens,
+                              parts, stream);
   else if (dtype == G2B_BF16)
-    g2b_launch(latent_pair_kernel<bf16>, dim3(blocks), dim3(LPAIR_WARPS * 32), 0, stream, (const bf16 *)d, rank, width, d_w,
-               (bf16 *)pages, page_table, P, page_size, tok_pos, tok_seq, (const bf16 *)e, e_rank, e_w, (bf16 *)e_out,
-               stride, eps, n_tokens, parts);
+    launch_latent_pair<bf16>(d, rank, width, d_w, pages, page_table, P, page_size, tok_pos, tok_seq, e, e_rank, e_w, e_out, stride, eps, n_tokens,
+                             parts, stream);
   else
     G2B_REFUSE("latent_pair: unknown dtype %d", dtype);
   return g2b_check_launch("latent_pair");

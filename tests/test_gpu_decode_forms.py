@@ -112,3 +112,74 @@ def test_pooled_entries_in_runs(hd, T, nh, nkv, window, pool):
         qt = q[t].double().view(nkv, nh // nkv, hd)
         a = torch.softmax(torch.einsum("kgd,ked->kge", qt, kv[0]) * hd ** -0.5, -1)
         near(out[t].view(nkv, nh // nkv, hd), torch.einsum("kge,ked->kgd", a, kv[1]), torch.bfloat16, 16 * torch.einsum("kge,ked->kgd", a, kv[1].abs()))
+
+
+@pytest.mark.parametrize("nh,nkv,nvh,D,V,rot,interleaved", [(1, 1, 1, 4, 4, 4, True), (5, 2, 2, 20, 12, 8, False), (20, 4, 4, 128, 128, 128, False),
+                                                            (7, 3, 1, 64, 128, 32, True), (4, 2, 2, 124, 124, 0, True), (3, 0, 0, 128, 128, 64, False), (6, 2, 2, 8, 100, 8, False)])
+@pytest.mark.parametrize("form", ["norm", "norm q", "unit", "values"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norms_per_head(nh, nkv, nvh, D, V, rot, interleaved, form, dtype):
+    from gguf2bin_b200 import kernels
+    T, page, hd = 3, 4, max(D, V)
+    n = (nh + nkv) * D + nvh * V
+    x, b = rnd(T, n, dtype=dtype, seed=1), rnd(n, seed=2) if form != "unit" else None
+    q_w, k_w = rnd(D, seed=3) if "norm" in form else None, rnd(D, seed=4) if form == "norm" else None
+    unit, v_eps = 1e-6 if form in ("unit", "norm q") else 0.0, 1e-6 if form == "values" else 0.0
+    angle = rnd(T, max(rot // 2, 1), seed=4)
+    rope = torch.stack([angle.cos(), angle.sin()], -1).contiguous() if rot else None
+    ctx = SimpleNamespace(tok_pos=torch.tensor([0, 5, 3], dtype=torch.int32, device=DEV), tok_seq=torch.tensor([1, 0, 2], dtype=torch.int32, device=DEV),
+                          page_table=torch.tensor([[0, 1], [2, 3], [4, 5]], dtype=torch.int32, device=DEV))
+    y = x.double() + (b.double() if b is not None else 0)
+    qk, v = y[:, :(nh + nkv) * D].reshape(T, nh + nkv, D).clone(), y[:, (nh + nkv) * D:].reshape(T, nvh, V)
+    rms = lambda z, eps: (z.square().mean(-1, keepdim=True) + eps).sqrt()
+    for w, heads in ((q_w, slice(0, nh)), (k_w, slice(nh, nh + nkv))):
+        if w is not None:
+            qk[:, heads] = qk[:, heads] / rms(qk[:, heads], 1e-5) * w.double()
+    size = qk.abs()
+    if rot:
+        c, s = rope[:, None, :, 0].double(), rope[:, None, :, 1].double()
+        one, two = (slice(0, rot, 2), slice(1, rot, 2)) if interleaved else (slice(0, rot // 2), slice(rot // 2, rot))
+        u, w = qk[..., one].clone(), qk[..., two].clone()
+        qk[..., one], qk[..., two] = u * c - w * s, w * c + u * s
+        size[..., one] = size[..., two] = u.abs() + w.abs()
+    if unit:
+        qk, size = qk / rms(qk, unit), size / rms(qk, unit)
+    if v_eps:
+        v = v / rms(v, v_eps)
+    for general in (False, True):
+        cache, q_out = torch.full((6, 2, max(nkv, 1), page, hd), 9.0, dtype=dtype, device=DEV), torch.empty(T, nh * hd, dtype=dtype, device=DEV)
+        kernels.proj_norm_rope_cache(apart(x, general), b, nh, nkv, D, V, q_w, k_w, 1e-5, rope, rot, interleaved, ctx, cache if nkv else None, page, q_out,
+                                     v_norm_eps=v_eps, norm_per_head="norm" in form, unit_eps=unit, n_v_heads=nvh)
+        q = q_out.view(T, nh, hd)
+        near(q[..., :D], qk[:, :nh], dtype, size[:, :nh])
+        assert not q[..., D:].any()
+        left = torch.ones_like(cache, dtype=torch.bool)
+        for t, (p, at) in enumerate(((2, 0), (1, 1), (4, 3))):
+            near(cache[p, 0, :nkv, at, :D], qk[t, nh:], dtype, size[t, nh:])
+            near(cache[p, 1, :nvh, at, :V], v[t], dtype, v[t].abs())
+            assert not cache[p, 0, :nkv, at, D:].any() and not cache[p, 1, :nvh, at, V:].any()
+            left[p, 0, :nkv, at] = left[p, 1, :nvh, at] = False
+        assert (cache[left] == 9.0).all()
+
+
+@pytest.mark.parametrize("rank,width,e_rank", [(4, 4, 4), (96, 128, 512), (512, 576, 1536), (508, 1000, 1024), (2044, 2048, 2048), (2048, 2052, 8)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_latents(rank, width, e_rank, dtype):
+    from gguf2bin_b200 import kernels
+    T, page = 5, 4
+    d_w, e_w = rnd(rank, seed=2), rnd(e_rank, seed=3)
+    ctx = SimpleNamespace(tok_pos=torch.tensor([0, 5, 3, 7, 1], dtype=torch.int32, device=DEV), tok_seq=torch.arange(5, dtype=torch.int32, device=DEV),
+                          page_table=torch.arange(10, dtype=torch.int32, device=DEV).view(5, 2), page_size=page)
+    both = rnd(T, rank + e_rank, dtype=dtype, seed=1)
+    want = [x / (x.square().mean(-1, keepdim=True) + 1e-5).sqrt() * w.double() for x, w in ((both[:, :rank].double(), d_w), (both[:, rank:].double(), e_w))]
+    for general in (False, True):
+        x = apart(both, general)
+        pages, out = torch.full((10, page, width), 9.0, dtype=dtype, device=DEV), torch.empty(T, e_rank, dtype=dtype, device=DEV)
+        kernels.latent_pair(x[:, :rank], width, d_w, pages, x[:, rank:], e_w, out, 1e-5, ctx)
+        near(out, want[1], dtype, want[1].abs())
+        left = torch.ones_like(pages, dtype=torch.bool)
+        for t, (p, at) in enumerate(((0, 0), (3, 1), (4, 3), (7, 3), (8, 1))):
+            near(pages[p, at, :rank], want[0][t], dtype, want[0][t].abs())
+            assert not pages[p, at, rank:].any()
+            left[p, at] = False
+        assert (pages[left] == 9.0).all()
