@@ -31,7 +31,6 @@ class EngineBackend:
         self.max_context = min(limit, int(max_context)) if max_context else limit
         self.page_size = engine.cache.page_size
         self._ids = torch.empty(1024, dtype=torch.int32, device=engine.device)
-        self._slots = torch.empty(1024, dtype=torch.int32, device=engine.device)
         self.use_graph = use_graph
         self._session: Optional[DecodeSession] = None
         # wall-clock account of the decode calls, for measurements through this API
@@ -72,12 +71,11 @@ class EngineBackend:
             self.engine.close_sequence(handle.seq)
 
     def _sample(self, logits: torch.Tensor, handles: Sequence[_Handle]) -> list:
+        """The tokens behind the step that has just run for these handles: their slots are in its metadata."""
         R = len(handles)
         if self._ids.shape[0] < R:
             self._ids = torch.empty(2 * R, dtype=torch.int32, device=self.engine.device)
-            self._slots = torch.empty(2 * R, dtype=torch.int32, device=self.engine.device)
-        self._slots[:R].copy_(torch.tensor([h.seq.slot for h in handles], dtype=torch.int32))
-        self.sampler.sample(logits, self.params, self._slots[:R], self._ids[:R])
+        self.sampler.sample(logits, self.params, self.engine.last_slots[:R], self._ids[:R])
         out = self._ids[:R].tolist()
         self.engine.check()                    # never hand on tokens of a launch that gave up a wait
         return out

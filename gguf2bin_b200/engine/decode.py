@@ -119,7 +119,7 @@ class DecodeRunner:
             host[4 * B + r * P:4 * B + r * P + len(s.pages)] = s.pages
         first = B if keep_tokens else 0
         self._meta[first:].copy_(self._meta_host[first:], non_blocking=True)
-        self._uploaded.record()
+        self._uploaded.record(kernels.current_stream())
         self.ctx.slots = slots
         # the page table is as wide as what is reserved; kernels that size their work by the keys plan with what is there
         self.ctx.kv_len_hint = max(s.length for s in session.seqs) + 1
@@ -151,7 +151,7 @@ class DecodeRunner:
             return
         before = kernels.launch_count()
         if use_graph and self.plain_steps >= eager_steps:
-            torch.cuda.current_stream().synchronize()
+            kernels.current_stream().synchronize()
             generation = ws.generation
             g, _ = capture_graph(self._launch)
             self.launches_per_step = kernels.launch_count() - before
@@ -256,7 +256,7 @@ class DecodeSession:
         staged[:] = 0
         staged[self.rows] = tokens
         runner.tok_ids.copy_(runner.pinned_in, non_blocking=True)
-        runner.tokens_uploaded.record()
+        runner.tokens_uploaded.record(kernels.current_stream())
 
     def run(self) -> None:
         """One step: feeds ``tok_ids``, leaves the sampled tokens in ``tok_ids`` and the
@@ -288,7 +288,7 @@ class DecodeSession:
         turn = runner.out_turn
         runner.out_turn ^= 1
         runner.pinned_out[turn].copy_(runner.tok_ids, non_blocking=True)
-        runner.out_ready[turn].record()
+        runner.out_ready[turn].record(kernels.current_stream())
         return turn
 
     def _collect(self, turn: int) -> list:

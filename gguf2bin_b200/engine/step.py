@@ -15,6 +15,7 @@ the cache, positions); a refused step changes nothing.
 from __future__ import annotations
 
 import gc
+from array import array
 from collections import OrderedDict
 from dataclasses import dataclass, field
 from typing import Optional, Sequence as Seq
@@ -22,6 +23,7 @@ from typing import Optional, Sequence as Seq
 import numpy as np
 import torch
 
+from .. import kernels
 from ..cache.pool import CacheError, Sequence
 from ..cache.storage import Cache
 from ..parts.base import ATTN_TILE_ROWS, ATTN_WIDE_TILE_ROWS, StepContext
@@ -59,6 +61,40 @@ class StepEntry:
     seq: Sequence
     tokens: Seq[int]
     want: Seq[int] = field(default_factory=tuple)
+
+
+def token_ids(tokens: Seq[int], vocab: int) -> np.ndarray:
+    """A step's token ids as integers, each checked against the vocabulary.  A list of whole numbers (a prompt of thousands, as a
+    rule) is converted and checked as a whole; anything else, and a list with something wrong in it, one by one."""
+    if type(tokens) in (list, tuple):
+        try:
+            ids = np.frombuffer(array("q", tokens), dtype=np.int64)
+        except (TypeError, ValueError, OverflowError):
+            ids = None
+        if ids is not None and ids.size and ids.min() >= 0 and ids.max() < vocab:
+            return ids
+    for t in tokens:
+        if not (0 <= int(t) < vocab):
+            raise StepError(f"token id {t} outside the vocabulary 0..{vocab - 1}")
+    return np.asarray(tokens, dtype=np.int32)
+
+
+def attention_tiles(q_lens: Seq[int], past: Seq[int], rows: int) -> np.ndarray:
+    """The prompt attention's work list, int32 [tiles, 4]: sequence, first token, rows (at most ``rows``) and the position of the
+    first, of every tile; the longest key ranges first."""
+    if len(q_lens) <= 2 and sum(q_lens) <= 16 * rows:                # a few tiles: plain lists are quicker than arrays
+        tiles, t0 = [], 0
+        for b, n in enumerate(q_lens):
+            tiles += [(b, t0 + r, min(rows, n - r), past[b] + r) for r in range(0, n, rows)]
+            t0 += n
+        tiles.sort(key=lambda t: -(t[3] + t[2]))
+        return np.array(tiles, dtype=np.int32)
+    n, before = np.asarray(q_lens), np.asarray(past)
+    count = -(-n // rows)
+    seq = np.repeat(np.arange(len(n)), count)
+    r = (np.arange(len(seq)) - np.repeat(np.cumsum(count) - count, count)) * rows
+    tiles = np.stack([seq, (np.cumsum(n) - n)[seq] + r, np.minimum(rows, n[seq] - r), before[seq] + r], axis=1)
+    return tiles[np.argsort(-(tiles[:, 3] + tiles[:, 2]), kind="stable")].astype(np.int32)
 
 
 class _PaddingSequence:
@@ -103,6 +139,7 @@ class Engine:
         self._seen: "OrderedDict[tuple, int]" = OrderedDict()        # shapes run plainly so far
         self.decode_runners: "OrderedDict[tuple, object]" = OrderedDict()
         self._padding = _PaddingSequence(self.cache)
+        self.last_slots: Optional[torch.Tensor] = None     # the slots of the last step's sequences, on the device until the next
         self.step_graph_captures = 0       # CUDA graphs captured so far: of prompt-step shapes,
         self.decode_graph_captures = 0     # and of decode shapes (engine/decode.py)
 
@@ -127,7 +164,9 @@ class Engine:
             kernels_bf16.check_status()
 
     # ---- step ------------------------------------------------------------------
-    def _check(self, entries: Seq[StepEntry]) -> None:
+    def _check(self, entries: Seq[StepEntry]) -> list:
+        """Refuses a step that cannot run; the entries' token ids as arrays."""
+        ids = []
         if not entries:
             raise StepError("a step needs at least one sequence")
         V, maxpos = self.model.vocab, self.model.spec.max_positions
@@ -141,9 +180,7 @@ class Engine:
             n = len(e.tokens)
             if n < 1:
                 raise StepError("every sequence of a step needs at least one token")
-            for t in e.tokens:
-                if not (0 <= int(t) < V):
-                    raise StepError(f"token id {t} outside the vocabulary 0..{V - 1}")
+            ids.append(token_ids(e.tokens, V))
             if e.seq.length + n > maxpos:
                 raise StepError(f"sequence would reach {e.seq.length + n} positions; the model "
                                 f"allows {maxpos}")
@@ -155,9 +192,11 @@ class Engine:
         if need > self.cache.table.pages.n_free:
             raise StepError(f"the cache is full: the step needs {need} more pages of "
                             f"{self.cache.page_size} tokens, {self.cache.table.pages.n_free} free")
+        return ids
 
-    def build_context(self, entries: Seq[StepEntry]) -> tuple[StepContext, torch.Tensor, int]:
-        """Host metadata of the step packed into one pinned buffer and copied once."""
+    def build_context(self, entries: Seq[StepEntry], ids: Optional[list] = None) -> tuple[StepContext, torch.Tensor, int]:
+        """Host metadata of the step packed into one pinned buffer and copied once.  ``ids``: the
+        entries' tokens as arrays, where they exist already (of the last entries the rest may lack)."""
         B = len(entries)
         q_lens = [len(e.tokens) for e in entries]
         past = [e.seq.length for e in entries]
@@ -166,20 +205,10 @@ class Engine:
         if T == B:                   # one token each: the table's width in steps, so that the shape's graph lasts
             P = -(-P // SINGLE_TABLE_STEP) * SINGLE_TABLE_STEP
         n_want = sum(len(e.want) for e in entries)
-        # prompt-attention work list: tiles of 64 query rows, the longest key ranges first
-        tiles, wide = [], []
-        t0 = 0
-        for b, e in enumerate(entries):
-            for r in range(0, q_lens[b], ATTN_TILE_ROWS):
-                tiles.append((b, t0 + r, min(ATTN_TILE_ROWS, q_lens[b] - r), past[b] + r))
-            for r in range(0, q_lens[b], ATTN_WIDE_TILE_ROWS):
-                wide.append((b, t0 + r, min(ATTN_WIDE_TILE_ROWS, q_lens[b] - r), past[b] + r))
-            t0 += q_lens[b]
-        tiles.sort(key=lambda t: -(t[3] + t[2]))
-        wide.sort(key=lambda t: -(t[3] + t[2]))
-        n_narrow = len(tiles)
-        tiles = tiles + wide
-        n_tiles = len(tiles)
+        # prompt-attention work list: tiles of 64 query rows, the longest key ranges first, then of 128
+        narrow = attention_tiles(q_lens, past, ATTN_TILE_ROWS)
+        wide = attention_tiles(q_lens, past, ATTN_WIDE_TILE_ROWS)
+        n_narrow, n_tiles = len(narrow), len(narrow) + len(wide)
         # layout: tiles[n_tiles*4] tok_ids[T] tok_pos[T] tok_seq[T] want[n_want] seq_meta[B*4]
         #         page_table[B*P] seq_slots[B]   (the tiles come first: the kernel reads them 16 bytes at a time)
         total = 4 * n_tiles + 3 * T + n_want + 4 * B + B * P + B
@@ -191,24 +220,26 @@ class Engine:
         o_ids = 4 * n_tiles
         o_pos, o_seq, o_want = o_ids + T, o_ids + 2 * T, o_ids + 3 * T
         o_meta = o_want + n_want
-        host[:4 * n_tiles] = np.asarray(tiles, dtype=np.int32).reshape(-1)
+        host[:4 * n_narrow] = narrow.reshape(-1)
+        host[4 * n_narrow:4 * n_tiles] = wide.reshape(-1)
         o_pt = o_meta + 4 * B
         o_slots = o_pt + B * P
-        t0 = w0 = 0
-        for b, e in enumerate(entries):
-            n = q_lens[b]
-            host[o_ids + t0:o_ids + t0 + n] = np.asarray(e.tokens, dtype=np.int32)
-            host[o_pos + t0:o_pos + t0 + n] = np.arange(past[b], past[b] + n, dtype=np.int32)
-            host[o_seq + t0:o_seq + t0 + n] = b
+        lens, starts = np.asarray(q_lens), np.cumsum(q_lens) - q_lens
+        seq = np.repeat(np.arange(B), lens)
+        host[o_seq:o_want] = seq
+        host[o_pos:o_seq] = np.arange(T) + (np.asarray(past) - starts)[seq]
+        meta = host[o_meta:o_pt].reshape(B, 4)
+        meta[:, 0], meta[:, 1], meta[:, 2], meta[:, 3] = starts, lens, past, [e.seq.slot for e in entries]
+        host[o_slots:total] = [e.seq.slot for e in entries]
+        w0 = 0
+        for b, (e, t0) in enumerate(zip(entries, starts.tolist())):
+            host[o_ids + t0:o_ids + t0 + q_lens[b]] = ids[b] if ids is not None and b < len(ids) else np.asarray(e.tokens, dtype=np.int32)
             for w in e.want:
                 host[o_want + w0] = t0 + int(w)
                 w0 += 1
-            host[o_meta + 4 * b:o_meta + 4 * b + 4] = (t0, n, past[b], e.seq.slot)
             row = host[o_pt + b * P:o_pt + (b + 1) * P]
             row[:len(e.seq.pages)] = e.seq.pages
             row[len(e.seq.pages):] = 0
-            host[o_slots + b] = e.seq.slot
-            t0 += n
         dev = self._meta_dev
         dev[:total].copy_(self._meta_host[:total], non_blocking=True)
         ctx = StepContext(
@@ -228,14 +259,15 @@ class Engine:
         [number of wanted places, vocab] in the order of the entries and of their
         ``want`` (None when nothing is wanted).  The tensor is scratch memory: it is
         valid until the next step."""
-        self._check(entries)
+        ids = self._check(entries)
         for e in entries:
             self.cache.reserve(e.seq, e.seq.length + len(e.tokens))
         # the pinned staging buffer is reused: the previous step's copy must be over
-        torch.cuda.current_stream().synchronize()
+        kernels.current_stream().synchronize()
         self.check()                 # a kernel of an earlier step that gave up a wait is reported here
         run = self._filled_up(entries)
-        ctx, want_rows, n_want = self.build_context(run)
+        ctx, want_rows, n_want = self.build_context(run, ids)
+        self.last_slots = ctx.seq_slots
         logits = self._forward(run, ctx, want_rows, n_want)
         for e in entries:
             e.seq.length += len(e.tokens)
@@ -288,7 +320,7 @@ class Engine:
             # The shape ran plainly before, so every scratch buffer it needs exists already.  A prompt
             # shape is captured when it comes for the third time: a capture costs as much as two or three
             # plain steps, and of the shapes of ragged batches most never come back.
-            torch.cuda.current_stream().synchronize()
+            kernels.current_stream().synchronize()
             generation = self.workspace.generation
             graph, logits = capture_graph(lambda: self.model.forward(ctx, self.cache, want_rows, n_want))
             self.step_graph_captures += 1

@@ -57,6 +57,24 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+_stream_objects: dict = {}         # (device, handle) -> the stream's object
+
+
+def current_stream() -> torch.cuda.Stream:
+    """``torch.cuda.current_stream()`` without its way through the device's name and the environment: an object that stands for
+    the same handle is kept (recording an event asks for one several times a step)."""
+    if _raw_stream is None or _raw_device is None:
+        return torch.cuda.current_stream()
+    device = _raw_device()
+    key = (device, _raw_stream(device))
+    stream = _stream_objects.get(key)
+    if stream is None:
+        if len(_stream_objects) >= 64:
+            _stream_objects.clear()
+        stream = _stream_objects[key] = torch.cuda.current_stream()
+    return stream
+
+
 def _need(t: torch.Tensor, dtype: torch.dtype, what: str) -> None:
     if t.dtype != dtype:
         raise KernelError(f"{what} must be {dtype}, got {t.dtype}")

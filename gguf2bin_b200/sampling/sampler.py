@@ -22,9 +22,8 @@ class Sampler:
         self._cap = 0
 
     def seed(self, slots: Sequence[int], streams: Sequence[int], seed: int) -> None:
-        s = torch.tensor(list(slots), dtype=torch.int32, device=self.device)
-        t = torch.tensor(list(streams), dtype=torch.int32, device=self.device)
-        kernels.seed_slots(self.seq_state, s, t, int(seed))
+        both = torch.tensor([list(slots), list(streams)], dtype=torch.int32, device=self.device)
+        kernels.seed_slots(self.seq_state, both[0], both[1], int(seed))
 
     def set_recent(self, slots: Sequence[int], tokens: Sequence[Sequence[int]]) -> None:
         """Starts each slot's ring of recent ids with the last ``RECENT_USE`` of its tokens
