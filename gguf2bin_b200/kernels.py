@@ -1324,10 +1324,11 @@ def moe_gemm(a, row_pair, pairs_per_token: int, w, n_out: int, plan, n_real: int
 
 
 def moe_gemv(a, row_pair, pairs_per_token: int, gather: bool, idx, w, n_out: int, plan, n_real: int, n_rows: int,
-             swiglu: bool, out, blocked: bool = False, form: GluForm = SILU) -> bool:
+             swiglu: bool, out, blocked: bool = False, form: GluForm = SILU, plan_stands: bool = False) -> bool:
     """``moe_gemm`` for a step of few rows, the weight rows streamed with 16-byte loads: in bfloat16 once for all rows of
     an expert (``swiglu`` in the blocked layout), else by a warp per four output columns of one row.  ``gather``: row r reads a[pair / pairs_per_token], else a[r].  False
-    when the sizes do not allow 16-byte loads (the caller then takes ``moe_gemm``)."""
+    when the sizes do not allow 16-byte loads (the caller then takes ``moe_gemm``).  ``plan_stands``: a ``moe_gemv`` over this plan
+    is in front on the stream, so that this one may read the plan before its predecessor ends."""
     if w.dtype != a.dtype:
         raise KernelError("moe_gemv: activations and expert matrices must have one dtype")
     per = 8 if a.dtype == torch.bfloat16 else 4
@@ -1335,10 +1336,11 @@ def moe_gemv(a, row_pair, pairs_per_token: int, gather: bool, idx, w, n_out: int
         return False
     f = _fn("moe.cu", "g2b_moe_gemv",
             [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
-             c_int, c_void_p, c_int, c_int, *_GLU_TYPES, c_void_p])
+             c_int, c_void_p, c_int, c_int, *_GLU_TYPES, c_int, c_void_p])
     _call(f, _ptr(a), _code(a.dtype), _dense_rows(a, "a"), _ptr(row_pair), pairs_per_token, 1 if gather else 0,
           _ptr(idx), _ptr(w), n_out, a.shape[1], _ptr(plan), n_real, n_rows, 1 if swiglu else 0, _ptr(out),
-          1 if out.dtype == torch.float32 else 0, 1 if blocked else 0, *form, _stream())
+          1 if out.dtype == torch.float32 else 0, 1 if blocked else 0, *form, 1 if plan_stands else 0,
+          _stream())
     return True
 
 

@@ -381,10 +381,10 @@ class RoutedExperts:
             if not done:
                 kernels.moe_gemm(a, row_pair, top, self.w_gate_up, self.inter, plan, E, max_tiles, True, mid,
                                  self.blocked, self.form)
-            done = False
+            streamed, done = few and done, False
             if few:
                 done = kernels.moe_gemv(mid, row_pair, top, False, idx, self.w_down, self.hidden, plan, E, n_pairs,
-                                        False, rows32)
+                                        False, rows32, plan_stands=streamed)
             elif many:
                 done = kernels.moe_gemm_tc(mid, self.w_down, self.hidden, plan, E, max_tiles, False, rows32)
             if not done:

@@ -55,3 +55,31 @@ def test_rows_of_experts(T, top, E, spread, N, K):
         err = K * 2.0 ** -23 * size.view(-1, half // 8, 2, 8)
         slack = 1.2 * err[:, :, 0].flatten(1) * up.abs() + (gate.abs() + 1) * err[:, :, 1].flatten(1)      # |silu'| < 1.1
         assert ((mid[rows].double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-6).all()
+
+
+@pytest.mark.parametrize("T,top,E", [(1, 4, 16), (8, 3, 16), (2, 1, 40)])
+@pytest.mark.parametrize("hidden,inter", [(512, 768), (1024, 48)])
+def test_second_product_over_a_plan(T, top, E, hidden, inter):
+    """Plans that change from round to round, in one queue without a wait: the product that starts ahead of its predecessor's end
+    gives the bits of the one that does not."""
+    from gguf2bin_b200 import kernels
+    g = torch.Generator().manual_seed(T)
+    w1, w2 = (rnd(E, n, k, dtype=torch.bfloat16, scale=0.05, seed=s) for n, k, s in ((2 * inter, hidden, 1), (hidden, inter, 2)))
+    a = rnd(T, hidden, dtype=torch.bfloat16, seed=3)
+    choices = [torch.randint(E + 1, (T, top), generator=g).to(torch.int32).to(DEV) for _ in range(12)]
+    ones, zeros = torch.ones(T, top, device=DEV), torch.zeros(T, hidden, device=DEV)
+    got = []
+    for stands in (False, True):
+        n = T * top
+        max_tiles = -(-n // kernels.moe_tile_rows()) + E
+        plan = torch.zeros(E + 2 + 3 * max_tiles, dtype=torch.int32, device=DEV)
+        row_pair, pair_row = (torch.zeros(n, dtype=torch.int32, device=DEV) for _ in range(2))
+        mid, out = torch.empty(n, inter, dtype=torch.bfloat16, device=DEV), torch.empty(n, hidden, device=DEV)
+        kept = torch.zeros(12, T, hidden, device=DEV)
+        for i, idx in enumerate(choices):
+            kernels.moe_plan(idx, E, max_tiles, plan, row_pair, pair_row)
+            kernels.moe_gemv(a, row_pair, top, True, idx, w1, inter, plan, E, n, True, mid, True)
+            kernels.moe_gemv(mid, row_pair, top, False, idx, w2, hidden, plan, E, n, False, out, plan_stands=stands)
+            kernels.moe_combine(out, pair_row, ones, zeros, top, kept[i])
+        got.append(kept)
+    assert torch.equal(*got) and got[0].abs().sum() > 0
