@@ -59,6 +59,20 @@ __device__ __forceinline__ void rotate_in_place(float *x, const float2 *cs, int 
   }
 }
 
+// The same with the first two pairs of every lane at hand already.
+__device__ __forceinline__ void rotate_ahead(float *x, const float2 *turn, const float2 *cs, int rot, int interleaved, int lane) {
+  const int half = rot >> 1;
+  auto pair = [&](int i, float2 r) {
+    const int a = interleaved ? 2 * i : i, b = interleaved ? 2 * i + 1 : i + half;
+    const float u = x[a], v = x[b];
+    x[a] = u * r.x - v * r.y;
+    x[b] = v * r.x + u * r.y;
+  };
+  if (lane < half) pair(lane, turn[0]);
+  if (lane + 32 < half) pair(lane + 32, turn[1]);
+  for (int i = lane + 64; i < half; i += 32) pair(i, cs[i]);
+}
+
 // ---------------------------------------------------------------------------
 // attention prologue with a norm over the whole projection
 // ---------------------------------------------------------------------------
@@ -308,8 +322,8 @@ proj_rope_cache_headwise_kernel(const T *__restrict__ qkv, int row_stride, const
 
 // The same for heads of up to 128 entries in vectors: a lane keeps four neighbours of its warp's head from the load to the store,
 // the half-split rotation's other halves come from the lane that has them, and every load is on its way before the first is
-// used (the constants' before the wait for the kernel in front).  Prologues of decode steps: 2.8 us, 5.2 us through shared memory (eight tokens
-// of heads of 64 and 128, on average), 4.8 and 6.7 us (three prompts and their single tokens).
+// used (the constants' before the wait for the kernel in front).  Prologues of decode steps: 2.8 us, 5.2 us through shared memory (eight tokens,
+// heads of 128), 4.8 and 6.7 us (three prompts and their single tokens).
 template <typename T>
 __global__ void __launch_bounds__(HEADWISE_WARPS * 32)
 proj_rope_cache_heads4_kernel(const T *qkv, int row_stride, const float *__restrict__ bias, int nh, int nkv, int D, int V,
@@ -787,7 +801,18 @@ state_scan_kernel(const ScanArgs a, int L) {
       const int row = first_row + t0 + warp;
       const T *qp = qg + (size_t)row * a.q_stride + (size_t)qk_head * D;
       const T *kp = kg + (size_t)row * a.k_stride + (size_t)qk_head * D;
+      // everything that the preparation reads is on its way before the first of it is used: a decode step is this chain (one token,
+      // 8 heads of 128 x 256: 6.2 us, 7.0 with each read where it is needed; four tokens of 64 heads of 128 x 64: 7.9, 9.5)
+      const float2 *cs = a.rope + (size_t)row * (a.rot >> 1);
+      float2 turn[2];
+      float ab_x = 0.f, ab_y = 0.f;
+      if (a.rope)
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+          if (lane + 32 * m < a.rot >> 1) turn[m] = cs[lane + 32 * m];
+      if (MODE != 0) ab_x = a.ab[(size_t)row * 2 * H + h], ab_y = a.ab[(size_t)row * 2 * H + H + h];
       float nq = 0.f, nk = 0.f;
+#pragma unroll 4
       for (int j = lane; j < D; j += 32) {
         const float x = to_f32(qp[j]), y = to_f32(kp[j]);
         sq[warp][j] = x;
@@ -802,9 +827,8 @@ state_scan_kernel(const ScanArgs a, int L) {
         fk *= 1.f / sqrtf(warp_sum(nk) + a.unit_eps);
       }
       if (a.rope) {
-        const float2 *cs = a.rope + (size_t)row * (a.rot >> 1);
-        rotate_in_place(sq[warp], cs, a.rot, a.interleaved, lane);
-        rotate_in_place(sk[warp], cs, a.rot, a.interleaved, lane);
+        rotate_ahead(sq[warp], turn, cs, a.rot, a.interleaved, lane);
+        rotate_ahead(sk[warp], turn, cs, a.rot, a.interleaved, lane);
         __syncwarp();
       }
       for (int j = lane; j < D; j += 32) {
@@ -812,12 +836,12 @@ state_scan_kernel(const ScanArgs a, int L) {
         sk[warp][j] *= fk;
       }
       if (MODE != 0 && lane == 0) {
-        const float x = a.ab[(size_t)row * 2 * H + h], y = a.ab[(size_t)row * 2 * H + H + h];
-        sg[warp] = MODE == 1 ? expf(-A * softplus_f(x + dt)) : x;
-        sb[warp] = MODE == 1 ? sigmoid_f(y) : y;
+        sg[warp] = MODE == 1 ? expf(-A * softplus_f(ab_x + dt)) : ab_x;
+        sb[warp] = MODE == 1 ? sigmoid_f(ab_y) : ab_y;
       }
     }
-    for (int i = threadIdx.x; i < nt * cols; i += SCAN_THREADS) {
+    // from the second warp on: the first prepares the only token of a decode step
+    for (int i = (threadIdx.x + SCAN_THREADS - 32) % SCAN_THREADS; i < nt * cols; i += SCAN_THREADS) {
       const int tt = i / cols, cc = i % cols;
       const int col = blockIdx.x * cols + cc;
       sv[tt][cc] = col < Vin ? to_f32(vg[(size_t)(first_row + t0 + tt) * a.v_stride + (size_t)h * Vin + col])
