@@ -668,42 +668,107 @@ moe_gemv_kernel(const T *__restrict__ A, int a_stride, const int *__restrict__ r
 // ---------------------------------------------------------------------------
 // the same in bfloat16: an expert's matrices are read once for all of its rows
 // ---------------------------------------------------------------------------
-// The work is a line of tiles: for every eight rows of every expert in use, all tiles of 16 rows of its matrix over the whole K.
-// A block per SM takes an equal stretch of the line.  The matrix is the 16-row operand of mma.m16n8k16, the expert's rows
-// (staged whole in shared memory) the 8-wide one; eight warps split every 256 columns, a thread copies 16 bytes of rows g and
-// g + 8 and the eight values feed two products under one permutation of k for both operands.  The copies run RING blocks of
-// 8 KB ahead, across tiles and experts, through a ring that needs no barrier: a thread reads back only what it copied.  A
-// tile's eight partial sums are added in the order of the warps (two buffers, one barrier a tile).  Memory bounds it.
-// Eight tokens, 3 of 16 experts, width 4096: gate and up of 3072 106 us (6.2 TB/s), down 57 us (5.7) (a warp a row and four columns, which
-// read a matrix once for every row of its expert: 168 and 76 us; blocks of eight tiles with the stream in registers, 174 and 111).
+// The work is a line of items: for every eight rows of every expert in use, all quads of rows of its matrix (two gates and their
+// two ups with SWIGLU) over the whole K.  A block per SM takes an equal stretch of the line, its sixteen warps an item each in turn,
+// the expert's rows staged whole in shared memory.  A warp brings 512 bytes of each of its four matrix rows at a time, RING such
+// blocks ahead, across items and experts, through a ring that needs no barrier: a lane reads back only what it copied, and
+// multiplies it by the same eight columns of each of the expert's rows.
+//
+// A lane's columns, the order of its multiply-adds and the tree that adds the lanes' sums are moe_gemv_kernel's, so both kernels give
+// the same bits.  On mma.m16n8k16, which cuts off what it adds instead of rounding it, sums over K = 768 to 6,000 were 1.0e-7 to
+// 7.2e-7 off and always towards zero; here 0.7e-7 to 1.1e-7 and to either side.  Memory bounds one row and two, the conversions to 32 bits (half
+// rate) and the multiply-adds more: hence four matrix rows a lane behind each conversion of x, and fma.rn.f32x2, which rounds each half
+// by itself, for two rows of x.  A product behind a product (of a row at a time; on mma.sync), gate and up of 3072 / down, width 4096,
+// eight tokens: 3 of 16 experts 118 us (6.0 TB/s) / 62 (166 / 62; 116 / 62), 8 of 16 168 / 87 (293 / 109; 134 / 71); sixteen tokens,
+// 8 of 16 241 / 129 (493 / 193; 191 / 105).  One token, 4 of 16, 768 / width 2048: 6.1 / 4.7 (13.6 / 4.3; 8.7 / 7.2).
 //
 // The next kernel of the stream may start once every block here has seen the plan (and waited for the kernel that wrote it), not
 // before.  A second product over the same plan (`plan_stands`: the down product behind gate and up) can therefore read the plan and
-// fill its ring with weights while the first one still works, and waits only for the rows: one token, 4 of 16
-// experts, width 2048, 8.3 us for 9.7; the down product above 56 us for 57.7.
-#define MS_KB 256
-#define MS_PAD 32
-#define MS_PART (8 * 16 * 8)
-#define MS_BLOCK 8192
+// fill its ring with weights while the first one still works, and waits only for the rows.
+#define MS_WARPS 16
+#define MS_ROWS 8
+#define MS_COLS 256               // columns of a block: eight a lane
+#define MS_BLOCK 2048             // bytes of a block: four rows
+template <int N> struct Rows { static constexpr int value = N; };
+__device__ __forceinline__ float lower_half(uint32_t two) { return __uint_as_float(two << 16); }
+__device__ __forceinline__ float upper_half(uint32_t two) { return __uint_as_float(two & 0xffff0000u); }
+__device__ __forceinline__ float2 fma_both(float a, const float2 &x, const float2 &acc) {      // each half rounded by itself
+  float2 r;
+  asm("{\n\t.reg .b64 ra, rx, rc;\n\tmov.b64 ra, {%2, %2};\n\tmov.b64 rx, {%3, %4};\n\tmov.b64 rc, {%5, %6};\n\t"
+      "fma.rn.f32x2 rc, ra, rx, rc;\n\tmov.b64 {%0, %1}, rc;\n\t}\n"
+      : "=f"(r.x), "=f"(r.y) : "f"(a), "f"(x.x), "f"(x.y), "f"(acc.x), "f"(acc.y));
+  return r;
+}
+// dot_chunk of four matrix rows and 2 PAIRS rows x, two of them an instruction; acc[p][j]: rows 2p and 2p + 1 against matrix row j
+template <int PAIRS>
+__device__ __forceinline__ void dot_chunks(const uint4 (&w)[4], const bf16 *x, int xrow, float2 (&acc)[PAIRS][4]) {
+  uint32_t xx[2 * PAIRS][4];
+#pragma unroll
+  for (int m = 0; m < 2 * PAIRS; ++m) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(x + (size_t)m * xrow);
+    xx[m][0] = v.x, xx[m][1] = v.y, xx[m][2] = v.z, xx[m][3] = v.w;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      float ww[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t raw = i == 0 ? w[j].x : i == 1 ? w[j].y : i == 2 ? w[j].z : w[j].w;
+        ww[j] = half ? upper_half(raw) : lower_half(raw);
+      }
+#pragma unroll
+      for (int p = 0; p < PAIRS; ++p) {
+        const float2 xp = half ? make_float2(upper_half(xx[2 * p][i]), upper_half(xx[2 * p + 1][i]))
+                               : make_float2(lower_half(xx[2 * p][i]), lower_half(xx[2 * p + 1][i]));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[p][j] = fma_both(ww[j], xp, acc[p][j]);
+      }
+    }
+}
+
+// The sums of N values (a power of two up to 32) over a warp, in warp_sum's tree: value i ends in the lanes whose bits from the
+// highest on are i's.
+template <int N>
+__device__ __forceinline__ float sums_over_warp(float (&v)[N], int lane) {
+  int n = N;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i)
+        if (i < n) {
+          const bool upper = lane & o;
+          const float keep = upper ? v[i + n] : v[i], send = upper ? v[i] : v[i + n];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return v[0];
+}
+
 template <bool SWIGLU, int RING>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(MS_WARPS * 32, 1)
 moe_stream_kernel(const bf16 *A, int a_stride, const int *row_pair, int pairs_per_token, int gather, const bf16 *__restrict__ W, int N,
                   int K, const int *plan, int n_real, void *out, int out_f32, GluForm glu, int plan_stands) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int warp_units[8];
-  const int nkb = (K + MS_KB - 1) / MS_KB, xrow = nkb * MS_KB + MS_PAD;
-  const uint32_t ring = smem_u32(smem_raw) + threadIdx.x * 16;
-  float *red = reinterpret_cast<float *>(smem_raw + RING * MS_BLOCK);                       // [2][8 warps][16][8]
-  bf16 *xs = reinterpret_cast<bf16 *>(smem_raw + RING * MS_BLOCK + 2 * MS_PART * sizeof(float));      // [8][xrow]
-  int *ustart = reinterpret_cast<int *>(xs + (size_t)8 * xrow);                             // [n_real + 1]: units in front of an expert
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
-  const int w_rows = SWIGLU ? 2 * N : N, tiles = (w_rows + 15) / 16, kw = 32 * warp + 8 * c;
+  __shared__ int warp_units[MS_WARPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nkb = (K + MS_COLS - 1) / MS_COLS, xrow = nkb * MS_COLS;
+  const uint32_t ring = smem_u32(smem_raw) + warp * (RING * MS_BLOCK) + lane * 16, ring_end = ring + RING * MS_BLOCK;
+  bf16 *xs = reinterpret_cast<bf16 *>(smem_raw + MS_WARPS * RING * MS_BLOCK);                // [8][xrow]
+  int *ustart = reinterpret_cast<int *>(xs + (size_t)MS_ROWS * xrow);                       // [n_real + 1]: units in front of an expert
+  const int w_rows = SWIGLU ? 2 * N : N, quads = SWIGLU ? N / 2 : (N + 3) / 4;
   if (!plan_stands) pdl_wait();
   pdl_launch();
   int before = 0;
-  for (int e0 = 0; e0 < n_real; e0 += 256) {
+  for (int e0 = 0; e0 < n_real; e0 += MS_WARPS * 32) {
     const int e = e0 + threadIdx.x;
-    const int mine = e < n_real ? (__ldcg(plan + 2 + e) - __ldcg(plan + 1 + e) + 7) / 8 : 0;
+    const int mine = e < n_real ? (__ldcg(plan + 2 + e) - __ldcg(plan + 1 + e) + MS_ROWS - 1) / MS_ROWS : 0;
     int upto = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -714,7 +779,7 @@ moe_stream_kernel(const bf16 *A, int a_stride, const int *row_pair, int pairs_pe
     __syncthreads();
     int all = 0;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) {
+    for (int w = 0; w < MS_WARPS; ++w) {
       if (w < warp) upto += warp_units[w];
       all += warp_units[w];
     }
@@ -724,7 +789,7 @@ moe_stream_kernel(const bf16 *A, int a_stride, const int *row_pair, int pairs_pe
   }
   if (threadIdx.x == 0) ustart[n_real] = before;
   __syncthreads();
-  const long long total = (long long)before * tiles;
+  const long long total = (long long)before * quads;
   const int t_begin = (int)(total * blockIdx.x / gridDim.x), t_end = (int)(total * (blockIdx.x + 1) / gridDim.x);
   if (t_begin >= t_end) {
     if (plan_stands) pdl_wait();                        // every kernel's end stands for the end of those in front
@@ -740,93 +805,108 @@ moe_stream_kernel(const bf16 *A, int a_stride, const int *row_pair, int pairs_pe
     return lo;
   };
   // ---- the weight stream
-  int p_t = t_begin, p_d = 0;
-  uint32_t p_slot = 0;
-  const bf16 *p_w0 = nullptr, *p_w1 = nullptr;
+  int p_t = t_begin + warp, p_unit = -1, p_k = lane * 8;
+  uint32_t put = ring;
+  const bf16 *p_matrix = nullptr, *p_w[4];
   auto aim = [&]() {
-    const int unit = p_t / tiles, n = (p_t - unit * tiles) * 16 + g;
-    const bf16 *We = W + (size_t)expert_of(unit) * w_rows * K;
-    p_w0 = We + (size_t)min(n, w_rows - 1) * K;
-    p_w1 = We + (size_t)min(n + 8, w_rows - 1) * K;
+    const int unit = p_t / quads, q = p_t - unit * quads;
+    if (unit != p_unit) p_matrix = W + (size_t)expert_of(unit) * w_rows * K + lane * 8;
+    p_unit = unit;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {                       // SWIGLU: rows in blocks of eight gates and their eight ups
+      const int row = SWIGLU ? (q >> 2) * 16 + (q & 3) * 2 + (j & 1) + 8 * (j >> 1) : min(4 * q + j, N - 1);
+      p_w[j] = p_matrix + (size_t)row * K;
+    }
   };
   auto issue = [&]() {                                  // one block (or nothing), one group
     if (p_t < t_end) {
-      const int k = p_d * MS_KB + kw;
-      if (k < K) {
-        cp_async_16(ring + p_slot * MS_BLOCK, p_w0 + k);
-        cp_async_16(ring + p_slot * MS_BLOCK + 4096, p_w1 + k);
-      }
-      if (++p_d == nkb) {
-        p_d = 0;
-        if (++p_t < t_end) aim();
+      if (p_k < K)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) cp_async_16(put + j * 512, p_w[j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) p_w[j] += MS_COLS;
+      p_k += MS_COLS;
+      if (p_k - lane * 8 >= K) {
+        p_k = lane * 8;
+        p_t += MS_WARPS;
+        if (p_t < t_end) aim();
       }
     }
     cp_async_commit();
-    p_slot = (p_slot + 1) % RING;
+    put += MS_BLOCK;
+    if (put == ring_end) put = ring;
   };
-  aim();
+  if (p_t < t_end) aim();
 #pragma unroll 1
   for (int i = 0; i < RING; ++i) issue();
   if (plan_stands) pdl_wait();
   // ---- the products
-  int staged = -1, rows = 0, r0 = 0;
-  uint32_t slot = 0;
-  for (int t = t_begin; t < t_end; ++t) {
-    const int unit = t / tiles;
-    if (unit != staged) {
-      staged = unit;
-      const int e = expert_of(unit);
-      r0 = plan[1 + e] + 8 * (unit - ustart[e]);
-      rows = min(8, plan[2 + e] - r0);
-      __syncthreads();                                  // the rows before are no longer read
-      bf16 *dst = xs + (size_t)warp * xrow;
-      const bf16 *src = A + (size_t)(warp < rows ? (gather ? row_pair[r0 + warp] / pairs_per_token : r0 + warp) : 0) * a_stride;
-      for (int k = lane * 8; k < xrow; k += 256)
-        *reinterpret_cast<uint4 *>(dst + k) = warp < rows && k < K ? *reinterpret_cast<const uint4 *>(src + k) : make_uint4(0, 0, 0, 0);
-      __syncthreads();
+  uint32_t get = ring;
+  int t = t_begin + warp;
+  for (int unit = t_begin / quads; unit * (long long)quads < t_end; ++unit) {
+    const int e = expert_of(unit), r0 = plan[1 + e] + MS_ROWS * (unit - ustart[e]), rows = min(MS_ROWS, plan[2 + e] - r0);
+    __syncthreads();                                    // the rows before are no longer read
+    for (int m = warp & 7; m < rows; m += MS_ROWS) {    // two warps a row
+      bf16 *dst = xs + (size_t)m * xrow;
+      const bf16 *src = A + (size_t)(gather ? row_pair[r0 + m] / pairs_per_token : r0 + m) * a_stride;
+      for (int k = ((warp >> 3) * 32 + lane) * 8; k < K; k += 512) *reinterpret_cast<uint4 *>(dst + k) = *reinterpret_cast<const uint4 *>(src + k);
     }
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int d = 0; d < nkb; ++d) {
-      cp_async_wait<RING - 1>();                        // this thread's copies of the block have landed
-      uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-      if (d * MS_KB + kw < K) {
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w) : "r"(ring + slot * MS_BLOCK));
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "r"(ring + slot * MS_BLOCK + 4096));
-      }
-      slot = (slot + 1) % RING;
-      const uint32_t a1[4] = {lo.x, hi.x, lo.y, hi.y}, a2[4] = {lo.z, hi.z, lo.w, hi.w};
-      const uint4 xv = *reinterpret_cast<const uint4 *>(xs + (size_t)g * xrow + d * MS_KB + kw);
-      mma_bf16_16816(acc, a1, xv.x, xv.y);
-      mma_bf16_16816(acc, a2, xv.z, xv.w);
-      issue();                                          // the slot just read is filled again
-    }
-    float *part = red + (t & 1) * MS_PART;
-    *reinterpret_cast<float2 *>(part + (warp * 16 + g) * 8 + 2 * c) = make_float2(acc[0], acc[1]);
-    *reinterpret_cast<float2 *>(part + (warp * 16 + g + 8) * 8 + 2 * c) = make_float2(acc[2], acc[3]);
     __syncthreads();
-    const int m = threadIdx.x >> 4, r = threadIdx.x & 15;
-    if (m < rows && (!SWIGLU || r < 8)) {
-      float v = 0.f, up = 0.f;
+    const int end = (int)min((long long)t_end, (unit + 1ll) * quads);
+    auto walk = [&](auto held) {
+      constexpr int HELD = decltype(held)::value, PAIRS = (HELD + 1) / 2, SUMS = 4 * HELD;      // HELD: 1, 2, 4 or 8
+      for (; t < end; t += MS_WARPS) {
+        float acc[SUMS];
+        float2 both[PAIRS][4];
 #pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        v += part[(w * 16 + r) * 8 + m];
-        if (SWIGLU) up += part[(w * 16 + 8 + r) * 8 + m];
+        for (int i = 0; i < 4; ++i) {
+          acc[i] = 0.f;
+#pragma unroll
+          for (int p = 0; p < PAIRS; ++p) both[p][i] = make_float2(0.f, 0.f);
+        }
+        const bf16 *x = xs + lane * 8;
+        for (int k = lane * 8; k - lane * 8 < K; k += MS_COLS, x += MS_COLS) {
+          cp_async_wait<RING - 1>();                    // this lane's copies of the block have landed
+          uint4 w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(w[j].x), "=r"(w[j].y), "=r"(w[j].z), "=r"(w[j].w) : "r"(get + j * 512));
+          get += MS_BLOCK;
+          if (get == ring_end) get = ring;
+          issue();                                      // the slot just read is filled again
+          if (k >= K) continue;
+          if (HELD == 1) {
+            const uint4 xv = *reinterpret_cast<const uint4 *>(x);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[j] = dot_chunk(w[j], xv, acc[j], bf16());
+          } else {
+            dot_chunks<PAIRS>(w, x, xrow, both);
+          }
+        }
+        if (HELD > 1)
+#pragma unroll
+          for (int i = 0; i < SUMS; ++i) acc[i] = i & 4 ? both[i >> 3][i & 3].y : both[i >> 3][i & 3].x;
+        float v = sums_over_warp(acc, lane);
+        const int value = lane / (32 / SUMS), m = value >> 2, j = value & 3, q = t - unit * quads;
+        if (SWIGLU) v = glu_value(v, __shfl_xor_sync(0xffffffffu, v, 2 * (32 / SUMS)), glu);
+        const int n = SWIGLU ? 2 * q + j : 4 * q + j;
+        if (lane % (32 / SUMS) == 0 && m < rows && n < N && (!SWIGLU || j < 2)) {
+          const size_t at = (size_t)(r0 + m) * N + n;
+          if (out_f32) ((float *)out)[at] = v;
+          else ((bf16 *)out)[at] = __float2bfloat16_rn(v);
+        }
       }
-      if (SWIGLU) v = glu_value(v, up, glu);
-      const int n = (t - unit * tiles) * (SWIGLU ? 8 : 16) + r;
-      const size_t at = (size_t)(r0 + m) * N + n;
-      if (n < N) {
-        if (out_f32) ((float *)out)[at] = v;
-        else ((bf16 *)out)[at] = __float2bfloat16_rn(v);
-      }
-    }
+    };
+    if (rows == 1) walk(Rows<1>());
+    else if (rows == 2) walk(Rows<2>());
+    else if (rows <= 4) walk(Rows<4>());
+    else walk(Rows<8>());
   }
   cp_async_wait<0>();
 }
 
 static size_t stream_smem(int ring, int K, int n_real) {
-  return (size_t)ring * MS_BLOCK + 2 * MS_PART * sizeof(float) + (size_t)8 * ((K + MS_KB - 1) / MS_KB * MS_KB + MS_PAD) * sizeof(bf16) +
-         (size_t)(n_real + 1) * sizeof(int);
+  return (size_t)MS_WARPS * ring * MS_BLOCK + (size_t)MS_ROWS * ((K + MS_COLS - 1) / MS_COLS * MS_COLS) * sizeof(bf16) + (size_t)(n_real + 1) * sizeof(int);
 }
 #define MS_SMEM_MOST (226 * 1024)
 template <bool SWIGLU, int RING>
@@ -839,8 +919,8 @@ static int launch_stream(const bf16 *A, int a_stride, const int *row_pair, int p
       G2B_REFUSE("moe_gemv: %d bytes of shared memory are not available", MS_SMEM_MOST);
     if (dev >= 0) done.value[dev] = 1;
   }
-  const long long tiles = ((SWIGLU ? 2 * N : N) + 15) / 16, most = tiles * n_rows;
-  g2b_launch(moe_stream_kernel<SWIGLU, RING>, dim3(most < 148 ? (unsigned)most : 148u), dim3(256), stream_smem(RING, K, n_real), stream, A,
+  const long long most = (SWIGLU ? N / 2 : (N + 3ll) / 4) * n_rows;
+  g2b_launch(moe_stream_kernel<SWIGLU, RING>, dim3(most < 148 ? (unsigned)most : 148u), dim3(MS_WARPS * 32), stream_smem(RING, K, n_real), stream, A,
              a_stride, row_pair, pairs_per_token, gather, W, N, K, plan, n_real, out, out_f32, glu, plan_stands);
   return g2b_check_launch("moe_gemv");
 }
@@ -872,11 +952,11 @@ extern "C" int g2b_moe_gemv(const void *A, int dtype, int a_stride, const int *r
   const int epl = dtype == G2B_BF16 ? 8 : 4;
   if (K % epl || a_stride % epl || (((uintptr_t)A | (uintptr_t)W) & 15))
     G2B_REFUSE("moe_gemv: K = %d or the rows' distance %d is no multiple of %d, or a pointer is off 16 bytes", K, a_stride, epl);
-  // a ring of 128 KB where the rows leave room for it (K up to about 5,000), else of 64
-  const long long line = (((swiglu ? 2ll : 1ll) * N + 15) / 16) * n_rows;
-  if (dtype == G2B_BF16 && (!swiglu || (blocked && N % 8 == 0)) && line < (1ll << 31) && stream_smem(8, K, n_real) <= MS_SMEM_MOST) {
-    const bool deep = stream_smem(16, K, n_real) <= MS_SMEM_MOST;
-    const auto launch = swiglu ? (deep ? launch_stream<true, 16> : launch_stream<true, 8>) : (deep ? launch_stream<false, 16> : launch_stream<false, 8>);
+  // a ring of 128 KB where the rows leave room for it (K up to about 6,000), else of 64 (up to about 10,000)
+  const long long line = (swiglu ? N / 2 : (N + 3ll) / 4) * n_rows;
+  if (dtype == G2B_BF16 && (!swiglu || (blocked && N % 8 == 0)) && line < (1ll << 31) - 1024 && stream_smem(2, K, n_real) <= MS_SMEM_MOST) {
+    const bool deep = stream_smem(4, K, n_real) <= MS_SMEM_MOST;
+    const auto launch = swiglu ? (deep ? launch_stream<true, 4> : launch_stream<true, 2>) : (deep ? launch_stream<false, 4> : launch_stream<false, 2>);
     return launch((const bf16 *)A, a_stride, row_pair, pairs_per_token, gather, (const bf16 *)W, N, K, plan, n_real, n_rows, out, out_f32, glu,
                   plan_stands, stream);
   }

@@ -83,3 +83,39 @@ def test_second_product_over_a_plan(T, top, E, hidden, inter):
             kernels.moe_combine(out, pair_row, ones, zeros, top, kept[i])
         got.append(kept)
     assert torch.equal(*got) and got[0].abs().sum() > 0
+
+
+@pytest.mark.parametrize("T,top,E,spread", [(1, 2, 4, 4), (9, 2, 3, 3), (16, 8, 16, 16), (12, 1, 2, 3), (21, 2, 5, 4)])
+@pytest.mark.parametrize("N,K", [(8, 8), (24, 264), (136, 2048), (16, 8200)])
+def test_bits_of_a_row_at_a_time(T, top, E, spread, N, K):
+    """The matrices streamed past all rows of their experts give the bits of the kernel that takes them row by row (which the
+    layout with all gates in front of all ups still takes)."""
+    from gguf2bin_b200 import kernels
+    idx = torch.randint(spread, (T, top), generator=torch.Generator().manual_seed(T + N)).to(torch.int32).to(DEV)
+    a, w = rnd(T, K, dtype=torch.bfloat16, seed=1), rnd(E, 2 * N, K, dtype=torch.bfloat16, seed=2)
+    w_blocked = w.view(E, 2, N // 8, 8, K).transpose(1, 2).contiguous().view(E, 2 * N, K)
+    plan, row_pair, _ = plan_of(idx, E)
+    outs = []
+    for matrix, blocked in ((w, False), (w_blocked, True)):
+        out = torch.full((T * top, N), float("nan"), device=DEV)
+        assert kernels.moe_gemv(a, row_pair, top, True, idx, matrix, N, plan, E, T * top, True, out, blocked)
+        outs.append(out[:int(plan[1 + E])])
+    assert torch.isfinite(outs[0]).all() and torch.equal(*outs)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 8])
+@pytest.mark.parametrize("K", [256, 768, 3072, 6000])
+def test_sums_are_rounded_to_nearest(rows, K):
+    """Positive products: sums rounded to nearest are off to either side.  One of a run's K / 32 additions is off by at most 2^-24 of
+    the run so far, so a sum by sqrt(K / 32) / 2 of these in the mean square at most, and the mean over 2,048 rows' and
+    columns' sums, were they to either side alike, by a 45th of that; six times as much is what chance leaves."""
+    from gguf2bin_b200 import kernels
+    N, idx = 2048, torch.zeros(rows, 1, dtype=torch.int32, device=DEV)
+    a, w = rnd(rows, K, dtype=torch.bfloat16, seed=1).abs(), rnd(1, N, K, dtype=torch.bfloat16, seed=2).abs()
+    plan, row_pair, pair_row = plan_of(idx, 1)
+    out = torch.empty(rows, N, device=DEV)
+    assert kernels.moe_gemv(a, row_pair, 1, True, idx, w, N, plan, 1, rows, False, out)
+    want = a.double() @ w[0].double().T
+    off = (out[pair_row.long()].double() - want) / want
+    assert off.square().mean().sqrt() <= (K / 32) ** 0.5 / 2 * 2.0 ** -24 + 2.0 ** -25
+    assert off.mean().abs() <= 6 * (K / 32) ** 0.5 / 2 * 2.0 ** -24 / 45
