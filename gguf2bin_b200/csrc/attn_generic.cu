@@ -166,7 +166,7 @@ attn_generic_kernel(const T *__restrict__ q, T *__restrict__ out, const T *__res
 // a page's keys (a segment) are brought to shared memory once and serve many rows.  A score is the sum of four partial
 // dot products (d mod 4, each in increasing d); a segment's scores have one maximum; its probabilities are added pairwise
 // by a warp (keys i and i + 32 first); its weighted values are added in the order of the keys; segments are merged one after
-// the other from the lowest.  Both kernels keep that order, so a row's result depends neither on the kernel nor on the batch.
+// the other from the lowest.  Both kernels keep that order, so a row's result does not depend on which of the two computes it.
 //
 //   tile    a block per (64 rows of one prompt, query head) that walks the segments: prompts
 //   split   a block per (token, kv head, segment), for all query heads of the kv head, and a merge: single tokens, whose
@@ -219,20 +219,27 @@ __device__ __forceinline__ void dot4(float4 &d, const float4 a, const float4 b) 
   d.z = fmaf(a.z, b.z, d.z);
   d.w = fmaf(a.w, b.w, d.w);
 }
-// One warp: a row's 64 scores in shared memory (-inf: not seen) become probabilities against their maximum.
-__device__ __forceinline__ void soften(float *row, int lane, float &m, float &l) {
-  const float a = row[lane], b = row[lane + 32];
+// One warp: a row's 64 scores in shared memory become probabilities against the maximum of those that the token at `pos` sees, and
+// HIDDEN where it does not.  What is hidden is decided by the positions alone: a score or a value that is NaN or infinite and
+// seen, whatever its weight, reaches the result.
+#define HIDDEN -1.f
+__device__ __forceinline__ void soften(const F32Attn &p, float *row, int lane, int seg, int pos, float &m, float &l) {
+  const int lo = lowest_key(p, pos), key = seg * SEG + lane;
+  const bool see_a = key <= pos && sees(p, lo, key), see_b = key + 32 <= pos && sees(p, lo, key + 32);
+  const float a = see_a ? row[lane] : -INFINITY, b = see_b ? row[lane + 32] : -INFINITY;
   m = warp_max(fmaxf(a, b));
   const float pa = a == -INFINITY ? 0.f : expf(a - m), pb = b == -INFINITY ? 0.f : expf(b - m);
-  row[lane] = pa;
-  row[lane + 32] = pb;
+  row[lane] = see_a ? pa : HIDDEN;
+  row[lane + 32] = see_b ? pb : HIDDEN;
   l = warp_sum(pa + pb);
 }
-// Adds a part (maximum m, times e) to a running one: the factors for what is there and for what comes.
+__device__ __forceinline__ bool hidden(float probability) { return probability < 0.f; }
+// Adds a part (maximum m_part) to a running one: the factors for what is there and for what comes.  Where the maxima are equal both
+// factors are 1, also in front of the first part and behind parts whose every score is -inf.
 __device__ __forceinline__ void merge_factors(float &m, float m_part, float &old_factor, float &new_factor) {
   const float m_new = fmaxf(m, m_part);
-  old_factor = expf(m - m_new);                                     // 0 in front of the first part
-  new_factor = expf(m_part - m_new);
+  old_factor = m == m_new ? 1.f : expf(m - m_new);
+  new_factor = m_part == m_new ? 1.f : expf(m_part - m_new);
   m = m_new;
 }
 __device__ __forceinline__ float merged(float there, float old_factor, float part, float new_factor) {
@@ -298,26 +305,18 @@ attn_f32_tile_kernel(F32Attn p) {
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty + 16 * i, pos = pos0 + r, lo = lowest_key(p, pos);
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int key = seg * SEG + tx + 16 * j;
-        Ps[r * (SEG + 4) + tx + 16 * j] = r < rows && key <= pos && sees(p, lo, key) ? scored(p, S[i][j]) : -INFINITY;
-      }
-    }
+      for (int j = 0; j < 4; ++j) Ps[(ty + 16 * i) * (SEG + 4) + tx + 16 * j] = scored(p, S[i][j]);
     __syncthreads();
     for (int r = warp; r < F32_TILE_ROWS; r += 8) {
-      float m, l;
-      soften(Ps + r * (SEG + 4), lane, m, l);
+      float m, l;                                                   // rows behind the last see nothing, like rows before a window
+      soften(p, Ps + r * (SEG + 4), lane, seg, r < rows ? pos0 + r : -1, m, l);
       if (lane == 0) {
-        float of = 1.f, nf = 0.f;                                   // nothing of the segment is seen: all stays
-        if (m != -INFINITY) {
-          float there = row_m[r];
-          merge_factors(there, m, of, nf);
-          row_m[r] = there;
-          row_l[r] = merged(row_l[r], of, l, nf);
-        }
+        float there = row_m[r], of, nf;
+        merge_factors(there, m, of, nf);
+        row_m[r] = there;
+        row_l[r] = merged(row_l[r], of, l, nf);
         old_f[r] = of;
         new_f[r] = nf;
       }
@@ -338,7 +337,7 @@ attn_f32_tile_kernel(F32Attn p) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float pr = Ps[(ty + 16 * i) * (SEG + 4) + key];
-        if (pr != 0.f)                                              // a value that is not seen is not touched, whatever it holds
+        if (!hidden(pr))                                            // a value that is not seen is not touched, whatever it holds
 #pragma unroll
           for (int j = 0; j < HD4; ++j)
             if (64 * j + 4 * tx < hd) {
@@ -352,14 +351,13 @@ attn_f32_tile_kernel(F32Attn p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float of = old_f[ty + 16 * i], nf = new_f[ty + 16 * i];
-      if (nf != 0.f || of != 1.f)
 #pragma unroll
-        for (int j = 0; j < HD4; ++j) {
-          O[i][j].x = merged(O[i][j].x, of, acc[i][j].x, nf);
-          O[i][j].y = merged(O[i][j].y, of, acc[i][j].y, nf);
-          O[i][j].z = merged(O[i][j].z, of, acc[i][j].z, nf);
-          O[i][j].w = merged(O[i][j].w, of, acc[i][j].w, nf);
-        }
+      for (int j = 0; j < HD4; ++j) {
+        O[i][j].x = merged(O[i][j].x, of, acc[i][j].x, nf);
+        O[i][j].y = merged(O[i][j].y, of, acc[i][j].y, nf);
+        O[i][j].z = merged(O[i][j].z, of, acc[i][j].z, nf);
+        O[i][j].w = merged(O[i][j].w, of, acc[i][j].w, nf);
+      }
     }
   }
 #pragma unroll
@@ -393,19 +391,19 @@ attn_f32_split_kernel(F32Attn p) {
   }
   asm volatile("cp.async.wait_group 1;\n" ::);
   __syncthreads();
-  const int j = tid & (SEG - 1), key = seg * SEG + j;
+  const int j = tid & (SEG - 1);
   for (int r = tid / SEG; r < group; r += 128 / SEG) {
     float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int c = 0; c < hd; c += 4) dot4(d, *(const float4 *)(Qs + r * pitch + c), *(const float4 *)(Ks + j * pitch + c));
-    Ps[r * (SEG + 4) + j] = key <= pos && sees(p, lo, key) ? scored(p, d) : -INFINITY;
+    Ps[r * (SEG + 4) + j] = scored(p, d);
   }
   __syncthreads();
   const size_t part_size = hd + F32_PART_EXTRA;
   float *part = p.parts + (((size_t)t * p.nh + kvh * group) * p.segments + seg) * part_size;
   for (int r = warp; r < group; r += 4) {
     float m, l;
-    soften(Ps + r * (SEG + 4), lane, m, l);
+    soften(p, Ps + r * (SEG + 4), lane, seg, pos, m, l);
     if (lane == 0) {
       part[r * p.segments * part_size] = m;
       part[r * p.segments * part_size + 1] = l;
@@ -420,7 +418,7 @@ attn_f32_split_kernel(F32Attn p) {
 #pragma unroll 8
     for (int k = 0; k < n_keys; ++k) {
       const float pr = Ps[r * (SEG + 4) + k];
-      if (pr != 0.f) acc = fmaf(pr, Vs[k * pitch + d], acc);
+      if (!hidden(pr)) acc = fmaf(pr, Vs[k * pitch + d], acc);
     }
     part[r * p.segments * part_size + F32_PART_EXTRA + d] = acc;
   }

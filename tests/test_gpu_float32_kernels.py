@@ -116,3 +116,62 @@ def test_attention_reads_no_value_that_is_not_seen(tiles):
     q, out = rnd(100, 64, seed=4), torch.empty(100, 64, device=DEV)
     assert kernels.attn_f32(q, out, cache, ctx_of(lens, q_lens, table, tiles), 1, 1, 64, 64, 0, 0.125)
     assert torch.isfinite(out[:99]).all() and torch.isnan(out[99]).all()
+
+
+def plain_attention(q, K, V, scale, see, sink):
+    """64-bit attention of one head: q [T, d], K and V [n, d], ``see`` [T, n]; ``sink`` a score or None."""
+    s = (q.double() @ K.double().T * scale).masked_fill(~see, -math.inf)
+    if sink is not None:
+        s = torch.cat([s, torch.full_like(s[:, :1], sink)], 1)
+    p = torch.softmax(s, 1)[:, :K.shape[0]]
+    out = torch.zeros(q.shape[0], V.shape[1], dtype=torch.float64, device=DEV)
+    for t in range(q.shape[0]):                         # hidden values are not touched; a weight of zero times infinity is NaN
+        out[t] = (p[t, see[t], None] * V.double()[see[t]]).sum(0)
+    return out
+
+
+SPECIALS = {
+    "queries": lambda q, K, V: [q.__setitem__(t, math.nan) for t in (0, 40, 62, 63, 64, 199)],
+    "own key": lambda q, K, V: K.__setitem__((64, 3), math.nan),
+    "a segment's keys": lambda q, K, V: K.__setitem__(slice(64, 128), math.nan),
+    "last keys of a segment": lambda q, K, V: K.__setitem__(slice(60, 64), math.nan),
+    "infinite value without weight": lambda q, K, V: (K.__setitem__(7, -1e6), V.__setitem__((7, 5), math.inf)),
+    "NaN value without weight": lambda q, K, V: (K.__setitem__(70, -1e6), V.__setitem__((70, 5), math.nan)),
+    "first segment at -inf": lambda q, K, V: K.__setitem__(slice(0, 64), -math.inf),
+    "a key at -inf": lambda q, K, V: K.__setitem__(64, -math.inf),
+    "a key at inf": lambda q, K, V: K.__setitem__(64, math.inf),
+}
+
+
+@pytest.mark.parametrize("what", SPECIALS)
+@pytest.mark.parametrize("sink", [None, 0.0])
+@pytest.mark.parametrize("options", [dict(), dict(window=37), dict(window=64, keep_first=3), dict(chunk=64)], ids=lambda o: "-".join(o) or "plain")
+def test_attention_keeps_nan_and_infinities_that_are_seen(what, sink, options):
+    """A score or a value that is seen and not finite reaches its row, whichever keys of its segment are hidden; everything else
+    stays finite: both kernels alike, the pattern and the values of 64-bit attention."""
+    from gguf2bin_b200 import kernels
+    n, hd = 200, 64
+    cache, table, Ks, Vs = make_paged(1, [n], 1, hd, 64, torch.float32, seed=3)
+    q, K, V = rnd(n, hd, seed=4).abs(), Ks[0][:, 0].abs().clone(), Vs[0][:, 0].clone()
+    SPECIALS[what](q, K, V)
+    for p in range(-(-n // 64)):
+        rows = min(64, n - 64 * p)
+        cache[int(table[0, p]), 0, 0, :rows], cache[int(table[0, p]), 1, 0, :rows] = K[64 * p:64 * p + rows], V[64 * p:64 * p + rows]
+    t, key = torch.arange(n, device=DEV)[:, None], torch.arange(n, device=DEV)[None]
+    window, chunk = options.get("window", 0), options.get("chunk", 0)
+    lo = t // chunk * chunk if chunk else (t - window + 1).clamp(min=0) if window else torch.zeros_like(t)
+    see = (key <= t) & ((key >= lo) | (key < options.get("keep_first", 0)))
+    want = plain_attention(q, K, V, 0.125, see, sink)
+    outs = []
+    for tiles in (True, False):
+        out = torch.empty(n, hd, device=DEV)
+        more = {k: v for k, v in options.items() if k != "window"}
+        assert kernels.attn_f32(q, out, cache, ctx_of([n], [n], table, tiles), 1, 1, hd, 64, window, 0.125,
+                                None if sink is None else torch.full((1,), sink, device=DEV), **more)
+        outs.append(out)
+    assert torch.equal(outs[0].nan_to_num(nan=1e30), outs[1].nan_to_num(nan=1e30))
+    bad = ~torch.isfinite(want)
+    assert torch.equal(~torch.isfinite(outs[0]), bad)
+    # scores of at most 64 x 0.125 x 16 = 128, as in test_attention_tiles_and_segments
+    score = (hd + 2) * EPS * 128
+    assert (outs[0].double() - want)[~bad].abs().max() <= 2 * (2 * score + 400 * EPS) * V[torch.isfinite(V)].abs().max()
