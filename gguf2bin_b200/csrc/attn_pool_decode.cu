@@ -136,16 +136,17 @@ attn_pool_decode_kernel(const bf16 *__restrict__ q, bf16 *__restrict__ out, cons
       float mx = -INFINITY;
       for (int r = lane; r < n_here; r += 32) mx = fmaxf(mx, sc[warp][r]);
       const float m_old = s_m[warp];
-      const float m_new = fmaxf(m_old, warp_max(mx));  // finite: the pass has an entry
+      // -inf where every score so far is (a run may have a single entry): such an entry has no weight, wherever the others are
+      const float m_new = fmaxf(m_old, warp_max(mx));
       float sum = 0.f;
       for (int r = lane; r < n_here; r += 32) {
-        const float p = expf(sc[warp][r] - m_new);
+        const float p = sc[warp][r] == -INFINITY ? 0.f : expf(sc[warp][r] - m_new);
         sc[warp][r] = p;
         sum += p;
       }
       sum = warp_sum(sum);
       if (lane == 0) {
-        const float corr = expf(m_old - m_new);        // 0 in the first pass
+        const float corr = m_old == m_new ? 1.f : expf(m_old - m_new);      // 0 in the first pass
         s_corr[warp] = corr;
         s_l[warp] = s_l[warp] * corr + sum;
         s_m[warp] = m_new;
@@ -217,11 +218,11 @@ attn_pool_decode_kernel(const bf16 *__restrict__ q, bf16 *__restrict__ out, cons
   #pragma unroll
       for (int r = 0; r < SPLIT; ++r) {
         m[r] = cluster.map_shared_rank(s_m, r)[g];
-        top = fmaxf(top, m[r]);                          // finite: a run has the token's own key
+        top = fmaxf(top, m[r]);
       }
   #pragma unroll
       for (int r = 0; r < SPLIT; ++r) {
-        const float f = expf(m[r] - top);                // 0 for a run without entries
+        const float f = m[r] == top ? 1.f : expf(m[r] - top);      // 0 for a run without entries
         l = fmaf(cluster.map_shared_rank(s_l, r)[g], f, l);
         sum = fmaf(cluster.map_shared_rank(&red[0][0][0], r)[idx], f, sum);
       }

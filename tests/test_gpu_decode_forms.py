@@ -1,5 +1,6 @@
 """The decode steps' forms of kernels (vectors, runs shared by clusters) against the same sums in 64 bits, and against the
 general form, which the same rows a step apart that no vector fits take."""
+import math
 from types import SimpleNamespace
 
 import pytest
@@ -112,6 +113,25 @@ def test_pooled_entries_in_runs(hd, T, nh, nkv, window, pool):
         qt = q[t].double().view(nkv, nh // nkv, hd)
         a = torch.softmax(torch.einsum("kgd,ked->kge", qt, kv[0]) * hd ** -0.5, -1)
         near(out[t].view(nkv, nh // nkv, hd), torch.einsum("kge,ked->kgd", a, kv[1]), torch.bfloat16, 16 * torch.einsum("kge,ked->kgd", a, kv[1].abs()))
+
+
+@pytest.mark.parametrize("keys,nan", [([1], False), ([0, 1], False), ([0, 2, 3], False), ([3], False), ([0, 1, 2, 3], True)])
+@pytest.mark.parametrize("T", [1, 150])
+def test_pooled_runs_of_infinite_scores(keys, nan, T):
+    """A key whose score is -inf has no weight, also where it is the only entry of its run (four entries, four CTAs; 150 tokens go without runs)."""
+    from gguf2bin_b200 import kernels_bf16
+    cache, pooled = rnd(T, 2, 1, 64, 64, dtype=torch.bfloat16, seed=1), rnd(T, 2, 1, 4, 64, dtype=torch.bfloat16, seed=2)
+    cache[:, 0, :, keys] = -math.inf
+    ctx = SimpleNamespace(all_single=True, tok_pos=torch.full((T,), 3, dtype=torch.int32, device=DEV), tok_seq=torch.arange(T, dtype=torch.int32, device=DEV),
+                          page_table=torch.arange(T, dtype=torch.int32, device=DEV)[:, None])
+    q, out = rnd(T, 64, dtype=torch.bfloat16, seed=4).abs() + 0.1, torch.empty(T, 64, dtype=torch.bfloat16, device=DEV)
+    assert kernels_bf16.attention_pooled_bf16(q, out, cache, pooled, ctx, 1, 1, 64, 64, 64, 16, 0.125)
+    k, v = cache[:, 0, 0, :4].double(), cache[:, 1, 0, :4].double()
+    a = torch.softmax(torch.einsum("td,ted->te", q.double(), k) * 0.125, -1)
+    want = torch.einsum("te,ted->td", a, v)
+    assert torch.isnan(want).all() == nan and torch.equal(torch.isnan(out), torch.isnan(want))
+    if not nan:
+        near(out, want, torch.bfloat16, 16 * torch.einsum("te,ted->td", a, v.abs()))
 
 
 @pytest.mark.parametrize("nh,nkv,nvh,D,V,rot,interleaved", [(1, 1, 1, 4, 4, 4, True), (5, 2, 2, 20, 12, 8, False), (20, 4, 4, 128, 128, 128, False),
