@@ -80,10 +80,13 @@ __device__ __forceinline__ float2 two_floats(double x) {
   const float hi = (float)x;
   return make_float2(hi, (float)(x - (double)hi));
 }
-__device__ __forceinline__ float4 carry4(const float4 &a, float2 f, const float4 &b) {       // f a + b
-  return make_float4(fmaf(f.x, a.x, fmaf(f.y, a.x, b.x)), fmaf(f.x, a.y, fmaf(f.y, a.y, b.y)), fmaf(f.x, a.z, fmaf(f.y, a.z, b.z)),
-                     fmaf(f.x, a.w, fmaf(f.y, a.w, b.w)));
+__device__ __forceinline__ float carry1(float a, float2 f, float b) {         // f a + b; what f's rounding left changes no infinite a
+  return fmaf(f.x, a, fmaf(f.y, isinf(a) ? 0.f : a, b));
 }
+__device__ __forceinline__ float4 carry4(const float4 &a, float2 f, const float4 &b) {
+  return make_float4(carry1(a.x, f, b.x), carry1(a.y, f, b.y), carry1(a.z, f, b.z), carry1(a.w, f, b.w));
+}
+__device__ __forceinline__ float4 sum4(const float4 &a, const float4 &b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 template <typename T, bool OUT>
 __global__ void __launch_bounds__(THREADS, OUT ? 1 : 2)
@@ -337,7 +340,7 @@ chunk_segment_kernel(const ChunkArgs a) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int m = 0; m < 2; ++m) st[i][m] = carry4(st[i][m], tb ? make_float2(1.f, 0.f) : f2, sum[i][m]);
+          for (int m = 0; m < 2; ++m) st[i][m] = tb ? sum4(st[i][m], sum[i][m]) : carry4(st[i][m], f2, sum[i][m]);
       }
     }
     __syncthreads();                                     // g, tail, S and P are written again
@@ -677,7 +680,7 @@ delta_walk_kernel(const DeltaArgs a) {
           if (4 * dx + 64 * m < D) add4(sum[m], f, *reinterpret_cast<const float4 *>(K + j * pitch + 4 * dx + 64 * m));
       }
 #pragma unroll
-      for (int m = 0; m < 2; ++m) st[m] = carry4(st[m], jb ? make_float2(1.f, 0.f) : all, sum[m]);
+      for (int m = 0; m < 2; ++m) st[m] = jb ? sum4(st[m], sum[m]) : carry4(st[m], all, sum[m]);
     }
 #pragma unroll
     for (int m = 0; m < 2; ++m)

@@ -130,3 +130,23 @@ def test_later_values_reach_no_earlier_token():
     assert kernels._chunk_segment(T, 1, H, V, D)
     kernels.state_scan(q, k, v, state, ctx, out, H, H, D, V, decay=torch.tensor([0.9, 0.5], device=DEV))
     assert torch.isfinite(out[:150]).all() and not torch.isfinite(out[150]).any() and torch.isnan(out[171:]).all()
+
+
+def test_infinite_states_stay_infinite():
+    """Where nothing is negative, a value that is infinite makes its column of the state, and what is read from it, infinite for
+    good, over chunks and segments."""
+    from gguf2bin_b200 import kernels
+    from gguf2bin_b200.engine.workspace import Workspace
+    from types import SimpleNamespace
+    T, H, D, V = 500, 2, 32, 48
+    q, k, v = (rnd(T, n, seed=i).abs() + 0.1 for i, n in enumerate((H * D, H * D, H * V)))
+    v[70, 5], v[480, 50] = float("inf"), float("inf")
+    ctx = SimpleNamespace(seq_meta=torch.tensor([[0, T, 0, 0]], dtype=torch.int32, device=DEV), n_seqs=1, workspace=Workspace(DEV))
+    state, out = torch.zeros(1, H, V, D, device=DEV), torch.empty(T, H * V, device=DEV)
+    kernels.state_scan(q, k, v, state, ctx, out, H, H, D, V, decay=torch.tensor([0.9, 0.5], device=DEV))
+    want = torch.zeros(T, H * V, dtype=torch.bool, device=DEV)
+    want[70:, 5], want[480:, 50] = True, True
+    assert torch.equal(out == float("inf"), want) and torch.isfinite(out[~want]).all()
+    inf = torch.zeros(H, V, dtype=torch.bool, device=DEV)
+    inf[0, 5], inf[1, 2] = True, True
+    assert torch.equal((state[0] == float("inf")).all(-1), inf) and torch.isfinite(state[0][~inf]).all()
