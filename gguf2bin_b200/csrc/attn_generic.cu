@@ -253,6 +253,7 @@ __device__ __forceinline__ float last_factor(const F32Attn &p, int t, int h, flo
 }
 
 #define F32_TILE_ROWS 64
+template <bool B> struct Flag { static constexpr bool value = B; };
 template <int HD4>                                                  // float4 columns of a row per thread: ceil(hd / 64)
 __global__ void __launch_bounds__(256)
 attn_f32_tile_kernel(F32Attn p) {
@@ -328,26 +329,29 @@ attn_f32_tile_kernel(F32Attn p) {
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < HD4; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int n_keys = min(SEG, last_pos - seg * SEG + 1);
-    for (int key = 0; key < n_keys; ++key) {
-      float4 v[HD4];
+    auto weigh = [&](auto all_seen, int n_keys) {
+      for (int key = 0; key < n_keys; ++key) {
+        float4 v[HD4];
 #pragma unroll
-      for (int j = 0; j < HD4; ++j)
-        if (64 * j + 4 * tx < hd) v[j] = *(const float4 *)(Vs + key * pitch + 64 * j + 4 * tx);
+        for (int j = 0; j < HD4; ++j)
+          if (64 * j + 4 * tx < hd) v[j] = *(const float4 *)(Vs + key * pitch + 64 * j + 4 * tx);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float pr = Ps[(ty + 16 * i) * (SEG + 4) + key];
-        if (!hidden(pr))                                            // a value that is not seen is not touched, whatever it holds
+        for (int i = 0; i < 4; ++i) {
+          const float pr = Ps[(ty + 16 * i) * (SEG + 4) + key];
+          if (decltype(all_seen)::value || !hidden(pr))             // a value that is not seen is not touched, whatever it holds
 #pragma unroll
-          for (int j = 0; j < HD4; ++j)
-            if (64 * j + 4 * tx < hd) {
-              acc[i][j].x = fmaf(pr, v[j].x, acc[i][j].x);
-              acc[i][j].y = fmaf(pr, v[j].y, acc[i][j].y);
-              acc[i][j].z = fmaf(pr, v[j].z, acc[i][j].z);
-              acc[i][j].w = fmaf(pr, v[j].w, acc[i][j].w);
-            }
+            for (int j = 0; j < HD4; ++j)
+              if (64 * j + 4 * tx < hd) {
+                acc[i][j].x = fmaf(pr, v[j].x, acc[i][j].x);
+                acc[i][j].y = fmaf(pr, v[j].y, acc[i][j].y);
+                acc[i][j].z = fmaf(pr, v[j].z, acc[i][j].z);
+                acc[i][j].w = fmaf(pr, v[j].w, acc[i][j].w);
+              }
+        }
       }
-    }
+    };
+    if (rows == F32_TILE_ROWS && seg * SEG + SEG - 1 <= pos0 && seg * SEG >= lowest_key(p, last_pos)) weigh(Flag<true>(), SEG);
+    else weigh(Flag<false>(), min(SEG, last_pos - seg * SEG + 1));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float of = old_f[ty + 16 * i], nf = new_f[ty + 16 * i];
