@@ -3,21 +3,23 @@
 // with g, s numbers per token and head (or one g per head and s = 1).  seq_mix.cu has the recurrence as it stands; a prompt
 // of thousands of tokens is a chain of dependent steps there, whatever the GPU could do beside it.
 //
-// Here a sequence is cut into segments, a segment into chunks of 64 tokens, and inside a chunk the recurrence is products:
+// Here a sequence is cut into chunks of 64 tokens, and inside a chunk the recurrence is products:
 //   with D_ij = g_(j+1) ... g_i, c_i = g_0 ... g_i (from the chunk's start) and the state S at the chunk's start
 //   o_i = c_i (S q_i) + sum_(j<=i) (q_i . k_j) D_ij s_j v_j,      S' = c_last S + sum_j D_(last,j) s_j v_j k_j^T.
 // The decays are products of the g's themselves, in the order of the tokens (no logarithms, no quotients), so a g of zero is
-// exact.  They are taken in 64 bits and rounded once, and what carries a state over a chunk or a segment is a pair of floats: the
+// exact.  They are taken in 64 bits and rounded once, and what carries a state over a chunk is a pair of floats: the
 // rounding of one factor would fall on a whole state, again with every chunk.  All else is 32-bit multiply-adds, in sums of 16
 // that are added up, which rounds less than the chain of single tokens does (decay per head, 2,048 tokens, against 64 bits:
 // outputs 1.5e-7, states 1.2e-7, token by token 4.9e-7 and 5.7e-7; gates 0.9e-7 and 0.8e-7, 1.3e-7 and 0.9e-7).
-//   1. chunk_segment<false>: every segment by itself from a zero state: its own contribution, and the product of its g's
-//   2. chunk_carry: along a sequence, S at every segment's start from the contributions; the sequence's state in the end
-//   3. chunk_segment<true>: every segment from its start state: the outputs
-// A block of 256 threads takes a segment of one head and 64 columns; the state's share (64 x D) stays in registers (32 a
-// thread), q, k and v of the next chunk are on their way while one is computed.  Shared-memory reads bound it: 8 loads of 16
-// bytes feed 64 multiply-adds.  2,048 tokens, 8 heads of 128 x 256: 64 + 26 + 95 us (551 us as a chain); 1,501 tokens at
-// most in four sequences, 64 heads of 128 x 64 and 8 of 128 x 257, on average: 164 + 23 + 372 us (697 us).
+//   1. chunk_kernel<false>: every chunk by itself from a zero state: its own contribution, and the product of its g's
+//   2. chunk_carry: along a sequence, S at every chunk's start from the contributions; the sequence's state in the end
+//   3. chunk_kernel<true>: every chunk from its start state: the outputs
+// A block of 256 threads takes a chunk of one head and 64 columns.  Shared-memory reads bound it: 8 loads of 16
+// bytes feed 64 multiply-adds.  2,048 tokens, 8 heads of 128 x 256: 184 us (486 us as a chain), four prompts of 203 to 1,501 tokens, 64 heads of
+// 128 x 64: 641 us (889).  Chunks grouped into segments of up to 256 tokens, whose states alone went through memory: 189 and 709 us.
+//
+// Which sequences of a step come here is the caller's rule: those of more than `over` tokens, and sequence `pad`.  Of the
+// others nothing is read or written.
 #include "common.cuh"
 
 G2B_DEFINE_LAST_ERROR
@@ -28,6 +30,16 @@ G2B_DEFINE_LAST_ERROR
 #define MAX_D 128
 #define P_PITCH (CHUNK + 4)
 
+struct Members {
+  const int *meta;            // [n_seqs, 4]: first row, tokens, past, slot
+  int n_seqs, over, pad;
+  // chunks of `size` tokens of sequence b
+  __device__ __forceinline__ int chunks(int b, int size) const {
+    const int n = meta[4 * b + 1];
+    return n > over || b == pad ? (n + size - 1) / size : 0;
+  }
+};
+
 struct ChunkArgs {
   const float *qf, *kf;       // [T, G, D] prepared
   const void *v;              // compute type, rows of a wider buffer
@@ -35,19 +47,18 @@ struct ChunkArgs {
   const float *decay;         // [H], or null:
   const float *gates;         // [T, 2H]: g, then s
   float *state;               // [slots, H, V, D]
-  const int *seq_meta;
-  int n_seqs, seg;            // tokens of a segment, a multiple of CHUNK
-  float *parts;               // [segments, H, V, D]: contributions, then start states
-  float2 *part_decay;         // [segments, H]: the product of the g's, and what its rounding left
+  Members seqs;
+  float *parts;               // [chunks, H, V, D]: contributions, then start states
+  float2 *part_decay;         // [chunks, H]: the product of the g's, and what its rounding left
   float *out;                 // [T, H*V]
 };
 
-// The sequence and the place in it of segment `idx` of the step (sequences one after another); false behind the last one.
-__device__ __forceinline__ bool find_segment(const int *meta, int n_seqs, int seg, int idx, int &b, int &place) {
+// The sequence and the place in it of chunk `idx` of the step (sequences one after another); false behind the last one.
+__device__ __forceinline__ bool find_chunk(const Members &seqs, int size, int idx, int &b, int &place) {
   const int lane = threadIdx.x & 31;
   int before = 0;
-  for (int b0 = 0; b0 < n_seqs; b0 += 32) {
-    const int mine = b0 + lane < n_seqs ? (meta[4 * (b0 + lane) + 1] + seg - 1) / seg : 0;
+  for (int b0 = 0; b0 < seqs.n_seqs; b0 += 32) {
+    const int mine = b0 + lane < seqs.n_seqs ? seqs.chunks(b0 + lane, size) : 0;
     int upto = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -64,6 +75,17 @@ __device__ __forceinline__ bool find_segment(const int *meta, int n_seqs, int se
     before += __shfl_sync(0xffffffffu, upto, 31);
   }
   return false;
+}
+// Chunks of the sequences in front of b; every lane has the sum.
+__device__ __forceinline__ int chunks_before(const Members &seqs, int size, int b, int lane) {
+  int before = 0;
+  for (int b0 = 0; b0 < b; b0 += 32) {
+    int c = b0 + lane < b ? seqs.chunks(b0 + lane, size) : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    before += c;
+  }
+  return before;
 }
 
 __device__ __forceinline__ void copy16(float *dst, const float *src) {
@@ -90,303 +112,258 @@ __device__ __forceinline__ float4 sum4(const float4 &a, const float4 &b) { retur
 
 template <typename T, bool OUT>
 __global__ void __launch_bounds__(THREADS, OUT ? 1 : 2)
-chunk_segment_kernel(const ChunkArgs a) {
+chunk_kernel(const ChunkArgs a) {
   pdl_launch();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, col0 = blockIdx.x * COLS;
   int b, place;
-  if (!find_segment(a.seq_meta, a.n_seqs, a.seg, blockIdx.z, b, place)) return;
-  const int first = a.seq_meta[4 * b] + place * a.seg, n = min(a.seg, a.seq_meta[4 * b + 1] - place * a.seg);
+  if (!find_chunk(a.seqs, CHUNK, blockIdx.z, b, place)) return;
+  const int first = a.seqs.meta[4 * b] + place * CHUNK, n = min(CHUNK, a.seqs.meta[4 * b + 1] - place * CHUNK);
   const int qk_head = h / (H / a.G), tid = threadIdx.x;
-  float *K = sm, *Vs = K + 2 * CHUNK * pitch;            // two buffers of K and of V
+  float *K = sm, *Vs = K + CHUNK * pitch;
   // decays and strengths of the chunk's tokens; from the token on: to the end of its sixteen, of the chunk times its strength;
   // up to the token: from its sixteen's start; the sixteens' products; in_block[B][i][j] = D_ij inside sixteen B
-  double *tail16 = reinterpret_cast<double *>(Vs + 2 * CHUNK * COLS), *head = tail16 + CHUNK, *block = head + CHUNK;
+  double *tail16 = reinterpret_cast<double *>(Vs + CHUNK * COLS), *head = tail16 + CHUNK, *block = head + CHUNK;
   float *g = reinterpret_cast<float *>(block + 4), *s = g + CHUNK, *tail = s + CHUNK, *in_block = tail + CHUNK;
-  float *Q = in_block + CHUNK * 17, *S = Q + 2 * CHUNK * pitch, *P = S + COLS * pitch;            // OUT only
+  float *Q = in_block + CHUNK * 17, *S = Q + CHUNK * pitch, *P = S + COLS * pitch;            // OUT only
+  float *part = a.parts + ((size_t)blockIdx.z * H + h) * ((size_t)V * D);
+  for (int i = tid; i < CHUNK * (D / 4); i += THREADS) {
+    const int r = i / (D / 4), c = i % (D / 4) * 4;
+    float *kd = K + r * pitch + c, *qd = Q + r * pitch + c, *sd = S + r * pitch + c;
+    const size_t at = ((size_t)(first + r) * a.G + qk_head) * D + c;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < n) {
+      copy16(kd, a.kf + at);
+      if (OUT) copy16(qd, a.qf + at);
+    } else {
+      *reinterpret_cast<float4 *>(kd) = zero;
+      if (OUT) *reinterpret_cast<float4 *>(qd) = zero;
+    }
+    if (OUT) {                                           // column col0 + r of the state at the chunk's start
+      if (col0 + r < V) copy16(sd, part + (size_t)(col0 + r) * D + c);
+      else *reinterpret_cast<float4 *>(sd) = zero;
+    }
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+  {
+    const int c = col0 + (tid & 63);
+    const T *vg = (const T *)a.v;
+    T rv[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {                       // nothing here waits for a load
+      const int r = (tid >> 6) + 4 * i;
+      rv[i] = from_f32<T>(c < V && c >= a.Vin ? 1.f : 0.f);
+      if (r < n && c < a.Vin) rv[i] = vg[(size_t)(first + r) * a.v_stride + (size_t)h * a.Vin + c];
+    }
+    if (tid < CHUNK) {
+      float rg = 1.f, rs = tid < n ? 1.f : 0.f;
+      if (tid < n) {
+        const size_t at = (size_t)(first + tid) * 2 * H + h;
+        if (a.decay) rg = a.decay[h];
+        else rg = a.gates[at], rs = a.gates[at + H];
+      }
+      g[tid] = rg;
+      s[tid] = rs;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) Vs[((tid >> 6) + 4 * i) * COLS + (tid & 63)] = to_f32(rv[i]);
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  if (tid < CHUNK) {                                     // the decays from token `tid` on, to the end of its sixteen
+    const int b16 = tid & ~15, j = tid & 15;
+    double d = 1.0;
+    in_block[tid * 17 + j] = 1.f;                        // row i of its sixteen: in_block[(b16 + i) * 17 + j]
+    if (j == 0) head[tid] = g[tid];
+    for (int i = j + 1; i < 16; ++i) {
+      d *= g[b16 + i];
+      in_block[(b16 + i) * 17 + j] = (float)d;
+      if (j == 0) head[b16 + i] = g[b16] * d;
+    }
+    tail16[tid] = d;
+    if (j == 0) block[tid >> 4] = g[b16] * d;
+  }
+  if (OUT) {
+    const int tx = tid & 15, ty = tid >> 4;              // tokens ty + 16 i, columns (or keys) tx + 16 j
+    float p[4][4], o[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) p[i][j] = o[i][j] = 0.f;
+#pragma unroll 1
+    for (int d0 = 0; d0 < D; d0 += 16) {
+      float p16[4][4], o16[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p16[i][j] = o16[i][j] = 0.f;
+      const int d1 = min(d0 + 16, D);
+#pragma unroll 2
+      for (int d = d0; d < d1; d += 4) {
+        float4 q[4], k[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4 *>(Q + (ty + 16 * i) * pitch + d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(K + (tx + 16 * j) * pitch + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j <= i) p16[i][j] = dot4(q[i], k[j], p16[i][j]);   // later keys are not seen
+#pragma unroll
+        for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(S + (tx + 16 * j) * pitch + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o16[i][j] = dot4(q[i], k[j], o16[i][j]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[i][j] += p16[i][j], o[i][j] += o16[i][j];
+    }
+    __syncthreads();                                     // all decays stand
+    double before = 1.0;                                 // the sixteens in front
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = ty + 16 * i;
+      const double up = head[r];
+      const float from_start = (float)(before * up);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[i][j] *= from_start;
+      before *= block[i];
+      double between = up;                               // the sixteens between the key's and the row's, and the row's up to it
+#pragma unroll
+      for (int j = 3; j >= 0; --j) {
+        if (j > i) continue;
+        const int t = tx + 16 * j;
+        if (j == i) {
+          p[i][j] = tx <= ty ? p[i][j] * (in_block[r * 17 + tx] * s[t]) : 0.f;
+        } else {
+          p[i][j] *= (float)(tail16[t] * between * (double)s[t]);
+          between *= block[j];
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) P[(ty + 16 * i) * P_PITCH + tx + 16 * j] = p[i][j];
+    __syncwarp();                                        // a row's 16 threads are one half of a warp
+    // sixteen tokens at a time, for the rows that see them; later values are not touched, whatever they hold
+#pragma unroll
+    for (int tb = 0; tb < 4; ++tb) {
+      float o16[4][4];
+#pragma unroll
+      for (int i = tb; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o16[i][j] = 0.f;
+#pragma unroll 1
+      for (int t = 16 * tb; t < 16 * tb + 16; t += 4) {
+        float x[4][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) x[e][j] = Vs[(t + e) * COLS + tx + 16 * j];
+#pragma unroll
+        for (int i = tb; i < 4; ++i) {
+          const int r = ty + 16 * i;
+          const float4 w = *reinterpret_cast<const float4 *>(P + r * P_PITCH + t);
+          const bool all = i > tb;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (all || t <= r) o16[i][j] = fmaf(w.x, x[0][j], o16[i][j]);
+            if (all || t + 1 <= r) o16[i][j] = fmaf(w.y, x[1][j], o16[i][j]);
+            if (all || t + 2 <= r) o16[i][j] = fmaf(w.z, x[2][j], o16[i][j]);
+            if (all || t + 3 <= r) o16[i][j] = fmaf(w.w, x[3][j], o16[i][j]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = tb; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[i][j] += o16[i][j];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int r = ty + 16 * i, c = col0 + tx + 16 * j;
+        if (r < n && c < V) a.out[(size_t)(first + r) * H * V + (size_t)h * V + c] = o[i][j];
+      }
+    return;
+  }
+  __syncthreads();                                       // all decays stand
+  if (tid < CHUNK) {
+    double f = (double)s[tid] * tail16[tid];
+    for (int B = (tid >> 4) + 1; B < 4; ++B) f *= block[B];
+    tail[tid] = (float)f;
+  }
+  __syncthreads();                                       // `tail` stands
   // this thread's share of the state: columns 4 vy .. + 3, entries 4 dx .. + 3 and 64 further
   const int dx = tid & 15, vy = tid >> 4;
-  const size_t head_state = (size_t)V * D;
-  float *part = a.parts + ((size_t)blockIdx.z * H + h) * head_state;
   float4 st[4][2];
+#pragma unroll 1
+  for (int tb = 0; tb < n; tb += 16) {
+    float4 sum[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) sum[i][m] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int t1 = min(tb + 16, n);
+#pragma unroll 4
+    for (int t = tb; t < t1; ++t) {
+      const float f = tail[t];
+      const float4 x = *reinterpret_cast<const float4 *>(Vs + t * COLS + 4 * vy);
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+        if (4 * dx + 64 * m < D) {
+          const float4 k = *reinterpret_cast<const float4 *>(K + t * pitch + 4 * dx + 64 * m);
+          add4(sum[0][m], f * x.x, k);
+          add4(sum[1][m], f * x.y, k);
+          add4(sum[2][m], f * x.z, k);
+          add4(sum[3][m], f * x.w, k);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) st[i][m] = tb ? sum4(st[i][m], sum[i][m]) : sum[i][m];
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
       const int c = col0 + 4 * vy + i, d = 4 * dx + 64 * m;
-      st[i][m] = OUT && c < V && d < D ? *reinterpret_cast<const float4 *>(part + (size_t)c * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < V && d < D) *reinterpret_cast<float4 *>(part + (size_t)c * D + d) = st[i][m];
     }
-  double whole = 1.0;                                    // the product of the segment's g's
-  const T *vg = (const T *)a.v;
-  T rv[16];                                              // the next chunk's values, decay and strength, on their way
-  float rg = 1.f, rs = 0.f;
-  auto fetch = [&](int t0, int buf) {
-    const int nt = min(CHUNK, n - t0);
-    for (int i = tid; i < CHUNK * (D / 4); i += THREADS) {
-      const int r = i / (D / 4), c = i % (D / 4) * 4;
-      float *kd = K + (buf * CHUNK + r) * pitch + c, *qd = Q + (buf * CHUNK + r) * pitch + c;
-      const size_t at = ((size_t)(first + t0 + r) * a.G + qk_head) * D + c;
-      if (r < nt) {
-        copy16(kd, a.kf + at);
-        if (OUT) copy16(qd, a.qf + at);
-      } else {
-        *reinterpret_cast<float4 *>(kd) = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (OUT) *reinterpret_cast<float4 *>(qd) = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-    const int c = col0 + (tid & 63);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {                       // nothing here waits for a load
-      const int r = (tid >> 6) + 4 * i;
-      rv[i] = from_f32<T>(c < V && c >= a.Vin ? 1.f : 0.f);
-      if (r < nt && c < a.Vin) rv[i] = vg[(size_t)(first + t0 + r) * a.v_stride + (size_t)h * a.Vin + c];
-    }
-    if (tid < CHUNK) {
-      rg = 1.f;
-      rs = tid < nt ? 1.f : 0.f;
-      if (tid < nt) {
-        const size_t at = (size_t)(first + t0 + tid) * 2 * H + h;
-        if (a.decay) rg = a.decay[h];
-        else rg = a.gates[at], rs = a.gates[at + H];
-      }
-    }
-  };
-  fetch(0, 0);
-  int buf = 0;
-  for (int t0 = 0; t0 < n; t0 += CHUNK, buf ^= 1) {
-    const int nt = min(CHUNK, n - t0);
-    const bool more = t0 + CHUNK < n;
-    float *Vc = Vs + buf * CHUNK * COLS;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) Vc[((tid >> 6) + 4 * i) * COLS + (tid & 63)] = to_f32(rv[i]);
-    if (tid < CHUNK) {
-      g[tid] = rg;
-      s[tid] = rs;
-    }
-    if (OUT)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-          if (4 * dx + 64 * m < D) *reinterpret_cast<float4 *>(S + (4 * vy + i) * pitch + 4 * dx + 64 * m) = st[i][m];
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-    if (more) fetch(t0 + CHUNK, buf ^ 1);
-    if (tid < CHUNK) {                                   // the decays from token `tid` on, to the end of its sixteen
-      const int b16 = tid & ~15, j = tid & 15;
-      double d = 1.0;
-      in_block[tid * 17 + j] = 1.f;                      // row i of its sixteen: in_block[(b16 + i) * 17 + j]
-      if (j == 0) head[tid] = g[tid];
-      for (int i = j + 1; i < 16; ++i) {
-        d *= g[b16 + i];
-        in_block[(b16 + i) * 17 + j] = (float)d;
-        if (j == 0) head[b16 + i] = g[b16] * d;
-      }
-      tail16[tid] = d;
-      if (j == 0) block[tid >> 4] = g[b16] * d;
-    }
-    const float *Kc = K + buf * CHUNK * pitch;
-    if (OUT) {
-      const int tx = tid & 15, ty = tid >> 4;            // tokens ty + 16 i, columns (or keys) tx + 16 j
-      const float *Qc = Q + buf * CHUNK * pitch;
-      float p[4][4], o[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) p[i][j] = o[i][j] = 0.f;
-#pragma unroll 1
-      for (int d0 = 0; d0 < D; d0 += 16) {
-        float p16[4][4], o16[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) p16[i][j] = o16[i][j] = 0.f;
-        const int d1 = min(d0 + 16, D);
-#pragma unroll 2
-        for (int d = d0; d < d1; d += 4) {
-          float4 q[4], k[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4 *>(Qc + (ty + 16 * i) * pitch + d);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(Kc + (tx + 16 * j) * pitch + d);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (j <= i) p16[i][j] = dot4(q[i], k[j], p16[i][j]); // later keys are not seen
-#pragma unroll
-          for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(S + (tx + 16 * j) * pitch + d);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) o16[i][j] = dot4(q[i], k[j], o16[i][j]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) p[i][j] += p16[i][j], o[i][j] += o16[i][j];
-      }
-      __syncthreads();                                   // all decays stand
-      if (tid < CHUNK) {
-        double f = (double)s[tid] * tail16[tid];
-        for (int B = (tid >> 4) + 1; B < 4; ++B) f *= block[B];
-        tail[tid] = (float)f;
-      }
-      double before = 1.0;                               // the sixteens in front
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = ty + 16 * i;
-        const double up = head[r];
-        const float from_start = (float)(before * up);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) o[i][j] *= from_start;
-        before *= block[i];
-        double between = up;                             // the sixteens between the key's and the row's, and the row's up to it
-#pragma unroll
-        for (int j = 3; j >= 0; --j) {
-          if (j > i) continue;
-          const int t = tx + 16 * j;
-          if (j == i) {
-            p[i][j] = tx <= ty ? p[i][j] * (in_block[r * 17 + tx] * s[t]) : 0.f;
-          } else {
-            p[i][j] *= (float)(tail16[t] * between * (double)s[t]);
-            between *= block[j];
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j <= i; ++j) P[(ty + 16 * i) * P_PITCH + tx + 16 * j] = p[i][j];
-      __syncwarp();                                      // a row's 16 threads are one half of a warp
-      // sixteen tokens at a time, for the rows that see them; later values are not touched, whatever they hold
-#pragma unroll
-      for (int tb = 0; tb < 4; ++tb) {
-        float o16[4][4];
-#pragma unroll
-        for (int i = tb; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) o16[i][j] = 0.f;
-#pragma unroll 1
-        for (int t = 16 * tb; t < 16 * tb + 16; t += 4) {
-          float x[4][4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) x[e][j] = Vc[(t + e) * COLS + tx + 16 * j];
-#pragma unroll
-          for (int i = tb; i < 4; ++i) {
-            const int r = ty + 16 * i;
-            const float4 w = *reinterpret_cast<const float4 *>(P + r * P_PITCH + t);
-            const bool all = i > tb;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (all || t <= r) o16[i][j] = fmaf(w.x, x[0][j], o16[i][j]);
-              if (all || t + 1 <= r) o16[i][j] = fmaf(w.y, x[1][j], o16[i][j]);
-              if (all || t + 2 <= r) o16[i][j] = fmaf(w.z, x[2][j], o16[i][j]);
-              if (all || t + 3 <= r) o16[i][j] = fmaf(w.w, x[3][j], o16[i][j]);
-            }
-          }
-        }
-#pragma unroll
-        for (int i = tb; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) o[i][j] += o16[i][j];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = ty + 16 * i, c = col0 + tx + 16 * j;
-          if (r < nt && c < V) a.out[(size_t)(first + t0 + r) * H * V + (size_t)h * V + c] = o[i][j];
-        }
-    } else {
-      __syncthreads();
-      if (tid < CHUNK) {
-        double f = (double)s[tid] * tail16[tid];
-        for (int B = (tid >> 4) + 1; B < 4; ++B) f *= block[B];
-        tail[tid] = (float)f;
-      }
-    }
-    __syncthreads();                                     // `tail` stands
-    if (!OUT || more) {
-      const double all = (block[0] * block[1]) * (block[2] * block[3]);
-      const float2 f2 = two_floats(all);
-      whole *= all;
-#pragma unroll 1
-      for (int tb = 0; tb < nt; tb += 16) {
-        float4 sum[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int m = 0; m < 2; ++m) sum[i][m] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const int t1 = min(tb + 16, nt);
-#pragma unroll 4
-        for (int t = tb; t < t1; ++t) {
-          const float f = tail[t];
-          const float4 x = *reinterpret_cast<const float4 *>(Vc + t * COLS + 4 * vy);
-#pragma unroll
-          for (int m = 0; m < 2; ++m)
-            if (4 * dx + 64 * m < D) {
-              const float4 k = *reinterpret_cast<const float4 *>(Kc + t * pitch + 4 * dx + 64 * m);
-              add4(sum[0][m], f * x.x, k);
-              add4(sum[1][m], f * x.y, k);
-              add4(sum[2][m], f * x.z, k);
-              add4(sum[3][m], f * x.w, k);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int m = 0; m < 2; ++m) st[i][m] = tb ? sum4(st[i][m], sum[i][m]) : carry4(st[i][m], f2, sum[i][m]);
-      }
-    }
-    __syncthreads();                                     // g, tail, S and P are written again
-  }
-  if (!OUT) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const int c = col0 + 4 * vy + i, d = 4 * dx + 64 * m;
-        if (c < V && d < D) *reinterpret_cast<float4 *>(part + (size_t)c * D + d) = st[i][m];
-      }
-    if (tid == 0 && blockIdx.x == 0) a.part_decay[(size_t)blockIdx.z * H + h] = two_floats(whole);
-  }
+  if (tid == 0 && blockIdx.x == 0) a.part_decay[(size_t)blockIdx.z * H + h] = two_floats((block[0] * block[1]) * (block[2] * block[3]));
 }
 
-// Four neighbours of a sequence's state a thread, along the sequence's segments.
+// Four neighbours of a sequence's state a thread, along the sequence's chunks.
 __global__ void __launch_bounds__(THREADS)
 chunk_carry_kernel(const ChunkArgs a) {
   pdl_launch();
   pdl_wait();
-  const int b = blockIdx.y, lane = threadIdx.x & 31;
-  int before = 0;                                        // segments of the sequences in front
-  for (int b0 = 0; b0 < b; b0 += 32) {
-    int c = b0 + lane < b ? (a.seq_meta[4 * (b0 + lane) + 1] + a.seg - 1) / a.seg : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    before += c;
-  }
+  const int b = blockIdx.y, before = chunks_before(a.seqs, CHUNK, b, threadIdx.x & 31), chunks = a.seqs.chunks(b, CHUNK);
   const size_t size = (size_t)a.H * a.V * a.D, e = ((size_t)blockIdx.x * THREADS + threadIdx.x) * 4;
-  if (e >= size) return;
-  const int h = (int)(e / ((size_t)a.V * a.D)), segments = (a.seq_meta[4 * b + 1] + a.seg - 1) / a.seg;
-  float4 *kept = reinterpret_cast<float4 *>(a.state + (size_t)a.seq_meta[4 * b + 3] * size + e);
+  if (!chunks || e >= size) return;
+  const int h = (int)(e / ((size_t)a.V * a.D));
+  float4 *kept = reinterpret_cast<float4 *>(a.state + (size_t)a.seqs.meta[4 * b + 3] * size + e);
   float4 s = *kept;
-  for (int i0 = 0; i0 < segments; i0 += 4) {
+  for (int i0 = 0; i0 < chunks; i0 += 4) {
     float4 x[4];
     float2 g[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const size_t at = (size_t)before + min(i0 + i, segments - 1);
+      const size_t at = (size_t)before + min(i0 + i, chunks - 1);
       x[i] = *reinterpret_cast<const float4 *>(a.parts + at * size + e);
       g[i] = a.part_decay[at * a.H + h];
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-      if (i0 + i < segments) {
+      if (i0 + i < chunks) {
         *reinterpret_cast<float4 *>(a.parts + ((size_t)before + i0 + i) * size + e) = s;
         s = carry4(s, g[i], x[i]);
       }
@@ -395,42 +372,41 @@ chunk_carry_kernel(const ChunkArgs a) {
 }
 
 template <typename T, bool OUT>
-static int launch_segments(const ChunkArgs &a, dim3 grid, cudaStream_t stream) {
+static int launch_chunks(const ChunkArgs &a, dim3 grid, cudaStream_t stream) {
   static G2bPerDevice done;
   auto bytes = [](int D) {
-    return sizeof(float) * ((size_t)2 * CHUNK * (D + 4) * (OUT ? 2 : 1) + 2 * CHUNK * COLS + 7 * CHUNK + 8 + CHUNK * 17 +
+    return sizeof(float) * ((size_t)CHUNK * (D + 4) * (OUT ? 2 : 1) + CHUNK * COLS + 7 * CHUNK + 8 + CHUNK * 17 +
                             (OUT ? (size_t)COLS * (D + 4) + CHUNK * P_PITCH : 0));
   };
   const int dev = g2b_current_device();
   if (dev < 0 || !done.value[dev]) {
-    if (cudaFuncSetAttribute(chunk_segment_kernel<T, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(MAX_D)) != cudaSuccess)
+    if (cudaFuncSetAttribute(chunk_kernel<T, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(MAX_D)) != cudaSuccess)
       G2B_REFUSE("chunk_scan: %zu bytes of shared memory are not available", bytes(MAX_D));
     if (dev >= 0) done.value[dev] = 1;
   }
-  g2b_launch(chunk_segment_kernel<T, OUT>, grid, dim3(THREADS), bytes(a.D), stream, a);
+  g2b_launch(chunk_kernel<T, OUT>, grid, dim3(THREADS), bytes(a.D), stream, a);
   return g2b_check_launch("chunk_scan");
 }
 
-// `segments`: how many there can be (n_tokens / seg + n_seqs); parts [segments, H, V, D], part_decay [segments, H, 2].
-extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D, int Vin,
-                              int extra_one, const float *decay, const float *gates, float *state, const int *seq_meta, int n_seqs,
-                              int seg, int segments, float *parts, float2 *part_decay, float *out, cudaStream_t stream) {
+// `chunks`: of 64 tokens, of all sequences that go here; parts [chunks, H, V, D], part_decay [chunks, H, 2].
+extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D, int Vin, int extra_one,
+                              const float *decay, const float *gates, float *state, const int *seq_meta, int n_seqs, int over, int pad,
+                              int chunks, float *parts, float2 *part_decay, float *out, cudaStream_t stream) {
   const int V = Vin + (extra_one ? 1 : 0);
-  if (n_seqs <= 0 || segments <= 0) return 0;
+  if (n_seqs <= 0 || chunks <= 0) return 0;
   if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("chunk_scan: unknown dtype %d", dtype);
   if (D <= 0 || D > MAX_D || D % 4) G2B_REFUSE("chunk_scan: key size %d (a multiple of 4 up to %d)", D, MAX_D);
   if (G <= 0 || H % G) G2B_REFUSE("chunk_scan: %d heads are not a multiple of %d query/key heads", H, G);
   if (!decay == !gates) G2B_REFUSE("chunk_scan: a decay per head or gates, not both");
-  if (seg <= 0 || seg % CHUNK) G2B_REFUSE("chunk_scan: segments of %d tokens (a multiple of %d)", seg, CHUNK);
-  if (H > 65535 || segments > 65535 || n_seqs > 65535) G2B_REFUSE("chunk_scan: %d heads, %d segments are too many", H, segments);
+  if (H > 65535 || chunks > 65535 || n_seqs > 65535) G2B_REFUSE("chunk_scan: %d heads, %d chunks are too many", H, chunks);
   if (((uintptr_t)qf | (uintptr_t)kf | (uintptr_t)state | (uintptr_t)parts) & 15) G2B_REFUSE("chunk_scan: a buffer is off 16 bytes");
-  const ChunkArgs a = {qf, kf, v, v_stride, H, G, D, V, Vin, decay, gates, state, seq_meta, n_seqs, seg, parts, part_decay, out};
-  const dim3 grid((V + COLS - 1) / COLS, H, segments);
-  if (int rc = dtype == G2B_F32 ? launch_segments<float, false>(a, grid, stream) : launch_segments<bf16, false>(a, grid, stream)) return rc;
+  const ChunkArgs a = {qf, kf, v, v_stride, H, G, D, V, Vin, decay, gates, state, {seq_meta, n_seqs, over, pad}, parts, part_decay, out};
+  const dim3 grid((V + COLS - 1) / COLS, H, chunks);
+  if (int rc = dtype == G2B_F32 ? launch_chunks<float, false>(a, grid, stream) : launch_chunks<bf16, false>(a, grid, stream)) return rc;
   const size_t quads = (size_t)H * V * D / 4;
   g2b_launch(chunk_carry_kernel, dim3((unsigned)((quads + THREADS - 1) / THREADS), n_seqs), dim3(THREADS), 0, stream, a);
   if (int rc = g2b_check_launch("chunk_scan")) return rc;
-  return dtype == G2B_F32 ? launch_segments<float, true>(a, grid, stream) : launch_segments<bf16, true>(a, grid, stream);
+  return dtype == G2B_F32 ? launch_chunks<float, true>(a, grid, stream) : launch_chunks<bf16, true>(a, grid, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -446,7 +422,7 @@ extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const
 //      S' = c_last S + sum_j D_(last,j) u_j k_j^T.  A block has 8 columns of a head; the next chunk's operands are on their way.
 // The substitution takes the tokens in their order, as the recurrence does; decays and sums as above (errors against 64 bits as
 // token by token: outputs 1.5e-7, states 1.1e-7).  The walk's chain of products, read
-// from shared memory, bounds it.  2,048 tokens, 8 heads of 128 x 128: 40 + 250 us (714 us a token after a token).
+// from shared memory, bounds it.  2,048 tokens, 8 heads of 128 x 128: 40 + 257 us (713 us a token after a token).
 #define DELTA_CHUNK 32
 #define DELTA_COLS 8
 #define DELTA_WALK 128
@@ -459,8 +435,7 @@ struct DeltaArgs {
   const float *ab;            // [T, 2H]: decay input, then write-strength input
   const float *A_log, *dt_bias;
   float *state;               // [slots, H, V, D]
-  const int *seq_meta;
-  int n_seqs;
+  Members seqs;
   float *U0, *W, *P, *decays; // [chunks, H, 32, V], [.., 32, D], [.., 32, 32], [.., 68]: c, the decays to the chunk's end, what c_last's rounding left
   float *out;                 // [T, H*V]
 };
@@ -475,8 +450,8 @@ delta_chunk_kernel(const DeltaArgs a) {
   __shared__ float g[DELTA_CHUNK], beta[DELTA_CHUNK], beta_c[DELTA_CHUNK];
   const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, tid = threadIdx.x, qk_head = h / (H / a.G);
   int b, place;
-  if (!find_segment(a.seq_meta, a.n_seqs, DELTA_CHUNK, blockIdx.x, b, place)) return;
-  const int first = a.seq_meta[4 * b] + place * DELTA_CHUNK, nt = min(DELTA_CHUNK, a.seq_meta[4 * b + 1] - place * DELTA_CHUNK);
+  if (!find_chunk(a.seqs, DELTA_CHUNK, blockIdx.x, b, place)) return;
+  const int first = a.seqs.meta[4 * b] + place * DELTA_CHUNK, nt = min(DELTA_CHUNK, a.seqs.meta[4 * b + 1] - place * DELTA_CHUNK);
   float *K = sm, *Q = K + DELTA_CHUNK * pitch;
   for (int i = tid; i < DELTA_CHUNK * (D / 4); i += THREADS) {
     const int r = i / (D / 4), d = i % (D / 4) * 4;
@@ -576,16 +551,11 @@ delta_walk_kernel(const DeltaArgs a) {
   pdl_launch();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
-  const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31;
+  const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
   const int qk_head = h / (H / a.G), col0 = blockIdx.x * DELTA_COLS;
-  int before = 0;                                        // chunks of the sequences in front
-  for (int b0 = 0; b0 < b; b0 += 32) {
-    int n = b0 + lane < b ? (a.seq_meta[4 * (b0 + lane) + 1] + DELTA_CHUNK - 1) / DELTA_CHUNK : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    before += n;
-  }
-  const int first = a.seq_meta[4 * b], n = a.seq_meta[4 * b + 1], slot = a.seq_meta[4 * b + 3];
+  if (!a.seqs.chunks(b, DELTA_CHUNK)) return;
+  const int before = chunks_before(a.seqs, DELTA_CHUNK, b, tid & 31);
+  const int first = a.seqs.meta[4 * b], n = a.seqs.meta[4 * b + 1], slot = a.seqs.meta[4 * b + 3];
   // two buffers, each: W, Q, K [32, pitch], P [32, 36], U0 [32, 8], decays [68]
   const int rows = DELTA_CHUNK * pitch, P_AT = 3 * rows, U_AT = P_AT + DELTA_CHUNK * 36, G_AT = U_AT + DELTA_CHUNK * DELTA_COLS,
             SIZE = G_AT + DELTA_DECAYS;
@@ -693,10 +663,10 @@ delta_walk_kernel(const DeltaArgs a) {
   }
 }
 
-// `chunks`: how many there can be (n_tokens / 32 + n_seqs).
+// `chunks`: of 32 tokens, of all sequences that go here.
 extern "C" int g2b_delta_scan(int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D, int V,
                               const float *ab, const float *A_log, const float *dt_bias, float *state, const int *seq_meta, int n_seqs,
-                              int chunks, float *U0, float *W, float *P, float *decays, float *out, cudaStream_t stream) {
+                              int over, int pad, int chunks, float *U0, float *W, float *P, float *decays, float *out, cudaStream_t stream) {
   if (n_seqs <= 0 || chunks <= 0) return 0;
   if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("delta_scan: unknown dtype %d", dtype);
   if (D <= 0 || D > MAX_D || D % 4 || V <= 0 || V % 4) G2B_REFUSE("delta_scan: key size %d (a multiple of 4 up to %d), value size %d (of 4)", D, MAX_D, V);
@@ -704,7 +674,7 @@ extern "C" int g2b_delta_scan(int dtype, const float *qf, const float *kf, const
   if (H > 65535 || n_seqs > 65535) G2B_REFUSE("delta_scan: %d heads, %d sequences are too many", H, n_seqs);
   if (((uintptr_t)qf | (uintptr_t)kf | (uintptr_t)state | (uintptr_t)U0 | (uintptr_t)W | (uintptr_t)P | (uintptr_t)decays) & 15)
     G2B_REFUSE("delta_scan: a buffer is off 16 bytes");
-  const DeltaArgs a = {qf, kf, v, v_stride, H, G, D, V, ab, A_log, dt_bias, state, seq_meta, n_seqs, U0, W, P, decays, out};
+  const DeltaArgs a = {qf, kf, v, v_stride, H, G, D, V, ab, A_log, dt_bias, state, {seq_meta, n_seqs, over, pad}, U0, W, P, decays, out};
   auto prep_bytes = [](int d) { return sizeof(float) * (size_t)2 * DELTA_CHUNK * (d + 4); };
   auto walk_bytes = [](int d) {
     return sizeof(float) * ((size_t)2 * (3 * DELTA_CHUNK * (d + 4) + DELTA_CHUNK * 36 + DELTA_CHUNK * DELTA_COLS + DELTA_DECAYS) + DELTA_COLS * (d + 4) +

@@ -36,8 +36,9 @@
 //
 // A state column (all D entries that feed one output channel) never mixes with another, so a
 // block owns a range of columns of one head of one sequence and walks the step's tokens in
-// order: what it computes for a token depends on the tokens before it in the sequence only,
-// not on how they were cut into steps or on the batch.
+// order: what it computes for a token depends on the tokens before it in the sequence only, not on how they were cut into steps
+// or on the batch.  In which order a column's sums are added (how many lanes share it, and whether a prompt goes a
+// token after a token here or in chunks, chunk_scan.cu) does depend on the step's lengths.
 #include "common.cuh"
 #include "join.cuh"
 
@@ -1014,6 +1015,7 @@ struct PScanArgs {
   const int *seq_meta;
   float *out;                 // [T, H*V]
   int L, Dp, tile;
+  int over, pad;              // sequences of more than `over` tokens, and sequence `pad`, are not this kernel's (chunk_scan.cu)
 };
 
 template <typename T, int MODE, int L>
@@ -1029,6 +1031,7 @@ state_scan_prompt_kernel(const PScanArgs a) {
   float *small = psm + 2 * qk_buf;
   float *po = small + 2 * small_buf;               // [TT, threads]: every lane's share of a token's read-out
   const int b = blockIdx.z, h = blockIdx.y;
+  if (a.seq_meta[4 * b + 1] > a.over || b == a.pad) return;
   const int qk_head = h / (H / a.G);
   const int lane_in_col = threadIdx.x % L, col_local = threadIdx.x / L;
   const int c = blockIdx.x * cols + col_local;
@@ -1214,12 +1217,13 @@ static void launch_scan_prompt(const PScanArgs &a, dim3 grid, size_t smem, cudaS
   else g2b_launch(state_scan_prompt_kernel<T, MODE, 32>, grid, dim3(PSCAN_THREADS), smem, stream, a);
 }
 
-// The preparation alone: q and k of the step turned or divided by their norms, scaled, in float [T, G, D].
+// The preparation: q and k of the step turned or divided by their norms, scaled, in float [T, G, D].
 extern "C" int g2b_scan_prep(int dtype, const void *q, int q_stride, const void *k, int k_stride, int n_tokens, int G, int D,
                              const float *rope, int rot, int interleaved, float q_scale, float k_scale, int unit_norm, float unit_eps,
                              float *qf, float *kf, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (D <= 0 || D > SCAN_MAX_D) G2B_REFUSE("state_scan: key size %d outside 1..%d", D, SCAN_MAX_D);
+  if (G <= 0) G2B_REFUSE("state_scan: %d query/key heads", G);
   if (rope && (rot <= 0 || rot > D || (rot & 1))) G2B_REFUSE("state_scan: %d rotated entries of a head of %d", rot, D);
   const dim3 grid((unsigned)(((long long)n_tokens * G + 3) / 4));
   if (dtype == G2B_F32)
@@ -1233,37 +1237,29 @@ extern "C" int g2b_scan_prep(int dtype, const void *q, int q_stride, const void 
   return g2b_check_launch("state_scan_prep");
 }
 
-extern "C" int g2b_state_scan_prompt(int mode, int dtype, const void *q, int q_stride, const void *k, int k_stride,
-                                     const void *v, int v_stride, int H, int G, int D, int V, const float *rope, int rot,
-                                     int interleaved, float q_scale, float k_scale, int unit_norm, float unit_eps,
-                                     const float *decay, const float *ab, const float *A_log, const float *dt_bias,
-                                     float *state, const int *seq_meta, int n_tokens, int n_seqs, float *qf, float *kf,
-                                     float *out, int extra_one, cudaStream_t stream) {
-  if (n_tokens <= 0 || n_seqs <= 0) return 0;
+// The scan of the sequences of a prepared step (scan_prep) that have at most `over` tokens and are not `pad`; `n_real`: the step's
+// sequences without padding.
+extern "C" int g2b_state_scan_prompt(int mode, int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D,
+                                     int V, const float *decay, const float *ab, const float *A_log, const float *dt_bias, float *state,
+                                     const int *seq_meta, int n_seqs, int n_real, int over, int pad, float *out, int extra_one,
+                                     cudaStream_t stream) {
+  if (n_seqs <= 0) return 0;
   if (D <= 0 || D > SCAN_MAX_D) G2B_REFUSE("state_scan: key size %d outside 1..%d", D, SCAN_MAX_D);
   if (G <= 0 || H % G) G2B_REFUSE("state_scan: %d heads are not a multiple of %d query/key heads", H, G);
-  if (rope && (rot <= 0 || rot > D || (rot & 1))) G2B_REFUSE("state_scan: %d rotated entries of a head of %d", rot, D);
   if (mode == 0 ? !decay : (mode == 1 ? (!ab || !A_log || !dt_bias) : !ab)) G2B_REFUSE("state_scan: mode %d lacks its decay inputs", mode);
   const int Vin = V;
   V += extra_one ? 1 : 0;
   if (!seq_meta) G2B_REFUSE("state_scan: the prompt kernel needs the step's table of sequences");
   if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("state_scan: unknown dtype %d", dtype);
-  const unsigned prep_blocks = (unsigned)(((long long)n_tokens * G + 3) / 4);
-  if (dtype == G2B_F32)
-    g2b_launch(scan_prep_kernel<float>, dim3(prep_blocks), dim3(128), 0, stream, (const float *)q, q_stride, (const float *)k,
-               k_stride, n_tokens, G, D, (const float2 *)rope, rot, interleaved, q_scale, k_scale, unit_norm, unit_eps, qf, kf);
-  else
-    g2b_launch(scan_prep_kernel<bf16>, dim3(prep_blocks), dim3(128), 0, stream, (const bf16 *)q, q_stride, (const bf16 *)k,
-               k_stride, n_tokens, G, D, (const float2 *)rope, rot, interleaved, q_scale, k_scale, unit_norm, unit_eps, qf, kf);
   PScanArgs a;
   a.qf = qf; a.kf = kf; a.v = v; a.v_stride = v_stride; a.H = H; a.G = G; a.D = D; a.V = V; a.Vin = Vin; a.decay = decay; a.ab = ab;
-  a.A_log = A_log; a.dt_bias = dt_bias; a.state = state; a.seq_meta = seq_meta; a.out = out;
+  a.A_log = A_log; a.dt_bias = dt_bias; a.state = state; a.seq_meta = seq_meta; a.out = out; a.over = over; a.pad = pad;
   // Lanes per column: at least D / 16; more while the step has few columns, so that every scheduler
   // of the GPU gets a few warps (a token's work in a warp is a chain of short dependent steps).
   a.L = 8;
   while (a.L * 16 < D) a.L <<= 1;
   {
-    const long long columns = (long long)n_seqs * H * V;
+    const long long columns = (long long)n_real * H * V;
     while (a.L < 32 && columns * a.L * 2 <= 32LL * 2400) a.L <<= 1;
   }
   a.Dp = (D + 4 * a.L - 1) / (4 * a.L) * (4 * a.L);

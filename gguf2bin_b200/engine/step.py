@@ -139,6 +139,7 @@ class Engine:
         self._seen: "OrderedDict[tuple, int]" = OrderedDict()        # shapes run plainly so far
         self.decode_runners: "OrderedDict[tuple, object]" = OrderedDict()
         self._padding = _PaddingSequence(self.cache)
+        self.scan_kinds: set = set()       # kinds of state scans the model runs in prompt steps, as the first of them leaves them here
         self.last_slots: Optional[torch.Tensor] = None     # the slots of the last step's sequences, on the device until the next
         self.step_graph_captures = 0       # CUDA graphs captured so far: of prompt-step shapes,
         self.decode_graph_captures = 0     # and of decode shapes (engine/decode.py)
@@ -251,7 +252,7 @@ class Engine:
             seq_meta=dev[o_meta:o_meta + 4 * B].view(B, 4), seq_slots=dev[o_slots:o_slots + B],
             attn_tiles=dev[:4 * n_narrow].view(n_narrow, 4), n_attn_tiles=n_narrow,
             attn_tiles_wide=dev[4 * n_narrow:4 * n_tiles].view(n_tiles - n_narrow, 4),
-            n_attn_tiles_wide=n_tiles - n_narrow)
+            n_attn_tiles_wide=n_tiles - n_narrow, padded=entries[-1].seq is self._padding, scan_kinds=self.scan_kinds)
         return ctx, dev[o_want:o_want + n_want], n_want
 
     def step(self, entries: Seq[StepEntry]) -> Optional[torch.Tensor]:
@@ -305,9 +306,11 @@ class Engine:
                    self._meta_dev.data_ptr())
         else:
             # which tokens, positions, pages, tiles and places is data on the device; the launches see
-            # only how many there are (the same numbers fix where each table lies in the step's metadata)
+            # only how many there are (the same numbers fix where each table lies in the step's metadata),
+            # and the state scans which sequences are long
             key = ("prompt", ctx.n_tokens, ctx.n_seqs, ctx.n_attn_tiles, ctx.n_attn_tiles_wide, n_want,
-                   ctx.page_table.shape[1], self._meta_dev.data_ptr())
+                   ctx.page_table.shape[1], self._meta_dev.data_ptr(), ctx.padded,
+                   *((kind, kernels.scan_plan(ctx, kind)) for kind in sorted(self.scan_kinds)))
         hit = self._graphs.get(key)
         if hit is not None:
             graph, generation, logits = hit

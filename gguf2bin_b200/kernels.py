@@ -8,6 +8,7 @@ device raises ``KernelError``, and a missing or unbuildable extension raises
 from __future__ import annotations
 
 import ctypes
+import heapq
 import math
 from ctypes import c_float, c_int, c_ulonglong, c_void_p
 from typing import NamedTuple, Optional
@@ -964,32 +965,88 @@ def short_conv(x, w32, ring, ctx, out, act: bool = True, bias=None) -> None:
         count_launches(1)
 
 
-DELTA_CHUNK = 32                  # tokens of a chunk of the gated delta rule (csrc/chunk_scan.cu)
-CHUNK_PARTS_MOST = 1 << 30        # bytes of scratch that the segments' states, or the delta rule's chunks, may take
+SCAN_CHUNK, DELTA_CHUNK = 64, 32  # tokens of a chunk (csrc/chunk_scan.cu): decays and gates, the gated delta rule
+SCAN_LENGTH_STEP = 32             # prompt lengths are told apart in steps of this many tokens
+NO_CHUNKS = 0x7fffffff            # every sequence a token after a token
+SMS = 148                         # multiprocessors of a B200
+CHUNK_PARTS_MOST = 1 << 30        # bytes of scratch that the chunks' states, or the delta rule's products, may take
 
 
-def _chunk_segment(n_tokens: int, n_seqs: int, heads: int, cols: int, dim: int) -> int:
-    """Tokens of a segment of the scan in chunks (csrc/chunk_scan.cu), 0 where the scan of a token after a token is taken: key
-    sizes that the kernel has not, prompts of less than 96 tokens on average, whose chain is no longer than the
-    chunked scan's launches, and states that do not fit the scratch.  The longest of 256, 128 and 64 tokens that
-    leaves four blocks for every SM, longer where the scratch asks for it."""
-    if dim % 4 or dim > 128 or n_tokens < 96 * n_seqs or heads > 65535:
-        return 0
-    blocks = heads * -(-cols // 64)
-    seg = next((s for s in (256, 128) if n_tokens // s * blocks >= 4 * 148), 64)
-    while 4 * (n_tokens // seg + n_seqs) * heads * cols * dim > CHUNK_PARTS_MOST:
-        if seg > n_tokens:
-            return 0
-        seg *= 2
-    return seg if n_tokens // seg + n_seqs <= 65535 else 0
+def _chain_us(lens, n_seqs: int, mode: int, heads: int, cols: int, dim: int) -> float:
+    """About what the scan of a token after a token takes for sequences of these lengths: blocks of 128 threads start in the
+    sequences' order as slots of the GPU come free, and a token costs a block more the fewer lanes a column has and the more blocks
+    share its SM.  (The lanes and the shared memory are csrc/seq_mix.cu's, ``n_seqs`` the sequences they are chosen for.)"""
+    lanes = 8
+    while lanes * 16 < dim:
+        lanes *= 2
+    while lanes < 32 and n_seqs * heads * cols * lanes * 2 <= 76800:
+        lanes *= 2
+    padded = -(-dim // (4 * lanes)) * 4 * lanes
+    tile = 16 if padded <= 128 else 8 if padded <= 256 else 4
+    blocks = heads * -(-cols // (128 // lanes))
+    per_sm = min(16, 227 * 1024 // (4 * tile * (4 * padded + 2 * (128 // lanes + 2) + 128) + 1024))
+    first, more = {(1, 8): (0.42, 0.04), (1, 16): (0.33, 0.03), (1, 32): (0.31, 0.03)}.get(
+        (mode, lanes), {8: (0.25, 0.045), 16: (0.20, 0.03), 32: (0.15, 0.03)}[lanes])
+    token = first + more * min(blocks * len(lens) / SMS, per_sm)
+    free, end = [(0.0, SMS * per_sm)], 0.0         # slots by when they come free
+    for n in lens:
+        left = blocks
+        while left:
+            at, slots = heapq.heappop(free)
+            take = min(slots, left)
+            left -= take
+            if slots > take:
+                heapq.heappush(free, (at, slots - take))
+            heapq.heappush(free, (at + n * token, take))
+            end = max(end, at + n * token)
+    return 6.0 + end
 
 
-def _delta_chunks(n_tokens: int, n_seqs: int, heads: int, dim: int, v_dim: int) -> int:
-    """Chunks of the gated delta rule over a prompt, 0 where it goes a token after a token: _chunk_segment's rule on sizes
-    and lengths, with the scratch of the chunks' own products."""
-    chunks = n_tokens // DELTA_CHUNK + n_seqs
-    fits = 4 * chunks * heads * (DELTA_CHUNK * (v_dim + dim + DELTA_CHUNK + 2) + 4) <= CHUNK_PARTS_MOST and chunks <= 65535
-    return chunks if fits and v_dim % 4 == 0 and _chunk_segment(n_tokens, 1, heads, 1, dim) and n_tokens >= 96 * n_seqs else 0
+def _scan_chunks_over(q_lens, mode: int, heads: int, cols: int, dim: int) -> Optional[int]:
+    """Which of a step's sequences (their lengths in the step, without padding) the chunked scan takes: those of more tokens than
+    the number returned; None for none, and all go a token after a token.  A token after a token costs the longest chain's
+    latency, several times over once the sequences' blocks fill the GPU; chunks cost all tokens alike, but up to
+    twice as much as a chain that fills the GPU.  So a few long prompts gain and large batches lose (microseconds a layer, a token after a token and in
+    chunks: 8 heads of 128 x 256 with a decay, 2,048 tokens 486 and 184, 100 tokens 33 and 33, 11 x 200 186 and 230; the
+    delta rule with 8 heads of 128 x 128, 2,048 tokens 713 and 297, 8 x 512 303 and 568).  The times of chunks below are fitted to
+    such measurements; lengths count in steps, which a step's graph is captured for."""
+    step = SCAN_LENGTH_STEP
+    classes = [-(-n // step) if n > 8 else 0 for n in q_lens]                   # those of a few tokens as of four
+    lens = [(c - 0.5) * step if c else 4.0 for c in classes]
+    wide = heads * -(-cols // 64) * 64 * dim
+    link, token = (0.04 + 0.0007 * dim, heads * cols * dim * 1.06e-6) if mode == 1 else (0.0, wide * 3.3e-7)
+    best, over = 0.95 * _chain_us(lens, len(lens), mode, heads, cols, dim), None      # chunks where they are quicker by more than the fit's error
+    cuts = sorted({c for c in classes if c * step > SCAN_CHUNK})
+    if len(cuts) > 8:                              # eight places to cut at are enough to choose from
+        cuts = [cuts[i * len(cuts) // 8] for i in range(8)]
+    for cut in cuts:
+        long = [-(-c * step // SCAN_CHUNK) * SCAN_CHUNK for c in classes if c >= cut]
+        short = [n for n, c in zip(lens, classes) if c < cut]
+        us = 22.0 + max(max(long) * link, sum(long) * token)
+        if short and us < best:
+            us += _chain_us(short, len(lens), mode, heads, cols, dim)
+        if us < best:
+            best, over = us, max(max((c * step for c in classes if c < cut), default=0), SCAN_CHUNK)
+    return over
+
+
+def scan_plan(ctx, kind) -> tuple:
+    """What a prompt step's launches of state scans of one kind (mode, heads, columns, key size) depend on beside the step's
+    sizes: (sequences of more tokens than this go in chunks, chunks of SCAN_CHUNK tokens, does padding go with them, does any
+    sequence go a token after a token).  Padding decides nothing: it is at most a chunk, and goes where chunks are launched anyway."""
+    plans = getattr(ctx, "scan_plans", None)
+    if plans is not None and kind in plans:
+        return plans[kind]
+    padded = getattr(ctx, "padded", False)
+    lens = ctx.q_lens[:-1] if padded else ctx.q_lens
+    over = _scan_chunks_over(lens, *kind) if lens else None
+    plan = (NO_CHUNKS, 0, False, True)
+    if over is not None:
+        chunked = (*(n for n in lens if n > over), *ctx.q_lens[len(lens):])
+        plan = (over, sum(-(-n // SCAN_CHUNK) for n in chunked), padded, min(lens) <= over)
+    if plans is not None:
+        plans[kind] = plan
+    return plan
 
 
 def state_scan(q, k, v, state, ctx, out32, heads, qk_heads, qk_dim, v_dim, *, decay=None, ab=None, a_log=None,
@@ -1031,44 +1088,46 @@ def state_scan(q, k, v, state, ctx, out32, heads, qk_heads, qk_dim, v_dim, *, de
         # that fetches the next tokens while it works on the ones it has
         qf = ctx.workspace.buffer("scan.q", (T, qk_heads * qk_dim), torch.float32)
         kf = ctx.workspace.buffer("scan.k", (T, qk_heads * qk_dim), torch.float32)
-        chunks = seg = 0
-        if not state.data_ptr() & 15:
-            if mode == 1:
-                chunks = _delta_chunks(T, ctx.n_seqs, heads, qk_dim, v_dim)
-            else:
-                seg = _chunk_segment(T, ctx.n_seqs, heads, cols, qk_dim)
-        if seg or chunks:
-            f = _fn("seq_mix.cu", "g2b_scan_prep",
-                    [c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_float, c_float, c_int,
-                     c_float, c_void_p, c_void_p, c_void_p])
-            _call(f, _code(q.dtype), _ptr(q), _dense_rows(q, "q"), _ptr(k), _dense_rows(k, "k"), T, qk_heads, qk_dim, _ptr(rope),
-                  rotary_dim, 1 if interleaved else 0, q_scale, k_scale, 0 if unit_eps is None else 1, unit_eps or 0.0, _ptr(qf),
-                  _ptr(kf), _stream())
-            if chunks:
-                u0, w_, p_, dec = (ctx.workspace.buffer("delta." + n, (chunks, heads, *shape), torch.float32) for n, shape in (
-                    ("u0", (DELTA_CHUNK, v_dim)), ("w", (DELTA_CHUNK, qk_dim)), ("p", (DELTA_CHUNK, DELTA_CHUNK)), ("decays", (2 * DELTA_CHUNK + 4,))))
-                f = _fn("chunk_scan.cu", "g2b_delta_scan",
-                        [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p] * 5 + [c_int] * 2 + [c_void_p] * 6)
-                _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim, _ptr(ab),
-                      _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, chunks, _ptr(u0), _ptr(w_), _ptr(p_),
-                      _ptr(dec), _ptr(out32), _stream())
-                count_launches(1)
-                return
-            segments = T // seg + ctx.n_seqs
-            parts = ctx.workspace.buffer("scan.parts", (segments, heads, cols, qk_dim), torch.float32)
-            decays = ctx.workspace.buffer("scan.part_decay", (segments, heads, 2), torch.float32)
+        f = _fn("seq_mix.cu", "g2b_scan_prep",
+                [c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_float, c_float, c_int,
+                 c_float, c_void_p, c_void_p, c_void_p])
+        _call(f, _code(q.dtype), _ptr(q), _dense_rows(q, "q"), _ptr(k), _dense_rows(k, "k"), T, qk_heads, qk_dim, _ptr(rope),
+              rotary_dim, 1 if interleaved else 0, q_scale, k_scale, 0 if unit_eps is None else 1, unit_eps or 0.0, _ptr(qf),
+              _ptr(kf), _stream())
+        over, chunks, padding, chain = NO_CHUNKS, 0, False, True
+        if qk_dim % 4 == 0 and qk_dim <= 128 and (mode != 1 or v_dim % 4 == 0) and not state.data_ptr() & 15:
+            kind = (mode, heads, cols, qk_dim)
+            if getattr(ctx, "scan_kinds", None) is not None:
+                ctx.scan_kinds.add(kind)
+            over, chunks, padding, chain = scan_plan(ctx, kind)
+            chunks, row = (2 * chunks, DELTA_CHUNK * (v_dim + qk_dim + DELTA_CHUNK + 2) + 4) if mode == 1 else (chunks, cols * qk_dim + 2)
+            if chunks > 65535 or 4 * chunks * heads * row > CHUNK_PARTS_MOST:
+                over, chunks, padding, chain = NO_CHUNKS, 0, False, True
+        pad = ctx.n_seqs - 1 if padding else -1
+        if chunks and mode == 1:
+            u0, w_, p_, dec = (ctx.workspace.buffer("delta." + n, (chunks, heads, *shape), torch.float32) for n, shape in (
+                ("u0", (DELTA_CHUNK, v_dim)), ("w", (DELTA_CHUNK, qk_dim)), ("p", (DELTA_CHUNK, DELTA_CHUNK)), ("decays", (2 * DELTA_CHUNK + 4,))))
+            f = _fn("chunk_scan.cu", "g2b_delta_scan",
+                    [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p] * 5 + [c_int] * 4 + [c_void_p] * 6)
+            _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim, _ptr(ab),
+                  _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, over, pad, chunks, _ptr(u0), _ptr(w_),
+                  _ptr(p_), _ptr(dec), _ptr(out32), _stream())
+            count_launches(1)
+        elif chunks:
+            parts = ctx.workspace.buffer("scan.parts", (chunks, heads, cols, qk_dim), torch.float32)
+            decays = ctx.workspace.buffer("scan.part_decay", (chunks, heads, 2), torch.float32)
             f = _fn("chunk_scan.cu", "g2b_chunk_scan",
-                    [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p] * 4 + [c_int] * 3 + [c_void_p] * 4)
+                    [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p] * 4 + [c_int] * 4 + [c_void_p] * 4)
             _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim,
-                  1 if ones_column else 0, _ptr(decay), _ptr(gates), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, seg, segments,
+                  1 if ones_column else 0, _ptr(decay), _ptr(gates), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, over, pad, chunks,
                   _ptr(parts), _ptr(decays), _ptr(out32), _stream())
             count_launches(2)
-            return
-        f = _fn("seq_mix.cu", "g2b_state_scan_prompt",
-                types + [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p])
-        _call(f, *common, _ptr(ctx.seq_meta), T, ctx.n_seqs, _ptr(qf), _ptr(kf), _ptr(out32),
-              1 if ones_column else 0, _stream())
-        count_launches(1)
+        if chain:
+            f = _fn("seq_mix.cu", "g2b_state_scan_prompt",
+                    [c_int, c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p] * 6 + [c_int] * 4 + [c_void_p, c_int, c_void_p])
+            _call(f, mode, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim, _ptr(decay),
+                  _ptr(ab), _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs,
+                  ctx.n_seqs - bool(getattr(ctx, "padded", False)), over, pad, _ptr(out32), 1 if ones_column else 0, _stream())
         return
     f = _fn("seq_mix.cu", "g2b_state_scan",
             types + [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p])

@@ -59,6 +59,9 @@ class StepContext:
     n_attn_tiles: int = 0                            # of row 0; tiles of ATTN_TILE_ROWS query rows
     attn_tiles_wide: Optional[torch.Tensor] = None   # the same with ATTN_WIDE_TILE_ROWS rows (tcgen05 kernel)
     n_attn_tiles_wide: int = 0
+    padded: bool = False                             # the last sequence is padding (its tokens fill the step up; nothing reads its results)
+    scan_kinds: Optional[set] = None                 # kinds of state scans that steps have run, the engine's set
+    scan_plans: dict = field(default_factory=dict)   # kernels.scan_plan of each kind in this step
     step_cache: dict = field(default_factory=dict)   # tensors derived once per step (cleared by the model)
     next_block: Optional[object] = None              # the block that runs after the one running now (None: the last)
     next_add: Optional[torch.Tensor] = None          # what is added to the stream before the next block; a block that

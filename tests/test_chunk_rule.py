@@ -1,21 +1,62 @@
-"""When a prompt's state scan goes in chunks: within the scratch, and only where prompts are long."""
+"""Which sequences of a step the chunked state scans take: a few long ones, whatever lies beside them; padding and small differences
+of length decide nothing."""
+from types import SimpleNamespace
+
 import pytest
 
 from gguf2bin_b200 import kernels
 
-
-@pytest.mark.parametrize("T,B,H,cols,D,want", [(2048, 1, 64, 65, 64, True), (95, 1, 4, 64, 64, False), (96, 1, 4, 64, 64, True),
-                                               (200, 3, 4, 64, 64, False), (4096, 2, 8, 64, 66, False), (4096, 2, 8, 64, 132, False),
-                                               (256 * 96, 256, 128, 128, 128, False), (1 << 20, 2, 64, 129, 128, True)])
-def test_segment(T, B, H, cols, D, want):
-    seg = kernels._chunk_segment(T, B, H, cols, D)
-    assert bool(seg) == want
-    if seg:
-        assert seg % 64 == 0 and 4 * (T // seg + B) * H * cols * D <= kernels.CHUNK_PARTS_MOST
+KINDS = [(0, 8, 256, 128), (2, 64, 64, 128), (2, 8, 257, 128), (1, 8, 128, 128), (0, 4, 64, 32), (1, 2, 32, 32)]
 
 
-@pytest.mark.parametrize("T,B,H,V,D,want", [(2048, 1, 32, 128, 128, True), (2048, 1, 32, 126, 128, False), (190, 2, 32, 128, 128, False),
-                                            (1 << 17, 1, 32, 128, 128, False), (96, 1, 2, 4, 4, True)])
-def test_delta_chunks(T, B, H, V, D, want):
-    chunks = kernels._delta_chunks(T, B, H, D, V)
-    assert chunks == (T // kernels.DELTA_CHUNK + B if want else 0)
+def plan_of(lens, kind, pad=0):
+    return kernels.scan_plan(SimpleNamespace(q_lens=[*lens, pad] if pad else lens, padded=bool(pad)), kind)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("beside", [[], [1] * 30, [7, 60, 3], [1] * 8 + [50]])
+def test_a_long_prompt_goes_in_chunks_whatever_lies_beside_it(kind, beside):
+    for lens in ([*beside, 2048], [2048, *beside]):
+        over, chunks, padding, chain = plan_of(lens, kind)
+        assert 64 <= over < 2048 and (chunks, padding, chain) == (32, False, bool(beside))
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("lens", [[1, 2], [64], [33, 64, 2], [64] * 40])
+def test_no_prompt_of_a_chunk_or_less(kind, lens):
+    assert plan_of(lens, kind) == (kernels.NO_CHUNKS, 0, False, True) == plan_of(lens, kind, pad=30)
+
+
+@pytest.mark.parametrize("kind", KINDS[:4])
+def test_large_batches_keep_the_gpu_busy_a_token_after_a_token(kind):
+    assert plan_of([200] * 40, kind)[0] == kernels.NO_CHUNKS
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("rest", [[], [20], [1, 1, 300]])
+def test_a_bucket_of_lengths_has_one_plan(kind, rest):
+    """A prompt of 1 to 63 tokens less than a multiple of 64, with padding that fills it up, is one shape: one graph."""
+    for top in (128, 320, 2048):
+        free = sum(rest) % 64
+        plans = {plan_of([n, *rest], kind, pad=(-n - free) % 64) for n in range(top - 63, top) if (n + free) % 64}
+        if not rest:
+            assert len(plans) <= 2 and (top < 320 or len(plans) == 1)      # at most where the rule changes its mind inside a bucket
+        assert all(p[0] in (64, kernels.NO_CHUNKS) or p[0] % 32 == 0 for p in plans)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_padding_decides_nothing(kind):
+    for lens in ([100], [97], [500, 20], [130, 130], [2000]):
+        bare = plan_of(lens, kind)
+        for pad in (1, 28, 63):
+            over, chunks, padding, chain = plan_of(lens, kind, pad)
+            assert (over, chain) == (bare[0], bare[3])
+            assert (chunks, padding) == ((bare[1] + 1, True) if bare[1] else (0, False))
+
+
+def test_every_chunk_is_counted():
+    for kind in KINDS:
+        over, chunks, _, chain = plan_of([1501, 900, 400, 130, 64, 5], kind)
+        if over != kernels.NO_CHUNKS:
+            taken = [n for n in (1501, 900, 400, 130, 64, 5) if n > over]
+            assert chunks == sum(-(-n // 64) for n in taken) and chain and taken[0] == 1501

@@ -21,12 +21,13 @@ def recurrence(q, k, v, g, s, S):
 @pytest.mark.parametrize("lens", [[64, 130], [193], [129, 1, 63, 260], [300, 321, 64]])
 @pytest.mark.parametrize("kind", ["decay", "gates"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("seg", [64, 256])
-def test_against_the_recurrence(H, G, D, V, ones, lens, kind, dtype, seg, monkeypatch):
+@pytest.mark.parametrize("over", [0, 64])
+def test_against_the_recurrence(H, G, D, V, ones, lens, kind, dtype, over, monkeypatch):
+    """``over`` 64: the sequences of up to 64 tokens go a token after a token in the same step."""
     from gguf2bin_b200 import kernels
     from gguf2bin_b200.engine.workspace import Workspace
     from types import SimpleNamespace
-    monkeypatch.setattr(kernels, "_chunk_segment", lambda *a: seg)
+    monkeypatch.setattr(kernels, "_scan_chunks_over", lambda *a: over)
     T, B, cols = sum(lens), len(lens), V + ones
     wide = rnd(T, 2 * G * D + H * V + 3, dtype=dtype, seed=1)
     q, k, v = wide[:, :G * D], wide[:, G * D:2 * G * D], wide[:, 2 * G * D:2 * G * D + H * V]
@@ -36,7 +37,7 @@ def test_against_the_recurrence(H, G, D, V, ones, lens, kind, dtype, seg, monkey
     for b, n in enumerate(lens):
         meta.append((at, n, 5, slots[b]))
         at += n
-    ctx = SimpleNamespace(seq_meta=torch.tensor(meta, dtype=torch.int32, device=DEV), n_seqs=B, workspace=Workspace(DEV))
+    ctx = SimpleNamespace(seq_meta=torch.tensor(meta, dtype=torch.int32, device=DEV), n_seqs=B, workspace=Workspace(DEV), q_lens=lens)
     gen = torch.Generator().manual_seed(3)
     if kind == "decay":
         decay = (1 - 2.0 ** -torch.randint(1, 12, (H,), generator=gen).float()).to(DEV)
@@ -87,10 +88,10 @@ def test_delta_rule(H, G, D, V, lens, dtype):
         at += n
     outs = []
     for chunked in (True, False):
-        ctx = SimpleNamespace(seq_meta=torch.tensor(meta, dtype=torch.int32, device=DEV), n_seqs=B, workspace=Workspace(DEV))
+        ctx = SimpleNamespace(seq_meta=torch.tensor(meta, dtype=torch.int32, device=DEV), n_seqs=B, workspace=Workspace(DEV), q_lens=lens)
         now, out = state.clone(), torch.full((T, H * V), float("nan"), device=DEV)
         with pytest.MonkeyPatch.context() as patch:
-            patch.setattr(kernels, "_chunk_segment", lambda *a: 64 * chunked)
+            patch.setattr(kernels, "_scan_chunks_over", lambda *a: 32 if chunked else None)
             kernels.state_scan(q, k, v, now, ctx, out, H, G, D, V, ab=ab, a_log=a_log, dt_bias=dt_bias, q_scale=D ** -0.5, unit_eps=1e-6)
         outs.append((out, now))
     at = 0
@@ -125,9 +126,9 @@ def test_later_values_reach_no_earlier_token():
     T, H, D, V = 200, 2, 32, 48
     q, k, v = rnd(T, H * D, seed=1), rnd(T, H * D, seed=2), rnd(T, H * V, seed=3)
     v[150], k[170] = float("inf"), float("nan")
-    ctx = SimpleNamespace(seq_meta=torch.tensor([[0, T, 0, 0]], dtype=torch.int32, device=DEV), n_seqs=1, workspace=Workspace(DEV))
+    ctx = SimpleNamespace(seq_meta=torch.tensor([[0, T, 0, 0]], dtype=torch.int32, device=DEV), n_seqs=1, workspace=Workspace(DEV), q_lens=[T])
     state, out = torch.zeros(1, H, V, D, device=DEV), torch.empty(T, H * V, device=DEV)
-    assert kernels._chunk_segment(T, 1, H, V, D)
+    assert kernels._scan_chunks_over([T], 0, H, V, D) is not None
     kernels.state_scan(q, k, v, state, ctx, out, H, H, D, V, decay=torch.tensor([0.9, 0.5], device=DEV))
     assert torch.isfinite(out[:150]).all() and not torch.isfinite(out[150]).any() and torch.isnan(out[171:]).all()
 
@@ -141,7 +142,7 @@ def test_infinite_states_stay_infinite():
     T, H, D, V = 500, 2, 32, 48
     q, k, v = (rnd(T, n, seed=i).abs() + 0.1 for i, n in enumerate((H * D, H * D, H * V)))
     v[70, 5], v[480, 50] = float("inf"), float("inf")
-    ctx = SimpleNamespace(seq_meta=torch.tensor([[0, T, 0, 0]], dtype=torch.int32, device=DEV), n_seqs=1, workspace=Workspace(DEV))
+    ctx = SimpleNamespace(seq_meta=torch.tensor([[0, T, 0, 0]], dtype=torch.int32, device=DEV), n_seqs=1, workspace=Workspace(DEV), q_lens=[T])
     state, out = torch.zeros(1, H, V, D, device=DEV), torch.empty(T, H * V, device=DEV)
     kernels.state_scan(q, k, v, state, ctx, out, H, H, D, V, decay=torch.tensor([0.9, 0.5], device=DEV))
     want = torch.zeros(T, H * V, dtype=torch.bool, device=DEV)
@@ -150,3 +151,30 @@ def test_infinite_states_stay_infinite():
     inf = torch.zeros(H, V, dtype=torch.bool, device=DEV)
     inf[0, 5], inf[1, 2] = True, True
     assert torch.equal((state[0] == float("inf")).all(-1), inf) and torch.isfinite(state[0][~inf]).all()
+
+
+@pytest.mark.parametrize("lens", [[100], [300], [700, 5, 40], [130, 257]])
+def test_steps_with_and_without_graphs_agree_to_the_bit(lens, monkeypatch):
+    """A prompt step that is filled up with padding and, from its third time on, replayed gives the bits of one that is not: the
+    padding changes neither which prompts go in chunks nor any sum."""
+    from gguf2bin_b200 import kernels
+    from gguf2bin_b200.engine import Engine, Model, StepEntry
+    from levolix_helpers import CONFIGS, model_folder
+    calls = []
+    rule = kernels._scan_chunks_over
+    monkeypatch.setattr(kernels, "_scan_chunks_over", lambda q, *a: calls.append(tuple(q)) or rule(q, *a))
+    model = Model.from_folder(model_folder("u"), dtype="float32")
+    gen, got = torch.Generator().manual_seed(sum(lens)), []
+    prompts = [torch.randint(CONFIGS["u"]["vocab"], (n,), generator=gen).tolist() for n in lens]
+    for graphs in (False, True):
+        eng = Engine(model, max_tokens=4096, step_graphs=graphs)
+        for _ in range(4 if graphs else 1):
+            seqs = [eng.open_sequence() for _ in lens]
+            got.append(eng.step([StepEntry(s, p, range(len(p))) for s, p in zip(seqs, prompts)]).clone())
+            nxt = [eng.step([StepEntry(s, [7], (0,))]).clone() for s in seqs]          # from the states that were left
+            got[-1] = torch.cat([got[-1], *nxt])
+            for s in seqs:
+                eng.close_sequence(s)
+        assert bool([k for k in eng._graphs if k[0] == "prompt"]) == graphs
+    assert all(torch.equal(got[0], g) for g in got[1:]) and torch.isfinite(got[0]).all()
+    assert set(calls) == {tuple(lens)}, "padding is not part of the lengths that decide"
