@@ -15,8 +15,8 @@
 //   2. chunk_carry: along a sequence, S at every chunk's start from the contributions; the sequence's state in the end
 //   3. chunk_kernel<true>: every chunk from its start state: the outputs
 // A block of 256 threads takes a chunk of one head and 64 columns.  Shared-memory reads bound it: 8 loads of 16
-// bytes feed 64 multiply-adds.  2,048 tokens, 8 heads of 128 x 256: 184 us (486 us as a chain), four prompts of 203 to 1,501 tokens, 64 heads of
-// 128 x 64: 641 us (889).  Chunks grouped into segments of up to 256 tokens, whose states alone went through memory: 189 and 709 us.
+// bytes feed 64 multiply-adds.  2,048 tokens, 8 heads of 128 x 256: 182 us (486 us as a chain), four prompts of 203 to 1,501 tokens, 64 heads of
+// 128 x 64: 649 us (889).  Chunks grouped into segments of up to 256 tokens, whose states alone went through memory: 189 and 709 us.
 //
 // Which sequences of a step come here is the caller's rule: those of more than `over` tokens, and sequence `pad`.  Of the
 // others nothing is read or written.
@@ -48,6 +48,7 @@ struct ChunkArgs {
   const float *gates;         // [T, 2H]: g, then s
   float *state;               // [slots, H, V, D]
   Members seqs;
+  int base, chunks;           // the launch's chunks: so many from this one of the step on
   float *parts;               // [chunks, H, V, D]: contributions, then start states
   float2 *part_decay;         // [chunks, H]: the product of the g's, and what its rounding left
   float *out;                 // [T, H*V]
@@ -118,7 +119,7 @@ chunk_kernel(const ChunkArgs a) {
   extern __shared__ __align__(16) float sm[];
   const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, col0 = blockIdx.x * COLS;
   int b, place;
-  if (!find_chunk(a.seqs, CHUNK, blockIdx.z, b, place)) return;
+  if (!find_chunk(a.seqs, CHUNK, a.base + blockIdx.z, b, place)) return;
   const int first = a.seqs.meta[4 * b] + place * CHUNK, n = min(CHUNK, a.seqs.meta[4 * b + 1] - place * CHUNK);
   const int qk_head = h / (H / a.G), tid = threadIdx.x;
   float *K = sm, *Vs = K + CHUNK * pitch;
@@ -346,9 +347,11 @@ __global__ void __launch_bounds__(THREADS)
 chunk_carry_kernel(const ChunkArgs a) {
   pdl_launch();
   pdl_wait();
-  const int b = blockIdx.y, before = chunks_before(a.seqs, CHUNK, b, threadIdx.x & 31), chunks = a.seqs.chunks(b, CHUNK);
+  // `chunks` of the sequence's are the launch's, in places from `before` on
+  const int b = blockIdx.y, place = chunks_before(a.seqs, CHUNK, b, threadIdx.x & 31) - a.base, before = max(place, 0);
+  const int chunks = min(a.seqs.chunks(b, CHUNK) - max(0, -place), a.chunks - before);
   const size_t size = (size_t)a.H * a.V * a.D, e = ((size_t)blockIdx.x * THREADS + threadIdx.x) * 4;
-  if (!chunks || e >= size) return;
+  if (chunks <= 0 || e >= size) return;
   const int h = (int)(e / ((size_t)a.V * a.D));
   float4 *kept = reinterpret_cast<float4 *>(a.state + (size_t)a.seqs.meta[4 * b + 3] * size + e);
   float4 s = *kept;
@@ -388,10 +391,11 @@ static int launch_chunks(const ChunkArgs &a, dim3 grid, cudaStream_t stream) {
   return g2b_check_launch("chunk_scan");
 }
 
-// `chunks`: of 64 tokens, of all sequences that go here; parts [chunks, H, V, D], part_decay [chunks, H, 2].
+// Chunks base .. base + chunks - 1 of those (of 64 tokens) of all sequences that go here, whose states stand behind the chunks in
+// front; parts [chunks, H, V, D], part_decay [chunks, H, 2].
 extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D, int Vin, int extra_one,
                               const float *decay, const float *gates, float *state, const int *seq_meta, int n_seqs, int over, int pad,
-                              int chunks, float *parts, float2 *part_decay, float *out, cudaStream_t stream) {
+                              int base, int chunks, float *parts, float2 *part_decay, float *out, cudaStream_t stream) {
   const int V = Vin + (extra_one ? 1 : 0);
   if (n_seqs <= 0 || chunks <= 0) return 0;
   if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("chunk_scan: unknown dtype %d", dtype);
@@ -400,7 +404,7 @@ extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const
   if (!decay == !gates) G2B_REFUSE("chunk_scan: a decay per head or gates, not both");
   if (H > 65535 || chunks > 65535 || n_seqs > 65535) G2B_REFUSE("chunk_scan: %d heads, %d chunks are too many", H, chunks);
   if (((uintptr_t)qf | (uintptr_t)kf | (uintptr_t)state | (uintptr_t)parts) & 15) G2B_REFUSE("chunk_scan: a buffer is off 16 bytes");
-  const ChunkArgs a = {qf, kf, v, v_stride, H, G, D, V, Vin, decay, gates, state, {seq_meta, n_seqs, over, pad}, parts, part_decay, out};
+  const ChunkArgs a = {qf, kf, v, v_stride, H, G, D, V, Vin, decay, gates, state, {seq_meta, n_seqs, over, pad}, base, chunks, parts, part_decay, out};
   const dim3 grid((V + COLS - 1) / COLS, H, chunks);
   if (int rc = dtype == G2B_F32 ? launch_chunks<float, false>(a, grid, stream) : launch_chunks<bf16, false>(a, grid, stream)) return rc;
   const size_t quads = (size_t)H * V * D / 4;
@@ -422,7 +426,7 @@ extern "C" int g2b_chunk_scan(int dtype, const float *qf, const float *kf, const
 //      S' = c_last S + sum_j D_(last,j) u_j k_j^T.  A block has 8 columns of a head; the next chunk's operands are on their way.
 // The substitution takes the tokens in their order, as the recurrence does; decays and sums as above (errors against 64 bits as
 // token by token: outputs 1.5e-7, states 1.1e-7).  The walk's chain of products, read
-// from shared memory, bounds it.  2,048 tokens, 8 heads of 128 x 128: 40 + 257 us (713 us a token after a token).
+// from shared memory, bounds it.  2,048 tokens, 8 heads of 128 x 128: 261 us, of which the walk 237 (713 us a token after a token).
 #define DELTA_CHUNK 32
 #define DELTA_COLS 8
 #define DELTA_WALK 128
@@ -436,6 +440,7 @@ struct DeltaArgs {
   const float *A_log, *dt_bias;
   float *state;               // [slots, H, V, D]
   Members seqs;
+  int base, chunks;           // the launch's chunks: so many from this one of the step on
   float *U0, *W, *P, *decays; // [chunks, H, 32, V], [.., 32, D], [.., 32, 32], [.., 68]: c, the decays to the chunk's end, what c_last's rounding left
   float *out;                 // [T, H*V]
 };
@@ -450,7 +455,7 @@ delta_chunk_kernel(const DeltaArgs a) {
   __shared__ float g[DELTA_CHUNK], beta[DELTA_CHUNK], beta_c[DELTA_CHUNK];
   const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, tid = threadIdx.x, qk_head = h / (H / a.G);
   int b, place;
-  if (!find_chunk(a.seqs, DELTA_CHUNK, blockIdx.x, b, place)) return;
+  if (!find_chunk(a.seqs, DELTA_CHUNK, a.base + blockIdx.x, b, place)) return;
   const int first = a.seqs.meta[4 * b] + place * DELTA_CHUNK, nt = min(DELTA_CHUNK, a.seqs.meta[4 * b + 1] - place * DELTA_CHUNK);
   float *K = sm, *Q = K + DELTA_CHUNK * pitch;
   for (int i = tid; i < DELTA_CHUNK * (D / 4); i += THREADS) {
@@ -546,16 +551,19 @@ delta_chunk_kernel(const DeltaArgs a) {
   }
 }
 
-__global__ void __launch_bounds__(DELTA_WALK)
+// (two blocks of an SM asked for: without, ptxas settles on half the registers and loads later, 270 us for 237)
+__global__ void __launch_bounds__(DELTA_WALK, 2)
 delta_walk_kernel(const DeltaArgs a) {
   pdl_launch();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int D = a.D, pitch = D + 4, V = a.V, H = a.H, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
   const int qk_head = h / (H / a.G), col0 = blockIdx.x * DELTA_COLS;
-  if (!a.seqs.chunks(b, DELTA_CHUNK)) return;
-  const int before = chunks_before(a.seqs, DELTA_CHUNK, b, tid & 31);
-  const int first = a.seqs.meta[4 * b], n = a.seqs.meta[4 * b + 1], slot = a.seqs.meta[4 * b + 3];
+  // the sequence's n tokens from row `first` on are the launch's, its chunks in places from `before` on
+  const int place = chunks_before(a.seqs, DELTA_CHUNK, b, tid & 31) - a.base, skip = max(0, -place) * DELTA_CHUNK, before = max(place, 0);
+  const int first = a.seqs.meta[4 * b] + skip, slot = a.seqs.meta[4 * b + 3];
+  const int n = min(a.seqs.meta[4 * b + 1] - skip, (a.chunks - before) * DELTA_CHUNK);
+  if (n <= 0 || !a.seqs.chunks(b, DELTA_CHUNK)) return;
   // two buffers, each: W, Q, K [32, pitch], P [32, 36], U0 [32, 8], decays [68]
   const int rows = DELTA_CHUNK * pitch, P_AT = 3 * rows, U_AT = P_AT + DELTA_CHUNK * 36, G_AT = U_AT + DELTA_CHUNK * DELTA_COLS,
             SIZE = G_AT + DELTA_DECAYS;
@@ -663,10 +671,10 @@ delta_walk_kernel(const DeltaArgs a) {
   }
 }
 
-// `chunks`: of 32 tokens, of all sequences that go here.
+// Chunks base .. base + chunks - 1 of those (of 32 tokens) of all sequences that go here, whose states stand behind the chunks in front.
 extern "C" int g2b_delta_scan(int dtype, const float *qf, const float *kf, const void *v, int v_stride, int H, int G, int D, int V,
                               const float *ab, const float *A_log, const float *dt_bias, float *state, const int *seq_meta, int n_seqs,
-                              int over, int pad, int chunks, float *U0, float *W, float *P, float *decays, float *out, cudaStream_t stream) {
+                              int over, int pad, int base, int chunks, float *U0, float *W, float *P, float *decays, float *out, cudaStream_t stream) {
   if (n_seqs <= 0 || chunks <= 0) return 0;
   if (dtype != G2B_F32 && dtype != G2B_BF16) G2B_REFUSE("delta_scan: unknown dtype %d", dtype);
   if (D <= 0 || D > MAX_D || D % 4 || V <= 0 || V % 4) G2B_REFUSE("delta_scan: key size %d (a multiple of 4 up to %d), value size %d (of 4)", D, MAX_D, V);
@@ -674,7 +682,7 @@ extern "C" int g2b_delta_scan(int dtype, const float *qf, const float *kf, const
   if (H > 65535 || n_seqs > 65535) G2B_REFUSE("delta_scan: %d heads, %d sequences are too many", H, n_seqs);
   if (((uintptr_t)qf | (uintptr_t)kf | (uintptr_t)state | (uintptr_t)U0 | (uintptr_t)W | (uintptr_t)P | (uintptr_t)decays) & 15)
     G2B_REFUSE("delta_scan: a buffer is off 16 bytes");
-  const DeltaArgs a = {qf, kf, v, v_stride, H, G, D, V, ab, A_log, dt_bias, state, {seq_meta, n_seqs, over, pad}, U0, W, P, decays, out};
+  const DeltaArgs a = {qf, kf, v, v_stride, H, G, D, V, ab, A_log, dt_bias, state, {seq_meta, n_seqs, over, pad}, base, chunks, U0, W, P, decays, out};
   auto prep_bytes = [](int d) { return sizeof(float) * (size_t)2 * DELTA_CHUNK * (d + 4); };
   auto walk_bytes = [](int d) {
     return sizeof(float) * ((size_t)2 * (3 * DELTA_CHUNK * (d + 4) + DELTA_CHUNK * 36 + DELTA_CHUNK * DELTA_COLS + DELTA_DECAYS) + DELTA_COLS * (d + 4) +

@@ -738,7 +738,21 @@ def attn_generic(q, out, cache_pages, tok_pos, tok_seq, page_table, n_heads, n_k
           pooled.shape[3] if pool else 0, float(softcap), int(keep_first), int(v_heads), _stream())
 
 
-F32_PARTS_MOST = 512 << 20        # bytes of scratch that the segments of single tokens may take
+F32_PARTS_MOST = 128 << 20        # bytes of scratch that the segments of single tokens may take; more tokens go in portions
+
+
+def _portion(workspace, name: str, rows: int, row_shape, most: int):
+    """Float scratch [n, *row_shape] for n of ``rows``, and n: as many as ``most`` bytes hold, fewer where the device has no more
+    memory, at least one.  The caller goes through its rows in portions of n."""
+    row = 4 * math.prod(row_shape)
+    n = max(1, min(rows, most // row, 65535))
+    while True:
+        try:
+            return workspace.buffer(name, (n, *row_shape), torch.float32, most=max(most, row)), n
+        except torch.OutOfMemoryError:
+            if n == 1:
+                raise
+            n = -(-n // 2)
 
 
 def attn_f32(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window, scale, sink=None, planes: int = 2,
@@ -757,20 +771,25 @@ def attn_f32(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size,
     if tiles is None or ctx.all_single:
         tiles, workspace = None, getattr(ctx, "workspace", None)
         segments = -(-getattr(ctx, "max_kv_len", 0) // page_size)
-        shape = (q.shape[0], n_heads, segments, head_dim + 2)
-        if workspace is None or segments < 1 or segments > ctx.page_table.shape[1] or q.shape[0] > 65535 or \
-                4 * shape[0] * shape[1] * shape[2] * shape[3] > F32_PARTS_MOST:
+        if workspace is None or segments < 1 or segments > ctx.page_table.shape[1]:
             return False
-        parts = workspace.buffer("attn.f32.parts", shape, torch.float32)
+        parts, portion = _portion(workspace, "attn.f32.parts", q.shape[0], (n_heads, segments, head_dim + 2), F32_PARTS_MOST)
     f = _fn("attn_generic.cu", "g2b_attn_f32",
             [c_void_p] * 6 + [c_int] * 6 + [c_float, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_float, c_int, c_int,
                                             c_void_p, c_int, c_void_p, c_int, c_void_p])
-    _call(f, _ptr(q), _ptr(out), _ptr(cache_pages), _ptr(ctx.tok_pos), _ptr(ctx.tok_seq), _ptr(ctx.page_table),
-          ctx.page_table.shape[1], q.shape[0], n_heads, n_kv_heads, head_dim, window, scale, _ptr(sink), planes, q.stride(0),
-          _ptr(gate), gate.stride(0) if gate is not None else 0, int(chunk), float(softcap), int(keep_first), int(v_heads),
-          _ptr(tiles), ctx.n_attn_tiles if tiles is not None else 0, _ptr(parts), segments, _stream())
-    if tiles is None:
-        count_launches(1)                          # the segments, then their merge
+    def run(q, out, tok_pos, tok_seq, gate) -> None:
+        _call(f, _ptr(q), _ptr(out), _ptr(cache_pages), _ptr(tok_pos), _ptr(tok_seq), _ptr(ctx.page_table),
+              ctx.page_table.shape[1], q.shape[0], n_heads, n_kv_heads, head_dim, window, scale, _ptr(sink), planes, q.stride(0),
+              _ptr(gate), gate.stride(0) if gate is not None else 0, int(chunk), float(softcap), int(keep_first), int(v_heads),
+              _ptr(tiles), ctx.n_attn_tiles if tiles is not None else 0, _ptr(parts), segments, _stream())
+        if tiles is None:
+            count_launches(1)                      # the segments, then their merge
+
+    if tiles is not None or q.shape[0] <= portion:
+        run(q, out, ctx.tok_pos, ctx.tok_seq, gate)
+        return True
+    for t in range(0, q.shape[0], portion):        # the parts do not fit: tokens in portions, each the same arithmetic
+        run(*(None if x is None else x[t:t + portion] for x in (q, out, ctx.tok_pos, ctx.tok_seq, gate)))
     return True
 
 
@@ -969,7 +988,7 @@ SCAN_CHUNK, DELTA_CHUNK = 64, 32  # tokens of a chunk (csrc/chunk_scan.cu): deca
 SCAN_LENGTH_STEP = 32             # prompt lengths are told apart in steps of this many tokens
 NO_CHUNKS = 0x7fffffff            # every sequence a token after a token
 SMS = 148                         # multiprocessors of a B200
-CHUNK_PARTS_MOST = 1 << 30        # bytes of scratch that the chunks' states, or the delta rule's products, may take
+CHUNK_PARTS_MOST = 256 << 20      # bytes of scratch that the chunks' states, or the delta rule's products, may take; more chunks go in portions
 
 
 def _chain_us(lens, n_seqs: int, mode: int, heads: int, cols: int, dim: int) -> float:
@@ -1008,13 +1027,13 @@ def _scan_chunks_over(q_lens, mode: int, heads: int, cols: int, dim: int) -> Opt
     latency, several times over once the sequences' blocks fill the GPU; chunks cost all tokens alike, but up to
     twice as much as a chain that fills the GPU.  So a few long prompts gain and large batches lose (microseconds a layer, a token after a token and in
     chunks: 8 heads of 128 x 256 with a decay, 2,048 tokens 486 and 184, 100 tokens 33 and 33, 11 x 200 186 and 230; the
-    delta rule with 8 heads of 128 x 128, 2,048 tokens 713 and 297, 8 x 512 303 and 568).  The times of chunks below are fitted to
+    delta rule with 8 heads of 128 x 128, 2,048 tokens 713 and 261, 8 x 512 303 and 506).  The times of chunks below are fitted to
     such measurements; lengths count in steps, which a step's graph is captured for."""
     step = SCAN_LENGTH_STEP
     classes = [-(-n // step) if n > 8 else 0 for n in q_lens]                   # those of a few tokens as of four
     lens = [(c - 0.5) * step if c else 4.0 for c in classes]
     wide = heads * -(-cols // 64) * 64 * dim
-    link, token = (0.04 + 0.0007 * dim, heads * cols * dim * 1.06e-6) if mode == 1 else (0.0, wide * 3.3e-7)
+    link, token = (0.04 + 0.0006 * dim, heads * cols * dim * 0.95e-6) if mode == 1 else (0.0, wide * 3.3e-7)
     best, over = 0.95 * _chain_us(lens, len(lens), mode, heads, cols, dim), None      # chunks where they are quicker by more than the fit's error
     cuts = sorted({c for c in classes if c * step > SCAN_CHUNK})
     if len(cuts) > 8:                              # eight places to cut at are enough to choose from
@@ -1100,28 +1119,30 @@ def state_scan(q, k, v, state, ctx, out32, heads, qk_heads, qk_dim, v_dim, *, de
             if getattr(ctx, "scan_kinds", None) is not None:
                 ctx.scan_kinds.add(kind)
             over, chunks, padding, chain = scan_plan(ctx, kind)
-            chunks, row = (2 * chunks, DELTA_CHUNK * (v_dim + qk_dim + DELTA_CHUNK + 2) + 4) if mode == 1 else (chunks, cols * qk_dim + 2)
-            if chunks > 65535 or 4 * chunks * heads * row > CHUNK_PARTS_MOST:
-                over, chunks, padding, chain = NO_CHUNKS, 0, False, True
+            chunks *= SCAN_CHUNK // (DELTA_CHUNK if mode == 1 else SCAN_CHUNK)
         pad = ctx.n_seqs - 1 if padding else -1
+        # portions of chunks in the order of the sequences: a state stays in its slot from one to the next
         if chunks and mode == 1:
-            u0, w_, p_, dec = (ctx.workspace.buffer("delta." + n, (chunks, heads, *shape), torch.float32) for n, shape in (
-                ("u0", (DELTA_CHUNK, v_dim)), ("w", (DELTA_CHUNK, qk_dim)), ("p", (DELTA_CHUNK, DELTA_CHUNK)), ("decays", (2 * DELTA_CHUNK + 4,))))
+            sizes = [heads * DELTA_CHUNK * n for n in (v_dim, qk_dim, DELTA_CHUNK)]             # U0, W, P; behind them the decays
+            parts, portion = _portion(ctx.workspace, "delta.parts", chunks, (sum(sizes) + heads * (2 * DELTA_CHUNK + 4),), CHUNK_PARTS_MOST)
+            at = [4 * portion * sum(sizes[:i]) for i in range(4)]
             f = _fn("chunk_scan.cu", "g2b_delta_scan",
-                    [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p] * 5 + [c_int] * 4 + [c_void_p] * 6)
-            _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim, _ptr(ab),
-                  _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, over, pad, chunks, _ptr(u0), _ptr(w_),
-                  _ptr(p_), _ptr(dec), _ptr(out32), _stream())
-            count_launches(1)
+                    [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p] * 5 + [c_int] * 5 + [c_void_p] * 6)
+            for first in range(0, chunks, portion):
+                _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim, _ptr(ab),
+                      _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, over, pad, first, min(portion, chunks - first),
+                      *(parts.data_ptr() + x for x in at), _ptr(out32), _stream())
+                count_launches(1)
         elif chunks:
-            parts = ctx.workspace.buffer("scan.parts", (chunks, heads, cols, qk_dim), torch.float32)
-            decays = ctx.workspace.buffer("scan.part_decay", (chunks, heads, 2), torch.float32)
+            parts, portion = _portion(ctx.workspace, "scan.parts", chunks, (heads, cols, qk_dim), CHUNK_PARTS_MOST)
+            decays = ctx.workspace.buffer("scan.part_decay", (portion, heads, 2), torch.float32)
             f = _fn("chunk_scan.cu", "g2b_chunk_scan",
-                    [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p] * 4 + [c_int] * 4 + [c_void_p] * 4)
-            _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim,
-                  1 if ones_column else 0, _ptr(decay), _ptr(gates), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, over, pad, chunks,
-                  _ptr(parts), _ptr(decays), _ptr(out32), _stream())
-            count_launches(2)
+                    [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p] * 4 + [c_int] * 5 + [c_void_p] * 4)
+            for first in range(0, chunks, portion):
+                _call(f, _code(q.dtype), _ptr(qf), _ptr(kf), _ptr(v), _dense_rows(v, "v"), heads, qk_heads, qk_dim, v_dim,
+                      1 if ones_column else 0, _ptr(decay), _ptr(gates), _ptr(state), _ptr(ctx.seq_meta), ctx.n_seqs, over, pad, first,
+                      min(portion, chunks - first), _ptr(parts), _ptr(decays), _ptr(out32), _stream())
+                count_launches(2)
         if chain:
             f = _fn("seq_mix.cu", "g2b_state_scan_prompt",
                     [c_int, c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p] * 6 + [c_int] * 4 + [c_void_p, c_int, c_void_p])

@@ -178,3 +178,35 @@ def test_steps_with_and_without_graphs_agree_to_the_bit(lens, monkeypatch):
         assert bool([k for k in eng._graphs if k[0] == "prompt"]) == graphs
     assert all(torch.equal(got[0], g) for g in got[1:]) and torch.isfinite(got[0]).all()
     assert set(calls) == {tuple(lens)}, "padding is not part of the lengths that decide"
+
+
+@pytest.mark.parametrize("kind", ["decay", "gates", "delta"])
+@pytest.mark.parametrize("portion", [1, 3, 7])
+def test_chunks_in_portions(kind, portion, monkeypatch):
+    """Scratch for a few chunks at a time, whose borders lie inside sequences and between them: the bits of all chunks at once."""
+    from gguf2bin_b200 import kernels
+    from gguf2bin_b200.engine.workspace import Workspace
+    from types import SimpleNamespace
+    H, D, V, lens = 2, 36, 64, [130, 20, 64, 321, 65]
+    monkeypatch.setattr(kernels, "_scan_chunks_over", lambda *a: 32)
+    T, B = sum(lens), len(lens)
+    q, k, v = rnd(T, H * D, seed=1), rnd(T, H * D, seed=2), rnd(T, H * V, seed=3)
+    gates = torch.cat([torch.rand(T, H, device=DEV), torch.rand(T, H, device=DEV)], 1)
+    more = {"decay": dict(decay=torch.tensor([0.9, 0.99], device=DEV)), "gates": dict(gates=gates),
+            "delta": dict(ab=rnd(T, 2 * H, seed=4), a_log=rnd(H, seed=5), dt_bias=rnd(H, seed=6), unit_eps=1e-6)}[kind]
+    meta, at = [], 0
+    for b, n in enumerate(lens):
+        meta.append((at, n, 5, b))
+        at += n
+    got = []
+    for limit in (1 << 28, None):
+        ws = Workspace(DEV)
+        if limit is None:
+            limit = 4 * portion * H * (32 * (V + D + 34) + 4 if kind == "delta" else V * D)
+        monkeypatch.setattr(kernels, "CHUNK_PARTS_MOST", limit)
+        ctx = SimpleNamespace(seq_meta=torch.tensor(meta, dtype=torch.int32, device=DEV), n_seqs=B, workspace=ws, q_lens=lens)
+        state, out = rnd(B, H, V, D, seed=7), torch.full((T, H * V), float("nan"), device=DEV)
+        kernels.state_scan(q, k, v, state, ctx, out, H, H, D, V, **more)
+        got.append((state, out))
+    assert ws._buffers["delta.parts" if kind == "delta" else "scan.parts"].numel() == limit
+    assert torch.isfinite(got[0][1]).all() and all(torch.equal(a, b) for a, b in zip(*got))

@@ -175,3 +175,20 @@ def test_attention_keeps_nan_and_infinities_that_are_seen(what, sink, options):
     # scores of at most 64 x 0.125 x 16 = 128, as in test_attention_tiles_and_segments
     score = (hd + 2) * EPS * 128
     assert (outs[0].double() - want)[~bad].abs().max() <= 2 * (2 * score + 400 * EPS) * V[torch.isfinite(V)].abs().max()
+
+
+@pytest.mark.parametrize("portion", [1, 2, 5])
+def test_segments_in_portions_of_tokens(portion, monkeypatch):
+    """Scratch for the segments of a few tokens at a time: the bits of all tokens at once."""
+    from gguf2bin_b200 import kernels
+    nh, nkv, hd, lens = 4, 2, 64, [130, 321, 64, 200, 1, 77, 500]
+    cache, table, _, _ = make_paged(len(lens), lens, nkv, hd, 64, torch.float32, seed=7)
+    q, sink, gate = rnd(len(lens), nh * hd, seed=8), rnd(nh, seed=9), rnd(len(lens), nh, seed=10)
+    outs = []
+    for limit in (1 << 28, 4 * portion * nh * 8 * (hd + 2)):
+        monkeypatch.setattr(kernels, "F32_PARTS_MOST", limit)
+        ctx, out = ctx_of(lens, [1] * len(lens), table, False), torch.full((len(lens), nh * hd), math.nan, device=DEV)
+        assert kernels.attn_f32(q, out, cache, ctx, nh, nkv, hd, 64, 0, 0.125, sink, 2, gate)
+        outs.append(out)
+    assert ctx.workspace.bytes() == limit
+    assert torch.isfinite(outs[0]).all() and torch.equal(*outs)
