@@ -10,6 +10,8 @@
 // bfloat16 path for sizes or dtypes the tensor-core kernels refuse.
 #include "common.cuh"
 
+#include <math.h>
+
 G2B_DEFINE_LAST_ERROR
 
 #define BM 64
@@ -343,11 +345,49 @@ static int launch_tile(const float *A, const float *W, void *C, int M, int N, in
   return g2b_check_launch("gemm_simt");
 }
 
-// Float operands whose rows all start on 16 bytes.  Up to ROWS_MAX rows the weights' bytes decide; four rows of W a block
-// and long stages where 16 would leave SMs without a block.
+// Which kernel takes float operands whose rows all start on 16 bytes.  All give the same bits, so time decides: the estimates
+// below (microseconds; the sums behind them are waves of blocks times what a block takes) pick a kernel within 8 % of the quickest for 950 of
+// 976 combinations of K from 16 to 4,096, N from 64 to 8,192 and 1 to 2,048 rows, timed back to back.  Where the kernel for
+// any strides wins: K up to about 128 (64 x 4096, 1,024 rows: 24 us, 429 with the rows kernel, to which a rule on the matrix's size alone
+// sent it; 64 x 4096, 4 rows: 4.9 and 17.7).  The rows kernel: up to about two waves of its blocks (64 x 1024, 64 rows: 37 us in
+// tiles, 8 here), and up to ROWS_MAX rows.
+enum { F32_GENERAL, F32_TILE1, F32_TILE4, F32_ROWS };
+static double ceil_div(double a, double b) { return ceil(a / b); }
+static double us_general(int M, int N, int K) {
+  const double tiles = ceil_div(N, BN) * ceil_div(M, BM);
+  return (1.6 + 0.055 * K) * (tiles <= 74 ? 1.0 : 1.2 + tiles / 270.0);
+}
+static double us_tile(int G, int M, int N, int K) {
+  const double tiles = ceil_div(N, TILE) * ceil_div(M, TILE), ragged = M % TILE ? 0.0006 * N : 0.0;      // all blocks ask for the last row
+  if (G == 4) return 0.6 + ragged + ceil_div(tiles, 148) * (0.2 + 9.0 * ceil_div(K, 4 * SUM_CHUNK));
+  return ragged + (3.6 + 3.8 * ceil_div(K, SUM_CHUNK)) * (tiles <= 148 ? 1.0 : tiles <= 592 ? 1.65 : 1.65 * tiles / 592);
+}
+static double us_rows(int rows_each, int NB, int CH, int M, int N, int K) {
+  const double smem = sizeof(float) * (2.0 * (NB + rows_each) * CH * CHUNK_PITCH + rows_each * NB * (CH + 1.0));
+  const double per_sm = floor(227 * 1024 / (smem + 1024)), waves = ceil_div(ceil_div(N, NB) * ceil_div(M, rows_each), 148 * per_sm);
+  return 0.6 + waves * (0.5 + (CH == 8 ? 1.3 + 0.17 * rows_each : 1.2 + 0.25 * rows_each) * sqrt(per_sm) * ceil_div(K, CH * SUM_CHUNK));
+}
+static bool four_rows_of_w(int M, int N) { return M <= 8 && N < 16 * 2 * 148; }      // where 16 would leave SMs without a block
+static int choose_f32(int M, int N, int K) {
+  const double general = us_general(M, N, K);
+  if (M <= ROWS_MAX) {
+    const bool four = four_rows_of_w(M, N);
+    return general < us_rows(M, four ? 4 : 16, four ? 32 : 8, M, N, K) ? F32_GENERAL : F32_ROWS;
+  }
+  const double us[4] = {general, us_tile(1, M, N, K), us_tile(4, M, N, K), us_rows(8, 16, 8, M, N, K)};
+  int best = 0;
+  for (int i = 1; i < 4; ++i)
+    if (us[i] < us[best]) best = i;
+  return best == F32_ROWS && (M + 7) / 8 > 65535 ? F32_TILE4 : best;
+}
+extern "C" int g2b_gemm_f32_kernel(int M, int N, int K) { return choose_f32(M, N, K); }
+
 template <int EPI>
-static int launch_f32(const float *A, const float *W, void *C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-  if (M <= 8 && N < 16 * 2 * 148) {
+static int launch_f32(const float *A, const float *W, void *C, int M, int N, int K, int lda, int ldw, int ldc, int which, cudaStream_t stream) {
+  if (which == F32_TILE1) return launch_tile<1, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  if (which == F32_TILE4) return launch_tile<4, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  if (M > ROWS_MAX) return launch_rows<16, 8, 8, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream, 8);      // eight rows a block, the matrix from the L2
+  if (four_rows_of_w(M, N)) {
     if (M == 1) return launch_rows<4, 32, 1, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     if (M == 2) return launch_rows<4, 32, 2, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     if (M <= 4) return launch_rows<4, 32, 4, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
@@ -356,13 +396,7 @@ static int launch_f32(const float *A, const float *W, void *C, int M, int N, int
   if (M == 1) return launch_rows<16, 8, 1, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
   if (M == 2) return launch_rows<16, 8, 2, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
   if (M <= 4) return launch_rows<16, 8, 4, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-  if (M <= ROWS_MAX) return launch_rows<16, 8, 8, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-  // A small matrix against a few more rows (the tiny models' prompts, 64 rows at least): eight rows a block, the matrix from
-  // the L2.  128 x 64 and 64 rows: 3.7 us in the step, where the tile kernel's long code costs 12 us to fetch for a few blocks.
-  if ((long long)N * K <= 1 << 18 && M <= 1024) return launch_rows<16, 8, 8, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream, 8);
-  const long long tiles = (long long)((N + TILE - 1) / TILE) * ((M + TILE - 1) / TILE);
-  if (tiles >= 3 * 148) return launch_tile<1, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-  return launch_tile<4, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  return launch_rows<16, 8, 8, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
 }
 
 template <typename TA, typename TW>
@@ -398,9 +432,12 @@ extern "C" int g2b_gemm_simt(const void *A, int a_dtype, const void *W, int w_dt
   if (a_dtype == G2B_F32 && w_dtype == G2B_F32 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0 &&
       (M + TILE - 1) / TILE <= 65535) {
     const float *a = (const float *)A, *w = (const float *)W;
-    if (epi == EPI_STORE_F32) return launch_f32<EPI_STORE_F32>(a, w, C, M, N, K, lda, ldw, ldc, stream);
-    if (epi == EPI_STORE_BF16) return launch_f32<EPI_STORE_BF16>(a, w, C, M, N, K, lda, ldw, ldc, stream);
-    if (epi == EPI_ACCUM_F32) return launch_f32<EPI_ACCUM_F32>(a, w, C, M, N, K, lda, ldw, ldc, stream);
+    const int which = choose_f32(M, N, K);
+    if (which != F32_GENERAL) {
+      if (epi == EPI_STORE_F32) return launch_f32<EPI_STORE_F32>(a, w, C, M, N, K, lda, ldw, ldc, which, stream);
+      if (epi == EPI_STORE_BF16) return launch_f32<EPI_STORE_BF16>(a, w, C, M, N, K, lda, ldw, ldc, which, stream);
+      if (epi == EPI_ACCUM_F32) return launch_f32<EPI_ACCUM_F32>(a, w, C, M, N, K, lda, ldw, ldc, which, stream);
+    }
   }
   if (a_dtype == G2B_F32 && w_dtype == G2B_F32)
     return launch<float, float>(A, W, C, M, N, K, lda, ldw, ldc, epi, stream);

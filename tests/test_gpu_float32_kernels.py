@@ -192,3 +192,22 @@ def test_segments_in_portions_of_tokens(portion, monkeypatch):
         outs.append(out)
     assert ctx.workspace.bytes() == limit
     assert torch.isfinite(outs[0]).all() and torch.equal(*outs)
+
+
+# general, tiles by one group and by four, rows: sizes where the estimates choose each, with ragged edges
+@pytest.mark.parametrize("which,M,N,K", [(0, 40, 4097, 64), (0, 700, 515, 20), (0, 3, 4096, 64), (1, 701, 3000, 516), (1, 1030, 4100, 188), (2, 129, 2500, 700),
+                                         (2, 600, 300, 1028), (3, 70, 70, 4100), (3, 200, 500, 516), (3, 32, 3000, 1028), (3, 1, 5000, 260)])
+def test_every_kernel_of_the_product_gives_the_same_bits(which, M, N, K):
+    from ctypes import c_int
+
+    from gguf2bin_b200 import kernels
+    choice = kernels._fn("gemm_simt.cu", "g2b_gemm_f32_kernel", [c_int] * 3)
+    assert choice(M, N, K) == which
+    a, w = rnd(M, K, seed=1), rnd(N, K, seed=2)
+    out, ref = torch.full((M, N), math.nan, device=DEV), torch.full((M, N), math.nan, device=DEV)
+    kernels.gemm_simt(a, w, out)
+    shifted = torch.empty(M * (K + 1) + 1, device=DEV)[1:].view(M, K + 1)[:, :K].copy_(a)         # rows off 16 bytes: the kernel for any strides
+    kernels.gemm_simt(shifted, w, ref)
+    assert torch.equal(out, ref)
+    bound = (66 + K / 64) * EPS * (a.double().abs() @ w.double().abs().T)
+    assert ((out.double() - a.double() @ w.double().T).abs() <= bound).all()
