@@ -136,17 +136,18 @@ attn_pool_decode_kernel(const bf16 *__restrict__ q, bf16 *__restrict__ out, cons
       float mx = -INFINITY;
       for (int r = lane; r < n_here; r += 32) mx = fmaxf(mx, sc[warp][r]);
       const float m_old = s_m[warp];
-      // -inf where every score so far is (a run may have a single entry): such an entry has no weight, wherever the others are
       const float m_new = fmaxf(m_old, warp_max(mx));
+      // -inf where every score so far is (a run may have a single entry): such an entry has no weight, wherever the others are
+      const float from = m_new == -INFINITY ? 0.f : m_new;
       float sum = 0.f;
       for (int r = lane; r < n_here; r += 32) {
-        const float p = sc[warp][r] == -INFINITY ? 0.f : expf(sc[warp][r] - m_new);
+        const float p = expf(sc[warp][r] - from);
         sc[warp][r] = p;
         sum += p;
       }
       sum = warp_sum(sum);
       if (lane == 0) {
-        const float corr = m_old == m_new ? 1.f : expf(m_old - m_new);      // 0 in the first pass
+        const float corr = expf(m_old - from);         // 0 in the first pass
         s_corr[warp] = corr;
         s_l[warp] = s_l[warp] * corr + sum;
         s_m[warp] = m_new;
@@ -220,9 +221,10 @@ attn_pool_decode_kernel(const bf16 *__restrict__ q, bf16 *__restrict__ out, cons
         m[r] = cluster.map_shared_rank(s_m, r)[g];
         top = fmaxf(top, m[r]);
       }
+      if (top == -INFINITY) top = 0.f;
   #pragma unroll
       for (int r = 0; r < SPLIT; ++r) {
-        const float f = m[r] == top ? 1.f : expf(m[r] - top);      // 0 for a run without entries
+        const float f = expf(m[r] - top);                // 0 for a run without entries
         l = fmaf(cluster.map_shared_rank(s_l, r)[g], f, l);
         sum = fmaf(cluster.map_shared_rank(&red[0][0][0], r)[idx], f, sum);
       }
@@ -250,9 +252,10 @@ extern "C" int g2b_attn_pool_decode(const void *q, void *out, const void *cache,
   const long long tiles = (long long)nkv * ((group + GH - 1) / GH);
   if (tiles > 65535) G2B_REFUSE("attn_pool_decode: %lld head tiles are too many for one launch", tiles);
   // As many runs as leave the GPU with about a CTA an SM: four tokens of 16 heads on 8 with a window of 512: 11.6 us in a decode
-  // step with four runs, 31.9 us with one.
-  const long long items = n_tokens * tiles;
-  const unsigned split = items * 2 <= 148 ? 4 : items <= 148 ? 2 : 1;
+  // step with four runs, 31.9 us with one.  One run where a token never has more entries than half a pass: 60 keys and 4.9 us, 5.6 with
+  // four (the cluster's two barriers).
+  const long long items = n_tokens * tiles, entries = (window < P * PAGE ? window : P * PAGE) + (long long)P * PAGE / pool;
+  const unsigned split = entries <= PASS / 2 ? 1 : items * 2 <= 148 ? 4 : items <= 148 ? 2 : 1;
   const auto kernel = split == 4 ? attn_pool_decode_kernel<4> : split == 2 ? attn_pool_decode_kernel<2> : attn_pool_decode_kernel<1>;
   g2b_launch_cluster(kernel, dim3((unsigned)n_tokens * split, (unsigned)tiles), dim3(THREADS), 0, stream, split,
              (const bf16 *)q, (bf16 *)out, (const bf16 *)cache, (const bf16 *)pooled, tok_pos, tok_seq, page_table, P,
