@@ -21,6 +21,12 @@
 // Which sequences of a step come here is the caller's rule: those of more than `over` tokens, and sequence `pad`.  Of the
 // others nothing is read or written.
 #include "common.cuh"
+#include <math.h>
+#include <algorithm>
+#include <exception>
+#include <functional>
+#include <queue>
+#include <vector>
 
 G2B_DEFINE_LAST_ERROR
 
@@ -700,4 +706,102 @@ extern "C" int g2b_delta_scan(int dtype, const float *qf, const float *kf, const
   if (int rc = g2b_check_launch("delta_scan")) return rc;
   g2b_launch(delta_walk_kernel, dim3((V + DELTA_COLS - 1) / DELTA_COLS, H, n_seqs), dim3(DELTA_WALK), walk_bytes(D), stream, a);
   return g2b_check_launch("delta_scan");
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// which sequences go in chunks (host; gates on 64 heads: 64 prompts of up to 600 tokens 0.11 ms, 256 of up to 200 1.7 ms)
+// ---------------------------------------------------------------------------------------------------------
+#define LENGTH_STEP 32            // prompt lengths are told apart in steps of this many tokens
+#define SMS 148                   // of the B200 that the times below were taken on; the rule is also asked where no GPU is
+
+struct ScanKind { int mode, heads, cols, dim; };      // mode: 0 a decay a head, 1 the delta rule, 2 gates
+
+// About what the scan of a token after a token takes for sequences of these lengths, in microseconds: blocks of 128 threads start
+// in the sequences' order as slots of the GPU come free, and a token costs a block more the fewer lanes a column has and the more
+// blocks share its SM.  (The lanes and the shared memory are seq_mix.cu's, `n_seqs` the sequences they are chosen for.)  Beyond `most`
+// the estimate ends early.
+static double chain_us(const std::vector<double> &lens, int n_seqs, const ScanKind &k, double most) {
+  int lanes = 8;
+  while (lanes * 16 < k.dim) lanes *= 2;
+  while (lanes < 32 && (double)n_seqs * k.heads * k.cols * lanes * 2 <= 76800) lanes *= 2;
+  const long long padded = (k.dim + 4 * lanes - 1) / (4 * lanes) * 4 * lanes, tile = padded <= 128 ? 16 : padded <= 256 ? 8 : 4;
+  const long long groups = 128 / lanes, blocks = k.heads * ((k.cols + groups - 1) / groups);
+  const long long per_sm = std::min(16ll, 227 * 1024 / (4 * tile * (4 * padded + 2 * (groups + 2) + 128) + 1024));
+  const int wide = lanes == 8 ? 0 : lanes == 16 ? 1 : 2;
+  static const double one[2][3] = {{0.25, 0.20, 0.15}, {0.42, 0.33, 0.31}}, more[2][3] = {{0.045, 0.03, 0.03}, {0.04, 0.03, 0.03}};
+  const double token = one[k.mode == 1][wide] +
+                       more[k.mode == 1][wide] * std::min((double)(blocks * (long long)lens.size()) / SMS, (double)per_sm);
+  typedef std::pair<double, long long> Slots;           // when they come free, and how many
+  std::priority_queue<Slots, std::vector<Slots>, std::greater<Slots>> free;
+  free.push({0.0, SMS * per_sm});
+  double end = 0.0;
+  for (const double n : lens) {
+    if (6.0 + end >= most) break;
+    for (long long left = blocks; left > 0;) {
+      const Slots s = free.top();
+      free.pop();
+      const long long take = std::min(s.second, left);
+      left -= take;
+      if (s.second > take) free.push({s.first, s.second - take});
+      free.push({s.first + n * token, take});
+      end = std::max(end, s.first + n * token);
+    }
+  }
+  return 6.0 + end;
+}
+
+// Sequences of more tokens than the number returned go in chunks; 0: none does.  A token after a token costs the longest chain's latency, several
+// times over once the sequences' blocks fill the GPU; chunks cost all tokens alike, but up to twice as much as a chain that
+// fills the GPU.  So a few long prompts gain and large batches lose (microseconds a layer, a token after a token and in chunks:
+// 8 heads of 128 x 256 with a decay, 2,048 tokens 486 and 184, 100 tokens 33 and 33, 11 x 200 186 and 230; the delta rule with 8
+// heads of 128 x 128, 2,048 tokens 713 and 261, 8 x 512 303 and 506).  The times of chunks below are fitted to such measurements;
+// lengths count in steps, which a step's graph is captured for.
+static int chunks_over(const int *tokens, int n, const ScanKind &k) {
+  std::vector<int> classes(n), cuts;                    // those of a few tokens as of four
+  std::vector<double> lens(n), few;
+  for (int i = 0; i < n; ++i) {
+    classes[i] = tokens[i] > 8 ? (tokens[i] + LENGTH_STEP - 1) / LENGTH_STEP : 0;
+    lens[i] = classes[i] ? (classes[i] - 0.5) * LENGTH_STEP : 4.0;
+    if (classes[i] * LENGTH_STEP > CHUNK) cuts.push_back(classes[i]);
+  }
+  std::sort(cuts.begin(), cuts.end());
+  cuts.erase(std::unique(cuts.begin(), cuts.end()), cuts.end());
+  if (cuts.empty()) return 0;
+  const double wide = (double)k.heads * ((k.cols + COLS - 1) / COLS) * COLS * k.dim;
+  const double link = k.mode == 1 ? 0.04 + 0.0006 * k.dim : 0.0, token = k.mode == 1 ? (double)k.heads * k.cols * k.dim * 0.95e-6 : wide * 3.3e-7;
+  double best = 0.95 * chain_us(lens, n, k, HUGE_VAL);            // chunks where they are quicker by more than the fit's error
+  int over = 0;
+  const int places = std::min<int>(8, (int)cuts.size());      // eight places to cut at are enough to choose from
+  for (int c = 0; c < places; ++c) {
+    const int cut = cuts[(size_t)c * cuts.size() / places];
+    double longest = 0.0, sum = 0.0;
+    int below = 0;
+    few.clear();
+    for (int i = 0; i < n; ++i) {
+      if (classes[i] < cut) {
+        few.push_back(lens[i]);
+        below = std::max(below, classes[i] * LENGTH_STEP);
+      } else {
+        const double whole = (double)((classes[i] * LENGTH_STEP + CHUNK - 1) / CHUNK * CHUNK);
+        longest = std::max(longest, whole);
+        sum += whole;
+      }
+    }
+    double us = 22.0 + std::max(longest * link, sum * token);
+    if (!few.empty() && us < best) us += chain_us(few, n, k, best - us);
+    if (us < best) best = us, over = std::max(below, CHUNK);
+  }
+  return over;
+}
+
+// `tokens` [n]: the lengths of a step's sequences, without padding.
+extern "C" int g2b_scan_chunks_over(const int *tokens, int n, int mode, int heads, int cols, int dim, int *over) {
+  if (n <= 0 || heads <= 0 || cols <= 0 || dim <= 0 || dim > MAX_D)
+    G2B_REFUSE("chunk_scan: no rule for %d sequences on %d heads of %d x %d", n, heads, dim, cols);
+  try {
+    *over = chunks_over(tokens, n, {mode, heads, cols, dim});
+  } catch (const std::exception &e) {
+    G2B_REFUSE("chunk_scan: %s", e.what());
+  }
+  return 0;
 }

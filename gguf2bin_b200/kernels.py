@@ -8,9 +8,8 @@ device raises ``KernelError``, and a missing or unbuildable extension raises
 from __future__ import annotations
 
 import ctypes
-import heapq
 import math
-from ctypes import c_float, c_int, c_ulonglong, c_void_p
+from ctypes import byref, c_float, c_int, c_ulonglong, c_void_p
 from typing import NamedTuple, Optional
 
 import torch
@@ -985,68 +984,18 @@ def short_conv(x, w32, ring, ctx, out, act: bool = True, bias=None) -> None:
 
 
 SCAN_CHUNK, DELTA_CHUNK = 64, 32  # tokens of a chunk (csrc/chunk_scan.cu): decays and gates, the gated delta rule
-SCAN_LENGTH_STEP = 32             # prompt lengths are told apart in steps of this many tokens
 NO_CHUNKS = 0x7fffffff            # every sequence a token after a token
-SMS = 148                         # multiprocessors of a B200
 CHUNK_PARTS_MOST = 256 << 20      # bytes of scratch that the chunks' states, or the delta rule's products, may take; more chunks go in portions
-
-
-def _chain_us(lens, n_seqs: int, mode: int, heads: int, cols: int, dim: int) -> float:
-    """About what the scan of a token after a token takes for sequences of these lengths: blocks of 128 threads start in the
-    sequences' order as slots of the GPU come free, and a token costs a block more the fewer lanes a column has and the more blocks
-    share its SM.  (The lanes and the shared memory are csrc/seq_mix.cu's, ``n_seqs`` the sequences they are chosen for.)"""
-    lanes = 8
-    while lanes * 16 < dim:
-        lanes *= 2
-    while lanes < 32 and n_seqs * heads * cols * lanes * 2 <= 76800:
-        lanes *= 2
-    padded = -(-dim // (4 * lanes)) * 4 * lanes
-    tile = 16 if padded <= 128 else 8 if padded <= 256 else 4
-    blocks = heads * -(-cols // (128 // lanes))
-    per_sm = min(16, 227 * 1024 // (4 * tile * (4 * padded + 2 * (128 // lanes + 2) + 128) + 1024))
-    first, more = {(1, 8): (0.42, 0.04), (1, 16): (0.33, 0.03), (1, 32): (0.31, 0.03)}.get(
-        (mode, lanes), {8: (0.25, 0.045), 16: (0.20, 0.03), 32: (0.15, 0.03)}[lanes])
-    token = first + more * min(blocks * len(lens) / SMS, per_sm)
-    free, end = [(0.0, SMS * per_sm)], 0.0         # slots by when they come free
-    for n in lens:
-        left = blocks
-        while left:
-            at, slots = heapq.heappop(free)
-            take = min(slots, left)
-            left -= take
-            if slots > take:
-                heapq.heappush(free, (at, slots - take))
-            heapq.heappush(free, (at + n * token, take))
-            end = max(end, at + n * token)
-    return 6.0 + end
 
 
 def _scan_chunks_over(q_lens, mode: int, heads: int, cols: int, dim: int) -> Optional[int]:
     """Which of a step's sequences (their lengths in the step, without padding) the chunked scan takes: those of more tokens than
-    the number returned; None for none, and all go a token after a token.  A token after a token costs the longest chain's
-    latency, several times over once the sequences' blocks fill the GPU; chunks cost all tokens alike, but up to
-    twice as much as a chain that fills the GPU.  So a few long prompts gain and large batches lose (microseconds a layer, a token after a token and in
-    chunks: 8 heads of 128 x 256 with a decay, 2,048 tokens 486 and 184, 100 tokens 33 and 33, 11 x 200 186 and 230; the
-    delta rule with 8 heads of 128 x 128, 2,048 tokens 713 and 261, 8 x 512 303 and 506).  The times of chunks below are fitted to
-    such measurements; lengths count in steps, which a step's graph is captured for."""
-    step = SCAN_LENGTH_STEP
-    classes = [-(-n // step) if n > 8 else 0 for n in q_lens]                   # those of a few tokens as of four
-    lens = [(c - 0.5) * step if c else 4.0 for c in classes]
-    wide = heads * -(-cols // 64) * 64 * dim
-    link, token = (0.04 + 0.0006 * dim, heads * cols * dim * 0.95e-6) if mode == 1 else (0.0, wide * 3.3e-7)
-    best, over = 0.95 * _chain_us(lens, len(lens), mode, heads, cols, dim), None      # chunks where they are quicker by more than the fit's error
-    cuts = sorted({c for c in classes if c * step > SCAN_CHUNK})
-    if len(cuts) > 8:                              # eight places to cut at are enough to choose from
-        cuts = [cuts[i * len(cuts) // 8] for i in range(8)]
-    for cut in cuts:
-        long = [-(-c * step // SCAN_CHUNK) * SCAN_CHUNK for c in classes if c >= cut]
-        short = [n for n, c in zip(lens, classes) if c < cut]
-        us = 22.0 + max(max(long) * link, sum(long) * token)
-        if short and us < best:
-            us += _chain_us(short, len(lens), mode, heads, cols, dim)
-        if us < best:
-            best, over = us, max(max((c * step for c in classes if c < cut), default=0), SCAN_CHUNK)
-    return over
+    the number returned; None for none, and all go a token after a token (the rule and its reasons: csrc/chunk_scan.cu)."""
+    f = _fn("chunk_scan.cu", "g2b_scan_chunks_over", [c_void_p] + [c_int] * 5 + [c_void_p])
+    lens, over = (c_int * len(q_lens))(*q_lens), c_int()
+    if f(lens, len(q_lens), mode, heads, cols, dim, byref(over)) != 0:
+        raise KernelError(f._lib.g2b_last_error().decode("utf-8", "replace"))
+    return over.value or None
 
 
 def scan_plan(ctx, kind) -> tuple:

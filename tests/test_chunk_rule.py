@@ -1,5 +1,7 @@
 """Which sequences of a step the chunked state scans take: a few long ones, whatever lies beside them; padding and small differences
 of length decide nothing."""
+import heapq
+import random
 from types import SimpleNamespace
 
 import pytest
@@ -60,3 +62,61 @@ def test_every_chunk_is_counted():
         if over != kernels.NO_CHUNKS:
             taken = [n for n in (1501, 900, 400, 130, 64, 5) if n > over]
             assert chunks == sum(-(-n // 64) for n in taken) and chain and taken[0] == 1501
+
+
+def plain_chain_us(lens, n_seqs, mode, heads, cols, dim):
+    lanes = 8
+    while lanes * 16 < dim:
+        lanes *= 2
+    while lanes < 32 and n_seqs * heads * cols * lanes * 2 <= 76800:
+        lanes *= 2
+    padded = -(-dim // (4 * lanes)) * 4 * lanes
+    tile = 16 if padded <= 128 else 8 if padded <= 256 else 4
+    blocks = heads * -(-cols // (128 // lanes))
+    per_sm = min(16, 227 * 1024 // (4 * tile * (4 * padded + 2 * (128 // lanes + 2) + 128) + 1024))
+    first, more = {(1, 8): (0.42, 0.04), (1, 16): (0.33, 0.03), (1, 32): (0.31, 0.03)}.get(
+        (mode, lanes), {8: (0.25, 0.045), 16: (0.20, 0.03), 32: (0.15, 0.03)}[lanes])
+    token = first + more * min(blocks * len(lens) / 148, per_sm)
+    free, end = [(0.0, 148 * per_sm)], 0.0   # slots of the GPU by when they come free
+    for n in lens:
+        left = blocks
+        while left:
+            at, slots = heapq.heappop(free)
+            take = min(slots, left)
+            left -= take
+            if slots > take:
+                heapq.heappush(free, (at, slots - take))
+            heapq.heappush(free, (at + n * token, take))
+            end = max(end, at + n * token)
+    return 6.0 + end
+
+
+def plain_rule(q_lens, mode, heads, cols, dim):
+    step = 32
+    classes = [-(-n // step) if n > 8 else 0 for n in q_lens]
+    lens = [(c - 0.5) * step if c else 4.0 for c in classes]
+    wide = heads * -(-cols // 64) * 64 * dim
+    link, token = (0.04 + 0.0006 * dim, heads * cols * dim * 0.95e-6) if mode == 1 else (0.0, wide * 3.3e-7)
+    best, over = 0.95 * plain_chain_us(lens, len(lens), mode, heads, cols, dim), None
+    cuts = sorted({c for c in classes if c * step > 64})
+    if len(cuts) > 8:
+        cuts = [cuts[i * len(cuts) // 8] for i in range(8)]
+    for cut in cuts:
+        long = [-(-c * step // 64) * 64 for c in classes if c >= cut]
+        short = [n for n, c in zip(lens, classes) if c < cut]
+        us = 22.0 + max(max(long) * link, sum(long) * token)
+        if short and us < best:
+            us += plain_chain_us(short, len(lens), mode, heads, cols, dim)
+        if us < best:
+            best, over = us, max(max((c * step for c in classes if c < cut), default=0), 64)
+    return over
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_the_rule_as_it_is_written(kind):
+    """The estimates restated, for few and many sequences, ragged, equal and with single tokens among them."""
+    rng = random.Random(sum(kind))
+    for n in (1, 2, 5, 9, 17, 33, 64, 150):
+        for most in (60, 400, 3000):
+            for lens in ([rng.randint(1, most) for _ in range(n)], [most] * n, [rng.choice((1, 1, rng.randint(1, most))) for _ in range(n)]):
+                assert kernels._scan_chunks_over(lens, *kind) == plain_rule(lens, *kind), lens
