@@ -714,7 +714,7 @@ norm_shift_kernel(const float *__restrict__ x, const float *__restrict__ w, cons
 }
 
 // The same for rows of a multiple of 4 up to 8,192 entries: a thread keeps PER groups of four neighbours of its row and of the
-// row before (or the sequence's last) in registers, both sums go through one pair of barriers, and the weights are asked for in
+// row before (or the sequence's last) in registers, both sums go through one barrier, and the weights are asked for in
 // front of the wait.  Four rows of 2,048 in a decode step: 4.6 us (13.3 us an entry at a time).
 template <typename TO, int PER>
 __global__ void __launch_bounds__(256)

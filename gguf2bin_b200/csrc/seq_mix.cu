@@ -79,7 +79,7 @@ __device__ __forceinline__ void rotate_ahead(float *x, const float2 *turn, const
 // ---------------------------------------------------------------------------
 // The common form (the norms span the heads, neighbours turn together, heads of one size that is the rows' in the pages): a
 // block a token, a thread keeps PER groups of four neighbours of [q | k | v] in registers from the load to the store, both
-// norms share one pair of barriers, and biases and weights are asked for before the wait for the kernel in front.  One token of
+// norms share one barrier, and biases and weights are asked for before the wait for the kernel in front.  One token of
 // 16 + 8 + 8 heads of 128 in a decode step: 5.3 us (21.8 us an entry at a time with 256 threads).
 template <typename T, int PER>
 __global__ void __launch_bounds__(1024)

@@ -203,3 +203,43 @@ def test_latents(rank, width, e_rank, dtype):
             assert not pages[p, at, rank:].any()
             left[p, at] = False
         assert (pages[left] == 9.0).all()
+
+
+@pytest.mark.parametrize("H", [61, 1028, 2052, 4096, 8192])
+@pytest.mark.parametrize("top", [5, 8])
+def test_experts_sums(H, top):
+    """More choices than one round of loads, some of them without a row (they read the token's own x): the sum stored and added, and
+    joined to the stream with and without a base and a next norm."""
+    from gguf2bin_b200 import kernels
+    T, R = 3, 7
+    g = torch.Generator().manual_seed(H + top)
+    pair_row = torch.randint(-1, R, (T, top), generator=g).to(torch.int32)
+    pair_row[0, top - 1], pair_row[1, 0] = -1, R - 1
+    rows, x, base, w = rnd(R, H, seed=1), rnd(T, H, seed=2), rnd(T, H, seed=3), rnd(H, seed=4)
+    weight = torch.rand((T, top), generator=g).to(DEV)
+    picked = torch.where((pair_row < 0)[..., None].to(DEV), x[:, None], rows[pair_row.clamp(min=0).long().to(DEV)]).double()
+    total, size = (weight.double()[..., None] * picked).sum(1), (weight.double()[..., None] * picked.abs()).sum(1)
+    pair_row = pair_row.to(DEV)
+    for add in (False, True):
+        out = base.clone() if add else torch.full_like(base, 7.0)
+        kernels.moe_combine(rows, pair_row, weight, x, top, out, add)
+        near(out, total + base.double() * add, torch.float32, size + base.double().abs() * add)
+
+    def unit(z):
+        return z / (z.square().mean(1, keepdim=True) + 1e-3).sqrt()
+
+    for dtype in (torch.float32, torch.bfloat16):
+        xs, cast = x.clone(), torch.empty((T, H), dtype=dtype, device=DEV)
+        if kernels.moe_combine_norm_add(rows, pair_row, weight, xs, w, 1e-3, top, cast):
+            want, most = x.double() + unit(total) * w.double(), x.double().abs() + size / total.square().mean(1, keepdim=True).sqrt() * w.double().abs()
+            near(xs, want, torch.float32, most)
+            near(cast, want, dtype, most)
+        else:
+            assert H > 4096 and torch.equal(xs, x)
+        for b in (None, base):
+            xs, y = x.clone(), total if b is None else total + b.double()
+            kernels.moe_combine_join(rows, pair_row, weight, b, top, xs, w, 1e-3, (w, 1e-3), cast)
+            want = x.double() + unit(y) * w.double()
+            most = x.double().abs() + (size + base.double().abs()) / y.square().mean(1, keepdim=True).sqrt() * w.double().abs()
+            near(xs, want, torch.float32, most)
+            near(cast, unit(want) * w.double(), dtype, most / want.square().mean(1, keepdim=True).sqrt() * w.double().abs())

@@ -310,7 +310,7 @@ def test_a_token_far_back_still_counts(kind):
 # the block's norm and token shift, the feed-forwards
 # ----------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("width", [60, 256, 1000])
+@pytest.mark.parametrize("width", [60, 61, 256, 1000, 1028, 2048, 4096, 8192])
 def test_norm_and_token_shift_over_steps(width, dtype):
     """h = norm(x) and the mixer's copy h + (h_before - h) mu, the row before taken from the step where
     there is one and from the slot otherwise; slots hold junk beyond what a sequence wrote, and
