@@ -1689,15 +1689,14 @@ static int launch_grouped(const CUtensorMap &ma, const CUtensorMap &mw, void *C,
 // (epi = EPI_STORE_F32) or [rows, Nw / 2] bfloat16 (EPI_SWIGLU_BF16: W's rows alternate eight
 // gates and eight ups).
 extern "C" int g2b_gemm_tc_grouped(const void *A, const void *W, void *C, int rows, int n_groups, int Nw, int K,
-                                   int lda, int ldc, int epi, const int *plan, int max_tiles, int *status,
+                                   int lda, int ldc, int epi, const int *plan, int *status,
                                    float glu_limit, float glu_offset, float glu_c1, float glu_c3, cudaStream_t stream) {
   [[maybe_unused]] ProductTail glu;
   glu.limit = glu_limit, glu.offset = glu_offset, glu.c1 = glu_c1, glu.c3 = glu_c3, glu.a_group = 0;
-  if (rows <= 0 || Nw <= 0 || n_groups <= 0 || max_tiles <= 0) return 0;
+  if (rows <= 0 || Nw <= 0 || n_groups <= 0) return 0;
   if (K <= 0 || K % 8 || lda % 8) G2B_REFUSE("gemm_tc: K=%d and the row stride %d must be multiples of 8", K, lda);
   if (((uintptr_t)A | (uintptr_t)W) & 15) G2B_REFUSE("gemm_tc: operands must be 16-byte aligned");
   if (epi == EPI_SWIGLU_BF16 && Nw % 16) G2B_REFUSE("gemm_tc: gated output needs N %% 16 == 0, N=%d", Nw);
-  if (max_tiles > 65535) G2B_REFUSE("gemm_tc: %d row tiles are too many for one launch", max_tiles);
   if (!status || !plan) G2B_REFUSE("gemm_tc: no status word or no plan");
   if ((long long)n_groups * Nw > 0x7fffffffLL) G2B_REFUSE("gemm_tc: %d groups of %d rows of W", n_groups, Nw);
   if (n_groups > GROUPS_MOST) G2B_REFUSE("gemm_tc: %d groups (at most %d)", n_groups, GROUPS_MOST);
