@@ -819,6 +819,16 @@ def attention(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size
                  softcap=softcap, keep_first=keep_first, v_heads=v_heads)
 
 
+def attention_qkv(qkv, q_w, k_w, eps, rope, rotary_dim, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window,
+                  scale, sink=None, chunk: int = 0, softcap: float = 0.0, keep_first: int = 0) -> bool:
+    """``qknorm_rope_cache`` of the projection ``qkv`` and the attention behind it in one kernel, for steps of one token per
+    sequence in bfloat16; False when no kernel takes the case (the caller then runs the two)."""
+    if qkv.dtype != torch.bfloat16:
+        return False
+    return (_bf16 or _bf16_mod()).attn_decode_qkv(qkv, q_w, k_w, eps, rope, rotary_dim, out, cache_pages, ctx, n_heads, n_kv_heads,
+                                                  head_dim, page_size, window, scale, sink, chunk, softcap, keep_first)
+
+
 def normed_product(x32, eps, w, out, gate_block=None) -> bool:
     """out = rmsnorm_without_weight(x32) @ w.T (or its SiLU gate) in one kernel; False when no
     kernel takes the case (the caller then runs the norm and the product one after the other)."""

@@ -13,7 +13,7 @@ from .kernels import SILU, _GLU_TYPES, KernelError, _call, _fn, _ptr, _stream
 FAST_HEAD_SIZES = (64, 128)          # head sizes the tensor-core attention kernels are written for
 DECODE_CHUNK_KEYS = 256              # keys per CTA of the decode kernel (attn_decode.cu)
 
-units.SPECIALISED_SOURCES[:] = [("attn_decode.cu", ()), ("attn_decode.cu", ("ATTN_DECODE_PAGES=2",)),
+units.SPECIALISED_SOURCES[:] = [("attn_decode.cu", ()), ("attn_decode_short.cu", ()),
                                 ("attn_decode.cu", ("ATTN_DECODE_PAGES=6",)), ("attn_decode.cu", ("ATTN_DECODE_PAGES=8",)),
                                 ("attn_decode_noalloc.cu", ()),
                                 ("attn_prefill.cu", ()), ("attn_prefill_tc.cu", ()),
@@ -491,31 +491,41 @@ def decode_chunk_pages(units: int, pages: int, head_dim: int, slots: int) -> int
     return best
 
 
+DECODE_CLUSTER_MOST = 16      # chunks of 128 keys that attn_decode_short.cu merges inside a thread-block cluster
+
+
+def _decode_pages(ctx, T, n_heads, n_kv_heads, head_dim, fine) -> int:
+    """Pages of 64 keys that a CTA takes."""
+    if fine is not None:
+        return 2 if fine else 4
+    tiles = n_kv_heads * -(-(n_heads // n_kv_heads) // 16)
+    keys = getattr(ctx, "kv_len_hint", 0) or ctx.max_kv_len       # max_kv_len may be the reserved length
+    return decode_chunk_pages(T * tiles, -(-max(int(keys), 1) // 64), head_dim, DECODE_CTAS_PER_SM * _sm_count(ctx.tok_pos.device))
+
+
+def _decode_scratch(ctx, T, n_heads, head_dim, pages):
+    """Scratch for the chunks' partial outputs and their statistics; none where clusters merge them."""
+    n_chunks = -(-max(int(ctx.max_kv_len), 1) // (64 * pages))
+    if pages == 2 and n_chunks <= DECODE_CLUSTER_MOST:
+        return None, None
+    kernels.count_launches(1)                      # the merge of the chunks
+    ws = ctx.workspace
+    return (ws.buffer("attn.part_o", (T * n_heads * n_chunks * head_dim,), torch.float32),
+            ws.buffer("attn.part_ml", (T * n_heads * n_chunks * 2,), torch.float32))
+
+
 def attn_decode(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window,
                 scale, fine=None, pages=None, sink=None, planes: int = 2, gate=None, softcap: float = 0.0,
                 keep_first: int = 0, v_heads: int = 0) -> None:
-    """One token per sequence: split-key attention with partial results in scratch memory
-    and a combine pass.  A CTA takes a chunk of keys of one kv head: 256 as a rule, 128, 384 or
+    """One token per sequence: split-key attention and a merge of the chunks, in one launch or two.  A CTA takes a chunk of keys of
+    one kv head: 256 as a rule, 128 (``attn_decode_short.cu``), 384 or
     512 where ``decode_chunk_pages`` says so (``fine`` = 128; ``pages`` = pages of 64 keys per
     CTA, 2 to 8; default by that rule)."""
     T = q.shape[0]
-    defines = (f"HD={head_dim}",)
-    if pages is None:
-        if fine is None:
-            tiles = n_kv_heads * -(-(n_heads // n_kv_heads) // 16)
-            keys = getattr(ctx, "kv_len_hint", 0) or ctx.max_kv_len       # max_kv_len may be the reserved length
-            pages = decode_chunk_pages(T * tiles, -(-max(int(keys), 1) // 64), head_dim,
-                                       DECODE_CTAS_PER_SM * _sm_count(q.device))
-        else:
-            pages = 2 if fine else 4
-    if pages != 4:
-        defines = defines + (f"ATTN_DECODE_PAGES={pages}",)
-    chunk_keys = 64 * pages
-    n_chunks = -(-max(int(ctx.max_kv_len), 1) // chunk_keys)
-    ws = ctx.workspace
-    part_o = ws.buffer("attn.part_o", (T * n_heads * n_chunks * head_dim,), torch.float32)
-    part_ml = ws.buffer("attn.part_ml", (T * n_heads * n_chunks * 2,), torch.float32)
-    f = _fn("attn_decode.cu", "g2b_attn_decode_ex",
+    pages = pages or _decode_pages(ctx, T, n_heads, n_kv_heads, head_dim, fine)
+    part_o, part_ml = _decode_scratch(ctx, T, n_heads, head_dim, pages)
+    defines = (f"HD={head_dim}",) if pages in (2, 4) else (f"HD={head_dim}", f"ATTN_DECODE_PAGES={pages}")
+    f = _fn(*(("attn_decode_short.cu", "g2b_attn_decode_short") if pages == 2 else ("attn_decode.cu", "g2b_attn_decode_ex")),
             [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
              c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
              c_int, c_float, c_int, c_int, c_void_p],
@@ -525,4 +535,29 @@ def attn_decode(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_si
           page_size, window, scale, int(ctx.max_kv_len), _ptr(part_o), _ptr(part_ml), _ptr(sink), planes,
           q.stride(0), _ptr(gate), gate.stride(0) if gate is not None else 0, float(softcap), int(keep_first),
           int(v_heads), _stream())
-    kernels.count_launches(1)                      # the attention and the merge of its chunks
+
+
+def attn_decode_qkv(qkv, q_w, k_w, eps, rope, rotary_dim, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window,
+                    scale, sink=None, chunk: int = 0, softcap: float = 0.0, keep_first: int = 0, fine=None) -> bool:
+    """``qknorm_rope_cache`` and the attention of a step of single tokens in one kernel; False: the case is left to the two.  Only where
+    chunks are short (``decode_chunk_pages``): with more to read the attention's copies run ahead while the prologue kernel is busy, and one
+    launch was slower (``attn_decode_short.cu``)."""
+    if not ctx.all_single or head_dim not in FAST_HEAD_SIZES or page_size != 64 or cache_pages.dtype != torch.bfloat16:
+        return False
+    if not scale > 0.0 or (chunk and (window or softcap or keep_first)) or (rope is not None and rotary_dim != head_dim):
+        return False
+    if not qkv.is_contiguous() or not out.is_contiguous() or qkv.shape[1] != (n_heads + 2 * n_kv_heads) * head_dim:
+        return False
+    if any(x is not None and x.data_ptr() % 16 for x in (qkv, out, q_w, k_w, rope, cache_pages)):
+        return False
+    if _decode_pages(ctx, qkv.shape[0], n_heads, n_kv_heads, head_dim, fine) != 2:
+        return False
+    part_o, part_ml = _decode_scratch(ctx, qkv.shape[0], n_heads, head_dim, 2)
+    f = _fn("attn_decode_short.cu", "g2b_attn_decode_short_qkv",
+            [c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+             c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p], defines=(f"HD={head_dim}",))
+    _call(f, _ptr(qkv), _ptr(q_w), _ptr(k_w), float(eps), _ptr(rope), _ptr(out), _ptr(cache_pages), _ptr(ctx.tok_pos), _ptr(ctx.tok_seq),
+          _ptr(ctx.page_table), ctx.page_table.shape[1], qkv.shape[0], n_heads, n_kv_heads, head_dim, page_size,
+          -int(chunk) if chunk else window, scale, int(ctx.max_kv_len), _ptr(part_o), _ptr(part_ml), _ptr(sink), float(softcap),
+          int(keep_first), _stream())
+    return True

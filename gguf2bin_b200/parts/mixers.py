@@ -293,28 +293,31 @@ class GQAAttention:
         nkv_own = 0 if self.shared_kv else self.nkv        # kv heads this layer projects
         nk = nkv_own * self.hd
         ws = ctx.workspace
-        q = ws.buffer("attn.q", (T, nq), self.dtype)
         fused = self.position.fused_rotation()
-        if fused is not None:
-            inv_freq, rot = fused
-            rope = ctx.rope_table(inv_freq) if inv_freq is not None else None
-            kernels.qknorm_rope_cache(qkv, self.nh, nkv_own, self.hd, self.q_norm_w,
-                                      self.k_norm_w, self.qk_eps, rope, rot, ctx.tok_pos,
-                                      ctx.tok_seq, ctx.page_table, view.pages, view.page_size, q)
-        else:
-            k = ws.buffer("attn.k", (T, nk), self.dtype)
-            v = ws.buffer("attn.v", (T, nk), self.dtype)
-            kernels.qknorm_rope_cache(qkv, self.nh, nkv_own, self.hd, self.q_norm_w,
-                                      self.k_norm_w, self.qk_eps, None, 0, ctx.tok_pos,
-                                      ctx.tok_seq, None, None, view.page_size, q, k, v)
-            self.position.apply(q, k, ctx)
-            if nkv_own:
-                kernels.cache_write(k, v, self.nkv, self.hd, ctx.tok_pos, ctx.tok_seq,
-                                    ctx.page_table, view.pages, view.page_size)
         o = ws.buffer("attn.o", (T, nq), self.dtype)
-        kernels.attention(q, o, view.pages, ctx, self.nh, self.nkv, self.hd, view.page_size,
-                          self.window, self.scale, sink=self.sink, chunk=self.chunk, softcap=self.softcap,
-                          keep_first=self.keep_first)
+        rope = ctx.rope_table(fused[0]) if fused is not None and fused[0] is not None else None
+        if fused is None or not nkv_own or not kernels.attention_qkv(
+                qkv, self.q_norm_w, self.k_norm_w, self.qk_eps, rope, fused[1], o, view.pages, ctx, self.nh, self.nkv, self.hd,
+                view.page_size, self.window, self.scale, sink=self.sink, chunk=self.chunk, softcap=self.softcap,
+                keep_first=self.keep_first):
+            q = ws.buffer("attn.q", (T, nq), self.dtype)
+            if fused is not None:
+                kernels.qknorm_rope_cache(qkv, self.nh, nkv_own, self.hd, self.q_norm_w,
+                                          self.k_norm_w, self.qk_eps, rope, fused[1], ctx.tok_pos,
+                                          ctx.tok_seq, ctx.page_table, view.pages, view.page_size, q)
+            else:
+                k = ws.buffer("attn.k", (T, nk), self.dtype)
+                v = ws.buffer("attn.v", (T, nk), self.dtype)
+                kernels.qknorm_rope_cache(qkv, self.nh, nkv_own, self.hd, self.q_norm_w,
+                                          self.k_norm_w, self.qk_eps, None, 0, ctx.tok_pos,
+                                          ctx.tok_seq, None, None, view.page_size, q, k, v)
+                self.position.apply(q, k, ctx)
+                if nkv_own:
+                    kernels.cache_write(k, v, self.nkv, self.hd, ctx.tok_pos, ctx.tok_seq,
+                                        ctx.page_table, view.pages, view.page_size)
+            kernels.attention(q, o, view.pages, ctx, self.nh, self.nkv, self.hd, view.page_size,
+                              self.window, self.scale, sink=self.sink, chunk=self.chunk, softcap=self.softcap,
+                              keep_first=self.keep_first)
         if self.out_scale != 1.0:
             og = ws.buffer("attn.gated", (T, nq), self.dtype)
             kernels.gate_mul(o, self.hd, None, self.nh, self.hd, self.out_scale, og)
