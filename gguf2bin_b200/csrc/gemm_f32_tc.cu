@@ -1,0 +1,450 @@
+// float32 products of many rows on the 5th-generation tensor cores:  C[M,N] (=|+=) A[M,K] * W[N,K]^T, everything float.
+//
+// A float is the sum of three bfloat16, x = x1 + x2 + x3, each the rest of the one before rounded to nearest (24 bits in 3 x 8 and two
+// signs; what is left is below 2^-26 of x).  Of the nine products of two such sums the six largest,
+//   a1 w3 + a3 w1 + a2 w2 + a1 w2 + a2 w1 + a1 w1,
+// are exact in 32 bits; the three left out are below 2^-25 of a1 w1.  The tensor cores' own sums cut low bits off, so they are kept
+// short: for every 64-wide block of K the 24 products of 16 are added in a fresh accumulator, the small ones first (the cuts then fall
+// on a small sum, and on the four last products), and a block's sum is added to a float in registers, rounded to nearest, block after block.
+// That is the order of sums of gemm_simt.cu (chunks of 64, then the chunks), with other rounding inside a chunk.
+// Relative error against 64 bits (2-norm, normal entries): 0.8 to 1.2e-7 for K = 68 to 3,072, where gemm_simt.cu has 1.5 to 1.9e-7; the largest
+// difference over the sum of magnitudes is 0.4 to 0.6 of that kernel's.
+//
+// Two launches.  `split_kernel` writes the three parts of A and W, [3 * rows][K] each, a warp a row, and says for every row whether the sum of
+// three is good for it.  `gemm_f32_tc_kernel`: a pair of CTAs takes a 256 x 256 tile (cta_group::2: each brings its own 128 rows of A and half
+// of W's 256) and, where the tiles are fewer than the SMs, a part of K (up to four pairs in a cluster, each of which adds all pairs' sums, in
+// their order, for a range of columns).  Roles by warp:
+//   warp 8   copies: per block of K the three parts of A and of W (128-byte swizzle), two blocks in flight; a part's place is filled again
+//            as soon as the last product that reads it is done
+//   warp 9   products, in the pair's first CTA: 24 tcgen05.mma a block (kind::f16, M = N = 256, K = 16) into one of two accumulators
+//   warps 0-7  add: warp w reads lanes 32 (w % 4) .. + 31 and columns 128 (w / 4) .. + 127 of a finished accumulator and adds them to its
+//              128 floats a thread, while the other accumulator is filled; at the end they write C, through shared memory, in rows
+//
+// Rows with an entry that is not finite, or whose largest entry is 2^120 and more (its parts may round to infinity) or below 2^-80 (its third
+// part would fall under bfloat16's range), are flagged; an output of a flagged row of A or W is summed from the floats themselves in the order
+// of gemm_simt.cu, by the warps that would have written it.
+//
+// What bounds it: the tensor cores do six products for one and need a block's 24 in 3,072 cycles (128 x 256 x 64 a CTA at 8,192 operations a
+// cycle), in which the copies bring 96 KB a CTA from the L2; with 128 x 128 tiles a CTA, or 256 x 128 a pair (96 and 72 KB in 1,536 cycles),
+// the L2's rate bounded it (about 10 TB/s, 2,070 cycles a block).
+// Measured: 3,065 cycles a block at the 1.57 GHz that the clock falls to.  701 rows, parts included: 45 us for 4096 x 1024, 50 for 6144 x 1024, 38
+// for 1024 x 2048, 51 for 1024 x 3072 (228, 230, 140 and 210 by gemm_f32_tile_kernel); 2,100 rows: 127 us for 6144 x 1024, 208 TFLOP/s (685).
+//
+// Every wait gives up after a bounded number of polls and leaves a code in `*status`, as in gemm_tc.cu.
+#include "common.cuh"
+#include "mma.cuh"
+#include "tc_common.cuh"
+
+#include <math.h>
+
+G2B_DEFINE_LAST_ERROR
+
+using namespace tc;
+
+constexpr int BM = 128, BN = 256, BK = 64;               // BM: rows of a CTA
+constexpr int PART_BYTES = BM * BK * 2;                  // one part of a CTA's rows of A, or of its half of W
+static_assert(BN / 2 == BM, "the parts of A and W have one size");
+constexpr int STAGES = 2, SLOT_BYTES = 2 * PART_BYTES;   // a slot: the part p of A and of W; slots [stage][p]
+constexpr int ADDERS = 8, THREADS = (ADDERS + 4) * 32;    // the last two warps only complete a group of four
+// Registers: 384 threads start with 168 each (64,512); the adders hold 128 sums and take 224, the others keep 40: 256 * 224 + 128 * 40 = 62,464.
+constexpr int ADDER_REGS = 224, OTHER_REGS = 40;
+constexpr int COLS = BN / 2;                             // columns of an adder
+constexpr int SPLIT_MOST = 4;
+constexpr int SUM_CHUNK = 64;
+constexpr int RING_BYTES = STAGES * 3 * SLOT_BYTES;
+constexpr int PITCH = 36;                                // floats a row of an adder's 32 x 32 outputs on their way to C
+constexpr int OUT_BYTES = ADDERS * 32 * PITCH * 4;
+constexpr int RECEIVED_BYTES = (SPLIT_MOST - 1) * (BN / SPLIT_MOST) * BM * 4;          // 96 KB; 64 with two parts
+constexpr int SMEM = RING_BYTES + 1024 + 256;            // + the swizzle's alignment, + barriers
+static_assert(RECEIVED_BYTES + OUT_BYTES <= RING_BYTES, "both lie where the ring was");
+enum { ST_PRODUCER_TIMEOUT = 21, ST_MMA_TIMEOUT = 22, ST_ADDER_TIMEOUT = 23 };
+
+// ---- parts ---------------------------------------------------------------------------------------------
+// Two floats as their parts, packed pairs of bfloat16.
+__device__ __forceinline__ void split2(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    p[i] = pack_bf16(x, y);
+    x -= __uint_as_float(p[i] << 16);
+    y -= __uint_as_float(p[i] & 0xffff0000u);
+  }
+}
+
+// A warp a row of A (rows 0 .. M - 1) or of W (M .. M + N - 1); `ld` is the parts' row length, a multiple of 8, zeros behind K.
+__global__ void __launch_bounds__(256)
+split_kernel(const float *A, const float *__restrict__ W, int M, int N, int K, int lda, int ldw, bf16 *parts_a, bf16 *parts_w, int ld, int *flags) {
+  pdl_launch();
+  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  pdl_wait();
+  if (r >= M + N) return;
+  const bool of_a = r < M;
+  const float *x = of_a ? A + (size_t)r * lda : W + (size_t)(r - M) * ldw;
+  const size_t plane = (size_t)(of_a ? M : N) * ld;
+  bf16 *to = (of_a ? parts_a + (size_t)r * ld : parts_w + (size_t)(r - M) * ld);
+  float most = 0.f, odd = 0.f;
+  constexpr int AHEAD = 2;
+  for (int k0 = lane * 8; k0 < ld; k0 += 256 * AHEAD) {
+    float4 v[AHEAD][2];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int k = k0 + 256 * u;                        // K is a multiple of 4
+      v[u][0] = k < K ? *reinterpret_cast<const float4 *>(x + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[u][1] = k + 4 < K ? *reinterpret_cast<const float4 *>(x + k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int k = k0 + 256 * u;
+      if (k >= ld) continue;
+      uint32_t p[4][3];
+      split2(v[u][0].x, v[u][0].y, p[0]);
+      split2(v[u][0].z, v[u][0].w, p[1]);
+      split2(v[u][1].x, v[u][1].y, p[2]);
+      split2(v[u][1].z, v[u][1].w, p[3]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4 *>(to + i * plane + k) = make_uint4(p[0][i], p[1][i], p[2][i], p[3][i]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float first = __uint_as_float(p[i][0] << 16), second = __uint_as_float(p[i][0] & 0xffff0000u);
+        most = fmaxf(most, fmaxf(fabsf(first), fabsf(second)));
+        odd = fmaf(first, 0.f, fmaf(second, 0.f, odd));  // NaN behind an infinity or a NaN
+      }
+    }
+  }
+  most = warp_max(most);
+  odd = warp_sum(odd);
+  if (lane == 0) flags[r] = !(odd == 0.f) || most >= 0x1p120f || (most > 0.f && most < 0x1p-80f);
+}
+
+// ---- the product -----------------------------------------------------------------------------------------
+__device__ __forceinline__ void st_cluster16(uint32_t addr, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+// Maps of the parts: [3 M][K] and [3 N][K], boxes of 128 rows.  Rows behind the last of a part belong to the next one (or are zeros):
+// they fill rows and columns of the tile that are not written.
+template <bool ACCUM, int SPLIT>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const float *A,
+                   const float *__restrict__ W, float *C, int M, int N, int K, int lda, int ldw, int ldc, const int *flags,
+                   int *__restrict__ status) {
+  pdl_launch();
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + RING_BYTES);
+  const uint32_t full0 = smem_addr(bars), empty0 = full0 + 8 * 3 * STAGES, sum_full0 = empty0 + 8 * 3 * STAGES, sum_empty0 = sum_full0 + 16;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 6 * STAGES + 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank(), half = rank & 1, first = rank & ~1u;          // the pair's first CTA issues its products
+  const int part = (int)(rank >> 1);
+  const int n0 = (int)(blockIdx.x / (2 * SPLIT)) * BN, m0 = (int)blockIdx.y * 2 * BM + (int)half * BM;
+  const int all = (K + BK - 1) / BK, per = (all + SPLIT - 1) / SPLIT;
+  const int kb0 = part * per, nkb = max(0, min(all, kb0 + per) - kb0);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 3 * STAGES; ++s) {
+      mbar_init(full0 + 8 * s, 1);               // in the first CTA, with both CTAs' bytes
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(sum_full0 + 8 * b, 1);
+      mbar_init(sum_empty0 + 8 * b, 2 * ADDERS); // in the first CTA: both CTAs' adders
+    }
+    mbar_init_fence();
+  }
+  if (warp == ADDERS + 1) tmem_alloc_pair(smem_addr(tmem_slot), 2 * BN);
+  tc_fence_before();
+  cluster_sync_all();                            // both CTAs' barriers and tensor memory exist
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();
+
+  const int row0 = 32 * (warp % 4), col0 = COLS * (warp / 4);                // an adder's first row and column of the CTA's tile
+  uint32_t row_flags = 0, col_flags[COLS / 32] = {};       // a bit a row, a bit a column
+  // Parts of K: pair p owns range p of SPLIT ranges of columns; every pair sends the others theirs, and a pair adds them in the order of
+  // the parts.
+  if (warp >= ADDERS) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(OTHER_REGS));
+    if (warp == ADDERS && lane == 0 && PRODUCER_RUNS) {
+      const uint32_t first_full0 = map_to_cta(full0, first);
+      bool ok = true;
+      for (int i = 0; i < nkb && ok; ++i) {
+        const int k = (kb0 + i) * BK;
+#pragma unroll
+        for (int p = 2; p >= 0; --p) {           // in the order in which the places become free
+          const int s = (i % STAGES) * 3 + p;
+          if (i >= STAGES && !mbar_wait(empty0 + 8 * s, (i / STAGES - 1) & 1)) {
+            atomicExch(status, ST_PRODUCER_TIMEOUT);
+            ok = false;
+            break;
+          }
+          const uint32_t to = smem_addr(smem + s * SLOT_BYTES);
+          if (half == 0) mbar_expect_tx(full0 + 8 * s, 2 * SLOT_BYTES);
+          tma_load_2d_pair(to, &map_a, k, p * M + m0, first_full0 + 8 * s);
+          tma_load_2d_pair(to + PART_BYTES, &map_w, k, p * N + n0 + (int)half * BM, first_full0 + 8 * s);
+        }
+      }
+    }
+    if (warp == ADDERS + 1 && lane == 0 && half == 0) {
+      constexpr uint32_t idesc = instr_desc(2 * BM, BN, false);
+      const uint16_t both = (uint16_t)(3u << rank);
+      bool ok = true;
+      for (int i = 0; i < nkb && ok; ++i) {
+        const int b = i & 1, s0 = (i % STAGES) * 3;
+        const uint32_t at = smem_addr(smem + s0 * SLOT_BYTES), parity = (i / STAGES) & 1;
+        auto arrived = [&](int p) { return mbar_wait(full0 + 8 * (s0 + p), parity); };
+        auto products = [&](int pa, int pw, uint32_t fresh) {
+          const uint64_t da = desc_k_major(at + pa * SLOT_BYTES), db = desc_k_major(at + pw * SLOT_BYTES + PART_BYTES);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) umma_bf16_pair(tmem + b * BN, da + 2 * k, db + 2 * k, idesc, (fresh && k == 0) ? 0u : 1u);
+        };
+        ok = (i < 2 || mbar_wait_cluster(sum_empty0 + 8 * b, (i / 2 - 1) & 1)) && arrived(2) && arrived(0);
+        if (ok) {
+          tc_fence_after();
+          products(0, 2, 1);
+          products(2, 0, 0);
+          umma_commit_pair(empty0 + 8 * (s0 + 2), both);
+          ok = arrived(1);
+        }
+        if (!ok) {
+          atomicExch(status, ST_MMA_TIMEOUT);
+          break;
+        }
+        tc_fence_after();
+        products(1, 1, 0);
+        products(0, 1, 0);
+        products(1, 0, 0);
+        umma_commit_pair(empty0 + 8 * (s0 + 1), both);
+        products(0, 0, 0);
+        umma_commit_pair(empty0 + 8 * s0, both);
+        umma_commit_pair(sum_full0 + 8 * b, both);
+      }
+    }
+    __syncwarp();
+    if (SPLIT > 1) {
+      cluster_sync_all();
+      cluster_sync_all();
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(ADDER_REGS));
+    float sum[COLS];
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+    row_flags = __ballot_sync(0xffffffffu, m0 + row0 + lane < M && flags[m0 + row0 + lane] != 0);
+#pragma unroll
+    for (int h = 0; h < COLS / 32; ++h) {
+      const int n = n0 + col0 + 32 * h + lane;
+      col_flags[h] = __ballot_sync(0xffffffffu, n < N && flags[M + n] != 0);
+    }
+    const uint32_t first_empty0 = map_to_cta(sum_empty0, first);
+    const uint32_t mine = tmem + ((uint32_t)row0 << 16) + col0;
+    for (int i = 0; i < nkb; ++i) {
+      const int b = i & 1;
+      if (!mbar_wait(sum_full0 + 8 * b, (i / 2) & 1)) {
+        if (lane == 0) atomicExch(status, ST_ADDER_TIMEOUT);
+        break;
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int h = 0; h < COLS / 32; ++h) {
+        uint32_t v[32];
+        tmem_ld32(mine + b * BN + 32 * h, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum[32 * h + j] += __uint_as_float(v[j]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(first_empty0 + 8 * b);
+    }
+    constexpr int RANGE = BN / SPLIT, OWN = COLS < RANGE ? COLS : RANGE;         // columns of a pair, of them in an adder's reach
+    if (SPLIT > 1) {
+      cluster_sync_all();                                  // all rings are free
+      // [source among the others][piece of four columns of the range][row] float4
+      auto place = [&](int source, int col) { return ((source * (RANGE / 4) + col % RANGE / 4) * BM + row0 + lane) * 16; };
+#pragma unroll
+      for (int j0 = 0; j0 < COLS; j0 += OWN) {
+        const int to = (col0 + j0) / RANGE;
+        if (to == part) continue;
+        const uint32_t at = map_to_cta(smem_addr(smem) + place(part - (part > to), col0 + j0), 2 * to + half);
+#pragma unroll
+        for (int j = 0; j < OWN; j += 4) st_cluster16(at + j / 4 * BM * 16, make_float4(sum[j0 + j], sum[j0 + j + 1], sum[j0 + j + 2], sum[j0 + j + 3]));
+      }
+      cluster_sync_all();
+#pragma unroll
+      for (int j0 = 0; j0 < COLS; j0 += OWN) {
+        if ((col0 + j0) / RANGE != part) continue;
+        const unsigned char *at = smem + place(0, col0 + j0);
+#pragma unroll
+        for (int j = 0; j < OWN; j += 4) {
+          float4 v[SPLIT];
+#pragma unroll
+          for (int o = 0; o < SPLIT - 1; ++o) v[o] = *reinterpret_cast<const float4 *>(at + ((o * (RANGE / 4) + j / 4) * BM) * 16);
+          const float4 mine4 = make_float4(sum[j0 + j], sum[j0 + j + 1], sum[j0 + j + 2], sum[j0 + j + 3]);
+          float4 t = part == 0 ? mine4 : v[0];
+#pragma unroll
+          for (int o = 1; o < SPLIT; ++o) {
+            const float4 x = o == part ? mine4 : (o < part ? v[o] : v[o - 1]);
+            t.x += x.x; t.y += x.y; t.z += x.z; t.w += x.w;
+          }
+          sum[j0 + j] = t.x; sum[j0 + j + 1] = t.y; sum[j0 + j + 2] = t.z; sum[j0 + j + 3] = t.w;
+        }
+      }
+    }
+    if (m0 + row0 < M) {
+      float *const mid = reinterpret_cast<float *>(smem + RECEIVED_BYTES) + warp * 32 * PITCH;
+      const bool vector = ldc % 4 == 0 && ((uintptr_t)C & 15) == 0;
+#pragma unroll
+      for (int h = 0; h < COLS / 32; ++h) {
+        if ((col0 + 32 * h) / RANGE != part) continue;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<float4 *>(mid + lane * PITCH + 4 * j) =
+              make_float4(sum[32 * h + 4 * j], sum[32 * h + 4 * j + 1], sum[32 * h + 4 * j + 2], sum[32 * h + 4 * j + 3]);
+        __syncwarp();
+        const int c = 4 * (lane % 8), n = n0 + col0 + 32 * h + c;               // a lane's columns: eight lanes a row
+        const uint32_t flagged = col_flags[h] >> c & 15;
+        if (n < N) {
+#pragma unroll 4
+          for (int i = 0; i < 8; ++i) {
+            const int r = 4 * i + lane / 8, m = m0 + row0 + r;
+            if (m >= M) break;
+            float4 v = *reinterpret_cast<const float4 *>(mid + r * PITCH + c);
+            float *to = C + (size_t)m * ldc + n;
+            const uint32_t odd = flagged | (row_flags >> r & 1 ? 15u : 0u);
+            if (vector && !odd && n + 4 <= N) {
+              if (ACCUM) {
+                const float4 old = *reinterpret_cast<const float4 *>(to);
+                v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
+              }
+              *reinterpret_cast<float4 *>(to) = v;
+            } else {
+              const float each[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                if (n + e >= N) break;
+                float x = each[e];
+                if (odd >> e & 1) {
+                  const float *a = A + (size_t)m * lda, *w = W + (size_t)(n + e) * ldw;
+                  x = 0.f;
+                  for (int k0 = 0; k0 < K; k0 += SUM_CHUNK) {
+                    float chunk = 0.f;
+#pragma unroll 4
+                    for (int k = k0; k < min(K, k0 + SUM_CHUNK); ++k) chunk = fmaf(a[k], w[k], chunk);
+                    x += chunk;
+                  }
+                }
+                to[e] = ACCUM ? to[e] + x : x;
+              }
+            }
+          }
+        }
+        __syncwarp();
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_all();                            // neither CTA's products, copies and arrivals meet a peer that is gone
+  if (warp == ADDERS + 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem, 2 * BN);
+  }
+}
+
+template <bool ACCUM, int SPLIT>
+static cudaError_t allow(int &clusters) {
+  cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<ACCUM, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * SPLIT), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = SMEM;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2 * SPLIT, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr, cfg.numAttrs = 1;
+  return cudaOccupancyMaxActiveClusters(&clusters, gemm_f32_tc_kernel<ACCUM, SPLIT>, &cfg);
+}
+// How many clusters of one, two and four pairs the device holds at once.
+struct Clusters { int of[SPLIT_MOST + 1]; };
+static int count_clusters(Clusters &out) {
+  static G2bPerDevice configured;
+  static Clusters kept[G2B_MAX_DEVICES];
+  const int dev = g2b_current_device();
+  if (dev >= 0 && configured.value[dev]) {
+    out = kept[dev];
+    return 0;
+  }
+  cudaError_t e = allow<false, 1>(out.of[1]);
+  if (e == cudaSuccess) e = allow<true, 1>(out.of[1]);
+  if (e == cudaSuccess) e = allow<false, 2>(out.of[2]);
+  if (e == cudaSuccess) e = allow<true, 2>(out.of[2]);
+  if (e == cudaSuccess) e = allow<false, 4>(out.of[4]);
+  if (e == cudaSuccess) e = allow<true, 4>(out.of[4]);
+  if (e != cudaSuccess || out.of[1] < 1) G2B_REFUSE("gemm_f32_tc: %d bytes of shared memory: %s", SMEM, cudaGetErrorString(e));
+  if (dev >= 0) {
+    kept[dev] = out;
+    configured.value[dev] = 1;
+  }
+  return 0;
+}
+
+// Pairs per tile.  A round takes its blocks of K and about as long as two and a half more for what stands around them, four with parts.
+static double rounds_of_blocks(int s, int tiles, int blocks, const Clusters &clusters) {
+  return (double)((tiles + clusters.of[s] - 1) / clusters.of[s]) * ((blocks + s - 1) / s + (s > 1 ? 4.0 : 2.5));
+}
+static int pick_split(int tiles, int blocks, const Clusters &clusters) {
+  int best = 1;
+  for (int s = 2; s <= SPLIT_MOST; s *= 2)
+    if (blocks >= 2 * s && clusters.of[s] > 0 && rounds_of_blocks(s, tiles, blocks, clusters) < rounds_of_blocks(best, tiles, blocks, clusters)) best = s;
+  return best;
+}
+static int tiles_of(int M, int N) { return ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN); }
+
+// Nanoseconds that both launches are estimated to take: the parts at 6.7 TB/s, a block 2.05 us under the clock that such products leave, and what a
+// launch takes whatever it does (fitted to 32 sizes of 32 to 2,100 rows, K = 1,024 to 3,072).
+extern "C" int g2b_gemm_f32_tc_estimate(int M, int N, int K) {
+  Clusters clusters;
+  if (count_clusters(clusters)) return 2000000000;
+  const int tiles = tiles_of(M, N), blocks = (K + BK - 1) / BK;
+  const double us = 7.0 + 1.5e-6 * ((double)M + N) * K + 2.05 * rounds_of_blocks(pick_split(tiles, blocks, clusters), tiles, blocks, clusters);
+  return us < 2e6 ? (int)(1e3 * us) : 2000000000;
+}
+
+template <int SPLIT>
+static void launch_product(bool accumulate, dim3 tiles, cudaStream_t stream, const CUtensorMap &map_a, const CUtensorMap &map_w, const float *A,
+                           const float *W, float *C, int M, int N, int K, int lda, int ldw, int ldc, const int *flags, int *status) {
+  const dim3 grid(tiles.x * 2 * SPLIT, tiles.y);
+  if (accumulate)
+    g2b_launch_cluster(gemm_f32_tc_kernel<true, SPLIT>, grid, dim3(THREADS), SMEM, stream, 2u * SPLIT, map_a, map_w, A, W, C, M, N, K, lda, ldw,
+                       ldc, flags, status);
+  else
+    g2b_launch_cluster(gemm_f32_tc_kernel<false, SPLIT>, grid, dim3(THREADS), SMEM, stream, 2u * SPLIT, map_a, map_w, A, W, C, M, N, K, lda, ldw,
+                       ldc, flags, status);
+}
+
+// Rows of A and W on 16 bytes, K a multiple of 4.  parts: bfloat16 [3 (M + N) * ld], ld = K rounded up to 8; flags: int [M + N].
+// accumulate: add into C.
+extern "C" int g2b_gemm_f32_tc(const float *A, const float *W, float *C, int M, int N, int K, int lda, int ldw, int ldc, int accumulate,
+                               void *parts, int *flags, int *status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || K % 4 || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)parts) & 15))
+    G2B_REFUSE("gemm_f32_tc: K=%d and row strides (%d, %d) must be multiples of 4, rows on 16 bytes", K, lda, ldw);
+  const int ld = (K + 7) / 8 * 8, tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (N + BN - 1) / BN;
+  if (3ll * M > INT32_MAX || 3ll * N > INT32_MAX || (long long)M + N > INT32_MAX || tiles_m > 65535)
+    G2B_REFUSE("gemm_f32_tc: M=%d, N=%d are too large for one launch", M, N);
+  bf16 *parts_a = (bf16 *)parts, *parts_w = parts_a + (size_t)3 * M * ld;
+  CUtensorMap map_a, map_w;
+  int rc = get_map(&map_a, parts_a, 3ll * M, ld, ld, BM);
+  if (!rc) rc = get_map(&map_w, parts_w, 3ll * N, ld, ld, BM);
+  if (rc) G2B_REFUSE("gemm_f32_tc: cuTensorMapEncodeTiled failed (%d)", rc);
+  Clusters clusters;
+  if (count_clusters(clusters)) return 1;
+  g2b_launch(split_kernel, dim3((unsigned)((M + (long long)N + 7) / 8)), dim3(256), 0, stream, A, W, M, N, K, lda, ldw, parts_a, parts_w, ld,
+             flags);
+  rc = g2b_check_launch("gemm_f32_tc split");
+  if (rc) return rc;
+  const int split = pick_split(tiles_of(M, N), (K + BK - 1) / BK, clusters);
+  const dim3 tiles((unsigned)tiles_n, (unsigned)tiles_m);
+  auto *launch = split == 4 ? launch_product<4> : (split == 2 ? launch_product<2> : launch_product<1>);
+  launch(accumulate != 0, tiles, stream, map_a, map_w, A, W, C, M, N, K, lda, ldw, ldc, flags, status);
+  return g2b_check_launch("gemm_f32_tc");
+}

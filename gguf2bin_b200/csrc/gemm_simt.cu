@@ -381,6 +381,11 @@ static int choose_f32(int M, int N, int K) {
   return best == F32_ROWS && (M + 7) / 8 > 65535 ? F32_TILE4 : best;
 }
 extern "C" int g2b_gemm_f32_kernel(int M, int N, int K) { return choose_f32(M, N, K); }
+// Nanoseconds that the kernel chosen for more than ROWS_MAX rows is estimated to take.
+extern "C" int g2b_gemm_f32_estimate(int M, int N, int K) {
+  const double us = fmin(fmin(us_general(M, N, K), us_rows(8, 16, 8, M, N, K)), fmin(us_tile(1, M, N, K), us_tile(4, M, N, K)));
+  return us < 2e6 ? (int)(1e3 * us) : 2000000000;
+}
 
 template <int EPI>
 static int launch_f32(const float *A, const float *W, void *C, int M, int N, int K, int lda, int ldw, int ldc, int which, cudaStream_t stream) {

@@ -5,7 +5,8 @@ from __future__ import annotations
 
 GENERIC_UNITS = [("elementwise.cu", ()), ("gemm_simt.cu", ()), ("attn_generic.cu", ()),
                  ("sampling.cu", ()), ("random_init.cu", ()), ("stream_ops.cu", ()),
-                 ("seq_mix.cu", ()), ("moe.cu", ()), ("channel_scan.cu", ()), ("chunk_scan.cu", ()), ("streams.cu", ())]
+                 ("seq_mix.cu", ()), ("moe.cu", ()), ("channel_scan.cu", ()), ("chunk_scan.cu", ()), ("streams.cu", ()),
+                 ("gemm_f32_tc.cu", ())]
 
 # head sizes built ahead of time (what the tests and the benchmark use)
 HEAD_SIZES = (64, 128)
@@ -27,4 +28,4 @@ def all_units() -> list:
 # that issues nothing, so that a test can see every other role give up and the kernel return.
 WAITS_RUN_OUT = ("G2B_SPIN_LIMIT=4096", "G2B_TEST_NO_PRODUCER")
 TEST_UNITS = [("gemm_tc.cu", WAITS_RUN_OUT), ("attn_prefill_tc.cu", ("HD=128",) + WAITS_RUN_OUT),
-              ("attn_prefill_tc_split.cu", ("HD=128",) + WAITS_RUN_OUT)]
+              ("attn_prefill_tc_split.cu", ("HD=128",) + WAITS_RUN_OUT), ("gemm_f32_tc.cu", WAITS_RUN_OUT)]

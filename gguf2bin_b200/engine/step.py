@@ -160,7 +160,7 @@ class Engine:
         waits gave up (its output is then invalid).  Reads a word from the device, so it waits
         for the stream; callers that are about to read logits or tokens on the host call it
         where they synchronise anyway."""
-        if self.model.dtype == torch.bfloat16:
+        if self.model.dtype == torch.bfloat16 or self.workspace.waits:
             from .. import kernels_bf16
             kernels_bf16.check_status()
 

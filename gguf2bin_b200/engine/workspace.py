@@ -13,6 +13,7 @@ class Workspace:
         self._views: dict = {}         # (name, shape, dtype) -> view of the buffer as it is now
         self.generation = 0            # bumps whenever a buffer moves (captured graphs go stale)
         self._refused: dict[str, int] = {}       # name -> bytes that the device did not have
+        self.waits = False             # a float32 step launched a kernel with bounded waits (bfloat16 steps always may)
 
     def buffer(self, name: str, shape, dtype: torch.dtype, most: int = 0) -> torch.Tensor:
         """The buffer of that name as a tensor of this shape.  ``most``: the bytes it may grow to (a larger request gets just what

@@ -111,10 +111,11 @@ def check_status() -> None:
             if code == 14:
                 raise KernelError(f"attn_prefill_tc on {dev}: dynamic shared memory does not start on a "
                                   "1024-byte boundary; nothing was computed")
-            kernel = "attn_prefill_tc" if code > 10 else "gemm_tc"
+            kernel = "gemm_f32_tc" if code > 20 else "attn_prefill_tc" if code > 10 else "gemm_tc"
             what = {1: "the TMA producer", 2: "the MMA issuer", 3: "the epilogue",
                     4: "a CTA of a pair, for its peer at the end of the kernel,",
-                    11: "the TMA producer", 12: "the MMA issuer", 13: "a softmax warp"}.get(code, "a role")
+                    11: "the TMA producer", 12: "the MMA issuer", 13: "a softmax warp",
+                    21: "the TMA producer", 22: "the MMA issuer", 23: "an adder"}.get(code, "a role")
             raise KernelError(f"{kernel} on {dev}: {what} gave up waiting on a barrier (code {code}); "
                               "the result of that launch is invalid")
 

@@ -332,7 +332,7 @@ class GatedPreNormBlock:
             if self.taps > 1:
                 keep = (h, ring, self.taps)
         gate = ws.buffer("gated.gate", (T, H), self.dtype)
-        kernels.linear(h, self.g1, gate)
+        kernels.linear(h, self.g1, gate, workspace=ctx.workspace)
         y = ws.buffer("gated.result", (T, H), torch.float32)
         if hasattr(self.mixer, "forward_into"):
             self.mixer.forward_into(u, ctx, view.get("mixer"), y, keep=keep)
@@ -361,7 +361,7 @@ class GatedPreNormBlock:
         if self._g2_rides:
             gate = ff.side_out
         else:
-            kernels.linear(h, self.g2, gate)
+            kernels.linear(h, self.g2, gate, workspace=ctx.workspace)
         self._add_or_leave(ctx, x32, y, gate, self.b2)
 
     @staticmethod

@@ -116,7 +116,7 @@ class LMHead:
 
     def forward(self, h: torch.Tensor, logits32: torch.Tensor, ctx) -> None:
         """logits32 [n, vocab] float32 = h [n, hidden] . matrix^T."""
-        kernels.linear(h, self.matrix, logits32)
+        kernels.linear(h, self.matrix, logits32, workspace=ctx.workspace)
 
 
 class PairEmbedding:

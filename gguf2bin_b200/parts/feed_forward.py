@@ -93,9 +93,9 @@ class SwiGLU:
         mid = ws.buffer("ffn.mid", (T, self.inter), self.dtype)
         if not kernels.gate_up_fused(h, self.w_gate_up, mid, self.block, self.form):
             gu = ws.buffer("ffn.gate_up", (T, 2 * self.inter), self.dtype)
-            kernels.linear(h, self.w_gate_up, gu)
+            kernels.linear(h, self.w_gate_up, gu, workspace=ctx.workspace)
             kernels.swiglu(gu, mid, self.block, form=self.form)
-        kernels.linear(mid, self.w_down, out32, accumulate=accumulate)
+        kernels.linear(mid, self.w_down, out32, accumulate=accumulate, workspace=ctx.workspace)
 
     def forward_from_stream(self, x32: torch.Tensor, norm, ctx, residual32: torch.Tensor) -> None:
         """The same with the block's norm folded into the gate/up product."""
@@ -105,7 +105,7 @@ class SwiGLU:
             return self.forward(h, ctx, residual32)
         mid = ctx.workspace.buffer("ffn.mid", (x32.shape[0], self.inter), self.dtype)
         normed_linear(x32, norm, self.w_gate_up, mid, ctx, gate_block=self.block)
-        kernels.linear(mid, self.w_down, residual32, accumulate=True)
+        kernels.linear(mid, self.w_down, residual32, accumulate=True, workspace=ctx.workspace)
 
 
 class ActMLP:
@@ -177,10 +177,10 @@ class ActMLP:
         if self.activation == "gelu_tanh" and not self.n_side:
             mid = ws.buffer("mlp.mid", (T, self.inter), self.dtype)
             if kernels.linear_act(h, self.w_up, mid, kernels.GluForm.gelu_tanh()):
-                kernels.linear(mid, self.w_down, out32, accumulate=accumulate)
+                kernels.linear(mid, self.w_down, out32, accumulate=accumulate, workspace=ctx.workspace)
                 return
         up = ws.buffer("mlp.up", (T, self.w_up.shape[0]), self.dtype)
-        kernels.linear(h, self.w_up, up)
+        kernels.linear(h, self.w_up, up, workspace=ctx.workspace)
         self.side_out = up[:, self.inter:self.inter + self.n_side] if self.n_side else None
         mid = ws.buffer("mlp.mid", (T, self.inter), self.dtype)
         if self.activation == "relu2":
@@ -189,7 +189,7 @@ class ActMLP:
             kernels.act_form(up[:, :self.inter], mid, kernels.GluForm.gelu_tanh())
         else:
             kernels.xielu(up[:, :self.inter], self.act, mid)
-        kernels.linear(mid, self.w_down, out32, accumulate=accumulate)
+        kernels.linear(mid, self.w_down, out32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 class RoutedExperts:
@@ -344,7 +344,7 @@ class RoutedExperts:
         """Routing, plan and the experts' products: (rows, pair -> row, weights)."""
         T, ws, top, E = h.shape[0], ctx.workspace, self.top, self.E
         z = ws.buffer("moe.logits", (T, E + self.I), torch.float32)
-        kernels.linear(h, self.w_router, z)
+        kernels.linear(h, self.w_router, z, workspace=ctx.workspace)
         idx = ws.buffer("moe.idx", (T, top), torch.int32)
         weight = ws.buffer("moe.weight", (T, top), torch.float32)
         n_pairs = T * top

@@ -28,8 +28,8 @@ def normed_linear(x32: torch.Tensor, norm, w: torch.Tensor, out: torch.Tensor, c
     h = ctx.workspace.buffer("fused.normed", (n, x32.shape[1]), ctx.dtype)
     norm.forward(x32, h, rows)
     if gate_block is None:
-        kernels.linear(h, w, out)
+        kernels.linear(h, w, out, workspace=ctx.workspace)
     elif not kernels.gate_up_fused(h, w, out, gate_block):
         gu = ctx.workspace.buffer("fused.gate_up", (n, w.shape[0]), ctx.dtype)
-        kernels.linear(h, w, gu)
+        kernels.linear(h, w, gu, workspace=ctx.workspace)
         kernels.swiglu(gu, out, gate_block)

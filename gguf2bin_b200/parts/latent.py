@@ -253,7 +253,7 @@ class LatentAttention:
         if view is None or view.planes != 1:
             raise kernels.KernelError("latent_attention: needs latent pages (one panel per page)")
         proj = ws.buffer("latent.in", (T, self.w_in.shape[0]), self.dtype)
-        kernels.linear(u, self.w_in, proj)
+        kernels.linear(u, self.w_in, proj, workspace=ctx.workspace)
         q = proj[:, :self.n_q]
         d = proj[:, self.n_q:self.n_q + self.n_c] if self.n_c else None
         gate = proj[:, self.n_q + self.n_c:self.n_q + self.n_c + self.n_g] if self.n_g else None
@@ -264,7 +264,7 @@ class LatentAttention:
             cq = ws.buffer("latent.cq", (T, self.q_rank), self.dtype)
             kernels.latent_pair(d, self.rank, self.c_norm, view.pages, q, self.q_norm, cq, self.eps, ctx)
             q = ws.buffer("latent.uq", (T, self.w_uq.shape[0]), self.dtype)
-            kernels.linear(cq, self.w_uq, q)
+            kernels.linear(cq, self.w_uq, q, workspace=ctx.workspace)
         elif self.rot:
             if ring is not None:
                 kernels.latent_keep(None, None, 0.0, None, rows, ring, taps, ctx)
@@ -291,7 +291,7 @@ class LatentAttention:
         else:
             o = ws.buffer("latent.o", (T, self.nh * self.dv), self.dtype)
             self._per_head(mix, self.w_uv, o, True, gate)
-        kernels.linear(o, self.w_o, out32, accumulate=accumulate)
+        kernels.linear(o, self.w_o, out32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 register_mixer("latent_attention", LatentAttention)

@@ -229,13 +229,13 @@ class GQAAttention:
     # ---- step ----------------------------------------------------------------
     def forward(self, h: torch.Tensor, ctx, view: KVView, residual32: torch.Tensor) -> None:
         qkv = ctx.workspace.buffer("attn.qkv", (h.shape[0], self.w_qkv.shape[0]), self.dtype)
-        kernels.linear(h, self.w_qkv, qkv)
+        kernels.linear(h, self.w_qkv, qkv, workspace=ctx.workspace)
         self._attend(qkv, ctx, view, residual32)
 
     def forward_store(self, h: torch.Tensor, ctx, view: KVView, out32: torch.Tensor) -> None:
         """Stores the result instead of adding it."""
         qkv = ctx.workspace.buffer("attn.qkv", (h.shape[0], self.w_qkv.shape[0]), self.dtype)
-        kernels.linear(h, self.w_qkv, qkv)
+        kernels.linear(h, self.w_qkv, qkv, workspace=ctx.workspace)
         self._attend(qkv, ctx, view, out32, accumulate=False)
 
     def forward_from_stream(self, x32: torch.Tensor, norm, ctx, view: KVView,
@@ -283,7 +283,7 @@ class GQAAttention:
             og = ctx.workspace.buffer("attn.gated", (T, no), self.dtype)
             kernels.gate_mul(o, hd, gate, self.nh, self.vd, self.out_scale, og)
             o = og
-        kernels.linear(o, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(o, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
     def _attend(self, qkv: torch.Tensor, ctx, view: KVView, residual32: torch.Tensor, accumulate: bool = True) -> None:
         if self.wide:
@@ -322,7 +322,7 @@ class GQAAttention:
             og = ws.buffer("attn.gated", (T, nq), self.dtype)
             kernels.gate_mul(o, self.hd, None, self.nh, self.hd, self.out_scale, og)
             o = og
-        kernels.linear(o, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(o, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 class DiffAttention(GQAAttention):
@@ -368,7 +368,7 @@ class DiffAttention(GQAAttention):
     def _project_out(self, o, qkv, gate_at: int, ctx, residual32, accumulate: bool) -> None:
         og = ctx.workspace.buffer("attn.gated", (o.shape[0], self.H * self.vd), self.dtype)
         kernels.diff_combine(o, self.H, self.cache_hd, self.vd, self.lam, self.out_eps, (1.0 - self.diff) * self.out_scale, og)
-        kernels.linear(og, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(og, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 register_mixer("gqa_attention", GQAAttention)

@@ -132,7 +132,7 @@ class RetentionMixer:
         T, ws = h.shape[0], ctx.workspace
         nq, nv = self.H * self.D, self.H * self.V
         proj = ws.buffer("retention.in", (T, 2 * nq + 2 * nv), self.dtype)
-        kernels.linear(h, self.w_in, proj)
+        kernels.linear(h, self.w_in, proj, workspace=ctx.workspace)
         inv_freq, rot, interleaved = self.position.table_rotation()
         rope = ctx.rope_table(inv_freq) if inv_freq is not None else None
         o32 = ws.buffer("retention.o", (T, nv), torch.float32)
@@ -141,7 +141,7 @@ class RetentionMixer:
                            interleaved=interleaved, k_scale=self.k_scale)
         og = ws.buffer("retention.gated", (T, nv), self.dtype)
         kernels.head_norm_gate(o32, self.H, self.V, None, self.eps, proj[:, 2 * nq + nv:], self.out_scale, og)
-        kernels.linear(og, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(og, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 class GatedDeltaMixer:
@@ -215,9 +215,9 @@ class GatedDeltaMixer:
         T, ws = h.shape[0], ctx.workspace
         C, nq, nv = self.channels, self.G * self.D, self.H * self.V
         proj = ws.buffer("delta.in", (T, C + nv), self.dtype)
-        kernels.linear(h, self.w_in, proj)
+        kernels.linear(h, self.w_in, proj, workspace=ctx.workspace)
         ab = ws.buffer("delta.ab", (T, 2 * self.H), torch.float32)
-        kernels.linear(h, self.w_ab, ab)
+        kernels.linear(h, self.w_ab, ab, workspace=ctx.workspace)
         mixed = ws.buffer("delta.conv", (T, C), self.dtype)
         ring = view["conv"].states if self.taps > 1 else None
         kernels.short_conv(proj[:, :C], self.w_conv, ring, ctx, mixed, act=True)
@@ -227,7 +227,7 @@ class GatedDeltaMixer:
                            q_scale=self.D ** -0.5, unit_eps=self.unit_eps)
         og = ws.buffer("delta.gated", (T, nv), self.dtype)
         kernels.head_norm_gate(o32, self.H, self.V, self.norm_w, self.eps, proj[:, C:], self.out_scale, og)
-        kernels.linear(og, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(og, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 def _padded_rows(parts, multiple: int = 8):
@@ -313,7 +313,7 @@ class SSDMixer:
         T, ws = h.shape[0], ctx.workspace
         inner, C, gn = self.inner, self.channels, self.G * self.N
         proj = ws.buffer("ssd.in", (T, self.w_in.shape[0]), self.dtype)
-        kernels.linear(h, self.w_in, proj)
+        kernels.linear(h, self.w_in, proj, workspace=ctx.workspace)
         mixed = ws.buffer("ssd.conv", (T, C), self.dtype)
         ring = view["conv"].states if self.taps > 1 else None
         kernels.short_conv(proj[:, inner:inner + C], self.w_conv, ring, ctx, mixed, act=True, bias=self.b_conv)
@@ -326,7 +326,7 @@ class SSDMixer:
         kernels.state_readout(o32, self.H, self.V, og, skip_x=mixed[:, :inner], skip_w=self.skip, gate=proj[:, :inner],
                               gate_act="silu", gate_first=True, group=inner // self.norm_groups, eps=self.eps,
                               w=self.norm_w)
-        kernels.linear(og, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(og, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 class SelectiveSSM:
@@ -388,18 +388,18 @@ class SelectiveSSM:
         T, ws = h.shape[0], ctx.workspace
         inner, N, R = self.inner, self.N, self.R
         proj = ws.buffer("ssm.in", (T, self.w_in.shape[0]), self.dtype)
-        kernels.linear(h, self.w_in, proj)
+        kernels.linear(h, self.w_in, proj, workspace=ctx.workspace)
         x = ws.buffer("ssm.conv", (T, inner), self.dtype)
         ring = view["conv"].states if self.taps > 1 else None
         kernels.short_conv(proj[:, :inner], self.w_conv, ring, ctx, x, act=True, bias=self.b_conv)
         p = ws.buffer("ssm.x", (T, self.w_x.shape[0]), self.dtype)
-        kernels.linear(x, self.w_x, p)
+        kernels.linear(x, self.w_x, p, workspace=ctx.workspace)
         dt = ws.buffer("ssm.dt", (T, inner), torch.float32)           # before bias and softplus, which the scan applies
-        kernels.linear(p[:, :R], self.w_dt, dt)
+        kernels.linear(p[:, :R], self.w_dt, dt, workspace=ctx.workspace)
         og = ws.buffer("ssm.gated", (T, inner), self.dtype)
         kernels.selective_scan(x, dt, self.dt_bias, p[:, R:R + 2 * N], self.a, self.skip, proj[:, inner:2 * inner],
                                view["state"].states, ctx, og, self.out_scale)
-        kernels.linear(og, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(og, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 class MLSTMMixer:
@@ -460,7 +460,7 @@ class MLSTMMixer:
         T, ws = h.shape[0], ctx.workspace
         H, nq, nv = self.H, self.H * self.D, self.H * self.V
         proj = ws.buffer("mlstm.in", (T, self.w_in.shape[0]), self.dtype)
-        kernels.linear(h, self.w_in, proj)
+        kernels.linear(h, self.w_in, proj, workspace=ctx.workspace)
         at = 2 * nq + 2 * nv
         gates = ws.buffer("mlstm.gates", (T, 2 * H), torch.float32)
         m = ws.buffer("mlstm.max", (T, H), torch.float32)
@@ -473,7 +473,7 @@ class MLSTMMixer:
         kernels.state_readout(o32, H, self.V, og, stored_cols=self.V + 1, m=m, den_eps=self.DEN_EPS,
                               gate=proj[:, 2 * nq + nv:at], gate_act="sigmoid", gate_first=False, group=self.V,
                               eps=self.eps, w=self.norm_w)
-        kernels.linear(og, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(og, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 class GatedLinearAttention:
@@ -544,7 +544,7 @@ class GatedLinearAttention:
         T, ws = h.shape[0], ctx.workspace
         nq, nv = self.H * self.D, self.H * self.V
         proj = ws.buffer("gla.in", (T, self.w_in.shape[0]), self.dtype)
-        kernels.linear(h, self.w_in, proj)
+        kernels.linear(h, self.w_in, proj, workspace=ctx.workspace)
         o32 = ws.buffer("gla.o", (T, nv), torch.float32)
         kernels.channel_scan(proj[:, :nq], proj[:, nq:2 * nq], proj[:, 2 * nq:2 * nq + nv],
                              proj[:, self.low_at:self.low_at + self.rank], self.w_low, self.b_low, view.states, ctx, o32,
@@ -552,7 +552,7 @@ class GatedLinearAttention:
         og = ws.buffer("gla.gated", (T, nv), self.dtype)
         kernels.head_norm_gate(o32, self.H, self.V, self.norm_w, self.eps, proj[:, 2 * nq + nv:2 * nq + 2 * nv],
                                self.out_scale, og)
-        kernels.linear(og, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(og, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 class WKVMixer:
@@ -624,14 +624,14 @@ class WKVMixer:
         proj = ws.buffer("wkv.in", (T, 4 * n), self.dtype)
         kernels.linear_stacked(mixed[:4], self.w_in, proj)
         low = ws.buffer("wkv.low", (T, self.w_low1.shape[0]), torch.float32)           # 32-bit: it enters the decay
-        kernels.linear(mixed[4], self.w_low1, low)
+        kernels.linear(mixed[4], self.w_low1, low, workspace=ctx.workspace)
         o32 = ws.buffer("wkv.o", (T, n), torch.float32)
         kernels.channel_scan(proj[:, :n], proj[:, n:2 * n], proj[:, 2 * n:3 * n], low, self.w_low2, self.w0,
                              view["state"].states, ctx, o32, self.H, self.D, self.D, 1.0, decay="double_exp", low_tanh=True,
                              bonus=self.bonus)
         og = ws.buffer("wkv.gated", (T, n), self.dtype)
         kernels.head_norm_gate(o32, self.H, self.D, self.norm_w, self.eps, proj[:, 3 * n:], 1.0, og)
-        kernels.linear(og, self.w_o, residual32, accumulate=accumulate)
+        kernels.linear(og, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
 
 class ParallelMixer:

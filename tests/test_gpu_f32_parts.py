@@ -1,0 +1,102 @@
+"""float32 products of many rows as products of bfloat16 parts: against 64-bit sums and the kernel of multiply-adds."""
+import math
+
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, rnd
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -24
+
+
+def product(a, w, out, accumulate=False, **more):
+    from gguf2bin_b200 import kernels, kernels_bf16
+    from gguf2bin_b200.engine.workspace import Workspace
+    assert kernels.gemm_f32_tc(a, w, out, accumulate, Workspace(DEV), **more)
+    kernels_bf16.check_status()
+    return out
+
+
+# tiles of 256 x 256, blocks of 64 of K, one, two and four parts of K
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (33, 255, 60), (128, 256, 64), (129, 257, 68), (256, 300, 132), (257, 1024, 2048), (600, 515, 1028),
+                                   (701, 1024, 3072), (300, 4096, 1024), (1500, 4100, 200)])
+def test_error_of_32_bit_sums(M, N, K):
+    from gguf2bin_b200 import kernels
+    a, w = rnd(M, K, seed=1) * torch.logspace(-6, 6, M, device=DEV)[:, None], rnd(N, K, seed=2)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    out = product(a, w, torch.full((M, N), math.nan, device=DEV))
+    plain = torch.empty(M, N, device=DEV)
+    kernels.gemm_simt(a, w, plain)
+    # the bound of tests of the kernel of multiply-adds: chunks of 64, then the chunks
+    assert ((out.double() - ref).abs() <= (66 + K / 64) * EPS * size).all()
+    if K >= 64:                                   # below, a single rounding decides
+        assert ((out.double() - ref) / size).norm() <= ((plain.double() - ref) / size).norm()
+    base = rnd(M, N, seed=3)
+    acc = product(a, w, base.clone(), accumulate=True)
+    assert torch.equal(acc, base + out)
+    # rows of C off 16 bytes, of A and W with a stride of their own
+    wide = torch.full((M, N + 3), 7.0, device=DEV)
+    strided_a, strided_w = torch.zeros(M, K + 4, device=DEV), torch.zeros(N, K + 8, device=DEV)
+    strided_a[:, :K], strided_w[:, :K] = a, w
+    product(strided_a[:, :K], strided_w[:, :K], wide[:, 1:N + 1])
+    assert torch.equal(wide[:, 1:N + 1], out) and (wide[:, 0] == 7).all() and (wide[:, N + 1:] == 7).all()
+
+
+def test_rows_that_three_parts_do_not_hold():
+    """Infinities, NaN, the largest floats, rows of tiny entries: the bits of the kernel of multiply-adds there, and nothing of it elsewhere."""
+    from gguf2bin_b200 import kernels
+    a, w = rnd(300, 200, seed=1), rnd(400, 200, seed=2)
+    clean = product(a, w, torch.empty(300, 400, device=DEV))
+    a[3, 150], a[40, 0], a[128, 7], w[9, 9], w[300, 3] = math.inf, math.nan, -3.4e38, -math.inf, 3.39e38
+    a[200], a[201], a[202], w[255] = a[200] * 1e-30, 0.0, a[202] * 1e-40, w[255] * 1e-36
+    out = product(a, w, torch.full((300, 400), 5.0, device=DEV))
+    plain = torch.empty(300, 400, device=DEV)
+    kernels.gemm_simt(a, w, plain)
+    odd_a, odd_w = [3, 40, 128, 200, 202], [9, 255, 300]
+    same = lambda x, y: torch.equal(x.nan_to_num(nan=1e30, posinf=2e30, neginf=3e30), y.nan_to_num(nan=1e30, posinf=2e30, neginf=3e30))  # noqa: E731
+    assert same(out[odd_a], plain[odd_a]) and same(out[:, odd_w], plain[:, odd_w])
+    rows, cols = [i for i in range(300) if i not in odd_a + [201]], [i for i in range(400) if i not in odd_w]
+    assert torch.equal(out[rows][:, cols], clean[rows][:, cols]) and not out[201][cols].any()
+    acc = product(a, w, torch.ones(300, 400, device=DEV), accumulate=True)
+    assert same(acc, out + 1)
+
+
+def test_slices_of_the_matrix(monkeypatch):
+    from gguf2bin_b200 import kernels
+    a, w = rnd(200, 1024, seed=1), rnd(1000, 1024, seed=2)
+    whole = product(a, w, torch.empty(200, 1000, device=DEV))
+    monkeypatch.setattr(kernels, "F32_PARTS_ROWS", 300)
+    parts = product(a, w, torch.full((200, 1000), math.nan, device=DEV))
+    size = a.double().abs() @ w.double().abs().T
+    assert ((parts.double() - whole).abs() <= 2 * (66 + 16) * EPS * size).all()
+
+
+def test_route():
+    """Which kernel: by rows in steps of 64, so that a step filled up with padding keeps it; few rows, or no workspace, never."""
+    from gguf2bin_b200 import kernels
+    from gguf2bin_b200.engine.workspace import Workspace
+    assert all(kernels._f32_tc_wins(m, 4096, 1024) == kernels._f32_tc_wins(256, 4096, 1024) for m in range(193, 257))
+    ws, before = Workspace(DEV), kernels.launch_count()
+    big = rnd(4096, 1024, seed=4)
+    out = torch.empty(256, 4096, device=DEV)
+    kernels.linear(rnd(256, 1024, seed=3), big, out, workspace=ws)
+    assert kernels.launch_count() == before + 2 and ws.waits
+    kernels.linear(rnd(32, 1024, seed=3), big, out[:32], workspace=ws)
+    assert kernels.launch_count() == before + 3
+    kernels.linear(rnd(256, 1024, seed=3), big, out)
+    assert kernels.launch_count() == before + 4
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 1024, 2048), (1500, 4096, 520)])
+def test_copies_that_never_come(M, N, K):
+    from gguf2bin_b200 import kernels, kernels_bf16
+    from gguf2bin_b200.csrc.units import WAITS_RUN_OUT
+    from gguf2bin_b200.engine.workspace import Workspace
+    a, w, out = rnd(M, K, seed=1), rnd(N, K, seed=2), torch.zeros(M, N, device=DEV)
+    kernels.gemm_f32_tc(a, w, out, False, Workspace(DEV), defines=WAITS_RUN_OUT)
+    torch.cuda.synchronize()
+    with pytest.raises(kernels.KernelError, match=r"gemm_f32_tc.*(MMA issuer|adder).*gave up waiting"):
+        kernels_bf16.check_status()
+    product(a, w, out)
+    assert ((out.double() - a.double() @ w.double().T).abs() <= (66 + K / 64) * EPS * (a.double().abs() @ w.double().abs().T)).all()
