@@ -194,6 +194,67 @@ gemm_f32_rows_kernel(const float *A, const float *__restrict__ W, void *C, int r
   }
 }
 
+// Up to eight rows against a K whose rows of W fit shared memory whole: a block's NB rows are asked for at once, before the wait for the kernel
+// in front, so that the copies of all blocks of an SM (up to 192 KB of it) are on their way together and nothing is waited for but their
+// arrival; the kernel above has one stage of 32 KB on its way in front of the wait and, with 32 chunks a stage, moved zeros for half of a K of 1,024.
+// Thread (chunk, row) sums chunks c, c + CH, ... of its row for every row of A.  A chunk's 16 pieces of four floats lie in the order
+// piece ^ (chunk % 8): eight lanes that read one piece of eight chunks touch all banks once, without padding.  In a chain
+// of launches, two rows: 5.1 us for 4096 x 1024 (10.5 by the kernel above), 5.7 for 6144 x 1024 (9.3), 3.9 for 1024 x 2048 (4.1), 5.6 for 1024 x 3072
+// (5.9), 119 for 151936 x 1024 (139); a layer's four in turn 20.3 (29.5), with one row 17.5 (24.3), with eight 41 (64).
+template <int NB, int CH, int MT, int EPI>
+__global__ void __launch_bounds__(NB *CH)
+gemm_f32_whole_kernel(const float *A, const float *__restrict__ W, void *C, int M, int N, int K, int lda, int ldw, int ldc) {
+  constexpr int THREADS = NB * CH;
+  extern __shared__ __align__(16) float sm[];
+  const int tid = threadIdx.x, n0 = blockIdx.x * NB, chunks = (K + SUM_CHUNK - 1) / SUM_CHUNK, pitch = chunks * SUM_CHUNK;
+  float *Ws = sm, *As = Ws + NB * pitch, *part = As + M * pitch;                  // part [M][NB][chunks + 1]
+  auto bring = [&](float *to, const float *from, int rows, int ld, int last) {
+    for (int i = tid; i < rows * (pitch / 4); i += THREADS) {
+      const int r = i / (pitch / 4), q = i % (pitch / 4), chunk = q / 16;
+      const int bytes = bytes_left(q * 4, K);
+      copy16(to + r * pitch + chunk * SUM_CHUNK + ((q % 16) ^ (chunk & 7)) * 4, from + (size_t)min(r, last) * ld + (bytes ? q * 4 : 0), bytes);
+    }
+  };
+  bring(Ws, W + (size_t)n0 * ldw, NB, ldw, N - 1 - n0);
+  pdl_launch();
+  pdl_wait();
+  bring(As, A, M, lda, M - 1);
+  copies_commit();
+  copies_wait<0>();
+  __syncthreads();
+  const int row = tid / CH;
+  for (int chunk = tid % CH; chunk < chunks; chunk += CH) {
+    const float *w = Ws + row * pitch + chunk * SUM_CHUNK, *a = As + chunk * SUM_CHUNK;
+    const int turn = chunk & 7;
+    float acc[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) acc[m] = 0.f;
+#pragma unroll
+    for (int q = 0; q < SUM_CHUNK / 4; ++q) {
+      const int at = (q ^ turn) * 4;
+      const float4 wv = *(const float4 *)(w + at);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const float4 av = *(const float4 *)(a + min(m, M - 1) * pitch + at);
+        acc[m] = fmaf(av.x, wv.x, acc[m]);
+        acc[m] = fmaf(av.y, wv.y, acc[m]);
+        acc[m] = fmaf(av.z, wv.z, acc[m]);
+        acc[m] = fmaf(av.w, wv.w, acc[m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+      if (m < M) part[(m * NB + row) * (chunks + 1) + chunk] = acc[m];
+  }
+  __syncthreads();
+  for (int p = tid; p < M * NB; p += THREADS) {
+    float sum = 0.f;
+#pragma unroll 16
+    for (int c = 0; c < chunks; ++c) sum += part[p * (chunks + 1) + c];
+    if (n0 + p % NB < N) put<EPI>(C, (size_t)(p / NB) * ldc + n0 + p % NB, sum);
+  }
+}
+
 // Many rows: 64 x 64 outputs a block, 8 x 8 a thread, so that 16 loads of 16 bytes feed 256 multiply-adds and the FFMA
 // pipe bounds it.  G groups of 64 threads share a tile: group g sums chunks g, g + G, ... of it, and after every round
 // all threads add the groups' sums to their share of the tile in the chunks' order.  G = 1 where the tiles alone fill
@@ -335,6 +396,33 @@ static int launch_rows(const float *A, const float *W, void *C, int M, int N, in
   return g2b_check_launch("gemm_simt");
 }
 
+// Rows of W a block of the kernel that keeps them whole takes: 16, or 8 or 4 where fewer would leave SMs without a block; 0 where two blocks do not
+// fit an SM (then the kernel that goes through K in stages).
+static size_t whole_bytes(int NB, int M, int K) {
+  const size_t chunks = (K + SUM_CHUNK - 1) / SUM_CHUNK;
+  return sizeof(float) * ((NB + M) * chunks * SUM_CHUNK + (size_t)M * NB * (chunks + 1));
+}
+static int whole_rows(int M, int N, int K) {
+  if (M > 8 || K < 8 * SUM_CHUNK) return 0;        // a short K is nothing but latency: 0.2 us more here at K = 64
+  for (int NB = 16; NB >= 4; NB /= 2)
+    if ((NB == 4 || N >= 128 * NB) && whole_bytes(NB, M, K) <= 112 * 1024) return NB;
+  return 0;
+}
+template <int NB, int CH, int MT, int EPI>
+static int launch_whole(const float *A, const float *W, void *C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
+  static G2bPerDevice done;
+  if (allow_smem(gemm_f32_whole_kernel<NB, CH, MT, EPI>, 112 * 1024, done, "gemm_simt")) return 1;
+  g2b_launch(gemm_f32_whole_kernel<NB, CH, MT, EPI>, dim3((N + NB - 1) / NB), dim3(NB * CH), whole_bytes(NB, M, K), stream, A, W, C, M, N, K, lda,
+             ldw, ldc);
+  return g2b_check_launch("gemm_simt");
+}
+template <int MT, int EPI>
+static int launch_whole_rows(int NB, const float *A, const float *W, void *C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
+  if (NB == 16) return launch_whole<16, 16, MT, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  if (NB == 8) return launch_whole<8, 32, MT, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  return launch_whole<4, 32, MT, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+}
+
 template <int G, int EPI>
 static int launch_tile(const float *A, const float *W, void *C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
   static G2bPerDevice done;
@@ -391,6 +479,12 @@ template <int EPI>
 static int launch_f32(const float *A, const float *W, void *C, int M, int N, int K, int lda, int ldw, int ldc, int which, cudaStream_t stream) {
   if (which == F32_TILE1) return launch_tile<1, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
   if (which == F32_TILE4) return launch_tile<4, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  if (const int NB = whole_rows(M, N, K)) {
+    if (M == 1) return launch_whole_rows<1, EPI>(NB, A, W, C, M, N, K, lda, ldw, ldc, stream);
+    if (M == 2) return launch_whole_rows<2, EPI>(NB, A, W, C, M, N, K, lda, ldw, ldc, stream);
+    if (M <= 4) return launch_whole_rows<4, EPI>(NB, A, W, C, M, N, K, lda, ldw, ldc, stream);
+    return launch_whole_rows<8, EPI>(NB, A, W, C, M, N, K, lda, ldw, ldc, stream);
+  }
   if (M > ROWS_MAX) return launch_rows<16, 8, 8, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream, 8);      // eight rows a block, the matrix from the L2
   if (four_rows_of_w(M, N)) {
     if (M == 1) return launch_rows<4, 32, 1, EPI>(A, W, C, M, N, K, lda, ldw, ldc, stream);
