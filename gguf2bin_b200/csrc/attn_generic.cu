@@ -168,12 +168,12 @@ attn_generic_kernel(const T *__restrict__ q, T *__restrict__ out, const T *__res
 // by a warp (keys i and i + 32 first); its weighted values are added in the order of the keys; segments are merged one after
 // the other from the lowest.  Both kernels keep that order, so a row's result does not depend on which of the two computes it.
 //
-//   tile    a block per (64 rows of one prompt, query head) that walks the segments: prompts
+//   tile    a block per (32 rows of one prompt, query head) that walks the segments: prompts
 //   split   a block per (token, kv head, segment), for all query heads of the kv head, and a merge: single tokens, whose
 //           few rows leave the GPU to the segments
 //
 // 16 heads of 128 on 8 kv heads: two tokens behind 200 and 500 keys 7.4 + 4.2 us in a decode step (850 us with a warp a token
-// and head, whose lanes read rows of 512 bytes each for themselves); prompts of 201 and 500 tokens 181 us.
+// and head, whose lanes read rows of 512 bytes each for themselves); prompts of 201 and 500 tokens 131 us.
 #define SEG 64
 #define F32_MAX_HD 256
 #define F32_MAX_GROUP 32
@@ -252,27 +252,46 @@ __device__ __forceinline__ float last_factor(const F32Attn &p, int t, int h, flo
   return f;
 }
 
-#define F32_TILE_ROWS 64
+// Prompts: half a tile (32 rows) and a query head a block, two blocks an SM at head sizes up to 128, so that one's softmax and waits lie
+// beside the other's products and a long prompt's last tiles are dealt out in halves.  A segment's keys are asked for as soon as the scores
+// of the one in front are taken, its values behind that one's last sum.  All heads of the longest tiles come first: with head after head the last head's
+// longest tiles began when the rest was done, and the SMs idled for 0.31 of the time (1,024 tokens).  Prompts of 201 and 500 tokens 131 us (183 with 64
+// rows a block of 256 threads, panels brought when they were needed, head after head), one of 2,048 804 us (1,097); issue slots are half filled, 0.56 of
+// them with multiply-adds.
+#define F32_ROWS 32
+#define F32_THREADS 128
 template <bool B> struct Flag { static constexpr bool value = B; };
 template <int HD4>                                                  // float4 columns of a row per thread: ceil(hd / 64)
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(F32_THREADS, HD4 <= 2 ? 2 : 1)
 attn_f32_tile_kernel(F32Attn p) {
   pdl_launch();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
+  constexpr int RS = F32_THREADS / 16, PITCH = SEG + 4;             // a thread's rows are ty, ty + RS, ...
   const int hd = p.hd, pitch = hd + 4;
-  float *Qs = sm, *Ks = Qs + F32_TILE_ROWS * pitch, *Vs = Ks + SEG * pitch, *Ps = Vs + SEG * pitch;
-  float *row_m = Ps + F32_TILE_ROWS * (SEG + 4), *row_l = row_m + F32_TILE_ROWS, *old_f = row_l + F32_TILE_ROWS,
-        *new_f = old_f + F32_TILE_ROWS;
+  float *Qs = sm, *Ks = Qs + F32_ROWS * pitch, *Vs = Ks + SEG * pitch, *Ps = Vs + SEG * pitch;
+  float *row_m = Ps + F32_ROWS * PITCH, *row_l = row_m + F32_ROWS, *old_f = row_l + F32_ROWS, *new_f = old_f + F32_ROWS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
-  const int *tile = p.tiles + 4 * blockIdx.x;
-  const int seq = tile[0], t0 = tile[1], rows = tile[2], pos0 = tile[3], h = blockIdx.y, kvh = h / (p.nh / p.nkv);
-  for (int i = tid; i < F32_TILE_ROWS * (hd / 4); i += 256) {
+  const int half = blockIdx.x / p.nh, h = blockIdx.x % p.nh;        // all heads of the longest tiles first
+  const int *tile = p.tiles + 4 * (half / 2);
+  const int skip = F32_ROWS * (half % 2), rows = min(F32_ROWS, tile[2] - skip);
+  if (rows <= 0) return;
+  const int seq = tile[0], t0 = tile[1] + skip, pos0 = tile[3] + skip, kvh = h / (p.nh / p.nkv);
+  const int last_pos = pos0 + rows - 1, lo0 = lowest_key(p, pos0);  // the first row's window starts lowest
+  auto next_of = [&](int seg) {
+    do ++seg;
+    while (seg * SEG <= last_pos && !sees_segment(p, lo0, last_pos, seg));
+    return seg;
+  };
+  int seg = next_of(-1);                                            // there is one: the rows' own
+  bring_panel(Ks, panel_of(p, seq, seg, kvh, false), hd, tid, F32_THREADS);
+  bring_panel(Vs, panel_of(p, seq, seg, kvh, true), hd, tid, F32_THREADS);
+  for (int i = tid; i < F32_ROWS * (hd / 4); i += F32_THREADS) {
     const int r = i / (hd / 4), c = i % (hd / 4) * 4;
     *(float4 *)(Qs + r * pitch + c) =
         r < rows ? *(const float4 *)(p.q + (size_t)(t0 + r) * p.q_stride + (size_t)h * hd + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  if (tid < F32_TILE_ROWS) {
+  if (tid < F32_ROWS) {
     row_m[tid] = -INFINITY;
     row_l[tid] = 0.f;
   }
@@ -281,26 +300,24 @@ attn_f32_tile_kernel(F32Attn p) {
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < HD4; ++j) O[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int last_pos = pos0 + rows - 1, lo0 = lowest_key(p, pos0);
-  for (int seg = 0; seg * SEG <= last_pos; ++seg) {
-    if (!sees_segment(p, lo0, last_pos, seg)) continue;             // the first row's window starts lowest
-    __syncthreads();                                                // the last segment's panels and probabilities are read
-    bring_panel(Ks, panel_of(p, seq, seg, kvh, false), hd, tid, 256);
-    bring_panel(Vs, panel_of(p, seq, seg, kvh, true), hd, tid, 256);
-    asm volatile("cp.async.wait_group 1;\n" ::);
+  while (seg * SEG <= last_pos) {
+    const int next = next_of(seg);
+    const bool more = next * SEG <= last_pos;
+    asm volatile("cp.async.wait_group 1;\n" ::);                    // the keys; the values may be on their way
     __syncthreads();
     float4 S[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) S[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
     for (int d = 0; d < hd; d += 4) {
       float4 k[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) k[j] = *(const float4 *)(Ks + (tx + 16 * j) * pitch + d);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float4 q = *(const float4 *)(Qs + (ty + 16 * i) * pitch + d);
+        const float4 q = *(const float4 *)(Qs + (ty + RS * i) * pitch + d);
 #pragma unroll
         for (int j = 0; j < 4; ++j) dot4(S[i][j], q, k[j]);
       }
@@ -308,11 +325,14 @@ attn_f32_tile_kernel(F32Attn p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) Ps[(ty + 16 * i) * (SEG + 4) + tx + 16 * j] = scored(p, S[i][j]);
-    __syncthreads();
-    for (int r = warp; r < F32_TILE_ROWS; r += 8) {
+      for (int j = 0; j < 4; ++j) Ps[(ty + RS * i) * PITCH + tx + 16 * j] = scored(p, S[i][j]);
+    __syncthreads();                                                // the keys are read
+    if (more) bring_panel(Ks, panel_of(p, seq, next, kvh, false), hd, tid, F32_THREADS);
+    else asm volatile("cp.async.commit_group;\n" ::);
+#pragma unroll 4
+    for (int r = warp; r < F32_ROWS; r += F32_THREADS / 32) {
       float m, l;                                                   // rows behind the last see nothing, like rows before a window
-      soften(p, Ps + r * (SEG + 4), lane, seg, r < rows ? pos0 + r : -1, m, l);
+      soften(p, Ps + r * PITCH, lane, seg, r < rows ? pos0 + r : -1, m, l);
       if (lane == 0) {
         float there = row_m[r], of, nf;
         merge_factors(there, m, of, nf);
@@ -322,39 +342,46 @@ attn_f32_tile_kernel(F32Attn p) {
         new_f[r] = nf;
       }
     }
-    asm volatile("cp.async.wait_group 0;\n" ::);
+    asm volatile("cp.async.wait_group 1;\n" ::);                    // the values; the next keys may be on their way
     __syncthreads();
     float4 acc[4][HD4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < HD4; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // four keys at a time; a probability of 0 for a key behind n_keys is HIDDEN already
     auto weigh = [&](auto all_seen, int n_keys) {
-      for (int key = 0; key < n_keys; ++key) {
-        float4 v[HD4];
+      for (int key = 0; key < n_keys; key += 4) {
+        float4 pr[4];
 #pragma unroll
-        for (int j = 0; j < HD4; ++j)
-          if (64 * j + 4 * tx < hd) v[j] = *(const float4 *)(Vs + key * pitch + 64 * j + 4 * tx);
+        for (int i = 0; i < 4; ++i) pr[i] = *(const float4 *)(Ps + (ty + RS * i) * PITCH + key);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float pr = Ps[(ty + 16 * i) * (SEG + 4) + key];
-          if (decltype(all_seen)::value || !hidden(pr))             // a value that is not seen is not touched, whatever it holds
+        for (int u = 0; u < 4; ++u) {
+          float4 v[HD4];
 #pragma unroll
-            for (int j = 0; j < HD4; ++j)
-              if (64 * j + 4 * tx < hd) {
-                acc[i][j].x = fmaf(pr, v[j].x, acc[i][j].x);
-                acc[i][j].y = fmaf(pr, v[j].y, acc[i][j].y);
-                acc[i][j].z = fmaf(pr, v[j].z, acc[i][j].z);
-                acc[i][j].w = fmaf(pr, v[j].w, acc[i][j].w);
-              }
+          for (int j = 0; j < HD4; ++j)
+            if (64 * j + 4 * tx < hd) v[j] = *(const float4 *)(Vs + (key + u) * pitch + 64 * j + 4 * tx);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float w = u == 0 ? pr[i].x : (u == 1 ? pr[i].y : (u == 2 ? pr[i].z : pr[i].w));
+            if (decltype(all_seen)::value || !hidden(w))            // a value that is not seen is not touched, whatever it holds
+#pragma unroll
+              for (int j = 0; j < HD4; ++j)
+                if (64 * j + 4 * tx < hd) {
+                  acc[i][j].x = fmaf(w, v[j].x, acc[i][j].x);
+                  acc[i][j].y = fmaf(w, v[j].y, acc[i][j].y);
+                  acc[i][j].z = fmaf(w, v[j].z, acc[i][j].z);
+                  acc[i][j].w = fmaf(w, v[j].w, acc[i][j].w);
+                }
+          }
         }
       }
     };
-    if (rows == F32_TILE_ROWS && seg * SEG + SEG - 1 <= pos0 && seg * SEG >= lowest_key(p, last_pos)) weigh(Flag<true>(), SEG);
+    if (rows == F32_ROWS && seg * SEG + SEG - 1 <= pos0 && seg * SEG >= lowest_key(p, last_pos)) weigh(Flag<true>(), SEG);
     else weigh(Flag<false>(), min(SEG, last_pos - seg * SEG + 1));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float of = old_f[ty + 16 * i], nf = new_f[ty + 16 * i];
+      const float of = old_f[ty + RS * i], nf = new_f[ty + RS * i];
 #pragma unroll
       for (int j = 0; j < HD4; ++j) {
         O[i][j].x = merged(O[i][j].x, of, acc[i][j].x, nf);
@@ -363,10 +390,14 @@ attn_f32_tile_kernel(F32Attn p) {
         O[i][j].w = merged(O[i][j].w, of, acc[i][j].w, nf);
       }
     }
+    __syncthreads();                                                // the values, the probabilities and the factors are read
+    if (more) bring_panel(Vs, panel_of(p, seq, next, kvh, true), hd, tid, F32_THREADS);
+    else asm volatile("cp.async.commit_group;\n" ::);
+    seg = next;
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int r = ty + 16 * i;
+    const int r = ty + RS * i;
     if (r >= rows) continue;
     const float f = last_factor(p, t0 + r, h, row_m[r], row_l[r]);
     float *op = p.out + (size_t)(t0 + r) * p.nh * hd + (size_t)h * hd;
@@ -454,14 +485,14 @@ attn_f32_merge_kernel(F32Attn p) {
 template <int HD4>
 static int launch_f32_tiles(const F32Attn &p, int n_tiles, cudaStream_t stream) {
   static G2bPerDevice done;
-  auto bytes = [](int hd) { return sizeof(float) * ((size_t)(F32_TILE_ROWS + 2 * SEG) * (hd + 4) + F32_TILE_ROWS * (SEG + 4) + 4 * F32_TILE_ROWS); };
+  auto bytes = [](int hd) { return sizeof(float) * ((size_t)(F32_ROWS + 2 * SEG) * (hd + 4) + F32_ROWS * (SEG + 4) + 4 * F32_ROWS); };
   const int dev = g2b_current_device();
   if (dev < 0 || !done.value[dev]) {
     if (cudaFuncSetAttribute(attn_f32_tile_kernel<HD4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(64 * HD4)) != cudaSuccess)
       G2B_REFUSE("attn_f32: %zu bytes of shared memory are not available", bytes(64 * HD4));
     if (dev >= 0) done.value[dev] = 1;
   }
-  g2b_launch(attn_f32_tile_kernel<HD4>, dim3(n_tiles, p.nh), dim3(256), bytes(p.hd), stream, p);
+  g2b_launch(attn_f32_tile_kernel<HD4>, dim3(2u * n_tiles * p.nh), dim3(F32_THREADS), bytes(p.hd), stream, p);
   return g2b_check_launch("attn_f32");
 }
 
