@@ -94,29 +94,45 @@ attn_combine_kernel(const float *__restrict__ part_o, const float2 *__restrict__
   const size_t th = blockIdx.x;                                // t * nh + h
   const int t = (int)(th / nh);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // Without a window a token's chunks are 0, 1, ...: those of a short table are asked for before the position is there (what lies
+  // behind the token's last is not used), so that one round of loads is waited for instead of three: 2.9 us for eight tokens at 2,048 keys (3.2).
+  const float2 *ml = part_ml + th * n_chunks;
+  const bool active = 4 * lane < HD;
+  constexpr int AHEAD = 8;
+  const bool ahead = window == 0 && n_chunks <= AHEAD * COMBINE_WARPS;
+  float2 own = make_float2(-INFINITY, 0.f), mlv[AHEAD];
+  float4 ov[AHEAD];
+  if (ahead) {
+    if ((int)threadIdx.x < n_chunks) own = ml[threadIdx.x];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int i = warp + u * COMBINE_WARPS;
+      if (i < n_chunks) {
+        mlv[u] = ml[i];
+        if (active) ov[u] = *reinterpret_cast<const float4 *>(part_o + (th * n_chunks + i) * HD + 4 * lane);
+      }
+    }
+  }
   const int pos = tok_pos[t];
   const int lo = first_visible_key(pos, window);
   const Chunks chunk_of(pos, lo, kept_keys(lo, keep_first));
   const int total = chunk_of.total;
-  const float2 *ml = part_ml + th * n_chunks;
   float M = -INFINITY;
-  for (int i = (int)threadIdx.x; i < total; i += COMBINE_WARPS * 32) M = fmaxf(M, ml[chunk_of(i)].x);
+  if (ahead) M = (int)threadIdx.x < total ? own.x : -INFINITY;
+  else
+    for (int i = (int)threadIdx.x; i < total; i += COMBINE_WARPS * 32) M = fmaxf(M, ml[chunk_of(i)].x);
   M = warp_max(M);
   if (lane == 0) s_max[warp] = M;
   __syncthreads();
   M = fmaxf(fmaxf(s_max[0], s_max[1]), fmaxf(s_max[2], s_max[3]));
-  const bool active = 4 * lane < HD;
   float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
   float den = 0.f;
   // eight chunks' loads in flight at a time (a token far into its sequence has hundreds of chunks,
   // and one load after the other cost 20 us at 65,536 keys); they are added in the same order
-  constexpr int AHEAD = 8;
   for (int i0 = warp; i0 < total; i0 += AHEAD * COMBINE_WARPS) {
-    float2 mlv[AHEAD];
-    float4 ov[AHEAD];
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
-      if (i0 + u * COMBINE_WARPS < total) {
+      if (!ahead && i0 + u * COMBINE_WARPS < total) {
         const int i = chunk_of(i0 + u * COMBINE_WARPS);
         mlv[u] = ml[i];
         if (active) ov[u] = *reinterpret_cast<const float4 *>(part_o + (th * n_chunks + i) * HD + 4 * lane);

@@ -421,6 +421,14 @@ qknorm_rope_fast_kernel(
     ldE<E>(w + j, wa);
     ldE<E>(w + HH + j, wb);
   }
+  // A decode step's place in the cache: the batch's layout (sequences, pages) is older than the step's first kernel and may be read in front of
+  // the wait, and the position as it stands there nearly always names the page already: 2.5 us for eight tokens in a decode step (3.1).
+  int hint_page = -1, page = 0;
+  const bool stores = E == 4 && kind != 0 && !(kind == 1 ? k_out : v_out);
+  if (stores) {
+    hint_page = *(const volatile int *)(tok_pos + t) / page_size;
+    page = page_table[(size_t)tok_seq[t] * P + min(max(hint_page, 0), P - 1)];
+  }
   pdl_wait();
   ldE<E>(src + j, a);
   ldE<E>(src + HH + j, b);
@@ -439,7 +447,7 @@ qknorm_rope_fast_kernel(
       dst = flat + ((size_t)t * nkv + kvh) * HD;
     } else {
       const int pos = tok_pos[t];
-      const int page = page_table[(size_t)tok_seq[t] * P + pos / page_size];
+      if (!stores || pos / page_size != hint_page) page = page_table[(size_t)tok_seq[t] * P + pos / page_size];
       dst = cache + ((((size_t)page * 2 + (kind - 1)) * nkv + kvh) * page_size + pos % page_size) * HD;
     }
   }
