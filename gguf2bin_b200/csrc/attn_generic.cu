@@ -173,7 +173,7 @@ attn_generic_kernel(const T *__restrict__ q, T *__restrict__ out, const T *__res
 //           few rows leave the GPU to the segments
 //
 // 16 heads of 128 on 8 kv heads: two tokens behind 200 and 500 keys 7.4 + 4.2 us in a decode step (850 us with a warp a token
-// and head, whose lanes read rows of 512 bytes each for themselves); prompts of 201 and 500 tokens 131 us.
+// and head, whose lanes read rows of 512 bytes each for themselves); prompts of 201 and 500 tokens 123 us.
 #define SEG 64
 #define F32_MAX_HD 256
 #define F32_MAX_GROUP 32
@@ -213,12 +213,7 @@ __device__ __forceinline__ float scored(const F32Attn &p, float4 d) {
   const float s = ((d.x + d.y) + (d.z + d.w)) * p.scale;
   return p.softcap > 0.f ? p.softcap * tanhf(s / p.softcap) : s;
 }
-__device__ __forceinline__ void dot4(float4 &d, const float4 a, const float4 b) {
-  d.x = fmaf(a.x, b.x, d.x);
-  d.y = fmaf(a.y, b.y, d.y);
-  d.z = fmaf(a.z, b.z, d.z);
-  d.w = fmaf(a.w, b.w, d.w);
-}
+__device__ __forceinline__ void dot4(float4 &d, const float4 a, const float4 b) { fma4(d, a, b); }
 // One warp: a row's 64 scores in shared memory become probabilities against the maximum of those that the token at `pos` sees, and
 // HIDDEN where it does not.  What is hidden is decided by the positions alone: a score or a value that is NaN or infinite and
 // seen, whatever its weight, reaches the result.
@@ -255,9 +250,9 @@ __device__ __forceinline__ float last_factor(const F32Attn &p, int t, int h, flo
 // Prompts: half a tile (32 rows) and a query head a block, two blocks an SM at head sizes up to 128, so that one's softmax and waits lie
 // beside the other's products and a long prompt's last tiles are dealt out in halves.  A segment's keys are asked for as soon as the scores
 // of the one in front are taken, its values behind that one's last sum.  All heads of the longest tiles come first: with head after head the last head's
-// longest tiles began when the rest was done, and the SMs idled for 0.31 of the time (1,024 tokens).  Prompts of 201 and 500 tokens 131 us (183 with 64
-// rows a block of 256 threads, panels brought when they were needed, head after head), one of 2,048 804 us (1,097); issue slots are half filled, 0.56 of
-// them with multiply-adds.
+// longest tiles began when the rest was done, and the SMs idled for 0.31 of the time (1,024 tokens).  Multiply-adds go two an instruction, since a warp's
+// chain of instructions is what is waited for (131 and 804 us with one).  Prompts of 201 and 500 tokens 123 us (183 with 64 rows a block of 256 threads,
+// panels brought when they were needed, head after head), one of 2,048 737 us (1,097).
 #define F32_ROWS 32
 #define F32_THREADS 128
 template <bool B> struct Flag { static constexpr bool value = B; };
@@ -367,12 +362,7 @@ attn_f32_tile_kernel(F32Attn p) {
             if (decltype(all_seen)::value || !hidden(w))            // a value that is not seen is not touched, whatever it holds
 #pragma unroll
               for (int j = 0; j < HD4; ++j)
-                if (64 * j + 4 * tx < hd) {
-                  acc[i][j].x = fmaf(w, v[j].x, acc[i][j].x);
-                  acc[i][j].y = fmaf(w, v[j].y, acc[i][j].y);
-                  acc[i][j].z = fmaf(w, v[j].z, acc[i][j].z);
-                  acc[i][j].w = fmaf(w, v[j].w, acc[i][j].w);
-                }
+                if (64 * j + 4 * tx < hd) fma4(acc[i][j], make_float4(w, w, w, w), v[j]);
           }
         }
       }

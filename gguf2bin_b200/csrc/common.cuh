@@ -102,6 +102,23 @@ template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }
 
+// ---- two multiply-adds an instruction ----------------------------------------
+// c.x + a.x b.x and c.y + a.y b.y, each rounded once as by fmaf: half the issue slots of two fmaf.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ void fma4(float4 &c, float4 a, float4 b) {        // c += a b, element by element
+  const float2 lo = fma2(make_float2(a.x, a.y), make_float2(b.x, b.y), make_float2(c.x, c.y));
+  const float2 hi = fma2(make_float2(a.z, a.w), make_float2(b.z, b.w), make_float2(c.z, c.w));
+  c = make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
 // ---- which keys a token sees -------------------------------------------------
 // The lowest key position that the token at `pos` attends to.  `window` > 0: the last `window`
 // keys; `window` < 0: the keys of the token's own chunk of -window positions (chunks count from
