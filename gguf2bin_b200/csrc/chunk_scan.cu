@@ -14,9 +14,11 @@
 //   1. chunk_kernel<false>: every chunk by itself from a zero state: its own contribution, and the product of its g's
 //   2. chunk_carry: along a sequence, S at every chunk's start from the contributions; the sequence's state in the end
 //   3. chunk_kernel<true>: every chunk from its start state: the outputs
-// A block of 256 threads takes a chunk of one head and 64 columns.  Shared-memory reads bound it: 8 loads of 16
-// bytes feed 64 multiply-adds.  2,048 tokens, 8 heads of 128 x 256: 182 us (486 us as a chain), four prompts of 203 to 1,501 tokens, 64 heads of
-// 128 x 64: 649 us (889).  Chunks grouped into segments of up to 256 tokens, whose states alone went through memory: 189 and 709 us.
+// A block of 256 threads takes a chunk of one head and 64 columns.  Its phases (the loads, the decays, the products, the way out) bound it, so two
+// blocks share an SM: the outputs keep their products where the queries were and values in 16 bits as they came (one block an SM: 276 us a layer for
+// four prompts of 203 to 1,501 tokens, 64 heads of 128 x 64, now 233), and begin while half of the rows are on their way; the contributions'
+// multiply-adds go two an instruction (161 us, now 136).  The whole scan there 0.46 ms (0.53; 0.89 token by token); 2,048 tokens, 8 heads of 128 x 256:
+// 156 us (178; 486).  Chunks grouped into segments of up to 256 tokens, whose states alone went through memory: 189 and 709 us.
 //
 // Which sequences of a step come here is the caller's rule: those of more than `over` tokens, and sequence `pad`.  Of the
 // others nothing is read or written.
@@ -25,6 +27,7 @@
 #include <algorithm>
 #include <exception>
 #include <functional>
+#include <type_traits>
 #include <queue>
 #include <vector>
 
@@ -101,9 +104,7 @@ __device__ __forceinline__ void copy16(float *dst, const float *src) {
 __device__ __forceinline__ float dot4(const float4 &a, const float4 &b, float acc) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
-__device__ __forceinline__ void add4(float4 &a, float f, const float4 &b) {
-  a.x = fmaf(f, b.x, a.x), a.y = fmaf(f, b.y, a.y), a.z = fmaf(f, b.z, a.z), a.w = fmaf(f, b.w, a.w);
-}
+__device__ __forceinline__ void add4(float4 &a, float f, const float4 &b) { fma4(a, make_float4(f, f, f, f), b); }
 
 __device__ __forceinline__ float2 two_floats(double x) {
   const float hi = (float)x;
@@ -118,7 +119,7 @@ __device__ __forceinline__ float4 carry4(const float4 &a, float2 f, const float4
 __device__ __forceinline__ float4 sum4(const float4 &a, const float4 &b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 template <typename T, bool OUT>
-__global__ void __launch_bounds__(THREADS, OUT ? 1 : 2)
+__global__ void __launch_bounds__(THREADS, 2)
 chunk_kernel(const ChunkArgs a) {
   pdl_launch();
   pdl_wait();
@@ -128,31 +129,40 @@ chunk_kernel(const ChunkArgs a) {
   if (!find_chunk(a.seqs, CHUNK, a.base + blockIdx.z, b, place)) return;
   const int first = a.seqs.meta[4 * b] + place * CHUNK, n = min(CHUNK, a.seqs.meta[4 * b + 1] - place * CHUNK);
   const int qk_head = h / (H / a.G), tid = threadIdx.x;
-  float *K = sm, *Vs = K + CHUNK * pitch;
+  typedef typename std::conditional<OUT, T, float>::type Value;
+  float *K = sm;
+  Value *Vs = reinterpret_cast<Value *>(K + CHUNK * pitch);
   // decays and strengths of the chunk's tokens; from the token on: to the end of its sixteen, of the chunk times its strength;
   // up to the token: from its sixteen's start; the sixteens' products; in_block[B][i][j] = D_ij inside sixteen B
   double *tail16 = reinterpret_cast<double *>(Vs + CHUNK * COLS), *head = tail16 + CHUNK, *block = head + CHUNK;
-  float *g = reinterpret_cast<float *>(block + 4), *s = g + CHUNK, *tail = s + CHUNK, *in_block = tail + CHUNK;
-  float *Q = in_block + CHUNK * 17, *S = Q + CHUNK * pitch, *P = S + COLS * pitch;            // OUT only
+  float *g = reinterpret_cast<float *>(block + 4), *s = g + CHUNK, *in_block = s + CHUNK, *tail = in_block + CHUNK * 17;
+  float *Q = tail, *S = Q + CHUNK * pitch, *P = Q;       // OUT only (where there is no `tail`); the products where the queries were
   float *part = a.parts + ((size_t)blockIdx.z * H + h) * ((size_t)V * D);
-  for (int i = tid; i < CHUNK * (D / 4); i += THREADS) {
-    const int r = i / (D / 4), c = i % (D / 4) * 4;
-    float *kd = K + r * pitch + c, *qd = Q + r * pitch + c, *sd = S + r * pitch + c;
-    const size_t at = ((size_t)(first + r) * a.G + qk_head) * D + c;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < n) {
-      copy16(kd, a.kf + at);
-      if (OUT) copy16(qd, a.qf + at);
-    } else {
-      *reinterpret_cast<float4 *>(kd) = zero;
-      if (OUT) *reinterpret_cast<float4 *>(qd) = zero;
+  // the outputs start on the first 64 entries of keys, queries and states while the others are on their way
+  const int D1 = OUT ? min(D, 64) : D;
+  auto bring = [&](int d0, int d1) {
+    const int quads = (d1 - d0) / 4;
+    for (int i = tid; i < CHUNK * quads; i += THREADS) {
+      const int r = i / quads, c = d0 + i % quads * 4;
+      float *kd = K + r * pitch + c, *qd = Q + r * pitch + c, *sd = S + r * pitch + c;
+      const size_t at = ((size_t)(first + r) * a.G + qk_head) * D + c;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < n) {
+        copy16(kd, a.kf + at);
+        if (OUT) copy16(qd, a.qf + at);
+      } else {
+        *reinterpret_cast<float4 *>(kd) = zero;
+        if (OUT) *reinterpret_cast<float4 *>(qd) = zero;
+      }
+      if (OUT) {                                           // column col0 + r of the state at the chunk's start
+        if (col0 + r < V) copy16(sd, part + (size_t)(col0 + r) * D + c);
+        else *reinterpret_cast<float4 *>(sd) = zero;
+      }
     }
-    if (OUT) {                                           // column col0 + r of the state at the chunk's start
-      if (col0 + r < V) copy16(sd, part + (size_t)(col0 + r) * D + c);
-      else *reinterpret_cast<float4 *>(sd) = zero;
-    }
-  }
-  asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  bring(0, D1);
+  if (OUT) bring(D1, D);
   {
     const int c = col0 + (tid & 63);
     const T *vg = (const T *)a.v;
@@ -174,9 +184,10 @@ chunk_kernel(const ChunkArgs a) {
       s[tid] = rs;
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) Vs[((tid >> 6) + 4 * i) * COLS + (tid & 63)] = to_f32(rv[i]);
+    for (int i = 0; i < 16; ++i) Vs[((tid >> 6) + 4 * i) * COLS + (tid & 63)] = from_f32<Value>(to_f32(rv[i]));
   }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (OUT) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+  else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
   if (tid < CHUNK) {                                     // the decays from token `tid` on, to the end of its sixteen
     const int b16 = tid & ~15, j = tid & 15;
@@ -200,6 +211,10 @@ chunk_kernel(const ChunkArgs a) {
       for (int j = 0; j < 4; ++j) p[i][j] = o[i][j] = 0.f;
 #pragma unroll 1
     for (int d0 = 0; d0 < D; d0 += 16) {
+      if (d0 == 64) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+      }
       float p16[4][4], o16[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -230,7 +245,7 @@ chunk_kernel(const ChunkArgs a) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) p[i][j] += p16[i][j], o[i][j] += o16[i][j];
     }
-    __syncthreads();                                     // all decays stand
+    __syncthreads();                                     // all decays stand, and the queries are read
     double before = 1.0;                                 // the sixteens in front
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -272,7 +287,7 @@ chunk_kernel(const ChunkArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) x[e][j] = Vs[(t + e) * COLS + tx + 16 * j];
+          for (int j = 0; j < 4; ++j) x[e][j] = to_f32(Vs[(t + e) * COLS + tx + 16 * j]);
 #pragma unroll
         for (int i = tb; i < 4; ++i) {
           const int r = ty + 16 * i;
@@ -384,8 +399,9 @@ template <typename T, bool OUT>
 static int launch_chunks(const ChunkArgs &a, dim3 grid, cudaStream_t stream) {
   static G2bPerDevice done;
   auto bytes = [](int D) {
-    return sizeof(float) * ((size_t)CHUNK * (D + 4) * (OUT ? 2 : 1) + CHUNK * COLS + 7 * CHUNK + 8 + CHUNK * 17 +
-                            (OUT ? (size_t)COLS * (D + 4) + CHUNK * P_PITCH : 0));
+    const size_t rows = sizeof(float) * CHUNK * (size_t)(D + 4), products = sizeof(float) * CHUNK * P_PITCH;       // (where the queries were)
+    return rows + CHUNK * COLS * (OUT ? sizeof(T) : sizeof(float)) + sizeof(float) * (6 * CHUNK + 8 + CHUNK * 17) +
+           (OUT ? std::max(rows, products) + std::max(rows, sizeof(float) * COLS * (size_t)(D + 4)) : sizeof(float) * CHUNK);
   };
   const int dev = g2b_current_device();
   if (dev < 0 || !done.value[dev]) {
