@@ -35,7 +35,7 @@ constexpr int BM = 128;
 constexpr int BK = 64;                      // 64 bf16 = 128 bytes = one swizzle row
 constexpr int THREADS = 192;
 
-enum { EPI_STORE_BF16 = 0, EPI_STORE_F32 = 1, EPI_ACCUM_F32 = 2, EPI_SWIGLU_BF16 = 3 };
+enum { EPI_STORE_BF16 = 0, EPI_STORE_F32 = 1, EPI_ACCUM_F32 = 2, EPI_SWIGLU_BF16 = 3, EPI_HEADS = 4 };
 // The gate of the gated epilogue: SiLU; in a build with -DG2B_GLU, which holds that epilogue alone, the
 // general form that the launch gives (glu.cuh).
 // A build with -DG2B_ACT holds the bfloat16 store alone, and every value passes the form's activation on its way out.
@@ -346,6 +346,158 @@ __device__ __forceinline__ void epilogue_tile_bulk(uint32_t tmem, unsigned char 
   }
 }
 
+// ---- heads: the q, k and v of a prompt -----------------------------------------------------------
+// The columns of C are the heads of q, k and v, 128 of them each, and what is wanted is not C: q and k normed head by head and rotated, k
+// and v in the cache's pages.  As a kernel of its own behind the product that is a write and two reads of memory more (16,384 tokens of 32
+// heads: 268 MB, 76 us behind a product of 92).  Here a warp rounds the 128 columns of a head to bfloat16, as C would hold them, into its two
+// staging boxes (the head's halves: an element and its partner of the rotation lie at one place of the two), and eight lanes read a row
+// back, 16 bytes of each half: what qknorm_rope_fast_kernel<bf16, 8, 8> (elementwise.cu) has in its registers, and its arithmetic in its
+// order, so that q and the pages get the same bits.
+constexpr int HEAD = 128;
+struct HeadsTail : ProductTail {
+  const float *q_w, *k_w;                          // null: no norm
+  const float2 *rope;                              // [tokens, 64] (cos, sin); null: no rotation
+  const int *tok_pos, *tok_seq, *page_table;
+  bf16 *cache, *q_out;
+  float eps;
+  int P, nh, nkv, page_size;
+};
+// What the epilogue of a tile needs of its rows, asked for before the tile's products are done: the angles of a lane's columns in the eight
+// rows it works on (the same for every head), and where the lane's own row goes in the cache, in rows, as far as it is the same for all heads.
+struct HeadRows {
+  float4 turn[8][4];
+  long long place;
+  __device__ __forceinline__ void ask(int m0, int n0, int cols, int M, int warp, int lane, const HeadsTail &tail) {
+    const int y = m0 + warp * 32, first_head = n0 / HEAD;
+    place = 0;
+    if (n0 + cols > tail.nh * HEAD && y + lane < M) {
+      const int pos = tail.tok_pos[y + lane];
+      const int page = tail.page_table[(size_t)tail.tok_seq[y + lane] * tail.P + pos / tail.page_size];
+      place = (long long)page * 2 * tail.nkv * tail.page_size + pos % tail.page_size;
+    }
+    if (tail.rope && first_head < tail.nh + tail.nkv) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 *from = reinterpret_cast<const float4 *>(tail.rope + (size_t)min(y + 4 * i + (lane >> 3), M - 1) * (HEAD / 2) + 8 * (lane & 7));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) turn[i][j] = from[j];
+      }
+    }
+  }
+};
+
+// what a kernel with an epilogue is launched with, and keeps of a tile's rows
+struct NoRows {};
+template <int EPI> struct TailOf { using type = ProductTail; using Rows = NoRows; };
+template <> struct TailOf<EPI_HEADS> { using type = HeadsTail; using Rows = HeadRows; };
+
+template <int BN>
+__device__ __forceinline__ void epilogue_heads(uint32_t tmem, unsigned char *stage, int m0, int n0, int M, int N, int warp, int lane,
+                                               const HeadRows &rows, const HeadsTail &tail) {
+  static_assert(BN % HEAD == 0, "whole heads in a tile");
+  const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+  const int y = m0 + warp * 32, sub = lane >> 3, c = lane & 7;
+  const int first_head = n0 / HEAD, heads = min(BN, N - n0) / HEAD;
+  const uint32_t own_row = smem_addr(stage) + lane * 128;
+#pragma unroll 1
+  for (int i = 0; i < heads; ++i) {
+    const int head = first_head + i;
+    const int kind = head < tail.nh ? 0 : (head < tail.nh + tail.nkv ? 1 : 2);       // q, k, v
+    const float *w = kind == 0 ? tail.q_w : (kind == 1 ? tail.k_w : nullptr);
+    const bool turned = kind != 2 && tail.rope;
+    float wa[8], wb[8];
+    if (w) {
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        *reinterpret_cast<float4 *>(wa + j) = *reinterpret_cast<const float4 *>(w + 8 * c + j);
+        *reinterpret_cast<float4 *>(wb + j) = *reinterpret_cast<const float4 *>(w + HEAD / 2 + 8 * c + j);
+      }
+    }
+    __syncwarp();                                  // the boxes of the head in front have been read
+#pragma unroll
+    for (int part = 0; part < 4; ++part) {
+      uint32_t v[32];
+      tmem_ld32(lane_addr + i * HEAD + part * 32, v);
+      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t *u = v + 8 * j;
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::
+                     "r"(own_row + (part / 2) * 4096 + (((4 * (part % 2) + j) ^ (lane & 7)) << 4)),
+                     "r"(pack2(u[0], u[1], tail)), "r"(pack2(u[2], u[3], tail)), "r"(pack2(u[4], u[5], tail)),
+                     "r"(pack2(u[6], u[7], tail)) : "memory");
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r0 = 0; r0 < 8; r0 += 2) {            // two rows a lane at once: one row's chain of sums and its root behind the other's
+      float a[2][8], b[2][8];
+      long long at[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int r = 4 * (r0 + k) + sub;
+        const unsigned char *from = stage + r * 128 + ((c ^ (r & 7)) << 4);
+        const uint4 xa = *reinterpret_cast<const uint4 *>(from), xb = *reinterpret_cast<const uint4 *>(from + 4096);
+        at[k] = __shfl_sync(0xffffffffu, rows.place, r);
+        const uint32_t ua[4] = {xa.x, xa.y, xa.z, xa.w}, ub[4] = {xb.x, xb.y, xb.z, xb.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          a[k][2 * j] = __uint_as_float(ua[j] << 16);
+          a[k][2 * j + 1] = __uint_as_float(ua[j] & 0xffff0000u);
+          b[k][2 * j] = __uint_as_float(ub[j] << 16);
+          b[k][2 * j + 1] = __uint_as_float(ub[j] & 0xffff0000u);
+        }
+      }
+      if (w) {
+        float ss[2] = {0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            ss[k] = fmaf(a[k][j], a[k][j], ss[k]);
+            ss[k] = fmaf(b[k][j], b[k][j], ss[k]);
+          }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], o);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float inv = 1.f / sqrtf(ss[k] / (float)HEAD + tail.eps);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            a[k][j] = (wa[j] * a[k][j]) * inv;
+            b[k][j] = (wb[j] * b[k][j]) * inv;
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (turned) {
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            const float4 cs = rows.turn[r0 + k][j / 2];
+            const float a0 = a[k][j], b0 = b[k][j], a1 = a[k][j + 1], b1 = b[k][j + 1];
+            a[k][j] = a0 * cs.x - b0 * cs.y;
+            b[k][j] = a0 * cs.y + b0 * cs.x;
+            a[k][j + 1] = a1 * cs.z - b1 * cs.w;
+            b[k][j + 1] = a1 * cs.w + b1 * cs.z;
+          }
+        }
+        const int t = y + 4 * (r0 + k) + sub;
+        if (t < M) {
+          bf16 *to = kind == 0 ? tail.q_out + ((size_t)t * tail.nh + head) * HEAD
+                               : tail.cache + (size_t)(at[k] + (long long)(head - tail.nh) * tail.page_size) * HEAD;
+          *reinterpret_cast<uint4 *>(to + 8 * c) =
+              make_uint4(pack2f(a[k][0], a[k][1]), pack2f(a[k][2], a[k][3]), pack2f(a[k][4], a[k][5]), pack2f(a[k][6], a[k][7]));
+          *reinterpret_cast<uint4 *>(to + HEAD / 2 + 8 * c) =
+              make_uint4(pack2f(b[k][0], b[k][1]), pack2f(b[k][2], b[k][3]), pack2f(b[k][4], b[k][5]), pack2f(b[k][6], b[k][7]));
+        }
+      }
+    }
+  }
+}
+
 // ---- K in parts over a cluster ---------------------------------------------------------------
 // With fewer tiles than half the SMs, the CTAs of a cluster take the same tile and one part of
 // K each.  The tile's chunks of 32 columns are dealt out to the ranks in contiguous ranges
@@ -504,7 +656,7 @@ template <int BN, int STAGES, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                           const __grid_constant__ CUtensorMap map_c, int M, int N, int K, int group_m,
-                          int k_parts, int *__restrict__ status, ProductTail glu) {
+                          int k_parts, int *__restrict__ status, typename TailOf<EPI>::type glu) {
   pdl_launch();
   extern __shared__ unsigned char smem_raw[];
   using S = SmemP<BN, STAGES>;
@@ -644,6 +796,11 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     TICK(t_epi);
     for (int t = walker; t < n_tiles; t += walkers, ++j) {
       const uint32_t buf = j & 1;
+      int tm, tn;
+      tile_of(t, tiles_m, tiles_n, group_m, tm, tn);
+      const int m0 = tm * BM, n0 = tn * BN;
+      typename TailOf<EPI>::Rows rows;
+      if constexpr (EPI == EPI_HEADS) rows.ask(m0, n0, BN, M, warp, lane, glu);
       TICK(t_af);
       if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1)) {
         if (lane == 0) atomicExch(status, ST_EPILOGUE_TIMEOUT);
@@ -652,10 +809,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       TOCK(7, t_af);
       TOCK(8, t_af - 1 + clock64());               // counts tiles (adds 1)
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      int tm, tn;
-      tile_of(t, tiles_m, tiles_n, group_m, tm, tn);
-      const int m0 = tm * BM, n0 = tn * BN;
-      epilogue_tile_bulk<BN, EPI>(tmem + buf * BN, stage, &map_c, m0, n0, M, N, warp, lane, box, glu);
+      if constexpr (EPI == EPI_HEADS) epilogue_heads<BN>(tmem + buf * BN, stage, m0, n0, M, N, warp, lane, rows, glu);
+      else epilogue_tile_bulk<BN, EPI>(tmem + buf * BN, stage, &map_c, m0, n0, M, N, warp, lane, box, glu);
       // every load of this warp from the accumulator has completed (each is waited for)
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
@@ -665,7 +820,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     TOCK(6, t_epi);
     if (threadIdx.x == 0) { TFLUSH(6); TFLUSH(7); TFLUSH(8); }
   }
-  if (k_parts > 1) {
+  if (EPI != EPI_HEADS && k_parts > 1) {
     // every thread of every CTA of the cluster comes through here, whatever its waits did
     const bool have_tile = walker < n_tiles;
     bool have_acc = false;
@@ -905,7 +1060,7 @@ template <int BN, int STAGES, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_c, int M, int N, int K, int group_m,
-                    int *__restrict__ status, ProductTail glu) {
+                    int *__restrict__ status, typename TailOf<EPI>::type glu) {
   pdl_launch();
   extern __shared__ unsigned char smem_raw[];
   using S = SmemPair<BN, STAGES>;
@@ -1005,15 +1160,18 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint32_t j = 0, box = 0;
     for (int t = pair; t < n_tiles; t += pairs, ++j) {
       const uint32_t buf = j & 1;
+      int tm, tn;
+      tile_of(t, tiles_m, tiles_n, group_m, tm, tn);
+      const int m0 = tm * (2 * BM) + (int)rank * BM, n0 = tn * BN;
+      typename TailOf<EPI>::Rows rows;
+      if constexpr (EPI == EPI_HEADS) rows.ask(m0, n0, BN, M, warp, lane, glu);
       if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1)) {
         if (lane == 0) atomicExch(status, ST_EPILOGUE_TIMEOUT);
         break;
       }
       tc_fence_after();
-      int tm, tn;
-      tile_of(t, tiles_m, tiles_n, group_m, tm, tn);
-      const int m0 = tm * (2 * BM) + (int)rank * BM, n0 = tn * BN;
-      epilogue_tile_bulk<BN, EPI>(tmem + buf * BN, stage, &map_c, m0, n0, M, N, warp, lane, box, glu);
+      if constexpr (EPI == EPI_HEADS) epilogue_heads<BN>(tmem + buf * BN, stage, m0, n0, M, N, warp, lane, rows, glu);
+      else epilogue_tile_bulk<BN, EPI>(tmem + buf * BN, stage, &map_c, m0, n0, M, N, warp, lane, box, glu);
       // every load of this warp from the accumulator has completed (each is waited for)
       tc_fence_before();
       __syncwarp();
@@ -1439,7 +1597,7 @@ static_assert(SmemP<128, 6>::RING_BYTES == 196608 && SmemP<256, 4>::RING_BYTES =
 // want_parts: 1 to 4 parts of K
 template <int BN, int STAGES, int EPI>
 static int launch_persistent(const CUtensorMap &ma, const CUtensorMap &mw, void *C, int M, int N, int K, int ldc,
-                             int want_parts, int *status, ProductTail glu, cudaStream_t stream) {
+                             int want_parts, int *status, typename TailOf<EPI>::type glu, cudaStream_t stream) {
   static G2bPerDevice configured;
   const int smem = SmemP<BN, STAGES>::TOTAL;
   const int cfg_dev = g2b_current_device();
@@ -1453,11 +1611,11 @@ static int launch_persistent(const CUtensorMap &ma, const CUtensorMap &mw, void 
   if (tiles > 0x7fffffffLL) G2B_REFUSE("gemm_tc: %lld tiles", tiles);
   const bool is_float = EPI == EPI_STORE_F32 || EPI == EPI_ACCUM_F32;
   const int c_cols = EPI == EPI_SWIGLU_BF16 ? N / 2 : N;
-  if (((uintptr_t)C & 15) || (ldc * (is_float ? 4 : 2)) % 16)
+  if (EPI != EPI_HEADS && (((uintptr_t)C & 15) || (ldc * (is_float ? 4 : 2)) % 16))
     G2B_REFUSE("gemm_tc: the persistent kernel stores tiles of C: C must be 16-byte aligned with a row stride "
                "that is a multiple of 16 bytes (ldc = %d)", ldc);
-  CUtensorMap mc;
-  const int rc = make_map_c(&mc, C, M, c_cols, ldc, is_float);
+  CUtensorMap mc = ma;                             // heads: no C
+  const int rc = EPI == EPI_HEADS ? 0 : make_map_c(&mc, C, M, c_cols, ldc, is_float);
   if (rc) return rc;
   const int nkb = (K + BK - 1) / BK;
   const int parts = want_parts < 1 ? 1 : want_parts;
@@ -1478,7 +1636,7 @@ static int launch_persistent(const CUtensorMap &ma, const CUtensorMap &mw, void 
 
 template <int BN, int STAGES, int EPI>
 static int launch_pair(const CUtensorMap &ma, const CUtensorMap &mw, void *C, int M, int N, int K, int ldc,
-                       int *status, ProductTail glu, cudaStream_t stream) {
+                       int *status, typename TailOf<EPI>::type glu, cudaStream_t stream) {
   static G2bPerDevice configured;
   const int smem = SmemPair<BN, STAGES>::TOTAL;
   const int cfg_dev = g2b_current_device();
@@ -1492,11 +1650,11 @@ static int launch_pair(const CUtensorMap &ma, const CUtensorMap &mw, void *C, in
   if (tiles > 0x7fffffffLL) G2B_REFUSE("gemm_tc: %lld tiles", tiles);
   const bool is_float = EPI == EPI_STORE_F32 || EPI == EPI_ACCUM_F32;
   const int c_cols = EPI == EPI_SWIGLU_BF16 ? N / 2 : N;
-  if (((uintptr_t)C & 15) || (ldc * (is_float ? 4 : 2)) % 16)
+  if (EPI != EPI_HEADS && (((uintptr_t)C & 15) || (ldc * (is_float ? 4 : 2)) % 16))
     G2B_REFUSE("gemm_tc: the paired kernel stores tiles of C: C must be 16-byte aligned with a row stride "
                "that is a multiple of 16 bytes (ldc = %d)", ldc);
-  CUtensorMap mc;
-  const int rc = make_map_c(&mc, C, M, c_cols, ldc, is_float);
+  CUtensorMap mc = ma;                             // heads: no C
+  const int rc = EPI == EPI_HEADS ? 0 : make_map_c(&mc, C, M, c_cols, ldc, is_float);
   if (rc) return rc;
   const int max_pairs = sm_count() / 2;
   if (max_pairs < 1) G2B_REFUSE("gemm_tc: the paired kernel needs two SMs");
@@ -1666,6 +1824,45 @@ extern "C" int g2b_gemm_tc(const void *A, const void *W, void *C, int M, int N, 
 #undef G2B_CASE
   G2B_REFUSE("gemm_tc: no kernel for tile width %d with %d stages and epilogue %d", bn, stages, epi);
 }
+
+#if !defined(G2B_GLU) && !defined(G2B_ACT)
+// Whether the product of M rows with N columns runs in whole tiles 256 wide on the persistent kernel (not narrower, not K in parts).
+extern "C" int g2b_gemm_tc_heads_whole(int M, int N, int K) {
+  int bn = 0, parts = 0;
+  choose_persistent(M, N, K, EPI_STORE_BF16, &bn, &parts, 0);
+  return bn == 256 && parts == 1;
+}
+
+// The product of A [M, K] with the q, k and v rows of W [(nh + 2 nkv) 128, K], q and k normed by head (q_w, k_w; null: not) and rotated
+// (rope: the step's table; null: not), q to q_out [M, nh 128], k and v to the cache's pages: what g2b_gemm_tc into a buffer and
+// g2b_qknorm_rope_cache on it give.  pair: pairs of CTAs, else the persistent kernel, as the product alone would run.  Product and prologue kernel
+// before, and now: 16,384 tokens, 16 and 8 heads, K = 1,024: 92 + 76 us, 132 (the four warps of the epilogue set the pace: 9.6 us a tile whose
+// products take 6.3); 2,048 tokens: 16 + 10 us, 24; 12,000 tokens, 32 and 8 heads, K = 4,096: 301 + 63 us, 299 (hidden behind the products).
+extern "C" int g2b_gemm_tc_heads(const void *A, const void *W, int M, int K, int lda, int ldw, int pair, const float *q_w,
+                                 const float *k_w, float eps, const float *rope, const int *tok_pos, const int *tok_seq,
+                                 const int *page_table, int P, void *cache, int page_size, void *q_out, int nh, int nkv, int *status,
+                                 cudaStream_t stream) {
+  if (M <= 0) return 0;
+  if (K <= 0 || K % 8 || lda % 8 || ldw % 8) G2B_REFUSE("gemm_tc_heads: K=%d and the row strides (%d, %d) must be multiples of 8", K, lda, ldw);
+  if (((uintptr_t)A | (uintptr_t)W | (uintptr_t)q_w | (uintptr_t)k_w | (uintptr_t)rope | (uintptr_t)cache | (uintptr_t)q_out) & 15)
+    G2B_REFUSE("gemm_tc_heads: operands must be 16-byte aligned");
+  if (nh <= 0 || nkv < 0 || !q_out || (nkv > 0 && (!cache || !page_table || !tok_pos || !tok_seq || P <= 0 || page_size <= 0)))
+    G2B_REFUSE("gemm_tc_heads: %d and %d heads, no place for them", nh, nkv);
+  if (!status) G2B_REFUSE("gemm_tc_heads: no status word");
+  const int N = (nh + 2 * nkv) * HEAD;
+  HeadsTail tail;
+  tail.limit = tail.offset = tail.c1 = tail.c3 = 0.f, tail.a_group = 0;
+  tail.q_w = q_w, tail.k_w = k_w, tail.rope = (const float2 *)rope, tail.tok_pos = tok_pos, tail.tok_seq = tok_seq;
+  tail.page_table = page_table, tail.cache = (bf16 *)cache, tail.q_out = (bf16 *)q_out, tail.eps = eps, tail.P = P;
+  tail.nh = nh, tail.nkv = nkv, tail.page_size = page_size;
+  CUtensorMap ma, mw;
+  int rc = make_map(&ma, A, M, K, lda, BM);
+  if (!rc) rc = make_map(&mw, W, N, K, ldw, pair ? 128 : 256);
+  if (rc) return rc;
+  return pair ? launch_pair<256, 6, EPI_HEADS>(ma, mw, nullptr, M, N, K, 0, status, tail, stream)
+              : launch_persistent<256, 4, EPI_HEADS>(ma, mw, nullptr, M, N, K, 0, 1, status, tail, stream);
+}
+#endif
 
 template <int BN, int STAGES, int EPI>
 static int launch_grouped(const CUtensorMap &ma, const CUtensorMap &mw, void *C, int rows, const int *plan, int n_groups, int Nw, int K,

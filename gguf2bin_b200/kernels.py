@@ -882,6 +882,15 @@ def attention_qkv(qkv, q_w, k_w, eps, rope, rotary_dim, out, cache_pages, ctx, n
                                                   head_dim, page_size, window, scale, sink, chunk, softcap, keep_first)
 
 
+def heads_product(a, w, q_w, k_w, eps, rope, rotary_dim, ctx, cache_pages, page_size, q_out, n_heads, n_kv_heads, head_dim) -> bool:
+    """The product of a prompt's rows with the q, k and v matrix and ``qknorm_rope_cache`` of it in one kernel (bfloat16); False when no
+    kernel takes the case (the caller then runs the two)."""
+    if a.dtype != torch.bfloat16:
+        return False
+    return (_bf16 or _bf16_mod()).heads_product(a, w, q_w, k_w, eps, rope, rotary_dim, ctx, cache_pages, page_size, q_out, n_heads,
+                                                n_kv_heads, head_dim)
+
+
 def normed_product(x32, eps, w, out, gate_block=None) -> bool:
     """out = rmsnorm_without_weight(x32) @ w.T (or its SiLU gate) in one kernel; False when no
     kernel takes the case (the caller then runs the norm and the product one after the other)."""

@@ -206,6 +206,47 @@ def linear_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate:
     return False
 
 
+_heads_whole: dict = {}   # (rows, columns, K, device) -> the persistent kernel runs it in whole tiles 256 wide
+
+
+def heads_product(a, w, q_w, k_w, eps, rope, rotary_dim, ctx, cache_pages, page_size, q_out, n_heads: int, n_kv_heads: int,
+                  head_dim: int) -> bool:
+    """``qknorm_rope_cache`` of a @ w.T inside the product's epilogue; False: the case is left to the two kernels.  Only where
+    the product runs on the tcgen05 kernels with tiles 256 wide, one part of K and a second accumulator (the walk over a tile's heads
+    is hidden behind the next tile's products then), heads of 128, and the rotation over all of a head."""
+    M, K = a.shape
+    N = (n_heads + 2 * n_kv_heads) * head_dim
+    if head_dim != 128 or M <= 128 or w.shape[0] != N or w.shape[1] != K or w.dtype != torch.bfloat16 or not _tc_ok(a, w):
+        return False
+    if not q_out.is_contiguous() or q_out.dtype != torch.bfloat16 or (rope is not None and rotary_dim != head_dim):
+        return False
+    if n_kv_heads and (cache_pages.dtype != torch.bfloat16 or not cache_pages.is_contiguous()):
+        return False
+    if any(x is not None and x.data_ptr() % 16 for x in (q_out, q_w, k_w, rope, cache_pages)):
+        return False
+    choice, bn, stages, persistent = _route(a, w, q_out)
+    if choice != "tc":
+        return False
+    if persistent != 2:
+        if persistent is not True or bn:
+            return False
+        key = (M, N, K, a.device.index)
+        whole = _heads_whole.get(key)
+        if whole is None:
+            if len(_heads_whole) > 4096:
+                _heads_whole.clear()
+            whole = _heads_whole[key] = bool(_fn("gemm_tc.cu", "g2b_gemm_tc_heads_whole", [c_int, c_int, c_int])(M, N, K))
+        if not whole:
+            return False
+    f = _fn("gemm_tc.cu", "g2b_gemm_tc_heads",
+            [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
+             c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p])
+    _call(f, _ptr(a), _ptr(w), M, K, a.stride(0), w.stride(0), int(persistent == 2), _ptr(q_w), _ptr(k_w), float(eps), _ptr(rope),
+          _ptr(ctx.tok_pos), _ptr(ctx.tok_seq), _ptr(ctx.page_table), ctx.page_table.shape[1], _ptr(cache_pages), page_size, _ptr(q_out),
+          n_heads, n_kv_heads, _ptr(_status_word(a.device)), _stream())
+    return True
+
+
 def linear_stacked_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
     """out[:, i N:(i + 1) N] = a[i] @ w[i].T for a [G, M, K], w [G, N, K], out [M, G N], all bfloat16 and a, w contiguous, in
     one launch; False where a tile would lie across two of the products (or the sizes do not fit)."""

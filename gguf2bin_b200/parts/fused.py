@@ -17,6 +17,13 @@ import torch
 from .. import kernels
 
 
+def normed_rows(x32: torch.Tensor, norm, ctx, rows: Optional[torch.Tensor] = None, n: Optional[int] = None) -> torch.Tensor:
+    """norm(x32[rows]), ``n`` rows of it (default: all), in scratch memory."""
+    h = ctx.workspace.buffer("fused.normed", (x32.shape[0] if n is None else n, x32.shape[1]), ctx.dtype)
+    norm.forward(x32, h, rows)
+    return h
+
+
 def normed_linear(x32: torch.Tensor, norm, w: torch.Tensor, out: torch.Tensor, ctx,
                   rows: Optional[torch.Tensor] = None, gate_block: Optional[int] = None) -> None:
     """out = norm(x32[rows]) @ w.T, or, with ``gate_block``, out = silu(gate) * up of a fused
@@ -25,8 +32,7 @@ def normed_linear(x32: torch.Tensor, norm, w: torch.Tensor, out: torch.Tensor, c
     eps = getattr(norm, "plain_rms_eps", lambda: None)()
     if eps is not None and rows is None and kernels.normed_product(x32, eps, w, out, gate_block):
         return
-    h = ctx.workspace.buffer("fused.normed", (n, x32.shape[1]), ctx.dtype)
-    norm.forward(x32, h, rows)
+    h = normed_rows(x32, norm, ctx, rows, n)
     if gate_block is None:
         kernels.linear(h, w, out, workspace=ctx.workspace)
     elif not kernels.gate_up_fused(h, w, out, gate_block):

@@ -66,7 +66,7 @@ from .. import kernels
 from ..cache.storage import KVNeed, KVView
 from ..config.specs import ConfigError, PartSpec
 from ..weights.loader import Expected
-from .fused import normed_linear
+from .fused import normed_linear, normed_rows
 from .registry import norm_class, position_class, register_mixer
 
 
@@ -228,22 +228,37 @@ class GQAAttention:
 
     # ---- step ----------------------------------------------------------------
     def forward(self, h: torch.Tensor, ctx, view: KVView, residual32: torch.Tensor) -> None:
-        qkv = ctx.workspace.buffer("attn.qkv", (h.shape[0], self.w_qkv.shape[0]), self.dtype)
-        kernels.linear(h, self.w_qkv, qkv, workspace=ctx.workspace)
-        self._attend(qkv, ctx, view, residual32)
+        self._project(h, ctx, view, residual32)
 
     def forward_store(self, h: torch.Tensor, ctx, view: KVView, out32: torch.Tensor) -> None:
         """Stores the result instead of adding it."""
-        qkv = ctx.workspace.buffer("attn.qkv", (h.shape[0], self.w_qkv.shape[0]), self.dtype)
-        kernels.linear(h, self.w_qkv, qkv, workspace=ctx.workspace)
-        self._attend(qkv, ctx, view, out32, accumulate=False)
+        self._project(h, ctx, view, out32, accumulate=False)
 
     def forward_from_stream(self, x32: torch.Tensor, norm, ctx, view: KVView,
                             residual32: torch.Tensor) -> None:
         """The same with the block's norm folded into the q/k/v product."""
+        if self._prompt(x32.shape[0], ctx):
+            return self._project(normed_rows(x32, norm, ctx), ctx, view, residual32)
         qkv = ctx.workspace.buffer("attn.qkv", (x32.shape[0], self.w_qkv.shape[0]), self.dtype)
         normed_linear(x32, norm, self.w_qkv, qkv, ctx)
         self._attend(qkv, ctx, view, residual32)
+
+    def _prompt(self, rows: int, ctx) -> bool:
+        """Whether the step may have its q, k and v finished inside their product."""
+        return rows > 128 and not self.wide and not ctx.all_single and self.position.fused_rotation() is not None
+
+    def _project(self, h: torch.Tensor, ctx, view: KVView, out32: torch.Tensor, accumulate: bool = True) -> None:
+        T, ws = h.shape[0], ctx.workspace
+        if self._prompt(T, ctx):
+            inv_freq, rot = self.position.fused_rotation()
+            rope = ctx.rope_table(inv_freq) if inv_freq is not None else None
+            q = ws.buffer("attn.q", (T, self.nh * self.hd), self.dtype)
+            if kernels.heads_product(h, self.w_qkv, self.q_norm_w, self.k_norm_w, self.qk_eps, rope, rot, ctx, view.pages,
+                                     view.page_size, q, self.nh, 0 if self.shared_kv else self.nkv, self.hd):
+                return self._attend(None, ctx, view, out32, accumulate, q)
+        qkv = ws.buffer("attn.qkv", (T, self.w_qkv.shape[0]), self.dtype)
+        kernels.linear(h, self.w_qkv, qkv, workspace=ws)
+        self._attend(qkv, ctx, view, out32, accumulate)
 
     def _attend_wide(self, qkv: torch.Tensor, ctx, view: KVView, residual32: torch.Tensor, accumulate: bool = True) -> None:
         """q, k, v (and the gate's columns) of one product; the prologue adds the biases, norms q and k
@@ -285,10 +300,11 @@ class GQAAttention:
             o = og
         kernels.linear(o, self.w_o, residual32, accumulate=accumulate, workspace=ctx.workspace)
 
-    def _attend(self, qkv: torch.Tensor, ctx, view: KVView, residual32: torch.Tensor, accumulate: bool = True) -> None:
+    def _attend(self, qkv, ctx, view: KVView, residual32: torch.Tensor, accumulate: bool = True, q=None) -> None:
+        """From the projection on; with ``q`` its heads are finished and the pages written."""
         if self.wide:
             return self._attend_wide(qkv, ctx, view, residual32, accumulate)
-        T = qkv.shape[0]
+        T = (qkv if q is None else q).shape[0]
         nq = self.nh * self.hd
         nkv_own = 0 if self.shared_kv else self.nkv        # kv heads this layer projects
         nk = nkv_own * self.hd
@@ -296,16 +312,19 @@ class GQAAttention:
         fused = self.position.fused_rotation()
         o = ws.buffer("attn.o", (T, nq), self.dtype)
         rope = ctx.rope_table(fused[0]) if fused is not None and fused[0] is not None else None
-        if fused is None or not nkv_own or not kernels.attention_qkv(
+        if q is not None or fused is None or not nkv_own or not kernels.attention_qkv(
                 qkv, self.q_norm_w, self.k_norm_w, self.qk_eps, rope, fused[1], o, view.pages, ctx, self.nh, self.nkv, self.hd,
                 view.page_size, self.window, self.scale, sink=self.sink, chunk=self.chunk, softcap=self.softcap,
                 keep_first=self.keep_first):
-            q = ws.buffer("attn.q", (T, nq), self.dtype)
-            if fused is not None:
+            if q is not None:
+                pass
+            elif fused is not None:
+                q = ws.buffer("attn.q", (T, nq), self.dtype)
                 kernels.qknorm_rope_cache(qkv, self.nh, nkv_own, self.hd, self.q_norm_w,
                                           self.k_norm_w, self.qk_eps, rope, fused[1], ctx.tok_pos,
                                           ctx.tok_seq, ctx.page_table, view.pages, view.page_size, q)
             else:
+                q = ws.buffer("attn.q", (T, nq), self.dtype)
                 k = ws.buffer("attn.k", (T, nk), self.dtype)
                 v = ws.buffer("attn.v", (T, nk), self.dtype)
                 kernels.qknorm_rope_cache(qkv, self.nh, nkv_own, self.hd, self.q_norm_w,
