@@ -349,11 +349,22 @@ __device__ __forceinline__ void epilogue_tile_bulk(uint32_t tmem, unsigned char 
 // ---- heads: the q, k and v of a prompt -----------------------------------------------------------
 // The columns of C are the heads of q, k and v, 128 of them each, and what is wanted is not C: q and k normed head by head and rotated, k
 // and v in the cache's pages.  As a kernel of its own behind the product that is a write and two reads of memory more (16,384 tokens of 32
-// heads: 268 MB, 76 us behind a product of 92).  Here a warp rounds the 128 columns of a head to bfloat16, as C would hold them, into its two
-// staging boxes (the head's halves: an element and its partner of the rotation lie at one place of the two), and eight lanes read a row
-// back, 16 bytes of each half: what qknorm_rope_fast_kernel<bf16, 8, 8> (elementwise.cu) has in its registers, and its arithmetic in its
-// order, so that q and the pages get the same bits.
+// heads: 268 MB, 76 us behind a product of 92).  Here a warp rounds 32 rows of a head to bfloat16, as C would hold them, frees the accumulator
+// and lays them, sixteen rows at a time, into its staging buffer by the head's halves (an element and its partner of the rotation lie at one
+// place of the two); eight lanes read a row back, 16 bytes of each half: what qknorm_rope_fast_kernel<bf16, 8, 8> (elementwise.cu) has in its
+// registers, and its arithmetic in its order (the sum of a row's squares is taken where the row is one thread's, in the order of those eight
+// lanes), so that q and the pages get the same bits.  That is a chain of some 1,100 instructions a head with few of them independent: with
+// four warps, each both heads of a tile, it took 1.4 times as long as the tile's products at K = 1,024 (132 us); with eight, each a head, 118.
+// What is left above the product (92) is the angles: 128 KB a tile beside 512 KB of operands into the SM; without them it takes 108.
 constexpr int HEAD = 128;
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {     // as tmem_ld32, sixteen columns
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
 struct HeadsTail : ProductTail {
   const float *q_w, *k_w;                          // null: no norm
   const float2 *rope;                              // [tokens, 64] (cos, sin); null: no rotation
@@ -362,141 +373,161 @@ struct HeadsTail : ProductTail {
   float eps;
   int P, nh, nkv, page_size;
 };
-// What the epilogue of a tile needs of its rows, asked for before the tile's products are done: the angles of a lane's columns in the eight
-// rows it works on (the same for every head), and where the lane's own row goes in the cache, in rows, as far as it is the same for all heads.
+
+// One warp's part of a tile: a head of 32 rows; lane `sub` * 8 + c works on columns 8c .. 8c + 7 of both halves in rows 4i + sub.
 struct HeadRows {
-  float4 turn[8][4];
-  long long place;
-  __device__ __forceinline__ void ask(int m0, int n0, int cols, int M, int warp, int lane, const HeadsTail &tail) {
-    const int y = m0 + warp * 32, first_head = n0 / HEAD;
+  static constexpr int AHEAD = 2;                  // (three spill: 320 threads get 168 registers)
+  float4 turn[AHEAD][4];                           // the angles of its next rows
+  float wa[8], wb[8];
+  const float *w;
+  const float2 *rope;                              // null: neither
+  long long place;                                 // of the lane's own row in the cache, in rows
+  int head, y;
+
+  __device__ __forceinline__ void ask_turn(int i, int M, int lane) {
+    const float4 *from = reinterpret_cast<const float4 *>(rope + (size_t)min(y + 4 * i + (lane >> 3), M - 1) * (HEAD / 2) + 8 * (lane & 7));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) turn[i % AHEAD][j] = from[j];
+  }
+  // what does not depend on the products is asked for before they are done
+  __device__ __forceinline__ void ask(int m0, int n0, int M, int N, int warp, int lane, const HeadsTail &tail) {
+    y = m0 + (warp & 3) * 32;
+    head = n0 / HEAD + (warp >= 4);
+    if (head * HEAD >= N) return;
+    const bool value = head >= tail.nh + tail.nkv, query = head < tail.nh;
+    w = value ? nullptr : query ? tail.q_w : tail.k_w;
+    rope = value ? nullptr : tail.rope;
+    if (rope) {
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) ask_turn(i, M, lane);
+    }
+    if (w) {
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        *reinterpret_cast<float4 *>(wa + j) = *reinterpret_cast<const float4 *>(w + 8 * (lane & 7) + j);
+        *reinterpret_cast<float4 *>(wb + j) = *reinterpret_cast<const float4 *>(w + HEAD / 2 + 8 * (lane & 7) + j);
+      }
+    }
     place = 0;
-    if (n0 + cols > tail.nh * HEAD && y + lane < M) {
+    if (!query && y + lane < M) {
       const int pos = tail.tok_pos[y + lane];
       const int page = tail.page_table[(size_t)tail.tok_seq[y + lane] * tail.P + pos / tail.page_size];
-      place = (long long)page * 2 * tail.nkv * tail.page_size + pos % tail.page_size;
+      place = ((long long)page * 2 * tail.nkv + (head - tail.nh)) * tail.page_size + pos % tail.page_size;
     }
-    if (tail.rope && first_head < tail.nh + tail.nkv) {
+  }
+
+  // `drained` gives the accumulator back
+  template <typename Drained>
+  __device__ __forceinline__ void finish(uint32_t tmem, unsigned char *stage, int M, int N, int warp, int lane, const HeadsTail &tail,
+                                         Drained drained) {
+    if (head * HEAD >= N) return drained();        // the last tile may hold one head
+    const uint32_t from_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >= 4 ? HEAD : 0);
+    const int sub = lane >> 3, c = lane & 7;
+    uint32_t u[2][8][4];                           // the row, by halves and pieces of 16 bytes
+    float sums[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 *from = reinterpret_cast<const float4 *>(tail.rope + (size_t)min(y + 4 * i + (lane >> 3), M - 1) * (HEAD / 2) + 8 * (lane & 7));
+    for (int part = 0; part < 4; ++part) {         // sixteen columns of both halves at a time: the registers
+      uint32_t v[2][16];
+      tmem_ld16(from_tmem + part * 16, v[0]);
+      tmem_ld16(from_tmem + HEAD / 2 + part * 16, v[1]);
+      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 4; ++j) turn[i][j] = from[j];
+      for (int j = 0; j < 2; ++j) {
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+          for (int half = 0; half < 2; ++half) u[half][2 * part + j][e] = pack2(v[half][8 * j + 2 * e], v[half][8 * j + 2 * e + 1], tail);
+#pragma unroll
+          for (int odd = 0; odd < 2; ++odd)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              const uint32_t two = u[half][2 * part + j][e];
+              const float x = __uint_as_float(odd ? two & 0xffff0000u : two << 16);
+              ss = fmaf(x, x, ss);
+            }
+        }
+        sums[2 * part + j] = ss;
+      }
+    }
+    drained();
+    float own_inv = 1.f;
+    if (w) {
+      const float ss = ((sums[0] + sums[4]) + (sums[2] + sums[6])) + ((sums[1] + sums[5]) + (sums[3] + sums[7]));
+      own_inv = 1.f / sqrtf(ss / (float)HEAD + tail.eps);
+    }
+    const uint32_t own_row = smem_addr(stage) + (lane & 15) * 128;
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+      __syncwarp();                                // the rows in front have been read
+      if ((lane >> 4) == pass) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(own_row + half * 2048 + ((j ^ (lane & 7)) << 4)),
+                         "r"(u[half][j][0]), "r"(u[half][j][1]), "r"(u[half][j][2]), "r"(u[half][j][3]) : "memory");
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 4 * pass; i < 4 * pass + 4; ++i) {
+        const int r = 4 * i + sub;
+        const unsigned char *from = stage + (r & 15) * 128 + ((c ^ (r & 7)) << 4);
+        const uint4 xa = *reinterpret_cast<const uint4 *>(from), xb = *reinterpret_cast<const uint4 *>(from + 2048);
+        const long long at = __shfl_sync(0xffffffffu, place, r);
+        const float inv = __shfl_sync(0xffffffffu, own_inv, r);
+        const uint32_t ua[4] = {xa.x, xa.y, xa.z, xa.w}, ub[4] = {xb.x, xb.y, xb.z, xb.w};
+        float a[8], b[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          a[2 * j] = __uint_as_float(ua[j] << 16);
+          a[2 * j + 1] = __uint_as_float(ua[j] & 0xffff0000u);
+          b[2 * j] = __uint_as_float(ub[j] << 16);
+          b[2 * j + 1] = __uint_as_float(ub[j] & 0xffff0000u);
+        }
+        if (w) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            a[j] = (wa[j] * a[j]) * inv;
+            b[j] = (wb[j] * b[j]) * inv;
+          }
+        }
+        if (rope) {
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            const float4 cs = turn[i % AHEAD][j / 2];
+            const float a0 = a[j], b0 = b[j], a1 = a[j + 1], b1 = b[j + 1];
+            a[j] = a0 * cs.x - b0 * cs.y;
+            b[j] = a0 * cs.y + b0 * cs.x;
+            a[j + 1] = a1 * cs.z - b1 * cs.w;
+            b[j + 1] = a1 * cs.w + b1 * cs.z;
+          }
+          if (i + AHEAD < 8) ask_turn(i + AHEAD, M, lane);
+        }
+        if (y + r < M) {
+          bf16 *to = head < tail.nh ? tail.q_out + ((size_t)(y + r) * tail.nh + head) * HEAD : tail.cache + (size_t)at * HEAD;
+          *reinterpret_cast<uint4 *>(to + 8 * c) = make_uint4(pack2f(a[0], a[1]), pack2f(a[2], a[3]), pack2f(a[4], a[5]), pack2f(a[6], a[7]));
+          *reinterpret_cast<uint4 *>(to + HEAD / 2 + 8 * c) =
+              make_uint4(pack2f(b[0], b[1]), pack2f(b[2], b[3]), pack2f(b[4], b[5]), pack2f(b[6], b[7]));
+        }
       }
     }
   }
 };
 
-// what a kernel with an epilogue is launched with, and keeps of a tile's rows
+// what a kernel with an epilogue is launched with, keeps of a tile's rows, and how many warps finish tiles: 0 to 3 and 6 to 9 (the warps of
+// products and copies are 4 and 5; a warp reaches the accumulator's rows 32 (warp % 4) and on)
 struct NoRows {};
-template <int EPI> struct TailOf { using type = ProductTail; using Rows = NoRows; };
-template <> struct TailOf<EPI_HEADS> { using type = HeadsTail; using Rows = HeadRows; };
-
-template <int BN>
-__device__ __forceinline__ void epilogue_heads(uint32_t tmem, unsigned char *stage, int m0, int n0, int M, int N, int warp, int lane,
-                                               const HeadRows &rows, const HeadsTail &tail) {
-  static_assert(BN % HEAD == 0, "whole heads in a tile");
-  const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-  const int y = m0 + warp * 32, sub = lane >> 3, c = lane & 7;
-  const int first_head = n0 / HEAD, heads = min(BN, N - n0) / HEAD;
-  const uint32_t own_row = smem_addr(stage) + lane * 128;
-#pragma unroll 1
-  for (int i = 0; i < heads; ++i) {
-    const int head = first_head + i;
-    const int kind = head < tail.nh ? 0 : (head < tail.nh + tail.nkv ? 1 : 2);       // q, k, v
-    const float *w = kind == 0 ? tail.q_w : (kind == 1 ? tail.k_w : nullptr);
-    const bool turned = kind != 2 && tail.rope;
-    float wa[8], wb[8];
-    if (w) {
-#pragma unroll
-      for (int j = 0; j < 8; j += 4) {
-        *reinterpret_cast<float4 *>(wa + j) = *reinterpret_cast<const float4 *>(w + 8 * c + j);
-        *reinterpret_cast<float4 *>(wb + j) = *reinterpret_cast<const float4 *>(w + HEAD / 2 + 8 * c + j);
-      }
-    }
-    __syncwarp();                                  // the boxes of the head in front have been read
-#pragma unroll
-    for (int part = 0; part < 4; ++part) {
-      uint32_t v[32];
-      tmem_ld32(lane_addr + i * HEAD + part * 32, v);
-      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t *u = v + 8 * j;
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::
-                     "r"(own_row + (part / 2) * 4096 + (((4 * (part % 2) + j) ^ (lane & 7)) << 4)),
-                     "r"(pack2(u[0], u[1], tail)), "r"(pack2(u[2], u[3], tail)), "r"(pack2(u[4], u[5], tail)),
-                     "r"(pack2(u[6], u[7], tail)) : "memory");
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int r0 = 0; r0 < 8; r0 += 2) {            // two rows a lane at once: one row's chain of sums and its root behind the other's
-      float a[2][8], b[2][8];
-      long long at[2];
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int r = 4 * (r0 + k) + sub;
-        const unsigned char *from = stage + r * 128 + ((c ^ (r & 7)) << 4);
-        const uint4 xa = *reinterpret_cast<const uint4 *>(from), xb = *reinterpret_cast<const uint4 *>(from + 4096);
-        at[k] = __shfl_sync(0xffffffffu, rows.place, r);
-        const uint32_t ua[4] = {xa.x, xa.y, xa.z, xa.w}, ub[4] = {xb.x, xb.y, xb.z, xb.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          a[k][2 * j] = __uint_as_float(ua[j] << 16);
-          a[k][2 * j + 1] = __uint_as_float(ua[j] & 0xffff0000u);
-          b[k][2 * j] = __uint_as_float(ub[j] << 16);
-          b[k][2 * j + 1] = __uint_as_float(ub[j] & 0xffff0000u);
-        }
-      }
-      if (w) {
-        float ss[2] = {0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            ss[k] = fmaf(a[k][j], a[k][j], ss[k]);
-            ss[k] = fmaf(b[k][j], b[k][j], ss[k]);
-          }
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-          for (int k = 0; k < 2; ++k) ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], o);
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const float inv = 1.f / sqrtf(ss[k] / (float)HEAD + tail.eps);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            a[k][j] = (wa[j] * a[k][j]) * inv;
-            b[k][j] = (wb[j] * b[k][j]) * inv;
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        if (turned) {
-#pragma unroll
-          for (int j = 0; j < 8; j += 2) {
-            const float4 cs = rows.turn[r0 + k][j / 2];
-            const float a0 = a[k][j], b0 = b[k][j], a1 = a[k][j + 1], b1 = b[k][j + 1];
-            a[k][j] = a0 * cs.x - b0 * cs.y;
-            b[k][j] = a0 * cs.y + b0 * cs.x;
-            a[k][j + 1] = a1 * cs.z - b1 * cs.w;
-            b[k][j + 1] = a1 * cs.w + b1 * cs.z;
-          }
-        }
-        const int t = y + 4 * (r0 + k) + sub;
-        if (t < M) {
-          bf16 *to = kind == 0 ? tail.q_out + ((size_t)t * tail.nh + head) * HEAD
-                               : tail.cache + (size_t)(at[k] + (long long)(head - tail.nh) * tail.page_size) * HEAD;
-          *reinterpret_cast<uint4 *>(to + 8 * c) =
-              make_uint4(pack2f(a[k][0], a[k][1]), pack2f(a[k][2], a[k][3]), pack2f(a[k][4], a[k][5]), pack2f(a[k][6], a[k][7]));
-          *reinterpret_cast<uint4 *>(to + HEAD / 2 + 8 * c) =
-              make_uint4(pack2f(b[k][0], b[k][1]), pack2f(b[k][2], b[k][3]), pack2f(b[k][4], b[k][5]), pack2f(b[k][6], b[k][7]));
-        }
-      }
-    }
-  }
-}
+template <int EPI> struct Finisher {
+  using Tail = ProductTail;
+  using Rows = NoRows;
+  static constexpr int WARPS = 4, STAGE = 2 * 4096;
+};
+template <> struct Finisher<EPI_HEADS> {
+  using Tail = HeadsTail;
+  using Rows = HeadRows;
+  static constexpr int WARPS = 8, STAGE = 4096;
+};
 
 // ---- K in parts over a cluster ---------------------------------------------------------------
 // With fewer tiles than half the SMs, the CTAs of a cluster take the same tile and one part of
@@ -653,10 +684,10 @@ template <int BN, int STAGES> struct SmemP {
 };
 
 template <int BN, int STAGES, int EPI>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(64 + 32 * Finisher<EPI>::WARPS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                           const __grid_constant__ CUtensorMap map_c, int M, int N, int K, int group_m,
-                          int k_parts, int *__restrict__ status, typename TailOf<EPI>::type glu) {
+                          int k_parts, int *__restrict__ status, typename Finisher<EPI>::Tail glu) {
   pdl_launch();
   extern __shared__ unsigned char smem_raw[];
   using S = SmemP<BN, STAGES>;
@@ -686,7 +717,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full0 + 8 * b, 1);
-      mbar_init(acc_empty0 + 8 * b, 4);            // one arrival per epilogue warp
+      mbar_init(acc_empty0 + 8 * b, Finisher<EPI>::WARPS);      // one arrival per epilogue warp
     }
     mbar_init(part_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -790,7 +821,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       TFLUSH(2); TFLUSH(3); TFLUSH(4); TFLUSH(5);
     }
   } else if (k_parts == 1) {
-    unsigned char *stage = smem + S::SCRATCH_OFFSET + warp * (2 * 4096);
+    unsigned char *stage = smem + S::SCRATCH_OFFSET + (warp < 4 ? warp : warp - 2) * Finisher<EPI>::STAGE;
     uint32_t j = 0, box = 0;
     TDECL(6); TDECL(7); TDECL(8);
     TICK(t_epi);
@@ -799,8 +830,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       int tm, tn;
       tile_of(t, tiles_m, tiles_n, group_m, tm, tn);
       const int m0 = tm * BM, n0 = tn * BN;
-      typename TailOf<EPI>::Rows rows;
-      if constexpr (EPI == EPI_HEADS) rows.ask(m0, n0, BN, M, warp, lane, glu);
+      typename Finisher<EPI>::Rows rows;
+      if constexpr (EPI == EPI_HEADS) rows.ask(m0, n0, M, N, warp, lane, glu);
       TICK(t_af);
       if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1)) {
         if (lane == 0) atomicExch(status, ST_EPILOGUE_TIMEOUT);
@@ -809,12 +840,17 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       TOCK(7, t_af);
       TOCK(8, t_af - 1 + clock64());               // counts tiles (adds 1)
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      if constexpr (EPI == EPI_HEADS) epilogue_heads<BN>(tmem + buf * BN, stage, m0, n0, M, N, warp, lane, rows, glu);
-      else epilogue_tile_bulk<BN, EPI>(tmem + buf * BN, stage, &map_c, m0, n0, M, N, warp, lane, box, glu);
-      // every load of this warp from the accumulator has completed (each is waited for)
-      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty0 + 8 * buf);
+      auto drained = [&] {                         // every load of this warp from the accumulator has completed (each is waited for)
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty0 + 8 * buf);
+      };
+      if constexpr (EPI == EPI_HEADS) {
+        rows.finish(tmem + buf * BN, stage, M, N, warp, lane, glu, drained);
+      } else {
+        epilogue_tile_bulk<BN, EPI>(tmem + buf * BN, stage, &map_c, m0, n0, M, N, warp, lane, box, glu);
+        drained();
+      }
     }
     if (lane == 0) bulk_wait<0>();                 // the staging buffers are read and C is written
     TOCK(6, t_epi);
@@ -1057,10 +1093,10 @@ template <int BN, int STAGES> struct SmemPair {
 enum { ST_PAIR_TIMEOUT = 4 };
 
 template <int BN, int STAGES, int EPI>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(64 + 32 * Finisher<EPI>::WARPS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_c, int M, int N, int K, int group_m,
-                    int *__restrict__ status, typename TailOf<EPI>::type glu) {
+                    int *__restrict__ status, typename Finisher<EPI>::Tail glu) {
   pdl_launch();
   extern __shared__ unsigned char smem_raw[];
   using S = SmemPair<BN, STAGES>;
@@ -1087,7 +1123,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full0 + 8 * b, 1);
-      mbar_init(acc_empty0 + 8 * b, 8);            // one arrival per epilogue warp of both CTAs
+      mbar_init(acc_empty0 + 8 * b, 2 * Finisher<EPI>::WARPS);  // one arrival per epilogue warp of both CTAs
     }
     mbar_init(done_bar, 1);
     mbar_init_fence();
@@ -1155,7 +1191,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
     }
   } else {
-    unsigned char *stage = smem + S::SCRATCH_OFFSET + warp * (2 * 4096);
+    unsigned char *stage = smem + S::SCRATCH_OFFSET + (warp < 4 ? warp : warp - 2) * Finisher<EPI>::STAGE;
     const uint32_t leader_acc_empty0 = map_to_cta(acc_empty0, 0);
     uint32_t j = 0, box = 0;
     for (int t = pair; t < n_tiles; t += pairs, ++j) {
@@ -1163,19 +1199,24 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       int tm, tn;
       tile_of(t, tiles_m, tiles_n, group_m, tm, tn);
       const int m0 = tm * (2 * BM) + (int)rank * BM, n0 = tn * BN;
-      typename TailOf<EPI>::Rows rows;
-      if constexpr (EPI == EPI_HEADS) rows.ask(m0, n0, BN, M, warp, lane, glu);
+      typename Finisher<EPI>::Rows rows;
+      if constexpr (EPI == EPI_HEADS) rows.ask(m0, n0, M, N, warp, lane, glu);
       if (!mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1)) {
         if (lane == 0) atomicExch(status, ST_EPILOGUE_TIMEOUT);
         break;
       }
       tc_fence_after();
-      if constexpr (EPI == EPI_HEADS) epilogue_heads<BN>(tmem + buf * BN, stage, m0, n0, M, N, warp, lane, rows, glu);
-      else epilogue_tile_bulk<BN, EPI>(tmem + buf * BN, stage, &map_c, m0, n0, M, N, warp, lane, box, glu);
-      // every load of this warp from the accumulator has completed (each is waited for)
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(leader_acc_empty0 + 8 * buf);
+      auto drained = [&] {                         // every load of this warp from the accumulator has completed (each is waited for)
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(leader_acc_empty0 + 8 * buf);
+      };
+      if constexpr (EPI == EPI_HEADS) {
+        rows.finish(tmem + buf * BN, stage, M, N, warp, lane, glu, drained);
+      } else {
+        epilogue_tile_bulk<BN, EPI>(tmem + buf * BN, stage, &map_c, m0, n0, M, N, warp, lane, box, glu);
+        drained();
+      }
     }
     if (lane == 0) bulk_wait<0>();                 // the staging buffers are read and C is written
   }
@@ -1597,7 +1638,7 @@ static_assert(SmemP<128, 6>::RING_BYTES == 196608 && SmemP<256, 4>::RING_BYTES =
 // want_parts: 1 to 4 parts of K
 template <int BN, int STAGES, int EPI>
 static int launch_persistent(const CUtensorMap &ma, const CUtensorMap &mw, void *C, int M, int N, int K, int ldc,
-                             int want_parts, int *status, typename TailOf<EPI>::type glu, cudaStream_t stream) {
+                             int want_parts, int *status, typename Finisher<EPI>::Tail glu, cudaStream_t stream) {
   static G2bPerDevice configured;
   const int smem = SmemP<BN, STAGES>::TOTAL;
   const int cfg_dev = g2b_current_device();
@@ -1628,7 +1669,7 @@ static int launch_persistent(const CUtensorMap &ma, const CUtensorMap &mw, void 
                  parts, room);
   }
   const unsigned grid = parts > 1 ? (unsigned)(tiles * parts) : (unsigned)(tiles < sm_count() ? tiles : sm_count());
-  g2b_launch_cluster(gemm_tc_persistent_kernel<BN, STAGES, EPI>, dim3(grid), dim3(THREADS), smem, stream,
+  g2b_launch_cluster(gemm_tc_persistent_kernel<BN, STAGES, EPI>, dim3(grid), dim3(64 + 32 * Finisher<EPI>::WARPS), smem, stream,
                      (unsigned)parts, ma, mw, mc, M, N, K, rows_of_tiles_per_group((M + BM - 1) / BM, BM, K), parts,
                      status, glu);
   return g2b_check_launch("gemm_tc (persistent)");
@@ -1636,7 +1677,7 @@ static int launch_persistent(const CUtensorMap &ma, const CUtensorMap &mw, void 
 
 template <int BN, int STAGES, int EPI>
 static int launch_pair(const CUtensorMap &ma, const CUtensorMap &mw, void *C, int M, int N, int K, int ldc,
-                       int *status, typename TailOf<EPI>::type glu, cudaStream_t stream) {
+                       int *status, typename Finisher<EPI>::Tail glu, cudaStream_t stream) {
   static G2bPerDevice configured;
   const int smem = SmemPair<BN, STAGES>::TOTAL;
   const int cfg_dev = g2b_current_device();
@@ -1659,7 +1700,7 @@ static int launch_pair(const CUtensorMap &ma, const CUtensorMap &mw, void *C, in
   const int max_pairs = sm_count() / 2;
   if (max_pairs < 1) G2B_REFUSE("gemm_tc: the paired kernel needs two SMs");
   const unsigned pairs = (unsigned)(tiles < max_pairs ? tiles : max_pairs);
-  g2b_launch_cluster(gemm_tc_pair_kernel<BN, STAGES, EPI>, dim3(2 * pairs), dim3(THREADS), smem, stream, 2u, ma, mw,
+  g2b_launch_cluster(gemm_tc_pair_kernel<BN, STAGES, EPI>, dim3(2 * pairs), dim3(64 + 32 * Finisher<EPI>::WARPS), smem, stream, 2u, ma, mw,
                      mc, M, N, K, rows_of_tiles_per_group((M + 2 * BM - 1) / (2 * BM), 2 * BM, K), status, glu);
   return g2b_check_launch("gemm_tc (pairs)");
 }
@@ -1836,8 +1877,8 @@ extern "C" int g2b_gemm_tc_heads_whole(int M, int N, int K) {
 // The product of A [M, K] with the q, k and v rows of W [(nh + 2 nkv) 128, K], q and k normed by head (q_w, k_w; null: not) and rotated
 // (rope: the step's table; null: not), q to q_out [M, nh 128], k and v to the cache's pages: what g2b_gemm_tc into a buffer and
 // g2b_qknorm_rope_cache on it give.  pair: pairs of CTAs, else the persistent kernel, as the product alone would run.  Product and prologue kernel
-// before, and now: 16,384 tokens, 16 and 8 heads, K = 1,024: 92 + 76 us, 132 (the four warps of the epilogue set the pace: 9.6 us a tile whose
-// products take 6.3); 2,048 tokens: 16 + 10 us, 24; 12,000 tokens, 32 and 8 heads, K = 4,096: 301 + 63 us, 299 (hidden behind the products).
+// before, and now: 16,384 tokens, 16 and 8 heads, K = 1,024: 92 + 76 us, 118; 2,048 tokens: 16 + 10 us, 20.6; 12,000 tokens, 32 and 8
+// heads, K = 4,096: 301 + 63 us, 299 (hidden behind the products).
 extern "C" int g2b_gemm_tc_heads(const void *A, const void *W, int M, int K, int lda, int ldw, int pair, const float *q_w,
                                  const float *k_w, float eps, const float *rope, const int *tok_pos, const int *tok_seq,
                                  const int *page_table, int P, void *cache, int page_size, void *q_out, int nh, int nkv, int *status,
