@@ -20,9 +20,9 @@
 //   warps 0-7  add: warp w reads lanes 32 (w % 4) .. + 31 and columns 128 (w / 4) .. + 127 of a finished accumulator and adds them to its
 //              128 floats a thread, while the other accumulator is filled; at the end they write C, through shared memory, in rows
 //
-// Rows with an entry that is not finite, or whose largest entry is 2^120 and more (its parts may round to infinity) or below 2^-80 (its third
-// part would fall under bfloat16's range), are flagged; an output of a flagged row of A or W is summed from the floats themselves in the order
-// of gemm_simt.cu, by the warps that would have written it.
+// Rows with an entry that is not finite, of 2^60 and more (sums of 64 products of smaller ones stay below 2^126, whatever their signs) or below
+// 2^-103 but not zero (its last bit is under 2^-126, the smallest normal number, so a part would lose bits) are flagged; an output of a flagged
+// row of A or W is summed from the floats themselves in the order of gemm_simt.cu, by the warps that would have written it.
 //
 // What bounds it: the tensor cores do six products for one and need a block's 24 in 3,072 cycles (128 x 256 x 64 a CTA at 8,192 operations a
 // cycle), in which the copies bring 96 KB a CTA from the L2; with 128 x 128 tiles a CTA, or 256 x 128 a pair (96 and 72 KB in 1,536 cycles),
@@ -70,6 +70,12 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t (&p)[3]) {
   }
 }
 
+// Three parts do not hold it, or its products (NaN too).
+__device__ __forceinline__ bool out_of_range(float x) {
+  const float size = fabsf(x);
+  return !(size < 0x1p60f) || (size < 0x1p-103f && size != 0.f);
+}
+
 // A warp a row of A (rows 0 .. M - 1) or of W (M .. M + N - 1); `ld` is the parts' row length, a multiple of 8, zeros behind K.
 __global__ void __launch_bounds__(256)
 split_kernel(const float *A, const float *__restrict__ W, int M, int N, int K, int lda, int ldw, bf16 *parts_a, bf16 *parts_w, int ld, int *flags) {
@@ -82,7 +88,7 @@ split_kernel(const float *A, const float *__restrict__ W, int M, int N, int K, i
   const float *x = of_a ? A + (size_t)r * lda : W + (size_t)(r - M) * ldw;
   const size_t plane = (size_t)(of_a ? M : N) * ld;
   bf16 *to = (of_a ? parts_a + (size_t)r * ld : parts_w + (size_t)(r - M) * ld);
-  float most = 0.f, odd = 0.f;
+  bool odd = false;
   constexpr int AHEAD = 2;
   for (int k0 = lane * 8; k0 < ld; k0 += 256 * AHEAD) {
     float4 v[AHEAD][2];
@@ -104,16 +110,11 @@ split_kernel(const float *A, const float *__restrict__ W, int M, int N, int K, i
 #pragma unroll
       for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4 *>(to + i * plane + k) = make_uint4(p[0][i], p[1][i], p[2][i], p[3][i]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float first = __uint_as_float(p[i][0] << 16), second = __uint_as_float(p[i][0] & 0xffff0000u);
-        most = fmaxf(most, fmaxf(fabsf(first), fabsf(second)));
-        odd = fmaf(first, 0.f, fmaf(second, 0.f, odd));  // NaN behind an infinity or a NaN
-      }
+      for (int i = 0; i < 2; ++i) odd |= out_of_range(v[u][i].x) | out_of_range(v[u][i].y) | out_of_range(v[u][i].z) | out_of_range(v[u][i].w);
     }
   }
-  most = warp_max(most);
-  odd = warp_sum(odd);
-  if (lane == 0) flags[r] = !(odd == 0.f) || most >= 0x1p120f || (most > 0.f && most < 0x1p-80f);
+  odd = __any_sync(0xffffffffu, odd);
+  if (lane == 0) flags[r] = odd;
 }
 
 // ---- the product -----------------------------------------------------------------------------------------

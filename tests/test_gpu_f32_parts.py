@@ -62,6 +62,35 @@ def test_rows_that_three_parts_do_not_hold():
     assert same(acc, out + 1)
 
 
+@pytest.mark.parametrize("where", ["a", "w"])
+def test_entries_that_three_parts_do_not_hold(where):
+    """A tiny entry beside ordinary ones whose partners are zero, and large ones whose partial products would be infinities of either sign: the
+    bits of the kernel of multiply-adds."""
+    from gguf2bin_b200 import kernels
+    x, y = torch.zeros(130, 96, device=DEV), torch.zeros(260, 96, device=DEV)
+    x[:, 0], x[:, 1] = 1.0, 1.2345679 * 2.0 ** -torch.arange(130.0, device=DEV)      # 1.23 * 2^0 .. 2^-129
+    y[:, 1] = 1.0                                 # meets the tiny entry alone
+    x[3, :], y[5, :] = 0.0, 0.0
+    x[3, 7], y[5, 7] = 1.9990001 * 2.0 ** 63, 1.9990001 * 2.0 ** 63                  # just within range; of the parts' products the first is not
+    a, w = (x, y) if where == "a" else (y, x)
+    M, N = a.shape[0], w.shape[0]
+    out, plain = product(a, w, torch.full((M, N), math.nan, device=DEV)), torch.empty(M, N, device=DEV)
+    kernels.gemm_simt(a, w, plain)
+    assert torch.equal(out, plain)
+    big = [3, 5] if where == "a" else [5, 3]
+    assert out[big[0], big[1]].isfinite()
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -40, 2.0 ** -52, 2.0 ** -56, 2.0 ** -60, 2.0 ** -63, 2.0 ** 30])
+def test_small_and_large_products(scale):
+    """Products down to the smallest normal numbers, whose parts' products lie under them, keep the error of 32-bit sums."""
+    a, w = (torch.where(x.abs() < 0.01, 0.01, x) * scale for x in (rnd(200, 320, seed=1), rnd(300, 320, seed=2)))
+    out = product(a, w, torch.full((200, 300), math.nan, device=DEV))
+    size = a.double().abs() @ w.double().abs().T
+    # a product or a sum that is no normal number may be off by half of the smallest number there is, 2^-149
+    assert ((out.double() - a.double() @ w.double().T).abs() <= (66 + 5) * EPS * size + 6 * 320 * 2.0 ** -150).all()
+
+
 def test_slices_of_the_matrix(monkeypatch):
     from gguf2bin_b200 import kernels
     a, w = rnd(200, 1024, seed=1), rnd(1000, 1024, seed=2)
