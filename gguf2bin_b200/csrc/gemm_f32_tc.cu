@@ -1,14 +1,18 @@
 // float32 products of many rows on the 5th-generation tensor cores:  C[M,N] (=|+=) A[M,K] * W[N,K]^T, everything float.
 //
-// A float is the sum of three bfloat16, x = x1 + x2 + x3, each the rest of the one before rounded to nearest (24 bits in 3 x 8 and two
-// signs; what is left is below 2^-26 of x).  Of the nine products of two such sums the six largest,
+// A float is the sum of three bfloat16, x = x1 + x2 + x3, each the rest of the one before rounded to nearest (7 + 8 + 8 bits and two
+// signs hold all 24).  Of the nine products of two such sums the six largest,
 //   a1 w3 + a3 w1 + a2 w2 + a1 w2 + a2 w1 + a1 w1,
-// are exact in 32 bits; the three left out are below 2^-25 of a1 w1.  The tensor cores' own sums cut low bits off, so they are kept
-// short: for every 64-wide block of K the 24 products of 16 are added in a fresh accumulator, the small ones first (the cuts then fall
-// on a small sum, and on the four last products), and a block's sum is added to a float in registers, rounded to nearest, block after block.
-// That is the order of sums of gemm_simt.cu (chunks of 64, then the chunks), with other rounding inside a chunk.
-// Relative error against 64 bits (2-norm, normal entries): 0.8 to 1.2e-7 for K = 68 to 3,072, where gemm_simt.cu has 1.5 to 1.9e-7; the largest
-// difference over the sum of magnitudes is 0.4 to 0.6 of that kernel's.
+// are exact in 32 bits; the three left out are below 2^-23 of a1 w1, 2^-26 in the mean square.  The tensor cores' own sums cut low bits off: always
+// toward zero, which sums of one sign do not average out.  So they are kept short: for every 64-wide block of K the small products and then
+// the first half of the a1 w1 are added in one fresh accumulator, the second half in another (the cuts then fall on a small sum and on halves; a
+// first part of seven bits leaves less to cut).  The two are added, rounded to nearest, and then to a sum in registers that carries along what
+// rounding takes from it, as two bfloat16 a register.
+// Relative error against 64 bits (2-norm), K = 64 to 3,072 and 17,408, gemm_simt.cu's in brackets:
+//   normal entries 0.5 to 0.8e-7 (1.4 to 3.3); their magnitudes 0.4 to 0.5e-7 (0.7 to 2.5); 1 + 0.1 normal 0.4 to 0.5e-7 (0.6 to 2.4); behind SiLU
+//   0.6 to 0.7e-7 (0.7 to 2.5).  Log-normal entries over ten powers of e, where a few products decide: 0.4 to 0.9e-7 (0.4 to 1.6).
+// Results of one sign are too small by 2 to 4e-8 in the mean, whatever K is (gemm_simt.cu: by nothing); with one accumulator, eight-bit first parts
+// and sums without rests by 8e-8, and the 2-norm error came to 1.6 of gemm_simt.cu's there.
 //
 // Two launches.  `split_kernel` writes the three parts of A and W, [3 * rows][K] each, a warp a row, and says for every row whether the sum of
 // three is good for it.  `gemm_f32_tc_kernel`: a pair of CTAs takes a 256 x 256 tile (cta_group::2: each brings its own 128 rows of A and half
@@ -16,19 +20,22 @@
 // their order, for a range of columns).  Roles by warp:
 //   warp 8   copies: per block of K the three parts of A and of W (128-byte swizzle), two blocks in flight; a part's place is filled again
 //            as soon as the last product that reads it is done
-//   warp 9   products, in the pair's first CTA: 24 tcgen05.mma a block (kind::f16, M = N = 256, K = 16) into one of two accumulators
-//   warps 0-7  add: warp w reads lanes 32 (w % 4) .. + 31 and columns 128 (w / 4) .. + 127 of a finished accumulator and adds them to its
-//              128 floats a thread, while the other accumulator is filled; at the end they write C, through shared memory, in rows
+//   warp 9   products, in the pair's first CTA: 24 tcgen05.mma a block (kind::f16, M = 256, N = 128, K = 16) for either half of the columns, into
+//            the half's two accumulators
+//   warps 0-7  add: warp w reads lanes 32 (w % 4) .. + 31 and a half (w / 4) of the columns of the accumulators of one half of the tile and adds
+//              them to 64 of its 128 floats a thread, while the other half's are filled; at the end they write C, through shared memory, in rows
+//   (half h takes rows 64 h .. + 63 of either CTA's 128 rows of W, so that a warp's columns are the 128 from 128 (w / 4) on)
 //
-// Rows with an entry that is not finite, of 2^60 and more (sums of 64 products of smaller ones stay below 2^126, whatever their signs) or below
+// Rows with an entry that is not finite, of 2^50 and more (sums of the products of smaller ones stay below 2^127 for any K) or below
 // 2^-103 but not zero (its last bit is under 2^-126, the smallest normal number, so a part would lose bits) are flagged; an output of a flagged
 // row of A or W is summed from the floats themselves in the order of gemm_simt.cu, by the warps that would have written it.
 //
-// What bounds it: the tensor cores do six products for one and need a block's 24 in 3,072 cycles (128 x 256 x 64 a CTA at 8,192 operations a
-// cycle), in which the copies bring 96 KB a CTA from the L2; with 128 x 128 tiles a CTA, or 256 x 128 a pair (96 and 72 KB in 1,536 cycles),
-// the L2's rate bounded it (about 10 TB/s, 2,070 cycles a block).
-// Measured: 3,065 cycles a block at the 1.57 GHz that the clock falls to.  701 rows, parts included: 45 us for 4096 x 1024, 50 for 6144 x 1024, 38
-// for 1024 x 2048, 51 for 1024 x 3072 (228, 230, 140 and 210 by gemm_f32_tile_kernel); 2,100 rows: 127 us for 6144 x 1024, 208 TFLOP/s (685).
+// What bounds it: the tensor cores do six products for one.  A block's 24 products of 256 columns would take 3,072 cycles (128 x 256 x 64 a CTA at
+// 8,192 operations a cycle); as 48 of 128 columns A is read from shared memory twice and they take 1.4 times that, and the adders, whose sums with
+// rests and loads from tensor memory come one after another, 1.6 times.  (With 256 columns there is no room for two accumulators a block beside
+// the next block's: 83 us where this takes 72.)  Sums without rests: 63 us; one accumulator a block as well, which the errors above forbid: 45.
+// Measured: 701 rows, parts included: 72 us for 4096 x 1024, 78 for 6144 x 1024, 53 for 1024 x 2048, 73 for 1024 x 3072 (229, 230, 140 and 209 by
+// gemm_f32_tile_kernel); 2,100 rows: 208 us for 6144 x 1024 (674).
 //
 // Every wait gives up after a bounded number of polls and leaves a code in `*status`, as in gemm_tc.cu.
 #include "common.cuh"
@@ -36,6 +43,8 @@
 #include "tc_common.cuh"
 
 #include <math.h>
+
+#include <type_traits>
 
 G2B_DEFINE_LAST_ERROR
 
@@ -46,9 +55,11 @@ constexpr int PART_BYTES = BM * BK * 2;                  // one part of a CTA's 
 static_assert(BN / 2 == BM, "the parts of A and W have one size");
 constexpr int STAGES = 2, SLOT_BYTES = 2 * PART_BYTES;   // a slot: the part p of A and of W; slots [stage][p]
 constexpr int ADDERS = 8, THREADS = (ADDERS + 4) * 32;    // the last two warps only complete a group of four
-// Registers: 384 threads start with 168 each (64,512); the adders hold 128 sums and take 224, the others keep 40: 256 * 224 + 128 * 40 = 62,464.
-constexpr int ADDER_REGS = 224, OTHER_REGS = 40;
-constexpr int COLS = BN / 2;                             // columns of an adder
+// Registers: 384 threads start with 168 each (64,512); the adders hold 128 sums and their 64 pairs of rests and take 232, the others keep 40:
+// 256 * 232 + 128 * 40 = 64,512.
+constexpr int ADDER_REGS = 232, OTHER_REGS = 40;
+constexpr int COLS = BN / 2;                             // columns of an adder, and of a half
+constexpr int AT_ONCE = 16;                              // columns read from an accumulator at a time
 constexpr int SPLIT_MOST = 4;
 constexpr int SUM_CHUNK = 64;
 constexpr int RING_BYTES = STAGES * 3 * SLOT_BYTES;
@@ -60,11 +71,15 @@ static_assert(RECEIVED_BYTES + OUT_BYTES <= RING_BYTES, "both lie where the ring
 enum { ST_PRODUCER_TIMEOUT = 21, ST_MMA_TIMEOUT = 22, ST_ADDER_TIMEOUT = 23 };
 
 // ---- parts ---------------------------------------------------------------------------------------------
-// Two floats as their parts, packed pairs of bfloat16.
+// Two floats as their parts, packed pairs of bfloat16; the first is rounded to seven bits.
+__device__ __forceinline__ float seven_bits(float x) {
+  const uint32_t u = __float_as_uint(x);
+  return __uint_as_float((u + 0xffffu + (u >> 17 & 1)) & 0xfffe0000u);
+}
 __device__ __forceinline__ void split2(float x, float y, uint32_t (&p)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    p[i] = pack_bf16(x, y);
+    p[i] = i == 0 ? pack_bf16(seven_bits(x), seven_bits(y)) : pack_bf16(x, y);
     x -= __uint_as_float(p[i] << 16);
     y -= __uint_as_float(p[i] & 0xffff0000u);
   }
@@ -73,7 +88,7 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t (&p)[3]) {
 // Three parts do not hold it, or its products (NaN too).
 __device__ __forceinline__ bool out_of_range(float x) {
   const float size = fabsf(x);
-  return !(size < 0x1p60f) || (size < 0x1p-103f && size != 0.f);
+  return !(size < 0x1p50f) || (size < 0x1p-103f && size != 0.f);
 }
 
 // A warp a row of A (rows 0 .. M - 1) or of W (M .. M + N - 1); `ld` is the parts' row length, a multiple of 8, zeros behind K.
@@ -120,6 +135,31 @@ split_kernel(const float *A, const float *__restrict__ W, int M, int N, int K, i
 // ---- the product -----------------------------------------------------------------------------------------
 __device__ __forceinline__ void st_cluster16(uint32_t addr, float4 v) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+// sum += v, two of each, with what was lost to rounding so far added to v first and what is lost now kept.
+__device__ __forceinline__ void add_with_rest(float &s0, float &s1, uint32_t &rest, float2 v) {
+  const float2 s = make_float2(s0, s1);
+  v = add2(v, make_float2(__uint_as_float(rest << 16), __uint_as_float(rest & 0xffff0000u)));
+  const float2 t = add2(s, v);
+  const float2 minus = make_float2(-1.f, -1.f);
+  const float2 lost = fma2(fma2(s, minus, t), minus, v);           // v - (t - s)
+  rest = pack_bf16(lost.x, lost.y);
+  s0 = t.x, s1 = t.y;
+}
+
+// D (+)= A * B of a pair; the descriptors' low words (their high words are one constant), so that the issuing thread keeps few registers
+template <bool ACC>
+__device__ __forceinline__ void umma_pair_lo(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+  constexpr uint32_t HIGH = (1024 >> 4) | (1u << 14) | (2u << 29);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 da, {%1, %4};\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}\n"
+      ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(HIGH), "n"(ACC ? 1 : 0)
+      : "memory");
 }
 
 // Maps of the parts: [3 M][K] and [3 N][K], boxes of 128 rows.  Rows behind the last of a part belong to the next one (or are zeros):
@@ -186,38 +226,52 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
     if (warp == ADDERS + 1 && lane == 0 && half == 0) {
-      constexpr uint32_t idesc = instr_desc(2 * BM, BN, false);
+      constexpr uint32_t idesc = instr_desc(2 * BM, COLS, false);
+      const std::true_type yes;                  // the first of a sum
+      const std::false_type no;
       const uint16_t both = (uint16_t)(3u << rank);
       bool ok = true;
       for (int i = 0; i < nkb && ok; ++i) {
-        const int b = i & 1, s0 = (i % STAGES) * 3;
+        const int s0 = (i % STAGES) * 3;
         const uint32_t at = smem_addr(smem + s0 * SLOT_BYTES), parity = (i / STAGES) & 1;
-        auto arrived = [&](int p) { return mbar_wait(full0 + 8 * (s0 + p), parity); };
-        auto products = [&](int pa, int pw, uint32_t fresh) {
-          const uint64_t da = desc_k_major(at + pa * SLOT_BYTES), db = desc_k_major(at + pw * SLOT_BYTES + PART_BYTES);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          // a part is there for the second half when it was for the first
+          auto arrived = [&](int p) { return h || mbar_wait(full0 + 8 * (s0 + p), parity); };
+          const uint32_t x = tmem + h * 2 * COLS, y = x + COLS;
+          uint32_t lo = ((at & 0x3FFFF) >> 4 | 1u << 16);
+          asm volatile("" : "+r"(lo));           // or all 48 descriptors are kept over the blocks, in memory
+          const uint32_t lo_w = lo + h * (PART_BYTES / 32);
+          auto products = [&](int pa, int pw, int k0, int k1, uint32_t to, auto fresh) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_bf16_pair(tmem + b * BN, da + 2 * k, db + 2 * k, idesc, (fresh && k == 0) ? 0u : 1u);
-        };
-        ok = (i < 2 || mbar_wait_cluster(sum_empty0 + 8 * b, (i / 2 - 1) & 1)) && arrived(2) && arrived(0);
-        if (ok) {
+            for (int k = k0; k < k1; ++k) {
+              const uint32_t da = lo + pa * (SLOT_BYTES / 16) + 2 * k, db = lo_w + (pw * SLOT_BYTES + PART_BYTES) / 16 + 2 * k;
+              if (decltype(fresh)::value && k == k0) umma_pair_lo<false>(to, da, db, idesc);
+              else umma_pair_lo<true>(to, da, db, idesc);
+            }
+          };
+          ok = (i < 1 || mbar_wait_cluster(sum_empty0 + 8 * h, (i - 1) & 1)) && arrived(2) && arrived(0);
+          if (ok) {
+            tc_fence_after();
+            products(0, 2, 0, 4, x, yes);
+            products(2, 0, 0, 4, x, no);
+            if (h) umma_commit_pair(empty0 + 8 * (s0 + 2), both);
+            ok = arrived(1);
+          }
+          if (!ok) {
+            atomicExch(status, ST_MMA_TIMEOUT);
+            break;
+          }
           tc_fence_after();
-          products(0, 2, 1);
-          products(2, 0, 0);
-          umma_commit_pair(empty0 + 8 * (s0 + 2), both);
-          ok = arrived(1);
+          products(1, 1, 0, 4, x, no);
+          products(0, 1, 0, 4, x, no);
+          products(1, 0, 0, 4, x, no);
+          if (h) umma_commit_pair(empty0 + 8 * (s0 + 1), both);
+          products(0, 0, 0, 2, x, no);
+          products(0, 0, 2, 4, y, yes);
+          if (h) umma_commit_pair(empty0 + 8 * s0, both);
+          umma_commit_pair(sum_full0 + 8 * h, both);
         }
-        if (!ok) {
-          atomicExch(status, ST_MMA_TIMEOUT);
-          break;
-        }
-        tc_fence_after();
-        products(1, 1, 0);
-        products(0, 1, 0);
-        products(1, 0, 0);
-        umma_commit_pair(empty0 + 8 * (s0 + 1), both);
-        products(0, 0, 0);
-        umma_commit_pair(empty0 + 8 * s0, both);
-        umma_commit_pair(sum_full0 + 8 * b, both);
       }
     }
     __syncwarp();
@@ -237,26 +291,39 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       col_flags[h] = __ballot_sync(0xffffffffu, n < N && flags[M + n] != 0);
     }
     const uint32_t first_empty0 = map_to_cta(sum_empty0, first);
-    const uint32_t mine = tmem + ((uint32_t)row0 << 16) + col0;
-    for (int i = 0; i < nkb; ++i) {
-      const int b = i & 1;
-      if (!mbar_wait(sum_full0 + 8 * b, (i / 2) & 1)) {
-        if (lane == 0) atomicExch(status, ST_ADDER_TIMEOUT);
-        break;
-      }
-      tc_fence_after();
+    const uint32_t from0 = tmem + ((uint32_t)row0 << 16) + COLS / 2 * (warp / 4);
+    uint32_t rest[COLS / 2];                               // what rounding has taken from the sums, two bfloat16 a register
 #pragma unroll
-      for (int h = 0; h < COLS / 32; ++h) {
-        uint32_t v[32];
-        tmem_ld32(mine + b * BN + 32 * h, v);
-        tmem_ld_wait();
+    for (int j = 0; j < COLS / 2; ++j) rest[j] = 0u;
+    bool ok = true;
+    for (int i = 0; i < nkb && ok; ++i)
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sum[32 * h + j] += __uint_as_float(v[j]);
+      for (int h = 0; h < 2; ++h) {
+        if (ok && !mbar_wait(sum_full0 + 8 * h, i & 1)) {
+          if (lane == 0) atomicExch(status, ST_ADDER_TIMEOUT);
+          ok = false;
+        }
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < COLS / 2; c += AT_ONCE) {
+          const uint32_t from = from0 + h * 2 * COLS + c;
+          uint32_t x[AT_ONCE], y[AT_ONCE];
+          tmem_ld16(from, x);
+          tmem_ld16(from + COLS, y);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < AT_ONCE; j += 2) {
+            const int k = h * (COLS / 2) + c + j;
+            const float2 v = add2(make_float2(__uint_as_float(x[j]), __uint_as_float(x[j + 1])), make_float2(__uint_as_float(y[j]), __uint_as_float(y[j + 1])));
+            add_with_rest(sum[k], sum[k + 1], rest[k / 2], v);
+          }
+          if (K < 0) break;                                // never: the pieces one after another, or the compiler mixes them and keeps 240 registers in memory
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(first_empty0 + 8 * h);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(first_empty0 + 8 * b);
-    }
     constexpr int RANGE = BN / SPLIT, OWN = COLS < RANGE ? COLS : RANGE;         // columns of a pair, of them in an adder's reach
     if (SPLIT > 1) {
       cluster_sync_all();                                  // all rings are free
@@ -400,13 +467,13 @@ static int pick_split(int tiles, int blocks, const Clusters &clusters) {
 }
 static int tiles_of(int M, int N) { return ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN); }
 
-// Nanoseconds that both launches are estimated to take: the parts at 6.7 TB/s, a block 2.05 us under the clock that such products leave, and what a
-// launch takes whatever it does (fitted to 32 sizes of 32 to 2,100 rows, K = 1,024 to 3,072).
+// Nanoseconds that both launches are estimated to take: the parts at 6.7 TB/s, a block 3.4 us, and what a launch
+// takes whatever it does (within 0.15 of 28 sizes of 64 to 2,100 rows, K = 1,024 to 3,072).
 extern "C" int g2b_gemm_f32_tc_estimate(int M, int N, int K) {
   Clusters clusters;
   if (count_clusters(clusters)) return 2000000000;
   const int tiles = tiles_of(M, N), blocks = (K + BK - 1) / BK;
-  const double us = 7.0 + 1.5e-6 * ((double)M + N) * K + 2.05 * rounds_of_blocks(pick_split(tiles, blocks, clusters), tiles, blocks, clusters);
+  const double us = 7.0 + 1.5e-6 * ((double)M + N) * K + 3.4 * rounds_of_blocks(pick_split(tiles, blocks, clusters), tiles, blocks, clusters);
   return us < 2e6 ? (int)(1e3 * us) : 2000000000;
 }
 

@@ -357,14 +357,6 @@ __device__ __forceinline__ void epilogue_tile_bulk(uint32_t tmem, unsigned char 
 // four warps, each both heads of a tile, it took 1.4 times as long as the tile's products at K = 1,024 (132 us); with eight, each a head, 118.
 // What is left above the product (92) is the angles: 128 KB a tile beside 512 KB of operands into the SM; without them it takes 108.
 constexpr int HEAD = 128;
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {     // as tmem_ld32, sixteen columns
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
 struct HeadsTail : ProductTail {
   const float *q_w, *k_w;                          // null: no norm
   const float2 *rope;                              // [tokens, 64] (cos, sin); null: no rotation

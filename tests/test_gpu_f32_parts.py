@@ -62,6 +62,26 @@ def test_rows_that_three_parts_do_not_hold():
     assert same(acc, out + 1)
 
 
+KINDS = {"one sign": lambda x: x.abs(), "offset": lambda x: 1 + 0.1 * x, "behind SiLU": lambda x: torch.nn.functional.silu(3 * x), "any sign": lambda x: x}
+
+
+# one block, several, parts of K; tiles enough for whole K (the last two)
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("M,N,K", [(300, 512, 64), (300, 512, 128), (300, 512, 1024), (300, 512, 3072), (300, 256, 17408), (1500, 4096, 256), (1500, 4096, 1024)])
+def test_cuts_of_one_sign(kind, M, N, K):
+    """Cuts toward zero add up where all sums have one sign: no larger an error than the multiply-adds' there either."""
+    from gguf2bin_b200 import kernels
+    a, w = (KINDS[kind](rnd(n, K, seed=s)) for n, s in ((M, 1), (N, 2)))
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    out, plain = product(a, w, torch.full((M, N), math.nan, device=DEV)), torch.empty(M, N, device=DEV)
+    kernels.gemm_simt(a, w, plain)
+    err = out.double() - ref
+    assert err.norm() <= (plain.double() - ref).norm()
+    # a cut takes half a unit in the last place of the sum it falls on, 0.72 * 2^-24 of it in the mean: two on a half of a block's sum and two on
+    # a quarter are 1.1 * 2^-24 where every product has bits to lose; a first part of seven bits leaves half of them none
+    assert (err * ref.sign() / size).mean().abs() <= EPS
+
+
 @pytest.mark.parametrize("where", ["a", "w"])
 def test_entries_that_three_parts_do_not_hold(where):
     """A tiny entry beside ordinary ones whose partners are zero, and large ones whose partial products would be infinities of either sign: the
