@@ -477,21 +477,42 @@ struct DecodeCall {
   int planes, q_stride, keep_first, v_heads;
 };
 
+// Shared memory of a launch, and the most that any launch of the kernel asks for: what is allowed once per device, so that threads that meet in
+// their first calls cannot lower it for one another.
+template <bool OWN, bool CLUSTER> static int launch_smem(int rows, int last, int n) {
+  const int a = Received(rows, n).bytes(n, rows), b = Received(last, n).bytes(n, last);
+  return received_at<OWN>() + (CLUSTER ? (a > b ? a : b) : 0);
+}
+template <bool OWN, bool CLUSTER> static int most_smem() {
+  int most = 0;
+  for (int n = 1; n <= (CLUSTER ? CLUSTER_MOST : 1); ++n)
+    for (int rows = 1; rows <= 16; ++rows) {
+      const int need = launch_smem<OWN, CLUSTER>(rows, rows, n);
+      most = need > most ? need : most;
+    }
+  return most;
+}
+template <bool OWN, bool CLUSTER> static int allow() {
+  static G2bPerDevice configured;
+  const int dev = g2b_current_device();
+  if (dev < 0 || !configured.value[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_short_kernel<OWN, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem<OWN, CLUSTER>());
+    if (e == cudaSuccess && CLUSTER)                                          // more than 8 CTAs
+      e = cudaFuncSetAttribute(attn_decode_short_kernel<OWN, CLUSTER>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess)
+      G2B_REFUSE("attn_decode_short: shared memory of %d bytes refused: %s", most_smem<OWN, CLUSTER>(), cudaGetErrorString(e));
+    if (dev >= 0) configured.value[dev] = 1;
+  }
+  return 0;
+}
+
 template <bool OWN, bool CLUSTER>
 static int launch_decode(const DecodeCall &c, cudaStream_t stream) {
   const int group = c.nh / c.nkv, head_tiles = (group + 15) / 16, rows = group < 16 ? group : 16;
   const int n = CLUSTER ? c.n_chunks : 1;
   const int last = (group - 1) % 16 + 1;         // heads of a kv head's last tile
-  const int smem = received_at<OWN>() + (CLUSTER ? max(Received(rows, n).bytes(n, rows), Received(last, n).bytes(n, last)) : 0);
-  static G2bPerDevice configured;
-  const int cfg_dev = g2b_current_device();
-  if (cfg_dev < 0 || configured.value[cfg_dev] < smem) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_short_kernel<OWN, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess && CLUSTER)                                          // more than 8 CTAs
-      e = cudaFuncSetAttribute(attn_decode_short_kernel<OWN, CLUSTER>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) G2B_REFUSE("attn_decode_short: shared memory of %d bytes refused: %s", smem, cudaGetErrorString(e));
-    if (cfg_dev >= 0) configured.value[cfg_dev] = smem;
-  }
+  const int smem = launch_smem<OWN, CLUSTER>(rows, last, n);
+  if (allow<OWN, CLUSTER>()) return 1;
   g2b_launch_cluster(attn_decode_short_kernel<OWN, CLUSTER>, dim3(c.n_chunks, c.nkv * head_tiles, c.T), dim3(THREADS), smem, stream,
                      (unsigned)n, c.q, c.pro, c.cache, c.tok_pos, c.tok_seq, c.page_table, c.P, c.nh, c.nkv, c.window, c.score, c.part_o,
                      c.part_ml, c.out, c.finish, c.n_chunks, c.planes, c.q_stride, c.keep_first, c.v_heads);
@@ -500,6 +521,18 @@ static int launch_decode(const DecodeCall &c, cudaStream_t stream) {
   g2b_launch(attn_combine_kernel, dim3((unsigned)((size_t)c.T * c.nh)), dim3(COMBINE_WARPS * 32), 0, stream,
              c.part_o, (const float2 *)c.part_ml, c.tok_pos, c.nh, c.window, c.n_chunks, c.out, c.finish, c.keep_first);
   return g2b_check_launch("attn_combine");
+}
+
+// What the device allows the form (own: with the prologue; cluster: merged in clusters) behind a launch of it, and the most that it may ask for.
+extern "C" int g2b_attn_decode_short_smem(int own, int cluster, int *allowed, int *most) {
+  const void *kernel = own ? (cluster ? (const void *)attn_decode_short_kernel<true, true> : (const void *)attn_decode_short_kernel<true, false>)
+                           : (cluster ? (const void *)attn_decode_short_kernel<false, true> : (const void *)attn_decode_short_kernel<false, false>);
+  cudaFuncAttributes attr;
+  const cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
+  if (e != cudaSuccess) G2B_REFUSE("attn_decode_short: %s", cudaGetErrorString(e));
+  *allowed = attr.maxDynamicSharedSizeBytes;
+  *most = own ? (cluster ? most_smem<true, true>() : most_smem<true, false>()) : (cluster ? most_smem<false, true>() : most_smem<false, false>());
+  return 0;
 }
 
 static int check_sizes(int T, int nh, int nkv, int hd, int page_size, int max_kv_len, float softcap, int window, int keep_first) {
