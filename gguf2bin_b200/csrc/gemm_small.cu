@@ -554,13 +554,16 @@ gemm_small_stream_kernel(const bf16 *A, const bf16 *__restrict__ W, void *__rest
   cp_async_wait<0>();
 }
 
+// What each whole-A kernel is allowed once per device: not what a call needs, which threads that meet in their first calls could lower for one another.
+constexpr int WHOLE_MOST = 200 * 1024;
+
 // shared memory the whole-A kernel needs, or 0 if the case does not fit
 static size_t whole_smem(int mrows, int K, int split = 1) {
   const int nkb = (K + KB - 1) / KB, per = (nkb + split - 1) / split;
   const size_t stage = ((size_t)mrows * (per * KB + XPAD) * sizeof(bf16) + 127) / 128 * 128;
   const size_t red = ((size_t)(WARPS + split) * 16 * mrows + mrows) * sizeof(float);    // + a factor per row
   const size_t need = stage + red;
-  return need <= 200 * 1024 ? need : 0;
+  return need <= WHOLE_MOST ? need : 0;
 }
 
 // CTAs per 16-row tile: narrow outputs with a long K are split over a cluster
@@ -589,11 +592,11 @@ static int launch_whole_depth(const void *A, const void *W, void *C, int M, int 
   do {                                                                                           \
     static G2bPerDevice configured;                                                              \
     const int cfg_dev = g2b_current_device();                                                    \
-    if (cfg_dev < 0 || configured.value[cfg_dev] < smem) {                                       \
+    if (cfg_dev < 0 || !configured.value[cfg_dev]) {                                             \
       cudaError_t e = cudaFuncSetAttribute(gemm_small_whole_kernel<MT, E, DEPTH_WHOLE, SPLIT>,       \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);   \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, WHOLE_MOST); \
       if (e != cudaSuccess) G2B_REFUSE("gemm_small: shared memory: %s", cudaGetErrorString(e));  \
-      if (cfg_dev >= 0) configured.value[cfg_dev] = smem;                                        \
+      if (cfg_dev >= 0) configured.value[cfg_dev] = 1;                                           \
     }                                                                                            \
     g2b_launch_cluster(gemm_small_whole_kernel<MT, E, DEPTH_WHOLE, SPLIT>, dim3(grid),           \
                        dim3(WARPS * 32), smem, stream, (unsigned)SPLIT, (const void *)A,         \
@@ -666,11 +669,11 @@ static int launch_normed(const float *X, const void *W, void *C, int M, int N, i
   do {                                                                                           \
     static G2bPerDevice configured;                                                              \
     const int cfg_dev = g2b_current_device();                                                    \
-    if (cfg_dev < 0 || configured.value[cfg_dev] < smem) {                                       \
+    if (cfg_dev < 0 || !configured.value[cfg_dev]) {                                             \
       cudaError_t e = cudaFuncSetAttribute(gemm_small_whole_kernel<MT, E, DEPTH_WHOLE, 1, true>, \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);   \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, WHOLE_MOST); \
       if (e != cudaSuccess) G2B_REFUSE("gemm_small: shared memory: %s", cudaGetErrorString(e));  \
-      if (cfg_dev >= 0) configured.value[cfg_dev] = smem;                                        \
+      if (cfg_dev >= 0) configured.value[cfg_dev] = 1;                                           \
     }                                                                                            \
     g2b_launch(gemm_small_whole_kernel<MT, E, DEPTH_WHOLE, 1, true>, dim3(grid), dim3(WARPS * 32), smem, \
                stream, (const void *)X, (const bf16 *)W, C, M, N, K, ldx, ldw, ldc, eps, glu);   \
@@ -728,6 +731,19 @@ static int launch_stream(const void *A, const void *W, void *C, int M, int N, in
              (const bf16 *)W, C, M, N, K, lda, ldw, ldc, epi, n_chunks, kbc, per, glu);
   return g2b_check_launch("gemm_small_stream");
 }
+
+#if !defined(G2B_GLU) && !defined(G2B_ACT)
+// What the device allows the whole-A kernel of up to eight rows and four blocks of K a CTA that stores floats (split: over a cluster of four) behind
+// its launches, and the most that one asks for.
+extern "C" int g2b_gemm_small_smem(int split, int *allowed, int *most) {
+  cudaFuncAttributes attr;
+  const cudaError_t e = cudaFuncGetAttributes(&attr, split ? (const void *)gemm_small_whole_kernel<1, EPI_STORE_F32, 4, 4>
+                                                           : (const void *)gemm_small_whole_kernel<1, EPI_STORE_F32, 4, 1>);
+  if (e != cudaSuccess) G2B_REFUSE("gemm_small: %s", cudaGetErrorString(e));
+  *allowed = attr.maxDynamicSharedSizeBytes, *most = WHOLE_MOST;
+  return 0;
+}
+#endif
 
 // A [M,K] and W [N,K] bfloat16 with unit inner stride; rows 16-byte aligned.
 // epi: 0 store bfloat16, 1 store float, 2 add into float, 3 gate (C is [M, N/2] bfloat16; N must be a

@@ -1,7 +1,6 @@
 """Decode attention with the token's norm, rotation and cache write in front of it, and the merge of its chunks inside a cluster:
 the bits of the kernels that do these one after another."""
 import math
-import os
 from types import SimpleNamespace
 
 import pytest
@@ -58,33 +57,3 @@ def test_prologue_and_cluster_give_the_bits_of_the_steps_one_by_one(width, nh, n
     assert torch.equal(out, outs[0]) and torch.equal(out, outs[1])
     # another split of the same sums: probabilities and the result are rounded to 8 bits, each against its segment's maximum
     assert (out.float() - outs[2].float()).abs().max() <= 2.0 ** -6 * cache.float().abs().max()
-
-
-@pytest.mark.parametrize("own", [False, True])
-@pytest.mark.parametrize("cluster", [False, True])
-def test_the_first_launch_allows_the_largest(own, cluster):
-    """The shared memory that the device allows the kernel does not depend on which shapes came in which order: two threads in their first calls
-    could leave the smaller of theirs.  (In a process of its own: attributes stay.)"""
-    import subprocess
-    import sys
-    code = f"""
-import torch, ctypes
-from types import SimpleNamespace
-from test_gpu_decode_attention import ctx_of
-from test_gpu_kernels import DEV, make_paged, rnd
-from gguf2bin_b200 import kernels, kernels_bf16
-from gguf2bin_b200.csrc.build import load_unit
-cache, table, _, _ = make_paged(1, [5], 1, 128, 64, torch.bfloat16, seed=40)
-ctx = ctx_of([5], table, {1 if cluster else 40})
-out = torch.empty(1, 128, dtype=torch.bfloat16, device=DEV)
-if {own}:
-    assert kernels_bf16.attn_decode_qkv(rnd(1, 384, dtype=torch.bfloat16, seed=1), None, None, 1e-6, None, 0, out, cache, ctx, 1, 1, 128, 64, 0, 0.1, fine=True)
-else:
-    kernels_bf16.attn_decode(rnd(1, 128, dtype=torch.bfloat16, seed=1), out, cache, ctx, 1, 1, 128, 64, 0, 0.1, pages=2)
-torch.cuda.synchronize()
-allowed, most = ctypes.c_int(), ctypes.c_int()
-assert load_unit("attn_decode_short.cu", ("HD=128",)).g2b_attn_decode_short_smem({int(own)}, {int(cluster)}, ctypes.byref(allowed), ctypes.byref(most)) == 0
-assert allowed.value >= most.value > 0, (allowed.value, most.value)
-"""
-    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env={**os.environ, "PYTHONPATH": os.pathsep.join(sys.path)})
-    assert done.returncode == 0, done.stderr[-2000:]
