@@ -456,7 +456,7 @@ attn_decode_short_kernel(const bf16 *__restrict__ q, Prologue pro, bf16 *cache,
         [&](int of) { return *reinterpret_cast<const float *>(received + rx.out(of, 0) + (e - e0) * 4); }, finish, t, head0 + e / HD));
 }
 
-// Scratch, used where a token has more than CLUSTER_MOST chunks: part_o float [T*nh*n_chunks*HD], part_ml float2 [T*nh*n_chunks], with
+// Scratch; without it (null) the chunks of a token, CLUSTER_MOST at most, are merged in a cluster: part_o float [T*nh*n_chunks*HD], part_ml float2 [T*nh*n_chunks], with
 // n_chunks = ceil(max_kv_len / 128).  q, out [T, nh*HD] bfloat16.
 // With programmatic dependent launch on (g2b_set_pdl(1)) the kernel reads tok_pos once above
 // the dependency line, as a hint for which old keys it may fetch early.  A caller whose own
@@ -548,8 +548,35 @@ static int check_sizes(int T, int nh, int nkv, int hd, int page_size, int max_kv
   return 0;
 }
 static int chunks_of(int max_kv_len) { return (max_kv_len + CHUNK_KEYS - 1) / CHUNK_KEYS; }
+static int check_form(const DecodeCall &c) {
+  if (!c.part_o && c.n_chunks > CLUSTER_MOST) G2B_REFUSE("attn_decode_short: %d chunks are more than a cluster (%d) and there is no scratch", c.n_chunks, CLUSTER_MOST);
+  if (c.part_o && !c.part_ml) G2B_REFUSE("attn_decode_short: no scratch for the statistics");
+  return 0;
+}
 
-// Arguments as g2b_attn_decode_ex (attn_decode.cu); the scratch may be null where clusters merge.
+// How many clusters of n_chunks CTAs the device holds at once; 0 where it holds none (own: with the prologue).
+template <bool OWN> static int count_clusters(int n) {
+  if (n > CLUSTER_MOST || allow<OWN, true>()) return 0;
+  int smem = 0, clusters = 0;
+  for (int rows = 1; rows <= 16; ++rows) smem = max(smem, launch_smem<OWN, true>(rows, rows, n));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = n, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr, cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&clusters, attn_decode_short_kernel<OWN, true>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters;
+}
+extern "C" int g2b_attn_decode_short_clusters(int own, int max_kv_len) {
+  const int n = max_kv_len > 0 ? chunks_of(max_kv_len) : 0;
+  return n <= 0 ? 0 : own ? count_clusters<true>(n) : count_clusters<false>(n);
+}
+
+// Arguments as g2b_attn_decode_ex (attn_decode.cu); scratch null: clusters merge.
 extern "C" int g2b_attn_decode_short(const void *q, void *out, const void *cache, const int *tok_pos,
                                   const int *tok_seq, const int *page_table, int P, int T, int nh,
                                   int nkv, int hd, int page_size, int window, float scale,
@@ -566,7 +593,8 @@ extern "C" int g2b_attn_decode_short(const void *q, void *out, const void *cache
                            nh, nkv, window, ScoreMap{scale * LOG2E, softcap > 0.f ? scale / softcap : 0.f, softcap * LOG2E},
                            chunks_of(max_kv_len), part_o, (float2 *)part_ml,
                            Finish{sink, (const bf16 *)gate, gate_stride}, planes, q_stride, keep_first, v_heads};
-  return call.n_chunks <= CLUSTER_MOST ? launch_decode<false, true>(call, stream) : launch_decode<false, false>(call, stream);
+  if (check_form(call)) return 1;
+  return call.part_o ? launch_decode<false, false>(call, stream) : launch_decode<false, true>(call, stream);
 }
 
 // The same from the projection of the step's tokens, qkv [T, (nh + 2 nkv) * HD] = [q heads | k heads | v heads] as g2b_qknorm_rope_cache
@@ -586,5 +614,6 @@ extern "C" int g2b_attn_decode_short_qkv(const void *qkv, const float *q_w, cons
                            ScoreMap{scale * LOG2E, softcap > 0.f ? scale / softcap : 0.f, softcap * LOG2E},
                            chunks_of(max_kv_len), part_o, (float2 *)part_ml, Finish{sink, nullptr, 0}, 2, 0, keep_first,
                            nkv};
-  return call.n_chunks <= CLUSTER_MOST ? launch_decode<true, true>(call, stream) : launch_decode<true, false>(call, stream);
+  if (check_form(call)) return 1;
+  return call.part_o ? launch_decode<true, false>(call, stream) : launch_decode<true, true>(call, stream);
 }

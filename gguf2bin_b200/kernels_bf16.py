@@ -534,6 +534,7 @@ def decode_chunk_pages(units: int, pages: int, head_dim: int, slots: int) -> int
 
 
 DECODE_CLUSTER_MOST = 16      # chunks of 128 keys that attn_decode_short.cu merges inside a thread-block cluster
+_clusters: dict = {}          # (device, head size, prologue, chunks) -> such clusters that the device holds at once
 
 
 def _decode_pages(ctx, T, n_heads, n_kv_heads, head_dim, fine) -> int:
@@ -545,10 +546,20 @@ def _decode_pages(ctx, T, n_heads, n_kv_heads, head_dim, fine) -> int:
     return decode_chunk_pages(T * tiles, -(-max(int(keys), 1) // 64), head_dim, DECODE_CTAS_PER_SM * _sm_count(ctx.tok_pos.device))
 
 
-def _decode_scratch(ctx, T, n_heads, head_dim, pages):
+def _clusters_at_once(device, head_dim: int, own: bool, n_chunks: int) -> int:
+    """Clusters of that many CTAs (own: with the prologue) that the device holds at once; 0: none, and the chunks go through scratch."""
+    key = (device.index, head_dim, own, n_chunks)
+    n = _clusters.get(key)
+    if n is None:
+        n = _clusters[key] = _fn("attn_decode_short.cu", "g2b_attn_decode_short_clusters", [c_int, c_int],
+                                 defines=(f"HD={head_dim}",))(int(own), 128 * n_chunks)
+    return n
+
+
+def _decode_scratch(ctx, T, n_heads, head_dim, pages, own=False):
     """Scratch for the chunks' partial outputs and their statistics; none where clusters merge them."""
     n_chunks = -(-max(int(ctx.max_kv_len), 1) // (64 * pages))
-    if pages == 2 and n_chunks <= DECODE_CLUSTER_MOST:
+    if pages == 2 and n_chunks <= DECODE_CLUSTER_MOST and _clusters_at_once(ctx.tok_pos.device, head_dim, own, n_chunks):
         return None, None
     kernels.count_launches(1)                      # the merge of the chunks
     ws = ctx.workspace
@@ -594,7 +605,7 @@ def attn_decode_qkv(qkv, q_w, k_w, eps, rope, rotary_dim, out, cache_pages, ctx,
         return False
     if _decode_pages(ctx, qkv.shape[0], n_heads, n_kv_heads, head_dim, fine) != 2:
         return False
-    part_o, part_ml = _decode_scratch(ctx, qkv.shape[0], n_heads, head_dim, 2)
+    part_o, part_ml = _decode_scratch(ctx, qkv.shape[0], n_heads, head_dim, 2, own=True)
     f = _fn("attn_decode_short.cu", "g2b_attn_decode_short_qkv",
             [c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
              c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p], defines=(f"HD={head_dim}",))

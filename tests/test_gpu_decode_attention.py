@@ -57,3 +57,39 @@ def test_prologue_and_cluster_give_the_bits_of_the_steps_one_by_one(width, nh, n
     assert torch.equal(out, outs[0]) and torch.equal(out, outs[1])
     # another split of the same sums: probabilities and the result are rounded to 8 bits, each against its segment's maximum
     assert (out.float() - outs[2].float()).abs().max() <= 2.0 ** -6 * cache.float().abs().max()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_a_device_without_room_for_a_cluster_merges_in_scratch(hd, monkeypatch):
+    from gguf2bin_b200 import kernels_bf16
+    lens, nh, nkv = [1, 129, 700], 4, 2
+    cache, table, _, _ = make_paged(len(lens), lens, nkv, hd, 64, torch.bfloat16, seed=40)
+    qkv = rnd(len(lens), (nh + 2 * nkv) * hd, dtype=torch.bfloat16, seed=41)
+    device = torch.device("cuda", 0)
+    assert kernels_bf16._clusters_at_once(device, hd, True, 1) > kernels_bf16._clusters_at_once(device, hd, True, 16) > 0
+    assert kernels_bf16._clusters_at_once(device, hd, False, 17) == 0
+    outs = []
+    for room in (None, 0):
+        if room is not None:
+            monkeypatch.setattr(kernels_bf16, "_clusters_at_once", lambda *a: room)
+        ctx, pages = ctx_of(lens, table, 16), cache.clone()
+        outs.append(torch.full((len(lens), nh * hd), math.nan, dtype=torch.bfloat16, device=DEV))
+        assert kernels_bf16.attn_decode_qkv(qkv, None, None, 1e-6, None, 0, outs[-1], pages, ctx, nh, nkv, hd, 64, 0, hd ** -0.5, fine=True)
+        assert (ctx.workspace.bytes() > 0) == (room == 0)
+        outs.append(torch.full((len(lens), nh * hd), math.nan, dtype=torch.bfloat16, device=DEV))
+        kernels_bf16.attn_decode(qkv[:, :nh * hd].contiguous(), outs[-1], pages, ctx, nh, nkv, hd, 64, 0, hd ** -0.5, pages=2)
+    assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[3]) and torch.equal(outs[0], outs[1])
+
+
+def test_the_launcher_refuses_what_has_no_place_to_merge():
+    from gguf2bin_b200 import kernels, kernels_bf16
+    lens = [5]
+    cache, table, _, _ = make_paged(1, lens, 1, 128, 64, torch.bfloat16, seed=40)
+    q, out = rnd(1, 128, dtype=torch.bfloat16, seed=1), torch.empty(1, 128, dtype=torch.bfloat16, device=DEV)
+    real = kernels_bf16._decode_scratch
+    try:
+        kernels_bf16._decode_scratch = lambda *a, **k: (None, None)
+        with pytest.raises(kernels.KernelError, match="17 chunks"):
+            kernels_bf16.attn_decode(q, out, cache, ctx_of(lens, table, 33), 1, 1, 128, 64, 0, 0.1, pages=2)
+    finally:
+        kernels_bf16._decode_scratch = real
