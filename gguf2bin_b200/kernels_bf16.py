@@ -13,7 +13,7 @@ from .kernels import SILU, _GLU_TYPES, KernelError, _call, _fn, _ptr, _stream
 FAST_HEAD_SIZES = (64, 128)          # head sizes the tensor-core attention kernels are written for
 DECODE_CHUNK_KEYS = 256              # keys per CTA of the decode kernel (attn_decode.cu)
 
-units.SPECIALISED_SOURCES[:] = [("attn_decode.cu", ()), ("attn_decode_short.cu", ()),
+units.SPECIALISED_SOURCES[:] = [("attn_decode.cu", ()), ("attn_decode.cu", ("ATTN_DECODE_PAGES=2",)), ("attn_decode_short.cu", ()),
                                 ("attn_decode.cu", ("ATTN_DECODE_PAGES=6",)), ("attn_decode.cu", ("ATTN_DECODE_PAGES=8",)),
                                 ("attn_decode_noalloc.cu", ()),
                                 ("attn_prefill.cu", ()), ("attn_prefill_tc.cu", ()),
@@ -537,15 +537,6 @@ DECODE_CLUSTER_MOST = 16      # chunks of 128 keys that attn_decode_short.cu mer
 _clusters: dict = {}          # (device, head size, prologue, chunks) -> such clusters that the device holds at once
 
 
-def _decode_pages(ctx, T, n_heads, n_kv_heads, head_dim, fine) -> int:
-    """Pages of 64 keys that a CTA takes."""
-    if fine is not None:
-        return 2 if fine else 4
-    tiles = n_kv_heads * -(-(n_heads // n_kv_heads) // 16)
-    keys = getattr(ctx, "kv_len_hint", 0) or ctx.max_kv_len       # max_kv_len may be the reserved length
-    return decode_chunk_pages(T * tiles, -(-max(int(keys), 1) // 64), head_dim, DECODE_CTAS_PER_SM * _sm_count(ctx.tok_pos.device))
-
-
 def _clusters_at_once(device, head_dim: int, own: bool, n_chunks: int) -> int:
     """Clusters of that many CTAs (own: with the prologue) that the device holds at once; 0: none, and the chunks go through scratch."""
     key = (device.index, head_dim, own, n_chunks)
@@ -556,11 +547,43 @@ def _clusters_at_once(device, head_dim: int, own: bool, n_chunks: int) -> int:
     return n
 
 
-def _decode_scratch(ctx, T, n_heads, head_dim, pages, own=False):
+def decode_plan(ctx, kind) -> tuple:
+    """(pages of 64 keys a CTA takes, the short kernel takes them, its chunks are merged in clusters) for the attention of a step of single tokens;
+    ``kind``: (kv heads x head tiles, head size, the token's norm, rotation and cache write come with it).  Chunks of two pages are the
+    short kernel's while its CTAs wait for nothing but their keys:
+    * clusters, where the device holds all of them at once (8 sequences of 492 keys, 512 reserved: 6.5 us, in three launches 9.3; of 640 keys, 2,048
+      reserved, 128 clusters of 16 where 14 fit at a time: 29.3 and 11.5);
+    * else partial outputs in scratch while the CTAs with keys run at once, two an SM, and those of the reserved length make four at most, since
+      each has to start to see that it has nothing to do (two sequences of 640 keys, 2,048 reserved: 6.2 and 8.7 us; of 40 keys, 8,192
+      reserved: 9.2 and 9.2; 64 of 640 and 128 of 40 keys with 4,096: 17 and 14, 22 and 14);
+    * else ``attn_decode.cu``, whose CTAs of 64 threads come and go more cheaply."""
+    tiles, head_dim, own = kind
+    units, device = ctx.tok_pos.shape[0] * tiles, ctx.tok_pos.device
+    keys = max(int(getattr(ctx, "kv_len_hint", 0) or ctx.max_kv_len), 1)       # max_kv_len may be the reserved length
+    sms = _sm_count(device)
+    pages = decode_chunk_pages(units, -(-keys // 64), head_dim, DECODE_CTAS_PER_SM * sms)
+    if pages != 2:
+        return pages, False, False
+    n_chunks = -(-max(int(ctx.max_kv_len), 1) // 128)
+    if n_chunks <= DECODE_CLUSTER_MOST and units <= _clusters_at_once(device, head_dim, own, n_chunks):
+        return 2, True, True
+    return 2, units * -(-keys // 128) <= 2 * sms and units * n_chunks <= 4 * sms, False
+
+
+def _asked_plan(ctx, kind, pages) -> tuple:
+    """The plan with ``pages`` asked for by the caller: two are the short kernel's, in clusters wherever they fit."""
+    if pages != 2:
+        return pages, False, False
+    n_chunks = -(-max(int(ctx.max_kv_len), 1) // 128)
+    return 2, True, n_chunks <= DECODE_CLUSTER_MOST and _clusters_at_once(ctx.tok_pos.device, kind[1], kind[2], n_chunks) > 0
+
+
+def _decode_scratch(ctx, T, n_heads, head_dim, plan):
     """Scratch for the chunks' partial outputs and their statistics; none where clusters merge them."""
-    n_chunks = -(-max(int(ctx.max_kv_len), 1) // (64 * pages))
-    if pages == 2 and n_chunks <= DECODE_CLUSTER_MOST and _clusters_at_once(ctx.tok_pos.device, head_dim, own, n_chunks):
+    pages, _, merged = plan
+    if merged:
         return None, None
+    n_chunks = -(-max(int(ctx.max_kv_len), 1) // (64 * pages))
     kernels.count_launches(1)                      # the merge of the chunks
     ws = ctx.workspace
     return (ws.buffer("attn.part_o", (T * n_heads * n_chunks * head_dim,), torch.float32),
@@ -571,14 +594,18 @@ def attn_decode(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_si
                 scale, fine=None, pages=None, sink=None, planes: int = 2, gate=None, softcap: float = 0.0,
                 keep_first: int = 0, v_heads: int = 0) -> None:
     """One token per sequence: split-key attention and a merge of the chunks, in one launch or two.  A CTA takes a chunk of keys of
-    one kv head: 256 as a rule, 128 (``attn_decode_short.cu``), 384 or
-    512 where ``decode_chunk_pages`` says so (``fine`` = 128; ``pages`` = pages of 64 keys per
-    CTA, 2 to 8; default by that rule)."""
+    one kv head: 256 as a rule, 128, 384 or 512 where ``decode_chunk_pages`` says so; which kernel and how its chunks meet is
+    ``decode_plan``'s.  ``fine`` (chunks of 128 keys, or of 256) and ``pages`` (pages of 64 keys a CTA, 2 to 8) ask for one, two
+    pages meaning ``attn_decode_short.cu``."""
     T = q.shape[0]
-    pages = pages or _decode_pages(ctx, T, n_heads, n_kv_heads, head_dim, fine)
-    part_o, part_ml = _decode_scratch(ctx, T, n_heads, head_dim, pages)
-    defines = (f"HD={head_dim}",) if pages in (2, 4) else (f"HD={head_dim}", f"ATTN_DECODE_PAGES={pages}")
-    f = _fn(*(("attn_decode_short.cu", "g2b_attn_decode_short") if pages == 2 else ("attn_decode.cu", "g2b_attn_decode_ex")),
+    if pages is None and fine is not None:
+        pages = 2 if fine else 4
+    kind = (n_kv_heads * -(-(n_heads // n_kv_heads) // 16), head_dim, False)
+    plan = decode_plan(ctx, kind) if pages is None else _asked_plan(ctx, kind, pages)
+    pages, short, _ = plan
+    part_o, part_ml = _decode_scratch(ctx, T, n_heads, head_dim, plan)
+    defines = (f"HD={head_dim}",) if short or pages == 4 else (f"HD={head_dim}", f"ATTN_DECODE_PAGES={pages}")
+    f = _fn(*(("attn_decode_short.cu", "g2b_attn_decode_short") if short else ("attn_decode.cu", "g2b_attn_decode_ex")),
             [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
              c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
              c_int, c_float, c_int, c_int, c_void_p],
@@ -593,7 +620,7 @@ def attn_decode(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_si
 def attn_decode_qkv(qkv, q_w, k_w, eps, rope, rotary_dim, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window,
                     scale, sink=None, chunk: int = 0, softcap: float = 0.0, keep_first: int = 0, fine=None) -> bool:
     """``qknorm_rope_cache`` and the attention of a step of single tokens in one kernel; False: the case is left to the two.  Only where
-    chunks are short (``decode_chunk_pages``): with more to read the attention's copies run ahead while the prologue kernel is busy, and one
+    ``decode_plan`` has the short kernel: with more to read the attention's copies run ahead while the prologue kernel is busy, and one
     launch was slower (``attn_decode_short.cu``)."""
     if not ctx.all_single or head_dim not in FAST_HEAD_SIZES or page_size != 64 or cache_pages.dtype != torch.bfloat16:
         return False
@@ -603,9 +630,11 @@ def attn_decode_qkv(qkv, q_w, k_w, eps, rope, rotary_dim, out, cache_pages, ctx,
         return False
     if any(x is not None and x.data_ptr() % 16 for x in (qkv, out, q_w, k_w, rope, cache_pages)):
         return False
-    if _decode_pages(ctx, qkv.shape[0], n_heads, n_kv_heads, head_dim, fine) != 2:
+    kind = (n_kv_heads * -(-(n_heads // n_kv_heads) // 16), head_dim, True)
+    plan = decode_plan(ctx, kind) if fine is None else _asked_plan(ctx, kind, 2 if fine else 4)
+    if not plan[1]:
         return False
-    part_o, part_ml = _decode_scratch(ctx, qkv.shape[0], n_heads, head_dim, 2, own=True)
+    part_o, part_ml = _decode_scratch(ctx, qkv.shape[0], n_heads, head_dim, plan)
     f = _fn("attn_decode_short.cu", "g2b_attn_decode_short_qkv",
             [c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
              c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p], defines=(f"HD={head_dim}",))

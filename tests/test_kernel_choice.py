@@ -66,3 +66,35 @@ def test_prompts_of_a_thousand_rows_and_a_long_k_go_to_pairs_of_ctas():
     assert _tc_shape(1000, 6144, out, 4096) == (0, 0, True)
     assert _tc_shape(2048, 6144, out, 1024) == (0, 0, True)          # the short K of a small model
     assert _tc_shape(2048, 1024, out, 4096) == (0, 0, True)          # few tiles: the persistent kernel may split K
+
+
+# clusters of n CTAs that a B200 holds at once
+AT_ONCE = {1: 296, 2: 148, 3: 93, 4: 71, 5: 56, 6: 45, 7: 37, 8: 33, 9: 30, 10: 26, 11: 21, 12: 21, 13: 17, 14: 14, 15: 14, 16: 14}
+
+
+@pytest.mark.parametrize("seqs,keys,reserved,want", [
+    # all clusters at once: one sequence whatever it reserves up to 2,048 keys, eight of up to 512, sixteen of up to 256
+    (1, 50, 256, (2, True, True)), (1, 2000, 2048, (2, True, True)), (2, 1000, 1024, (2, True, True)), (8, 492, 512, (2, True, True)),
+    (16, 40, 256, (2, True, True)),
+    # more clusters than fit: scratch while the CTAs with keys run at once and the reserved ones are few
+    (2, 40, 2048, (2, True, False)), (8, 240, 1024, (2, True, False)), (1, 4000, 4096, (2, True, False)), (16, 160, 512, (2, True, False)),
+    # short sequences in a long reservation, or many keys: the kernel of small CTAs
+    (8, 100, 2048, (2, False, False)), (8, 640, 2048, (2, False, False)), (8, 700, 768, (2, False, False)), (16, 40, 2048, (2, False, False)),
+    (24, 160, 1024, (2, False, False)), (4, 1000, 4096, (2, False, False)), (2, 3000, 3072, (2, False, False)),
+    # much to read: longer chunks
+    (8, 1000, 1024, (4, False, False)), (8, 2080, 2304, (6, False, False)),
+])
+def test_which_decode_attention(seqs, keys, reserved, want, monkeypatch):
+    """Eight kv heads of 128: what is reserved counts, what is there counts, not what the first step of a shape found."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from gguf2bin_b200 import kernels_bf16
+    monkeypatch.setattr(kernels_bf16, "_sm_count", lambda device: 148)
+    monkeypatch.setattr(kernels_bf16, "_clusters_at_once", lambda device, head_dim, own, n: AT_ONCE.get(n, 0))
+    ctx = SimpleNamespace(tok_pos=torch.zeros(seqs, dtype=torch.int32), max_kv_len=reserved, kv_len_hint=keys)
+    assert kernels_bf16.decode_plan(ctx, (8, 128, True)) == want
+    # a device that holds no cluster: as if every reservation were too long for one
+    monkeypatch.setattr(kernels_bf16, "_clusters_at_once", lambda *a: 0)
+    assert not kernels_bf16.decode_plan(ctx, (8, 128, True))[2]
