@@ -8,9 +8,10 @@ positions advance on the device.  It runs the same model, cache, kernels and sam
 
 The launches of one such step (the model's forward pass, sampling, the advance) depend on
 the step's shape only: how many sequences, how wide their page table, how it samples.
-Which sequences, pages, positions and tokens is data on the device.  So the device buffers
-of a shape and the CUDA graph captured over them belong to the engine, as a
-``DecodeRunner`` kept by shape: a new session of a shape that was seen before (another
+Which sequences, pages, positions and tokens is data on the device; only which kernels the
+attention runs also goes by how long the sequences are, which changes a few times while they
+grow.  So the device buffers of a shape and the CUDA graphs captured over them (one for each
+choice of kernels) belong to the engine, as a ``DecodeRunner`` kept by shape: a new session of a shape that was seen before (another
 call, or the batch that is left when a sequence ends and an earlier batch had that size)
 writes its sequences' data into the runner's buffers and replays the graph that is there.
 A graph is captured only once a shape has run plainly a few times, and a batch of more than
@@ -37,6 +38,7 @@ so a model with such a layer never runs ahead.
 from __future__ import annotations
 
 import weakref
+from collections import OrderedDict
 from typing import Optional, Sequence
 
 import numpy as np
@@ -60,9 +62,10 @@ def padded_rows(n_seqs: int) -> int:
 
 
 class DecodeRunner:
-    """Device buffers and, in time, the captured graph of decode steps of one shape."""
+    """Device buffers and, in time, the captured graphs of decode steps of one shape."""
 
     EAGER_STEPS = 4          # plain steps of a shape before its graph is captured
+    GRAPHS_KEPT = 4          # choices of attention kernels whose graphs are kept: the latest
 
     def __init__(self, engine: Engine, batch: int, table_width: int, params: Optional[SamplingParams]):
         self.engine, self.batch, self.table_width = engine, batch, table_width
@@ -83,7 +86,7 @@ class DecodeRunner:
             page_table=self.page_table, page_size=engine.cache.page_size,
             workspace=engine.workspace, dtype=engine.model.dtype, q_lens=[1] * B,
             past_lens=[0] * B, slots=[0] * B, max_kv_len=P * engine.cache.page_size,
-            seq_slots=self.slots)
+            seq_slots=self.slots, decode_kinds=engine.decode_kinds)
         # what a session needs to talk to the host, kept here so that a new session of a known
         # shape allocates nothing (pinned memory is slow to get)
         self.pinned_in = torch.empty(B, dtype=torch.int32, pin_memory=True)
@@ -93,9 +96,8 @@ class DecodeRunner:
         self.tokens_uploaded = torch.cuda.Event()
         self._owner = None                      # weak: the session holds the runner, not the other way round
         self.logits: Optional[torch.Tensor] = None
-        self._graph: Optional[torch.cuda.CUDAGraph] = None
-        self._graph_generation = -1
-        self.plain_steps = 0
+        self._graphs: "OrderedDict[tuple, tuple]" = OrderedDict()    # attention's plans -> (graph, generation, launches)
+        self._plain_steps: dict = {}            # attention's plans -> plain steps so far
         self.launches_per_step = 0
 
     def bind(self, session: "DecodeSession", keep_tokens: bool = False) -> None:
@@ -121,8 +123,6 @@ class DecodeRunner:
         self._meta[first:].copy_(self._meta_host[first:], non_blocking=True)
         self._uploaded.record(kernels.current_stream())
         self.ctx.slots = slots
-        # the page table is as wide as what is reserved; kernels that size their work by the keys plan with what is there
-        self.ctx.kv_len_hint = max(s.length for s in session.seqs) + 1
         self._owner = weakref.ref(session)
 
     def owned_by(self, session: "DecodeSession") -> bool:
@@ -142,28 +142,41 @@ class DecodeRunner:
                                     self.tok_ids)
             kernels.advance_positions(self.tok_pos, self.batch)
 
-    def run(self, use_graph: bool, eager_steps: int) -> None:
-        ws = self.engine.workspace
-        if self._graph is not None and ws.generation != self._graph_generation:
-            self._graph, self.plain_steps = None, 0           # scratch buffers moved: capture again
-        if self._graph is not None and use_graph:
-            self._graph.replay()
+    def run(self, use_graph: bool, eager_steps: int, longest: int) -> None:
+        """One step; ``longest``: the keys of the longest sequence with it.  The page table is as wide as what is reserved; kernels that size
+        their work by the keys plan with these."""
+        ws, eng = self.engine.workspace, self.engine
+        self.ctx.kv_len_hint = longest
+        plan = kernels.decode_plans(self.ctx, eng.decode_kinds)
+        hit = self._graphs.get(plan)
+        if hit is not None and hit[1] != ws.generation:           # scratch buffers moved: capture again
+            del self._graphs[plan]
+            self._plain_steps[plan], hit = 0, None
+        if hit is not None and use_graph:
+            self._graphs.move_to_end(plan)
+            self.launches_per_step = hit[2]
+            hit[0].replay()
             return
         before = kernels.launch_count()
-        if use_graph and self.plain_steps >= eager_steps:
+        if use_graph and self._plain_steps.get(plan, 0) >= eager_steps:
             kernels.current_stream().synchronize()
             generation = ws.generation
             g, _ = capture_graph(self._launch)
             self.launches_per_step = kernels.launch_count() - before
-            self.engine.decode_graph_captures += 1
+            eng.decode_graph_captures += 1
             if ws.generation == generation:
-                self._graph, self._graph_generation = g, generation
+                self._graphs[plan] = (g, generation, self.launches_per_step)
+                while len(self._graphs) > self.GRAPHS_KEPT:
+                    self._graphs.popitem(last=False)
                 g.replay()
                 return
             before = kernels.launch_count()        # a buffer appeared during the capture: run plainly
         self._launch()
         self.launches_per_step = kernels.launch_count() - before
-        self.plain_steps += 1
+        plan = kernels.decode_plans(self.ctx, eng.decode_kinds)     # the first step of a model leaves its kinds
+        if len(self._plain_steps) > 64:
+            self._plain_steps.clear()
+        self._plain_steps[plan] = self._plain_steps.get(plan, 0) + 1
 
 
 def decode_runner(engine: Engine, batch: int, pages: int, params: Optional[SamplingParams]) -> DecodeRunner:
@@ -270,7 +283,7 @@ class DecodeSession:
         for r, s in zip(self.rows, self.seqs):
             past[r] = s.length
         runner.ctx.past_lens = past
-        runner.run(self.use_graph, self.eager_steps)
+        runner.run(self.use_graph, self.eager_steps, max(past) + 1)
         if not self._sample_in_graph:
             self.sampler.sample(runner.logits, self.params, runner.slots, runner.tok_ids)
             kernels.advance_positions(runner.tok_pos, runner.batch)

@@ -139,6 +139,7 @@ class Engine:
         self._seen: "OrderedDict[tuple, int]" = OrderedDict()        # shapes run plainly so far
         self.decode_runners: "OrderedDict[tuple, object]" = OrderedDict()
         self._padding = _PaddingSequence(self.cache)
+        self.decode_kinds: set = set()     # kinds of decode attention of its steps of single tokens, likewise
         self.scan_kinds: set = set()       # kinds of state scans the model runs in prompt steps, as the first of them leaves them here
         self.last_slots: Optional[torch.Tensor] = None     # the slots of the last step's sequences, on the device until the next
         self.step_graph_captures = 0       # CUDA graphs captured so far: of prompt-step shapes,
@@ -252,7 +253,8 @@ class Engine:
             seq_meta=dev[o_meta:o_meta + 4 * B].view(B, 4), seq_slots=dev[o_slots:o_slots + B],
             attn_tiles=dev[:4 * n_narrow].view(n_narrow, 4), n_attn_tiles=n_narrow,
             attn_tiles_wide=dev[4 * n_narrow:4 * n_tiles].view(n_tiles - n_narrow, 4),
-            n_attn_tiles_wide=n_tiles - n_narrow, padded=entries[-1].seq is self._padding, scan_kinds=self.scan_kinds)
+            n_attn_tiles_wide=n_tiles - n_narrow, padded=entries[-1].seq is self._padding, scan_kinds=self.scan_kinds,
+            decode_kinds=self.decode_kinds)
         return ctx, dev[o_want:o_want + n_want], n_want
 
     def step(self, entries: Seq[StepEntry]) -> Optional[torch.Tensor]:
@@ -294,8 +296,8 @@ class Engine:
         single = ctx.all_single
         if single:
             # One token per sequence: the kernels take every position from device memory, so one
-            # graph serves the shape for as long as the page table keeps its width; the attention
-            # is laid out for all the keys the table covers and plans with those there are.
+            # graph serves the shape for as long as the page table keeps its width and the attention its plan: it
+            # is laid out for all the keys the table covers and chooses its kernels by those there are.
             ctx.kv_len_hint = ctx.max_kv_len
             ctx.max_kv_len = ctx.page_table.shape[1] * self.cache.page_size
         if not self.step_graphs or (ctx.n_tokens < self.GRAPH_MIN_TOKENS and not single):
@@ -303,7 +305,7 @@ class Engine:
         # everything a launch argument or a buffer address is derived from
         if single:
             key = ("single", ctx.n_seqs, tuple(len(e.want) for e in entries), ctx.page_table.shape[1],
-                   self._meta_dev.data_ptr())
+                   self._meta_dev.data_ptr(), kernels.decode_plans(ctx, self.decode_kinds))
         else:
             # which tokens, positions, pages, tiles and places is data on the device; the launches see
             # only how many there are (the same numbers fix where each table lies in the step's metadata),

@@ -872,6 +872,12 @@ def attention(q, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size
                  softcap=softcap, keep_first=keep_first, v_heads=v_heads)
 
 
+def decode_plans(ctx, kinds) -> tuple:
+    """Which kernels the attention of a step of single tokens runs for these kinds (``kernels_bf16.decode_plan``): by what is reserved and by what
+    is there, so a graph of such a step holds for one choice."""
+    return tuple((kind, (_bf16 or _bf16_mod()).decode_plan(ctx, kind)) for kind in sorted(kinds))
+
+
 def attention_qkv(qkv, q_w, k_w, eps, rope, rotary_dim, out, cache_pages, ctx, n_heads, n_kv_heads, head_dim, page_size, window,
                   scale, sink=None, chunk: int = 0, softcap: float = 0.0, keep_first: int = 0) -> bool:
     """``qknorm_rope_cache`` of the projection ``qkv`` and the attention behind it in one kernel, for steps of one token per

@@ -558,6 +558,8 @@ def decode_plan(ctx, kind) -> tuple:
       reserved: 9.2 and 9.2; 64 of 640 and 128 of 40 keys with 4,096: 17 and 14, 22 and 14);
     * else ``attn_decode.cu``, whose CTAs of 64 threads come and go more cheaply."""
     tiles, head_dim, own = kind
+    if getattr(ctx, "decode_kinds", None) is not None:
+        ctx.decode_kinds.add(kind)
     units, device = ctx.tok_pos.shape[0] * tiles, ctx.tok_pos.device
     keys = max(int(getattr(ctx, "kv_len_hint", 0) or ctx.max_kv_len), 1)       # max_kv_len may be the reserved length
     sms = _sm_count(device)

@@ -62,6 +62,7 @@ class StepContext:
     padded: bool = False                             # the last sequence is padding (its tokens fill the step up; nothing reads its results)
     scan_kinds: Optional[set] = None                 # kinds of state scans that steps have run, the engine's set
     scan_plans: dict = field(default_factory=dict)   # kernels.scan_plan of each kind in this step
+    decode_kinds: Optional[set] = None               # kinds of attention that steps of single tokens have run, the engine's set
     step_cache: dict = field(default_factory=dict)   # tensors derived once per step (cleared by the model)
     next_block: Optional[object] = None              # the block that runs after the one running now (None: the last)
     next_add: Optional[torch.Tensor] = None          # what is added to the stream before the next block; a block that
