@@ -638,19 +638,23 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: b
           w.stride(0), out.stride(0), epi, _stream())
 
 
-F32_PARTS_ROWS = 8192            # rows of a float32 matrix that are split at a time, fewer where a row is long: at most
-F32_PARTS_MOST_W = 128 << 20     # bytes of its parts (6 an entry), but 1,024 rows
+F32_PARTS_ROWS = 8192            # rows of a float32 matrix that are split at a time; of it and of the step's rows fewer where a row is long: at most
+F32_PARTS_MOST = 128 << 20       # bytes of parts (6 an entry) each, but 1,024 rows
 _f32_estimates: dict = {}        # (rows, rows of the matrix, K) -> whether the tensor cores are the quicker way
 
 
+def _f32_rows(K: int) -> int:
+    return max(1024, F32_PARTS_MOST // (6 * (-(-K // 8) * 8)) // 256 * 256)
+
+
 def _f32_slice(N: int, K: int) -> int:
-    return min(N, F32_PARTS_ROWS, max(1024, F32_PARTS_MOST_W // (6 * (-(-K // 8) * 8)) // 256 * 256))
+    return min(N, F32_PARTS_ROWS, _f32_rows(K))
 
 
 def _f32_tc_wins(M: int, N: int, K: int) -> bool:
     """More than 32 rows, and the estimate of the kernel on parts (csrc/gemm_f32_tc.cu) below nine tenths of the best of the kernels of
     multiply-adds (csrc/gemm_simt.cu).  Rows count in steps of 64, so that padding decides nothing."""
-    M = -(-M // 64) * 64
+    M = min(-(-M // 64) * 64, _f32_rows(K))
     wins = _f32_estimates.get((M, N, K))
     if wins is None:
         us = [_fn(unit, name, [c_int] * 3)(M, _f32_slice(N, K), K) for unit, name in (
@@ -664,25 +668,26 @@ def _f32_tc_wins(M: int, N: int, K: int) -> bool:
 def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool, workspace, defines=()) -> bool:
     """out (=|+=) a @ w.T in float32 by products of bfloat16 parts on the tensor cores, with the error of 32-bit sums
     (csrc/gemm_f32_tc.cu); False where the alignment is not its own or the device has no memory for the parts.  The matrix goes in
-    slices of rows (``_f32_slice``), which bound the scratch."""
+    slices of rows (``_f32_slice``), and so do the rows of ``a``, which bounds the scratch."""
     M, K = a.shape
     N = w.shape[0]
     if K % 4 or a.stride(0) % 4 or w.stride(0) % 4 or a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1 or \
             a.data_ptr() % 16 or w.data_ptr() % 16:
         return False
-    ld, rows = -(-K // 8) * 8, _f32_slice(N, K)
-    try:
-        parts = workspace.buffer("f32.parts", (3 * (M + rows) * ld,), torch.bfloat16, most=6 * (M + rows) * ld)
+    ld, rows, some = -(-K // 8) * 8, _f32_slice(N, K), min(M, _f32_rows(K))
+    try:                                           # the parts, and behind them a flag for each of their rows
+        scratch = workspace.buffer("f32.parts", ((some + rows) * (3 * ld + 2),), torch.bfloat16, most=2 * F32_PARTS_MOST)
     except torch.OutOfMemoryError:
         return False
-    flags = workspace.buffer("f32.flags", (M + rows,), torch.int32)
     status = (_bf16 or _bf16_mod())._status_word(a.device)
     workspace.waits = True
     f = _fn("gemm_f32_tc.cu", "g2b_gemm_f32_tc", [c_void_p] * 3 + [c_int] * 7 + [c_void_p] * 4, defines=tuple(defines))
-    for n in range(0, N, rows):
-        _call(f, _ptr(a), _ptr(w[n:n + rows]), _ptr(out[:, n:n + rows]), M, min(rows, N - n), K, a.stride(0), w.stride(0), out.stride(0),
-              1 if accumulate else 0, _ptr(parts), _ptr(flags), _ptr(status), _stream())
-        count_launches(1)                      # the parts, then the product
+    for m in range(0, M, some):
+        for n in range(0, N, rows):
+            _call(f, _ptr(a[m:m + some]), _ptr(w[n:n + rows]), _ptr(out[m:m + some, n:n + rows]), min(some, M - m), min(rows, N - n), K,
+                  a.stride(0), w.stride(0), out.stride(0), 1 if accumulate else 0, _ptr(scratch), _ptr(scratch[(some + rows) * 3 * ld:]),
+                  _ptr(status), _stream())
+            count_launches(1)                      # the parts, then the product
     return True
 
 

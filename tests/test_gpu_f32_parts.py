@@ -121,6 +121,30 @@ def test_slices_of_the_matrix(monkeypatch):
     assert ((parts.double() - whole).abs() <= 2 * (66 + 16) * EPS * size).all()
 
 
+def test_slices_of_the_rows(monkeypatch):
+    """More rows than are split at a time: scratch for a slice, the same sums."""
+    from gguf2bin_b200 import kernels
+    from gguf2bin_b200.engine.workspace import Workspace
+    a, w = rnd(700, 1024, seed=1), rnd(1000, 1024, seed=2)
+    whole = product(a, w, torch.empty(700, 1000, device=DEV))
+    monkeypatch.setattr(kernels, "_f32_rows", lambda K: 256)
+    ws, base = Workspace(DEV), rnd(700, 1000, seed=3)
+    parts = base.clone()
+    assert kernels.gemm_f32_tc(a, w, parts, True, ws) and ws.bytes() == 2 * 256 * (3 * 1024 + 2) * 2
+    size = a.double().abs() @ w.double().abs().T
+    assert ((parts.double() - base.double() - whole).abs() <= 2 * (66 + 16) * EPS * size + EPS * parts.double().abs()).all()
+
+
+def test_scratch_grows_with_room_to_spare():
+    """A buffer that moves makes every captured graph of an engine stale: prompts a little longer each time move it once, not each time."""
+    from gguf2bin_b200 import kernels
+    from gguf2bin_b200.engine.workspace import Workspace
+    ws, w = Workspace(DEV), rnd(256, 128, seed=2)
+    for M in range(256, 1024, 64):
+        assert kernels.gemm_f32_tc(rnd(M, 128, seed=1), w, torch.empty(M, 256, device=DEV), False, ws)
+    assert ws.generation <= 3                     # the first, twice that, four times that
+
+
 def test_route():
     """Which kernel: by rows in steps of 64, so that a step filled up with padding keeps it; few rows, or no workspace, never."""
     from gguf2bin_b200 import kernels
