@@ -28,7 +28,9 @@
 //
 // Rows with an entry that is not finite, of 2^50 and more (sums of the products of smaller ones stay below 2^127 for any K) or below
 // 2^-103 but not zero (its last bit is under 2^-126, the smallest normal number, so a part would lose bits) are flagged; an output of a flagged
-// row of A or W is summed from the floats themselves in the order of gemm_simt.cu, by the warps that would have written it.
+// row of A or W is summed from the floats themselves in the order of gemm_simt.cu, by the warp that would have written it.  701 rows by 6144 x 1024
+// (90 us; 235 by multiply-adds): 206 with a flagged row, 116 with a column, 277 with every 32nd row, 817 with all (950, 940, 910 and 6,800 by a lane
+// an output).
 //
 // What bounds it: the tensor cores do six products for one.  A block's 24 products of 256 columns would take 3,072 cycles (128 x 256 x 64 a CTA at
 // 8,192 operations a cycle); as 48 of 128 columns A is read from shared memory twice and they take 1.4 times that, and the adders, whose sums with
@@ -389,24 +391,91 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
               const float each[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                if (n + e >= N) break;
-                float x = each[e];
-                if (odd >> e & 1) {
-                  const float *a = A + (size_t)m * lda, *w = W + (size_t)(n + e) * ldw;
-                  x = 0.f;
-                  for (int k0 = 0; k0 < K; k0 += SUM_CHUNK) {
-                    float chunk = 0.f;
-#pragma unroll 4
-                    for (int k = k0; k < min(K, k0 + SUM_CHUNK); ++k) chunk = fmaf(a[k], w[k], chunk);
-                    x += chunk;
-                  }
-                }
-                to[e] = ACCUM ? to[e] + x : x;
+                if (n + e < N && !(odd >> e & 1)) to[e] = ACCUM ? to[e] + each[e] : each[e];
               }
             }
           }
         }
         __syncwarp();
+      }
+      // Outputs of flagged rows and columns, in the order of gemm_simt.cu: a few columns one after another, a lane a row; rows, and many
+      // columns, eight rows at a time, a lane every 32nd column.
+      constexpr int FEW = 8;
+      constexpr int PER_LANE = OWN / 32;
+#pragma unroll 1
+      for (int c0 = 0; c0 < COLS; c0 += OWN) {
+        if ((col0 + c0) / RANGE != part) continue;
+        const float *w[PER_LANE];
+        uint32_t own = 0, found[PER_LANE];                 // the lane's flagged columns, a bit each, and everybody's
+        int count = 0;
+#pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) {
+          const int n = n0 + col0 + c0 + 32 * j + lane;
+          w[j] = W + (size_t)min(n, N - 1) * ldw;
+          found[j] = __ballot_sync(0xffffffffu, n < N && flags[M + n] != 0);
+          own |= (found[j] >> lane & 1) << j;
+          count += __popc(found[j]);
+        }
+        if (count <= FEW) {
+          const float *a = A + (size_t)min(m0 + row0 + lane, M - 1) * lda;
+#pragma unroll
+          for (int j = 0; j < PER_LANE; ++j)
+            for (uint32_t left = found[j]; left; left &= left - 1) {
+              const int n = n0 + col0 + c0 + 32 * j + __ffs(left) - 1;
+              const float *wn = W + (size_t)n * ldw;
+              float total = 0.f;
+              for (int k0 = 0; k0 < K; k0 += SUM_CHUNK) {
+                float chunk = 0.f;
+#pragma unroll 8
+                for (int k = k0; k < min(K, k0 + SUM_CHUNK); k += 4) {
+                  const float4 wk = *reinterpret_cast<const float4 *>(wn + k), ak = *reinterpret_cast<const float4 *>(a + k);
+                  chunk = fmaf(ak.w, wk.w, fmaf(ak.z, wk.z, fmaf(ak.y, wk.y, fmaf(ak.x, wk.x, chunk))));
+                }
+                total += chunk;
+              }
+              if (m0 + row0 + lane < M && !(row_flags >> lane & 1)) {
+                float *to = C + (size_t)(m0 + row0 + lane) * ldc + n;
+                *to = ACCUM ? *to + total : total;
+              }
+            }
+          own = 0;
+        }
+#pragma unroll 1
+        for (int r0 = 0; r0 < 32; r0 += 8) {
+          const int m = m0 + row0 + r0;
+          if (m >= M || !(count > FEW || (row_flags >> r0 & 255))) continue;
+          float total[8][PER_LANE] = {};
+          for (int k0 = 0; k0 < K; k0 += SUM_CHUNK) {
+            float chunk[8][PER_LANE] = {};
+#pragma unroll 4
+            for (int k = k0; k < min(K, k0 + SUM_CHUNK); k += 4) {
+              float4 wk[PER_LANE];
+#pragma unroll
+              for (int j = 0; j < PER_LANE; ++j) wk[j] = *reinterpret_cast<const float4 *>(w[j] + k);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float4 ak = *reinterpret_cast<const float4 *>(A + (size_t)min(m + i, M - 1) * lda + k);
+#pragma unroll
+                for (int j = 0; j < PER_LANE; ++j)
+                  chunk[i][j] = fmaf(ak.w, wk[j].w, fmaf(ak.z, wk[j].z, fmaf(ak.y, wk[j].y, fmaf(ak.x, wk[j].x, chunk[i][j]))));
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+              for (int j = 0; j < PER_LANE; ++j) total[i][j] += chunk[i][j];
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < PER_LANE; ++j) {
+              const int n = n0 + col0 + c0 + 32 * j + lane;
+              if (m + i < M && n < N && ((own >> j | row_flags >> (r0 + i)) & 1)) {
+                float *to = C + (size_t)(m + i) * ldc + n;
+                *to = ACCUM ? *to + total[i][j] : total[i][j];
+              }
+            }
+        }
       }
     }
   }

@@ -111,6 +111,43 @@ def test_small_and_large_products(scale):
     assert ((out.double() - a.double() @ w.double().T).abs() <= (66 + 5) * EPS * size + 6 * 320 * 2.0 ** -150).all()
 
 
+# whole K and parts of it; columns flagged: none, few and many of a warp's 128, the last; rows: one, some of every eight, all
+@pytest.mark.parametrize("M,N,K", [(300, 900, 132), (1500, 4100, 68), (270, 515, 2052)])
+@pytest.mark.parametrize("columns,rows", [(slice(0, 0), slice(7, 8)), (slice(5, None, 130), slice(0, 0)), (slice(1, None, 13), slice(0, 0)),
+                                          (slice(0, None, 60), slice(3, None, 11)), (slice(-1, None), slice(None))])
+def test_flagged_rows_and_columns(M, N, K, columns, rows):
+    from gguf2bin_b200 import kernels
+    a, w = rnd(M, K, seed=1), rnd(N, K, seed=2)
+    clean = product(a, w, torch.empty(M, N, device=DEV))
+    a[rows, K // 2], w[columns, 3] = math.nan, 1e-33
+    out, plain = product(a, w, torch.full((M, N), 5.0, device=DEV)), torch.empty(M, N, device=DEV)
+    kernels.gemm_simt(a, w, plain)
+    flagged = torch.zeros(M, N, dtype=torch.bool, device=DEV)
+    flagged[rows], flagged[:, columns] = True, True
+    assert torch.equal(out[flagged].nan_to_num(nan=7e30), plain[flagged].nan_to_num(nan=7e30)) and torch.equal(out[~flagged], clean[~flagged])
+    acc = product(a, w, torch.ones(M, N, device=DEV), accumulate=True)
+    assert torch.equal(acc.nan_to_num(nan=7e30), (out + 1).nan_to_num(nan=7e30))
+
+
+def test_a_step_that_has_gone_to_nan_ends_in_time():
+    """All rows flagged: four times as long as the multiply-adds (thirty times by a lane an output)."""
+    from gguf2bin_b200 import kernels
+    from gguf2bin_b200.engine.workspace import Workspace
+    a, w, out, ws = torch.full((701, 1024), math.nan, device=DEV), rnd(6144, 1024, seed=2), torch.empty(701, 6144, device=DEV), Workspace(DEV)
+
+    def best(fn):
+        times = []
+        for _ in range(4):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            fn()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times)
+    assert best(lambda: kernels.gemm_f32_tc(a, w, out, False, ws)) < 10 * best(lambda: kernels.gemm_simt(a, w, out)) and out.isnan().all()
+
+
 def test_slices_of_the_matrix(monkeypatch):
     from gguf2bin_b200 import kernels
     a, w = rnd(200, 1024, seed=1), rnd(1000, 1024, seed=2)
