@@ -4,15 +4,14 @@
 // signs hold all 24).  Of the nine products of two such sums the six largest,
 //   a1 w3 + a3 w1 + a2 w2 + a1 w2 + a2 w1 + a1 w1,
 // are exact in 32 bits; the three left out are below 2^-23 of a1 w1, 2^-26 in the mean square.  The tensor cores' own sums cut low bits off: always
-// toward zero, which sums of one sign do not average out.  So they are kept short: for every 64-wide block of K the small products and then
-// the first half of the a1 w1 are added in one fresh accumulator, the second half in another (the cuts then fall on a small sum and on halves; a
-// first part of seven bits leaves less to cut).  The two are added, rounded to nearest, and then to a sum in registers that carries along what
-// rounding takes from it, as two bfloat16 a register.
+// toward zero, which sums of one sign do not average out.  So they are kept short: for every 32 of K the small products and then the a1 w1 are
+// added in a fresh accumulator (the cuts then fall on a small sum and on the two last products, of which first parts of seven bits leave less to
+// cut), and its sum is added, rounded to nearest, to a sum in registers that carries along what rounding takes from it, as two bfloat16 a register.
 // Relative error against 64 bits (2-norm), K = 64 to 3,072 and 17,408, gemm_simt.cu's in brackets:
-//   normal entries 0.5 to 0.8e-7 (1.4 to 3.3); their magnitudes 0.4 to 0.5e-7 (0.7 to 2.5); 1 + 0.1 normal 0.4 to 0.5e-7 (0.6 to 2.4); behind SiLU
-//   0.6 to 0.7e-7 (0.7 to 2.5).  Log-normal entries over ten powers of e, where a few products decide: 0.4 to 0.9e-7 (0.4 to 1.6).
-// Results of one sign are too small by 2 to 4e-8 in the mean, whatever K is (gemm_simt.cu: by nothing); with one accumulator, eight-bit first parts
-// and sums without rests by 8e-8, and the 2-norm error came to 1.6 of gemm_simt.cu's there.
+//   normal entries 0.6 to 0.8e-7 (1.4 to 3.3); their magnitudes 0.5 to 0.6e-7 (0.7 to 2.5); 1 + 0.1 normal 0.5 to 0.6e-7 (0.6 to 2.4); behind SiLU
+//   0.6 to 0.7e-7 (0.7 to 2.5).  Log-normal entries over ten powers of e, where a few products decide: 0.4 to 0.8e-7 (0.4 to 1.6).
+// Results of one sign are too small by 4 to 5e-8 in the mean, whatever K is (gemm_simt.cu: by nothing); with 64 of K an accumulator, eight-bit first
+// parts and sums without rests by 8e-8, and the 2-norm error came to 1.6 of gemm_simt.cu's there.
 //
 // Two launches.  `split_kernel` writes the three parts of A and W, [3 * rows][K] each, a warp a row, and says for every row whether the sum of
 // three is good for it.  `gemm_f32_tc_kernel`: a pair of CTAs takes a 256 x 256 tile (cta_group::2: each brings its own 128 rows of A and half
@@ -20,11 +19,9 @@
 // their order, for a range of columns).  Roles by warp:
 //   warp 8   copies: per block of K the three parts of A and of W (128-byte swizzle), two blocks in flight; a part's place is filled again
 //            as soon as the last product that reads it is done
-//   warp 9   products, in the pair's first CTA: 24 tcgen05.mma a block (kind::f16, M = 256, N = 128, K = 16) for either half of the columns, into
-//            the half's two accumulators
-//   warps 0-7  add: warp w reads lanes 32 (w % 4) .. + 31 and a half (w / 4) of the columns of the accumulators of one half of the tile and adds
-//              them to 64 of its 128 floats a thread, while the other half's are filled; at the end they write C, through shared memory, in rows
-//   (half h takes rows 64 h .. + 63 of either CTA's 128 rows of W, so that a warp's columns are the 128 from 128 (w / 4) on)
+//   warp 9   products, in the pair's first CTA: 12 tcgen05.mma (kind::f16, M = N = 256, K = 16) for either half of a block, into one of two accumulators
+//   warps 0-7  add: warp w reads lanes 32 (w % 4) .. + 31 and columns 128 (w / 4) .. + 127 of a finished accumulator and adds them to its
+//              128 floats a thread, while the other accumulator is filled; at the end they write C, through shared memory, in rows
 //
 // Rows with an entry that is not finite, of 2^50 and more (sums of the products of smaller ones stay below 2^127 for any K) or below
 // 2^-103 but not zero (its last bit is under 2^-126, the smallest normal number, so a part would lose bits) are flagged; an output of a flagged
@@ -32,12 +29,13 @@
 // (90 us; 235 by multiply-adds): 206 with a flagged row, 116 with a column, 277 with every 32nd row, 817 with all (950, 940, 910 and 6,800 by a lane
 // an output).
 //
-// What bounds it: the tensor cores do six products for one.  A block's 24 products of 256 columns would take 3,072 cycles (128 x 256 x 64 a CTA at
-// 8,192 operations a cycle); as 48 of 128 columns A is read from shared memory twice and they take 1.4 times that, and the adders, whose sums with
-// rests and loads from tensor memory come one after another, 1.6 times.  (With 256 columns there is no room for two accumulators a block beside
-// the next block's: 83 us where this takes 72.)  Sums without rests: 63 us; one accumulator a block as well, which the errors above forbid: 45.
-// Measured: 701 rows, parts included: 72 us for 4096 x 1024, 78 for 6144 x 1024, 53 for 1024 x 2048, 73 for 1024 x 3072 (229, 230, 140 and 209 by
-// gemm_f32_tile_kernel); 2,100 rows: 208 us for 6144 x 1024 (674).
+// What bounds it: the tensor cores do six products for one and need a block's 24 in 3,072 cycles (128 x 256 x 64 a CTA at 8,192 operations a
+// cycle); the adders, whose loads from tensor memory and sums with rests come one after another in two warps a scheduler, take about 1.4 times that
+// for its two accumulators.  Sums without rests 54 us where this takes 62, one accumulator a block as well 45: the errors above forbid both.  Two accumulators
+// for either half of the columns, emptied together, 72 (as 48 products of 128 columns, A is read from shared memory twice).  An adder's arrival
+// that released its stores to the cluster cost 20 us.
+// Measured: 701 rows, parts included: 62 us for 4096 x 1024, 67 for 6144 x 1024, 47 for 1024 x 2048, 64 for 1024 x 3072 (229, 230, 140 and 209 by
+// gemm_f32_tile_kernel); 2,100 rows: 172 us for 6144 x 1024 (674).
 //
 // Every wait gives up after a bounded number of polls and leaves a code in `*status`, as in gemm_tc.cu.
 #include "common.cuh"
@@ -60,7 +58,7 @@ constexpr int ADDERS = 8, THREADS = (ADDERS + 4) * 32;    // the last two warps 
 // Registers: 384 threads start with 168 each (64,512); the adders hold 128 sums and their 64 pairs of rests and take 232, the others keep 40:
 // 256 * 232 + 128 * 40 = 64,512.
 constexpr int ADDER_REGS = 232, OTHER_REGS = 40;
-constexpr int COLS = BN / 2;                             // columns of an adder, and of a half
+constexpr int COLS = BN / 2;                             // columns of an adder
 constexpr int AT_ONCE = 16;                              // columns read from an accumulator at a time
 constexpr int SPLIT_MOST = 4;
 constexpr int SUM_CHUNK = 64;
@@ -164,6 +162,12 @@ __device__ __forceinline__ void umma_pair_lo(uint32_t d, uint32_t a_lo, uint32_t
       : "memory");
 }
 
+// One arrival on a barrier of the pair: says that this warp's reads of tensor memory are done (they are waited for) and hands over no data, so it is no
+// release to the cluster, which waits for every store under way.
+__device__ __forceinline__ void arrive_read(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_bar) : "memory");
+}
+
 // Maps of the parts: [3 M][K] and [3 N][K], boxes of 128 rows.  Rows behind the last of a part belong to the next one (or are zeros):
 // they fill rows and columns of the tile that are not written.
 template <bool ACCUM, int SPLIT>
@@ -228,7 +232,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
     if (warp == ADDERS + 1 && lane == 0 && half == 0) {
-      constexpr uint32_t idesc = instr_desc(2 * BM, COLS, false);
+      constexpr uint32_t idesc = instr_desc(2 * BM, BN, false);
       const std::true_type yes;                  // the first of a sum
       const std::false_type no;
       const uint16_t both = (uint16_t)(3u << rank);
@@ -237,26 +241,24 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const int s0 = (i % STAGES) * 3;
         const uint32_t at = smem_addr(smem + s0 * SLOT_BYTES), parity = (i / STAGES) & 1;
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          // a part is there for the second half when it was for the first
+        for (int h = 0; h < 2; ++h) {            // the halves of the block; a part is there for the second when it was for the first
           auto arrived = [&](int p) { return h || mbar_wait(full0 + 8 * (s0 + p), parity); };
-          const uint32_t x = tmem + h * 2 * COLS, y = x + COLS;
-          uint32_t lo = ((at & 0x3FFFF) >> 4 | 1u << 16);
-          asm volatile("" : "+r"(lo));           // or all 48 descriptors are kept over the blocks, in memory
-          const uint32_t lo_w = lo + h * (PART_BYTES / 32);
-          auto products = [&](int pa, int pw, int k0, int k1, uint32_t to, auto fresh) {
+          const uint32_t to = tmem + h * BN;
+          uint32_t lo = ((at & 0x3FFFF) >> 4 | 1u << 16) + 4 * h;
+          asm volatile("" : "+r"(lo));           // or all descriptors are kept over the blocks, in memory
+          auto products = [&](int pa, int pw, auto fresh) {
 #pragma unroll
-            for (int k = k0; k < k1; ++k) {
-              const uint32_t da = lo + pa * (SLOT_BYTES / 16) + 2 * k, db = lo_w + (pw * SLOT_BYTES + PART_BYTES) / 16 + 2 * k;
-              if (decltype(fresh)::value && k == k0) umma_pair_lo<false>(to, da, db, idesc);
+            for (int k = 0; k < 2; ++k) {
+              const uint32_t da = lo + pa * (SLOT_BYTES / 16) + 2 * k, db = lo + (pw * SLOT_BYTES + PART_BYTES) / 16 + 2 * k;
+              if (decltype(fresh)::value && k == 0) umma_pair_lo<false>(to, da, db, idesc);
               else umma_pair_lo<true>(to, da, db, idesc);
             }
           };
           ok = (i < 1 || mbar_wait_cluster(sum_empty0 + 8 * h, (i - 1) & 1)) && arrived(2) && arrived(0);
           if (ok) {
             tc_fence_after();
-            products(0, 2, 0, 4, x, yes);
-            products(2, 0, 0, 4, x, no);
+            products(0, 2, yes);
+            products(2, 0, no);
             if (h) umma_commit_pair(empty0 + 8 * (s0 + 2), both);
             ok = arrived(1);
           }
@@ -265,12 +267,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             break;
           }
           tc_fence_after();
-          products(1, 1, 0, 4, x, no);
-          products(0, 1, 0, 4, x, no);
-          products(1, 0, 0, 4, x, no);
+          products(1, 1, no);
+          products(0, 1, no);
+          products(1, 0, no);
           if (h) umma_commit_pair(empty0 + 8 * (s0 + 1), both);
-          products(0, 0, 0, 2, x, no);
-          products(0, 0, 2, 4, y, yes);
+          products(0, 0, no);
           if (h) umma_commit_pair(empty0 + 8 * s0, both);
           umma_commit_pair(sum_full0 + 8 * h, both);
         }
@@ -293,7 +294,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       col_flags[h] = __ballot_sync(0xffffffffu, n < N && flags[M + n] != 0);
     }
     const uint32_t first_empty0 = map_to_cta(sum_empty0, first);
-    const uint32_t from0 = tmem + ((uint32_t)row0 << 16) + COLS / 2 * (warp / 4);
+    const uint32_t from0 = tmem + ((uint32_t)row0 << 16) + col0;
     uint32_t rest[COLS / 2];                               // what rounding has taken from the sums, two bfloat16 a register
 #pragma unroll
     for (int j = 0; j < COLS / 2; ++j) rest[j] = 0u;
@@ -308,23 +309,18 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
-        for (int c = 0; c < COLS / 2; c += AT_ONCE) {
-          const uint32_t from = from0 + h * 2 * COLS + c;
-          uint32_t x[AT_ONCE], y[AT_ONCE];
-          tmem_ld16(from, x);
-          tmem_ld16(from + COLS, y);
+        for (int c = 0; c < COLS; c += AT_ONCE) {
+          uint32_t x[AT_ONCE];
+          tmem_ld16(from0 + h * BN + c, x);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < AT_ONCE; j += 2) {
-            const int k = h * (COLS / 2) + c + j;
-            const float2 v = add2(make_float2(__uint_as_float(x[j]), __uint_as_float(x[j + 1])), make_float2(__uint_as_float(y[j]), __uint_as_float(y[j + 1])));
-            add_with_rest(sum[k], sum[k + 1], rest[k / 2], v);
-          }
+          for (int j = 0; j < AT_ONCE; j += 2)
+            add_with_rest(sum[c + j], sum[c + j + 1], rest[(c + j) / 2], make_float2(__uint_as_float(x[j]), __uint_as_float(x[j + 1])));
           if (K < 0) break;                                // never: the pieces one after another, or the compiler mixes them and keeps 240 registers in memory
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(first_empty0 + 8 * h);
+        if (lane == 0) arrive_read(first_empty0 + 8 * h);
       }
     constexpr int RANGE = BN / SPLIT, OWN = COLS < RANGE ? COLS : RANGE;         // columns of a pair, of them in an adder's reach
     if (SPLIT > 1) {
@@ -536,13 +532,13 @@ static int pick_split(int tiles, int blocks, const Clusters &clusters) {
 }
 static int tiles_of(int M, int N) { return ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN); }
 
-// Nanoseconds that both launches are estimated to take: the parts at 6.7 TB/s, a block 3.4 us, and what a launch
-// takes whatever it does (within 0.15 of 28 sizes of 64 to 2,100 rows, K = 1,024 to 3,072).
+// Nanoseconds that both launches are estimated to take: the parts at 6.7 TB/s, a block 2.8 us, and what a launch
+// takes whatever it does (within 0.13 of the time at 35 sizes of 64 to 2,100 rows, K = 1,024 to 4,096).
 extern "C" int g2b_gemm_f32_tc_estimate(int M, int N, int K) {
   Clusters clusters;
   if (count_clusters(clusters)) return 2000000000;
   const int tiles = tiles_of(M, N), blocks = (K + BK - 1) / BK;
-  const double us = 7.0 + 1.5e-6 * ((double)M + N) * K + 3.4 * rounds_of_blocks(pick_split(tiles, blocks, clusters), tiles, blocks, clusters);
+  const double us = 7.0 + 1.5e-6 * ((double)M + N) * K + 2.8 * rounds_of_blocks(pick_split(tiles, blocks, clusters), tiles, blocks, clusters);
   return us < 2e6 ? (int)(1e3 * us) : 2000000000;
 }
 

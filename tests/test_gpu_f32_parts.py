@@ -77,8 +77,8 @@ def test_cuts_of_one_sign(kind, M, N, K):
     kernels.gemm_simt(a, w, plain)
     err = out.double() - ref
     assert err.norm() <= (plain.double() - ref).norm()
-    # a cut takes half a unit in the last place of the sum it falls on, 0.72 * 2^-24 of it in the mean: two on a half of a block's sum and two on
-    # a quarter are 1.1 * 2^-24 where every product has bits to lose; a first part of seven bits leaves half of them none
+    # a cut takes half a unit in the last place of the sum it falls on, 0.72 * 2^-24 of it in the mean: of a sum of 32, its last and its last but
+    # one, on a half of it, 1.1 * 2^-24 where every product has bits to lose; a first part of seven bits leaves half of them none
     assert (err * ref.sign() / size).mean().abs() <= EPS
 
 
