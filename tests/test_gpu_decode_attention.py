@@ -27,8 +27,20 @@ def ctx_of(lens, table, width):
 @pytest.mark.parametrize("nh,nkv,hd", [(16, 8, 128), (5, 1, 128), (20, 1, 64), (40, 2, 128), (6, 2, 64)])
 @pytest.mark.parametrize("form", FORMS, ids=lambda f: "-".join(f) or "plain")
 def test_prologue_and_cluster_give_the_bits_of_the_steps_one_by_one(width, nh, nkv, hd, form):
+    bits_of_the_steps_one_by_one([1, 2, 16, 17, 63, 64, 65, 127, 129, 256, 257, 383, 513, 700, 1025], width, nh, nkv, hd, form)
+
+
+# clusters of one to eight CTAs: the last chunk whole, half or of one key
+@pytest.mark.parametrize("width", [1, 2, 3, 4, 6, 7, 8, 10, 11, 14, 16])
+@pytest.mark.parametrize("nh,nkv,hd", [(16, 8, 128), (20, 1, 64)])
+@pytest.mark.parametrize("form", [dict(), dict(window=70)], ids=lambda f: "-".join(f) or "plain")
+def test_short_clusters(width, nh, nkv, hd, form):
+    most = 64 * width
+    bits_of_the_steps_one_by_one(sorted({1, 33, most, max(1, most - 1), most // 2 + 1, max(1, most - 63)}), width, nh, nkv, hd, form)
+
+
+def bits_of_the_steps_one_by_one(lens, width, nh, nkv, hd, form):
     from gguf2bin_b200 import kernels, kernels_bf16
-    lens = [1, 2, 16, 17, 63, 64, 65, 127, 129, 256, 257, 383, 513, 700, 1025]
     cache, table, _, _ = make_paged(len(lens), lens, nkv, hd, 64, torch.bfloat16, seed=40)
     T = len(lens)
     qkv = rnd(T, (nh + 2 * nkv) * hd, dtype=torch.bfloat16, seed=41)

@@ -42,6 +42,13 @@ def test_heads_get_the_bits_of_product_and_prologue(rows, nh, nkv, K, form):
     assert torch.equal(q, q_ref) and torch.equal(own, ref)
 
 
+# from 129 rows on: fewer tiles than SMs, one of 128 rows and one of a row, a chat's prompt with its padding
+@pytest.mark.parametrize("rows,nh,nkv,K", [(129, 64, 8, 512), (255, 64, 16, 2048), (257, 40, 8, 5120), (576, 16, 8, 1024), (576, 32, 0, 520), (701, 16, 8, 64)])
+@pytest.mark.parametrize("form", [dict(), dict(norm=False, rope=False)], ids=lambda f: "-".join(f) or "plain")
+def test_heads_of_short_prompts(rows, nh, nkv, K, form):
+    test_heads_get_the_bits_of_product_and_prologue(rows, nh, nkv, K, form)
+
+
 def test_what_the_epilogue_cannot_do_is_left_to_the_two():
     from gguf2bin_b200 import kernels
     cache, table, _, _ = make_paged(1, [2048], 8, 128, 64, torch.bfloat16, seed=50)
