@@ -502,7 +502,7 @@ static int count_clusters(Clusters &out) {
   static G2bPerDevice configured;
   static Clusters kept[G2B_MAX_DEVICES];
   const int dev = g2b_current_device();
-  if (dev >= 0 && configured.value[dev]) {
+  if (dev >= 0 && __atomic_load_n(&configured.value[dev], __ATOMIC_ACQUIRE)) {
     out = kept[dev];
     return 0;
   }
@@ -514,8 +514,8 @@ static int count_clusters(Clusters &out) {
   if (e == cudaSuccess) e = allow<true, 4>(out.of[4]);
   if (e != cudaSuccess || out.of[1] < 1) G2B_REFUSE("gemm_f32_tc: %d bytes of shared memory: %s", SMEM, cudaGetErrorString(e));
   if (dev >= 0) {
-    kept[dev] = out;
-    configured.value[dev] = 1;
+    kept[dev] = out;                             // (two threads in their first calls write the same)
+    __atomic_store_n(&configured.value[dev], 1, __ATOMIC_RELEASE);
   }
   return 0;
 }
