@@ -98,6 +98,7 @@ class DecodeRunner:
         self.logits: Optional[torch.Tensor] = None
         self._graphs: "OrderedDict[tuple, tuple]" = OrderedDict()    # attention's plans -> (graph, generation, launches)
         self._plain_steps: dict = {}            # attention's plans -> plain steps so far
+        self._replaying: Optional[tuple] = None      # what the last step's plans were made for, its graph and launches
         self.launches_per_step = 0
 
     def bind(self, session: "DecodeSession", keep_tokens: bool = False) -> None:
@@ -144,8 +145,14 @@ class DecodeRunner:
 
     def run(self, use_graph: bool, eager_steps: int, longest: int) -> None:
         """One step; ``longest``: the keys of the longest sequence with it.  The page table is as wide as what is reserved; kernels that size
-        their work by the keys plan with these."""
+        their work by the keys plan with these (in pages, so the plans are made anew when a sequence gets to its next)."""
         ws, eng = self.engine.workspace, self.engine
+        made_for = (longest + 63 >> 6, len(eng.decode_kinds), ws.generation)
+        if use_graph and self._replaying is not None and self._replaying[0] == made_for:
+            _, graph, self.launches_per_step = self._replaying
+            graph.replay()
+            return
+        self._replaying = None
         self.ctx.kv_len_hint = longest
         plan = kernels.decode_plans(self.ctx, eng.decode_kinds)
         hit = self._graphs.get(plan)
@@ -154,8 +161,9 @@ class DecodeRunner:
             self._plain_steps[plan], hit = 0, None
         if hit is not None and use_graph:
             self._graphs.move_to_end(plan)
-            self.launches_per_step = hit[2]
-            hit[0].replay()
+            graph, _, self.launches_per_step = hit
+            self._replaying = (made_for, graph, self.launches_per_step)
+            graph.replay()
             return
         before = kernels.launch_count()
         if use_graph and self._plain_steps.get(plan, 0) >= eager_steps:
