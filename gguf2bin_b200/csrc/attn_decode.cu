@@ -15,7 +15,8 @@
 //
 // Each CTA writes an unnormalised partial output with its maximum and sum (log2 domain)
 // to scratch; `attn_combine_kernel` merges a token's chunks in an order that depends on its
-// position only.  Steps of one or two sequences take attn_decode_short.cu.
+// position only.  Steps whose keys make few CTAs, all of which the device holds at once, take attn_decode_short.cu
+// (`decode_plan` in kernels_bf16.py).
 //
 // Options of the extended entry point (`g2b_attn_decode_ex`): `softcap` > 0 turns a scaled score s into
 // softcap tanh(s / softcap); `keep_first` > 0 (with a window) keeps the keys at positions below it visible

@@ -1,4 +1,4 @@
-// Decode attention of steps with little to read: one or two sequences, or few heads.  Latency is what such a step waits for (a round of
+// Decode attention of steps with little to read: few sequences, few heads or few keys.  Latency is what such a step waits for (a round of
 // loads, the chain of products of a segment, the merge, a launch), so the keys are spread as widely as the sums allow, and what stands in
 // front of the attention and behind it runs in the same launch.
 //
@@ -8,9 +8,9 @@
 // eight warps takes 16 keys: 16 rows of K and V, copied with 16-byte cp.async, read back with ldmatrix.  Scores, softmax statistics and the
 // output are 32-bit; probabilities are rounded to bfloat16 for the P.V product.  The warps' partial outputs are added in warp order.
 //
-// How the chunks of a token meet.  Up to CLUSTER_MOST chunks (2,048 keys) are one thread-block cluster: every CTA sends each
+// How the chunks of a token meet.  Where the caller passes no scratch, they are one thread-block cluster (up to CLUSTER_MOST chunks, 2,048 keys): every CTA sends each
 // CTA of the cluster its share of the partial output (and all maxima and sums) through distributed
-// shared memory, and after one cluster barrier the CTAs write a share of the heads each.  More chunks
+// shared memory, and after one cluster barrier the CTAs write a share of the heads each.  Else the chunks
 // leave unnormalised partial outputs with their maxima and sums (log2 domain) in scratch, which
 // `attn_combine_kernel` merges.  Both add in the same order, which depends on the token's position only.
 //
@@ -18,10 +18,12 @@
 // rotation of the heads are done here, row by row as qknorm_rope_fast_kernel (elementwise.cu) does them, in every CTA that needs the row; the
 // token's own key and value are put among the rows of the cache from shared memory, and the warp whose keys they follow writes them to the cache.
 //
-// Measured in a chain of launches, norm, rotation and merge included, 16 query heads of 128 on 8: one sequence at 550 keys 4.0 us (8.5 by
-// qknorm_rope_fast_kernel, attn_decode_kernel with two warps of 64 keys and attn_combine_kernel), at 2,000 keys 5.9 (8.5), at 4,000 keys
-// 8.0 (9.2); two sequences at 1,000 keys 4.8 (8.7).  Not for steps whose keys fill the memory's rate (8 sequences at 2,048 keys): there
-// the three launches leave the memory time to run ahead, and one launch in their place was slower (90 ms against 82 for eight requests of 64 tokens).
+// Measured in a chain of launches, norm, rotation and merge included, 16 query heads of 128 on 8: one sequence at 550 keys 3.9 us (8.4 by
+// qknorm_rope_fast_kernel, attn_decode_kernel with two warps of 64 keys and attn_combine_kernel), at 2,000 keys 5.9 (8.4), at 4,000 keys
+// 7.5 (9.3); two at 1,000 keys 4.8 (8.8), four at 500 4.9 (8.9), eight at 500 6.7 (9.9), sixteen at 200 6.2 (10.1).  Not for clusters or CTAs that
+// have to wait for others to end (`decode_plan` in kernels_bf16.py draws the line), nor for steps whose keys fill the memory's rate (8 sequences at
+// 2,048 keys): there the three launches leave the memory time to run ahead, and one launch in their place was slower (90 ms against 82 for eight
+// requests of 64 tokens).
 //
 // Formula: src/l5_model.c:518, 559-577 of AnonymoDGH/gguf2bin.  Compiled per head size (-DHD=64 or 128); the page size is 64 keys.
 #include "common.cuh"
